@@ -155,7 +155,35 @@ def lib() -> ctypes.CDLL:
 
 
 def build_library(force: bool = False) -> str:
-    return _build.build_library(force=force)
+    path = _build.build_library(force=force)
+    _build.build_torch_calls(force=force)
+    return path
+
+
+class _NativeCalls:
+    """Stands for the native call path (csrc/torch_calls.cpp) until the first call loads it."""
+
+    def __getattr__(self, name):
+        global _native
+        if not os.path.exists(_build.TORCH_CALLS):
+            raise RuntimeError(
+                f"{_build.TORCH_CALLS} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`; "
+                "this provider has no CPU or PyTorch fallback"
+            )
+        import importlib.util
+
+        import torch  # noqa: F401 - its libraries have to be loaded first
+
+        lib()
+        spec = importlib.util.spec_from_file_location("_tcrv_torch", _build.TORCH_CALLS)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(_check)
+        _native = module
+        return getattr(module, name)
+
+
+_native = _NativeCalls()
 
 
 def _check(status: int, where: str) -> None:
@@ -193,18 +221,7 @@ def check_device_errors() -> None:
 
 
 def add(lhs, rhs, out=None):
-    import torch
-
-    if out is None:
-        out = torch.empty_like(lhs)
-    if lhs.dtype == torch.float32:
-        fn, name = lib().tcrv_cuda_add_f32, "tcrv_cuda_add_f32"
-    elif lhs.dtype == torch.int32:
-        fn, name = lib().tcrv_cuda_add_i32, "tcrv_cuda_add_i32"
-    else:
-        raise TypeError("add supports float32 and int32")
-    _check(fn(_dev(lhs), _dev(rhs, lhs.dtype), _dev(out, lhs.dtype), lhs.numel(), _stream()), name)
-    return out
+    return _native.add(lhs, rhs, out)
 
 
 def dequantize_i32_f32(lhs, scale: float, out=None):
@@ -226,49 +243,19 @@ def _rows(t, block_bytes: int):
 
 
 def dequantize_q8_0(vx, out=None):
-    import torch
-
-    nb = _rows(vx, Q8_0_BLOCK)
-    if out is None:
-        out = torch.empty(vx.shape[:-1] + (nb * QK,), dtype=torch.float32, device=vx.device)
-    _check(lib().tcrv_cuda_dequantize_row_q8_0(_dev(vx, torch.uint8), _dev(out, torch.float32), out.numel(), _stream()),
-           "tcrv_cuda_dequantize_row_q8_0")
-    return out
+    return _native.dequantize(vx, out, Q8_0_BLOCK)
 
 
 def dequantize_q4_0(vx, out=None):
-    import torch
-
-    nb = _rows(vx, Q4_0_BLOCK)
-    if out is None:
-        out = torch.empty(vx.shape[:-1] + (nb * QK,), dtype=torch.float32, device=vx.device)
-    _check(lib().tcrv_cuda_dequantize_row_q4_0(_dev(vx, torch.uint8), _dev(out, torch.float32), out.numel(), _stream()),
-           "tcrv_cuda_dequantize_row_q4_0")
-    return out
+    return _native.dequantize(vx, out, Q4_0_BLOCK)
 
 
 def quantize_q8_0(x, out=None):
-    import torch
-
-    if x.shape[-1] % QK != 0:
-        raise ValueError("last dimension must be a multiple of 32")
-    if out is None:
-        out = torch.empty(x.shape[:-1] + (x.shape[-1] // QK * Q8_0_BLOCK,), dtype=torch.uint8, device=x.device)
-    _check(lib().tcrv_cuda_quantize_row_q8_0(x.numel(), _dev(x, torch.float32), _dev(out, torch.uint8), _stream()),
-           "tcrv_cuda_quantize_row_q8_0")
-    return out
+    return _native.quantize(x, out, Q8_0_BLOCK)
 
 
 def quantize_q4_0(x, out=None):
-    import torch
-
-    if x.shape[-1] % QK != 0:
-        raise ValueError("last dimension must be a multiple of 32")
-    if out is None:
-        out = torch.empty(x.shape[:-1] + (x.shape[-1] // QK * Q4_0_BLOCK,), dtype=torch.uint8, device=x.device)
-    _check(lib().tcrv_cuda_quantize_row_q4_0(x.numel(), _dev(x, torch.float32), _dev(out, torch.uint8), _stream()),
-           "tcrv_cuda_quantize_row_q4_0")
-    return out
+    return _native.quantize(x, out, Q4_0_BLOCK)
 
 
 # ------------------------------------------------------------------- block dots
@@ -308,15 +295,7 @@ def vec_dot_q8_0_q8_0(w_row, x_row):
 
 def gemv(w, x, q8_weights: bool = False, flags: int = FLAG_NONE, out=None):
     """out[row, col] = block dot(weight row, activation column); x has at most 8 columns."""
-    wblock = Q8_0_BLOCK if q8_weights else Q4_0_BLOCK
-    n, nr, nc, bx, by, torch = _matrix_args(w, x, wblock)
-    if out is None:
-        out = torch.empty((nr, nc), dtype=torch.float32, device=w.device)
-    name = "tcrv_cuda_gemv_q8_0_q8_0" if q8_weights else "tcrv_cuda_gemv_q4_0_q8_0"
-    fn = getattr(lib(), name)
-    _check(fn(n, _dev(out, torch.float32), w.data_ptr(), x.data_ptr(), by, nr, nc, bx, out.stride(0), flags, _stream()),
-           name)
-    return out
+    return _native.gemv(w, x, q8_weights, flags, out)
 
 
 class GemvCall(ctypes.Structure):
@@ -339,8 +318,7 @@ def gemv_group_calls(problems, q8_weights: bool = False):
 
 def gemv_group(calls, q8_weights: bool = False, flags: int = FLAG_NONE):
     """Independent GEMVs as one request (tcrv_cuda_gemv_group_*): `calls` from gemv_group_calls."""
-    name = "tcrv_cuda_gemv_group_q8_0_q8_0" if q8_weights else "tcrv_cuda_gemv_group_q4_0_q8_0"
-    _check(getattr(lib(), name)(ctypes.addressof(calls), len(calls), flags, _stream()), name)
+    _native.gemv_group(ctypes.addressof(calls), len(calls), q8_weights, flags)
 
 
 def gemv_fold_order(w, x, q8_weights: bool = False, flags: int = FLAG_NONE) -> int:
@@ -389,31 +367,9 @@ def gemm(w, x, out=None, workspace=None):
     """out[row, col] = Q4_0 x Q8_0 block dot for any number of activation columns.
 
     `w` is either a (rows, row_bytes) uint8 tensor of block_q4_0 rows or a PreparedWeights."""
-    import torch
-
     if isinstance(w, PreparedWeights):
-        n, nr, nc, by = w.n, w.nr, x.shape[0], x.stride(0)
-        if _rows(x, Q8_0_BLOCK) * QK != n:
-            raise ValueError("weights and activations disagree on the number of blocks per row")
-        if out is None:
-            out = torch.empty((nr, nc), dtype=torch.float32, device=x.device)
-        need = lib().tcrv_cuda_gemm_acts_workspace_bytes(n, nc)
-        if workspace is None:
-            workspace = _workspace(need, x.device)
-        _check(lib().tcrv_cuda_gemm_q4_0_q8_0_prepared(n, _dev(out, torch.float32), w.buffer.data_ptr(), x.data_ptr(), by,
-                                                       nr, nc, out.stride(0), workspace.data_ptr(), workspace.numel(), 0,
-                                                       _stream()), "tcrv_cuda_gemm_q4_0_q8_0_prepared")
-        return out
-    n, nr, nc, bx, by, _ = _matrix_args(w, x, Q4_0_BLOCK)
-    if out is None:
-        out = torch.empty((nr, nc), dtype=torch.float32, device=w.device)
-    need = lib().tcrv_cuda_gemm_workspace_bytes(n, nr, nc)
-    if workspace is None:
-        workspace = _workspace(need, w.device)
-    _check(lib().tcrv_cuda_gemm_q4_0_q8_0(n, _dev(out, torch.float32), w.data_ptr(), x.data_ptr(), by, nr, nc, bx,
-                                          out.stride(0), workspace.data_ptr(), workspace.numel(), 0, _stream()),
-           "tcrv_cuda_gemm_q4_0_q8_0")
-    return out
+        return _native.gemm_prepared(w.buffer, w.n, w.nr, x, out, workspace)
+    return _native.gemm(w, x, out, workspace)
 
 
 def pack_q4_0_to_q4_0x16(src, out=None):
@@ -450,18 +406,7 @@ def repack_gemv(wx16, x, nc: int, q8_weights: bool = False, out=None, flags: int
     """Decode GEMV over 16-row interleaved weights: `wx16` is the flat block_q4_0x16 (or
     block_q8_0x16) stream of nc / 16 row groups, `x` one plain Q8_0 activation row; returns
     the nc fp32 results (tcrv_rvv.repack_gemv_q4_0_q8_0 / repack_gemv_q8_0_q8_0)."""
-    import torch
-
-    block = 544 if q8_weights else 288
-    nb = x.numel() // Q8_0_BLOCK
-    if x.numel() % Q8_0_BLOCK or nc % 16 or wx16.numel() != nc // 16 * nb * block:
-        raise ValueError("weights, activation and nc do not describe the same shape")
-    if out is None:
-        out = torch.empty(nc, dtype=torch.float32, device=wx16.device)
-    fn = lib().tcrv_cuda_repack_gemv_q8_0_q8_0 if q8_weights else lib().tcrv_cuda_repack_gemv_q4_0_q8_0
-    _check(fn(nb * QK, _dev(out, torch.float32), _dev(wx16, torch.uint8), _dev(x, torch.uint8), nc, flags, _stream()),
-           "tcrv_cuda_repack_gemv")
-    return out
+    return _native.repack_gemv(wx16, x, nc, q8_weights, out, flags)
 
 
 def repack_gemm(wx16, xx4, n: int, nr: int, nc: int, out=None, workspace=None):
@@ -529,18 +474,8 @@ SIBLING_STRIDES = {1: (20, 36), 2: (22, 34), 3: (24, 36)}  # (weight, activation
 def sibling_dot_rows(fmt: int, w, x, out=None):
     """out[row, col] = block dot of weight row `row` (format's weight blocks) and activation
     column `col` (Q8_0 or Q8_1 blocks), folded in strict ascending block order."""
-    import torch
-
     wb, ab = SIBLING_STRIDES[fmt]
-    if w.shape[1] % wb or x.shape[1] % ab or w.shape[1] // wb != x.shape[1] // ab:
-        raise ValueError("row bytes do not match the format's block sizes")
-    n, nr, nc = w.shape[1] // wb * QK, w.shape[0], x.shape[0]
-    if out is None:
-        out = torch.empty((nr, nc), dtype=torch.float32, device=w.device)
-    _check(lib().tcrv_cuda_sibling_dot_rows(fmt, n, _dev(out, torch.float32), _dev(w, torch.uint8), _dev(x, torch.uint8),
-                                            x.stride(0), nr, nc, w.stride(0), out.stride(0), _stream()),
-           "tcrv_cuda_sibling_dot_rows")
-    return out
+    return _native.sibling_dot_rows(fmt, wb, ab, w, x, out)
 
 
 def sibling_block_sums(fmt: int, w, x):
@@ -560,34 +495,17 @@ def sibling_block_sums(fmt: int, w, x):
 
 def vec_scale_(y, v: float):
     """y *= v in place."""
-    import torch
-
-    _check(lib().tcrv_cuda_vec_scale_f32(y.numel(), _dev(y, torch.float32), v, _stream()),
-           "tcrv_cuda_vec_scale_f32")
-    return y
+    return _native.vec_scale_(y, v)
 
 
 def vec_silu(x, out=None):
-    import torch
-
-    if out is None:
-        out = torch.empty_like(x)
-    _check(lib().tcrv_cuda_vec_silu_f32(x.numel(), _dev(x, torch.float32), _dev(out, torch.float32), _stream()), "tcrv_cuda_vec_silu_f32")
-    return out
+    return _native.vec_silu(x, out)
 
 
 def rms_norm(x, eps: float, out=None, flags: int = FLAG_NONE):
     """RMS norm over the last dimension of a 2-D (rows, ne00) tensor (row strides honoured).
     FLAG_STRICT_ORDER adds the squares in the reference's ascending chain."""
-    import torch
-
-    if x.dim() != 2 or x.stride(1) != 1 or x.dtype != torch.float32 or not x.is_cuda:
-        raise ValueError("x must be a 2-D float32 CUDA tensor with unit inner stride")
-    if out is None:
-        out = torch.empty((x.shape[0], x.shape[1]), dtype=torch.float32, device=x.device)
-    _check(lib().tcrv_cuda_rms_norm_f32_flags(x.shape[1], x.data_ptr(), out.data_ptr(), eps, x.shape[0], x.stride(0),
-                                              out.stride(0), flags, _stream()), "tcrv_cuda_rms_norm_f32_flags")
-    return out
+    return _native.rms_norm(x, eps, out, flags)
 
 
 def vec_soft_max(x, max_value: float, out=None):
@@ -617,15 +535,7 @@ def rope_cache(n_dims: int, theta_base: float, theta_scale: float, device="cuda"
 
 def rope_apply(x, cache, out=None):
     """Rotates the rows of a 2-D (rows, n_dims) tensor with one shared angle cache."""
-    import torch
-
-    if x.dim() != 2 or x.stride(1) != 1 or x.dtype != torch.float32 or not x.is_cuda:
-        raise ValueError("x must be a 2-D float32 CUDA tensor with unit inner stride")
-    if out is None:
-        out = torch.empty((x.shape[0], x.shape[1]), dtype=torch.float32, device=x.device)
-    _check(lib().tcrv_cuda_rope_apply_f32(x.shape[1], x.data_ptr(), out.data_ptr(), _dev(cache, torch.float32), x.shape[0],
-                                          x.stride(0), out.stride(0), _stream()), "tcrv_cuda_rope_apply_f32")
-    return out
+    return _native.rope_apply(x, cache, out)
 
 
 # ------------------------------------------------------------------ N-sharding (multi-GPU GEMM)

@@ -1,7 +1,9 @@
 """Build recipe for the provider's native code (sm_100a only, in-tree outputs).
 
 ``build_library()`` compiles ``csrc/*.cu`` into ``libtcrv_cuda.so`` next to this file with
-nvcc; it needs no GPU (nvcc cross-compiles).  Run as a script to force a rebuild.
+nvcc; it needs no GPU (nvcc cross-compiles).  ``build_torch_calls()`` compiles
+``csrc/torch_calls.cpp``, the package's native call path, into ``_tcrv_torch.so`` beside it with
+the host compiler.  Run as a script to force a rebuild.
 """
 from __future__ import annotations
 
@@ -15,6 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtcrv_cuda.so")
+TORCH_CALLS = os.path.join(HERE, "_tcrv_torch.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -53,5 +56,31 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_torch_calls(force: bool = False) -> str:
+    """The Python calls' native half; needs the C-ABI library (it links against it)."""
+    import sysconfig
+
+    import torch
+
+    source = os.path.join(CSRC, "torch_calls.cpp")
+    deps = [source, os.path.join(ROOT, "include", "tcrv_cuda.h")]
+    if not force and os.path.exists(TORCH_CALLS) and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_CALLS) for d in deps):
+        return TORCH_CALLS
+    torch_dir = os.path.dirname(torch.__file__)
+    torch_lib = os.path.join(torch_dir, "lib")
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    subprocess.run([
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"],
+        "-isystem", os.path.join(torch_dir, "include"), "-isystem", os.path.join(torch_dir, "include/torch/csrc/api/include"),
+        "-isystem", cuda_include, "-o", TORCH_CALLS, source,
+        "-L", HERE, "-ltcrv_cuda", "-L", torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+        "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}",
+    ], check=True)
+    return TORCH_CALLS
+
+
 if __name__ == "__main__":
     print(build_library(force=True, verbose="-v" in sys.argv))
+    print(build_torch_calls(force=True))

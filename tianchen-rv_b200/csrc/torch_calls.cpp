@@ -1,0 +1,442 @@
+// The Python package's hot calls as native functions: argument checks, the output's allocation
+// and the current stream are taken from torch in C++, then the C ABI (include/tcrv_cuda.h) is
+// called.  A decode step is dozens of launches of 3..10 us each; the same work done in the
+// interpreter (attribute reads, torch.empty, a ctypes call of eleven arguments) cost 12.4 us per
+// call, more than most of the kernels it launched.
+//
+// The functions take their arguments by position, exactly as the wrappers in __init__.py pass
+// them; a non-zero status goes to the package's `_check`, which raises TcrvCudaError.
+#include <Python.h>
+
+#include <ATen/ops/empty.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "tcrv_cuda.h"
+
+namespace {
+
+constexpr int64_t kQK = TCRV_QK;
+PyObject *g_check = nullptr;  // the package's _check(status, where)
+
+struct PyError {};  // a Python exception is set
+
+[[noreturn]] void fail(PyObject *type, const char *text) {
+  PyErr_SetString(type, text);
+  throw PyError{};
+}
+
+inline cudaStream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+inline const at::Tensor &tensor(PyObject *o) {
+  if (!THPVariable_Check(o))
+    fail(PyExc_TypeError, "operands must be CUDA torch tensors (device pointers cross the C ABI)");
+  const at::Tensor &t = THPVariable_Unpack(o);
+  if (!t.is_cuda())
+    fail(PyExc_TypeError, "operands must be CUDA torch tensors (device pointers cross the C ABI)");
+  return t;
+}
+
+// A contiguous CUDA tensor of the given type.
+inline const at::Tensor &dense(PyObject *o, at::ScalarType type) {
+  const at::Tensor &t = tensor(o);
+  if (t.scalar_type() != type) {
+    PyErr_Format(PyExc_TypeError, "expected dtype torch.%s, got %s",
+                 type == at::kFloat ? "float32" : type == at::kInt ? "int32" : type == at::kByte ? "uint8" : "float64",
+                 c10::toString(t.scalar_type()));
+    throw PyError{};
+  }
+  if (!t.is_contiguous())
+    fail(PyExc_ValueError, "operands must be contiguous");
+  return t;
+}
+
+inline uint8_t *bytes(const at::Tensor &t) { return static_cast<uint8_t *>(t.data_ptr()); }
+inline float *floats(const at::Tensor &t) { return static_cast<float *>(t.data_ptr()); }
+
+inline at::Tensor empty(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like) {
+  return at::empty(shape, like.options().dtype(type));
+}
+
+inline int64_t integer(PyObject *o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred())
+    throw PyError{};
+  return v;
+}
+
+inline double real(PyObject *o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred())
+    throw PyError{};
+  return v;
+}
+
+inline bool truth(PyObject *o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0)
+    throw PyError{};
+  return v != 0;
+}
+
+void check(int status, const char *where) {
+  if (status == TCRV_CUDA_OK)
+    return;
+  PyObject *r = PyObject_CallFunction(g_check, "is", status, where);
+  if (r != nullptr) {
+    Py_DECREF(r);
+    PyErr_SetString(PyExc_RuntimeError, where);
+  }
+  throw PyError{};
+}
+
+// Runs a launch without the interpreter lock, as a ctypes call does.
+template <typename F>
+inline int unlocked(F &&launch) {
+  int status;
+  Py_BEGIN_ALLOW_THREADS
+  status = launch();
+  Py_END_ALLOW_THREADS
+  return status;
+}
+
+inline int64_t blocks_of(int64_t row_bytes, int64_t block_bytes) {
+  if (row_bytes % block_bytes != 0) {
+    PyErr_Format(PyExc_ValueError, "last dimension %lld is not a whole number of %lld-byte blocks",
+                 static_cast<long long>(row_bytes), static_cast<long long>(block_bytes));
+    throw PyError{};
+  }
+  return row_bytes / block_bytes;
+}
+
+inline PyObject *given_or_wrapped(PyObject *given, at::Tensor &&made) {
+  if (given != Py_None) {
+    Py_INCREF(given);
+    return given;
+  }
+  return THPVariable_Wrap(std::move(made));
+}
+
+#define TCRV_CALL(name, count) \
+  PyObject *name##_body(PyObject *const *a); \
+  PyObject *name(PyObject *, PyObject *const *a, Py_ssize_t n) { \
+    if (n != (count)) { \
+      PyErr_SetString(PyExc_TypeError, #name ": wrong number of arguments"); \
+      return nullptr; \
+    } \
+    try { \
+      return name##_body(a); \
+    } catch (const PyError &) { \
+      return nullptr; \
+    } catch (const std::exception &e) { \
+      PyErr_SetString(PyExc_RuntimeError, e.what()); \
+      return nullptr; \
+    } \
+  } \
+  PyObject *name##_body(PyObject *const *a)
+
+// add(lhs, rhs, out)
+TCRV_CALL(add, 3) {
+  const at::Tensor &lhs = tensor(a[0]);
+  const at::ScalarType type = lhs.scalar_type();
+  if (type != at::kFloat && type != at::kInt)
+    fail(PyExc_TypeError, "add supports float32 and int32");
+  const at::Tensor &l = dense(a[0], type), &r = dense(a[1], type);
+  at::Tensor made;
+  if (a[2] == Py_None)
+    made = empty(l.sizes(), type, l);
+  void *out = a[2] == Py_None ? made.data_ptr() : dense(a[2], type).data_ptr();
+  const size_t n = static_cast<size_t>(l.numel());
+  const cudaStream_t st = stream();
+  if (type == at::kFloat)
+    check(unlocked([&] {
+            return tcrv_cuda_add_f32(floats(l), floats(r), static_cast<float *>(out), n, st);
+          }),
+          "tcrv_cuda_add_f32");
+  else
+    check(unlocked([&] {
+            return tcrv_cuda_add_i32(static_cast<const int32_t *>(l.data_ptr()), static_cast<const int32_t *>(r.data_ptr()),
+                                     static_cast<int32_t *>(out), n, st);
+          }),
+          "tcrv_cuda_add_i32");
+  return given_or_wrapped(a[2], std::move(made));
+}
+
+// dequantize(vx, out, block_bytes)
+TCRV_CALL(dequantize, 3) {
+  const int64_t block = integer(a[2]);
+  const at::Tensor &vx = dense(a[0], at::kByte);
+  if (vx.dim() == 0)
+    fail(PyExc_ValueError, "blocks come in rows");
+  const int64_t nb = blocks_of(vx.size(-1), block);
+  at::Tensor made;
+  if (a[1] == Py_None) {
+    auto shape = vx.sizes().vec();
+    shape.back() = nb * kQK;
+    made = empty(shape, at::kFloat, vx);
+  }
+  const at::Tensor &out = a[1] == Py_None ? made : dense(a[1], at::kFloat);
+  const size_t n = static_cast<size_t>(out.numel());
+  const cudaStream_t st = stream();
+  if (block == TCRV_Q8_0_BLOCK_BYTES)
+    check(unlocked([&] { return tcrv_cuda_dequantize_row_q8_0(bytes(vx), floats(out), n, st); }), "tcrv_cuda_dequantize_row_q8_0");
+  else
+    check(unlocked([&] { return tcrv_cuda_dequantize_row_q4_0(bytes(vx), floats(out), n, st); }), "tcrv_cuda_dequantize_row_q4_0");
+  return given_or_wrapped(a[1], std::move(made));
+}
+
+// quantize(x, out, block_bytes)
+TCRV_CALL(quantize, 3) {
+  const int64_t block = integer(a[2]);
+  const at::Tensor &x = tensor(a[0]);
+  if (x.dim() == 0 || x.size(-1) % kQK != 0)
+    fail(PyExc_ValueError, "last dimension must be a multiple of 32");
+  dense(a[0], at::kFloat);
+  at::Tensor made;
+  if (a[1] == Py_None) {
+    auto shape = x.sizes().vec();
+    shape.back() = shape.back() / kQK * block;
+    made = empty(shape, at::kByte, x);
+  }
+  const at::Tensor &out = a[1] == Py_None ? made : dense(a[1], at::kByte);
+  const size_t n = static_cast<size_t>(x.numel());
+  const cudaStream_t st = stream();
+  if (block == TCRV_Q8_0_BLOCK_BYTES)
+    check(unlocked([&] { return tcrv_cuda_quantize_row_q8_0(n, floats(x), bytes(out), st); }), "tcrv_cuda_quantize_row_q8_0");
+  else
+    check(unlocked([&] { return tcrv_cuda_quantize_row_q4_0(n, floats(x), bytes(out), st); }), "tcrv_cuda_quantize_row_q4_0");
+  return given_or_wrapped(a[1], std::move(made));
+}
+
+// gemv(w, x, q8_weights, flags, out)
+TCRV_CALL(gemv, 5) {
+  const bool q8 = truth(a[2]);
+  const unsigned flags = static_cast<unsigned>(integer(a[3]));
+  const at::Tensor &w = tensor(a[0]), &x = tensor(a[1]);
+  if (w.dim() != 2 || x.dim() != 2)
+    fail(PyExc_ValueError, "weights are (rows, row_bytes), activations are (columns, column_bytes)");
+  const int64_t nb = blocks_of(x.size(1), TCRV_Q8_0_BLOCK_BYTES);
+  if (blocks_of(w.size(1), q8 ? TCRV_Q8_0_BLOCK_BYTES : TCRV_Q4_0_BLOCK_BYTES) != nb)
+    fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
+  const int64_t nr = w.size(0), nc = x.size(0);
+  at::Tensor made;
+  if (a[4] == Py_None)
+    made = empty({nr, nc}, at::kFloat, w);
+  const at::Tensor &out = a[4] == Py_None ? made : dense(a[4], at::kFloat);
+  const size_t n = static_cast<size_t>(nb * kQK), bx = static_cast<size_t>(w.stride(0)),
+               by = static_cast<size_t>(x.stride(0)), bs = static_cast<size_t>(out.stride(0));
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return (q8 ? tcrv_cuda_gemv_q8_0_q8_0 : tcrv_cuda_gemv_q4_0_q8_0)(
+              n, floats(out), bytes(w), bytes(x), by, static_cast<size_t>(nr), static_cast<size_t>(nc), bx, bs, flags, st);
+        }),
+        q8 ? "tcrv_cuda_gemv_q8_0_q8_0" : "tcrv_cuda_gemv_q4_0_q8_0");
+  return given_or_wrapped(a[4], std::move(made));
+}
+
+// gemv_group(address of the calls, count, q8_weights, flags)
+TCRV_CALL(gemv_group, 4) {
+  const auto *calls = reinterpret_cast<const tcrv_cuda_gemv_call *>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLong(a[0])));
+  if (PyErr_Occurred())
+    throw PyError{};
+  const size_t count = static_cast<size_t>(integer(a[1]));
+  const bool q8 = truth(a[2]);
+  const unsigned flags = static_cast<unsigned>(integer(a[3]));
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return (q8 ? tcrv_cuda_gemv_group_q8_0_q8_0 : tcrv_cuda_gemv_group_q4_0_q8_0)(calls, count, flags, st);
+        }),
+        q8 ? "tcrv_cuda_gemv_group_q8_0_q8_0" : "tcrv_cuda_gemv_group_q4_0_q8_0");
+  Py_RETURN_NONE;
+}
+
+// Device scratch of at least `need` bytes: the caller's tensor, or a new one.  (A new one may go
+// back to torch's allocator as soon as the launches are queued: its next user on this stream
+// runs behind them.)
+inline const at::Tensor &scratch(PyObject *given, at::Tensor &made, size_t need, const at::Tensor &like) {
+  if (given != Py_None)
+    return tensor(given);
+  made = empty({static_cast<int64_t>(need < 256 ? 256 : need)}, at::kByte, like);
+  return made;
+}
+
+// gemm(w, x, out, workspace)
+TCRV_CALL(gemm, 4) {
+  const at::Tensor &w = tensor(a[0]), &x = tensor(a[1]);
+  if (w.dim() != 2 || x.dim() != 2)
+    fail(PyExc_ValueError, "weights are (rows, row_bytes), activations are (columns, column_bytes)");
+  const int64_t nb = blocks_of(x.size(1), TCRV_Q8_0_BLOCK_BYTES);
+  if (blocks_of(w.size(1), TCRV_Q4_0_BLOCK_BYTES) != nb)
+    fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
+  const size_t n = static_cast<size_t>(nb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
+  at::Tensor made, made_ws;
+  if (a[2] == Py_None)
+    made = empty({w.size(0), x.size(0)}, at::kFloat, w);
+  const at::Tensor &out = a[2] == Py_None ? made : dense(a[2], at::kFloat);
+  const at::Tensor &ws = scratch(a[3], made_ws, tcrv_cuda_gemm_workspace_bytes(n, nr, nc), w);
+  const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0)), bs = static_cast<size_t>(out.stride(0));
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return tcrv_cuda_gemm_q4_0_q8_0(n, floats(out), bytes(w), bytes(x), by, nr, nc, bx, bs, ws.data_ptr(),
+                                          static_cast<size_t>(ws.numel()), 0, st);
+        }),
+        "tcrv_cuda_gemm_q4_0_q8_0");
+  return given_or_wrapped(a[2], std::move(made));
+}
+
+// gemm_prepared(buffer, n, nr, x, out, workspace)
+TCRV_CALL(gemm_prepared, 6) {
+  const at::Tensor &buffer = tensor(a[0]), &x = tensor(a[3]);
+  const size_t n = static_cast<size_t>(integer(a[1])), nr = static_cast<size_t>(integer(a[2]));
+  if (x.dim() != 2)
+    fail(PyExc_ValueError, "activations are (columns, column_bytes)");
+  if (static_cast<size_t>(blocks_of(x.size(1), TCRV_Q8_0_BLOCK_BYTES) * kQK) != n)
+    fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
+  const size_t nc = static_cast<size_t>(x.size(0));
+  at::Tensor made, made_ws;
+  if (a[4] == Py_None)
+    made = empty({static_cast<int64_t>(nr), x.size(0)}, at::kFloat, x);
+  const at::Tensor &out = a[4] == Py_None ? made : dense(a[4], at::kFloat);
+  const at::Tensor &ws = scratch(a[5], made_ws, tcrv_cuda_gemm_acts_workspace_bytes(n, nc), x);
+  const size_t by = static_cast<size_t>(x.stride(0)), bs = static_cast<size_t>(out.stride(0));
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return tcrv_cuda_gemm_q4_0_q8_0_prepared(n, floats(out), buffer.data_ptr(), bytes(x), by, nr, nc, bs, ws.data_ptr(),
+                                                   static_cast<size_t>(ws.numel()), 0, st);
+        }),
+        "tcrv_cuda_gemm_q4_0_q8_0_prepared");
+  return given_or_wrapped(a[4], std::move(made));
+}
+
+// sibling_dot_rows(format, weight block bytes, activation block bytes, w, x, out)
+TCRV_CALL(sibling_dot_rows, 6) {
+  const int format = static_cast<int>(integer(a[0]));
+  const int64_t wb = integer(a[1]), ab = integer(a[2]);
+  const at::Tensor &w = dense(a[3], at::kByte), &x = dense(a[4], at::kByte);
+  if (w.dim() != 2 || x.dim() != 2 || w.size(1) % wb != 0 || x.size(1) % ab != 0 || w.size(1) / wb != x.size(1) / ab)
+    fail(PyExc_ValueError, "row bytes do not match the format's block sizes");
+  const size_t n = static_cast<size_t>(w.size(1) / wb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
+  at::Tensor made;
+  if (a[5] == Py_None)
+    made = empty({w.size(0), x.size(0)}, at::kFloat, w);
+  const at::Tensor &out = a[5] == Py_None ? made : dense(a[5], at::kFloat);
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return tcrv_cuda_sibling_dot_rows(format, n, floats(out), bytes(w), bytes(x), static_cast<size_t>(x.stride(0)), nr, nc,
+                                            static_cast<size_t>(w.stride(0)), static_cast<size_t>(out.stride(0)), st);
+        }),
+        "tcrv_cuda_sibling_dot_rows");
+  return given_or_wrapped(a[5], std::move(made));
+}
+
+inline const at::Tensor &row_matrix(PyObject *o) {
+  const bool is = THPVariable_Check(o);
+  if (!is || !THPVariable_Unpack(o).is_cuda() || THPVariable_Unpack(o).dim() != 2 || THPVariable_Unpack(o).stride(1) != 1 ||
+      THPVariable_Unpack(o).scalar_type() != at::kFloat)
+    fail(PyExc_ValueError, "x must be a 2-D float32 CUDA tensor with unit inner stride");
+  return THPVariable_Unpack(o);
+}
+
+// rms_norm(x, eps, out, flags)
+TCRV_CALL(rms_norm, 4) {
+  const at::Tensor &x = row_matrix(a[0]);
+  const float eps = static_cast<float>(real(a[1]));
+  const unsigned flags = static_cast<unsigned>(integer(a[3]));
+  at::Tensor made;
+  if (a[2] == Py_None)
+    made = empty({x.size(0), x.size(1)}, at::kFloat, x);
+  const at::Tensor &out = a[2] == Py_None ? made : tensor(a[2]);
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return tcrv_cuda_rms_norm_f32_flags(static_cast<size_t>(x.size(1)), floats(x), floats(out), eps,
+                                              static_cast<size_t>(x.size(0)), static_cast<size_t>(x.stride(0)),
+                                              static_cast<size_t>(out.stride(0)), flags, st);
+        }),
+        "tcrv_cuda_rms_norm_f32_flags");
+  return given_or_wrapped(a[2], std::move(made));
+}
+
+// rope_apply(x, cache, out)
+TCRV_CALL(rope_apply, 3) {
+  const at::Tensor &x = row_matrix(a[0]);
+  const at::Tensor &cache = dense(a[1], at::kFloat);
+  at::Tensor made;
+  if (a[2] == Py_None)
+    made = empty({x.size(0), x.size(1)}, at::kFloat, x);
+  const at::Tensor &out = a[2] == Py_None ? made : tensor(a[2]);
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return tcrv_cuda_rope_apply_f32(static_cast<size_t>(x.size(1)), floats(x), floats(out), floats(cache),
+                                          static_cast<size_t>(x.size(0)), static_cast<size_t>(x.stride(0)),
+                                          static_cast<size_t>(out.stride(0)), st);
+        }),
+        "tcrv_cuda_rope_apply_f32");
+  return given_or_wrapped(a[2], std::move(made));
+}
+
+// vec_silu(x, out)
+TCRV_CALL(vec_silu, 2) {
+  const at::Tensor &x = dense(a[0], at::kFloat);
+  at::Tensor made;
+  if (a[1] == Py_None)
+    made = empty(x.sizes(), at::kFloat, x);
+  const at::Tensor &out = a[1] == Py_None ? made : dense(a[1], at::kFloat);
+  const cudaStream_t st = stream();
+  check(unlocked([&] { return tcrv_cuda_vec_silu_f32(static_cast<size_t>(x.numel()), floats(x), floats(out), st); }),
+        "tcrv_cuda_vec_silu_f32");
+  return given_or_wrapped(a[1], std::move(made));
+}
+
+// vec_scale_(y, v)
+TCRV_CALL(vec_scale_, 2) {
+  const at::Tensor &y = dense(a[0], at::kFloat);
+  const float v = static_cast<float>(real(a[1]));
+  const cudaStream_t st = stream();
+  check(unlocked([&] { return tcrv_cuda_vec_scale_f32(static_cast<size_t>(y.numel()), floats(y), v, st); }),
+        "tcrv_cuda_vec_scale_f32");
+  Py_INCREF(a[0]);
+  return a[0];
+}
+
+// repack_gemv(wx16, x, nc, q8_weights, out, flags)
+TCRV_CALL(repack_gemv, 6) {
+  const at::Tensor &w = tensor(a[0]), &x = tensor(a[1]);
+  const int64_t nc = integer(a[2]);
+  const bool q8 = truth(a[3]);
+  const unsigned flags = static_cast<unsigned>(integer(a[5]));
+  const int64_t nb = x.numel() / TCRV_Q8_0_BLOCK_BYTES;
+  if (x.numel() % TCRV_Q8_0_BLOCK_BYTES != 0 || nc % 16 != 0 || w.numel() != nc / 16 * nb * (q8 ? 544 : 288))
+    fail(PyExc_ValueError, "weights, activation and nc do not describe the same shape");
+  dense(a[0], at::kByte);
+  dense(a[1], at::kByte);
+  at::Tensor made;
+  if (a[4] == Py_None)
+    made = empty({nc}, at::kFloat, w);
+  const at::Tensor &out = a[4] == Py_None ? made : dense(a[4], at::kFloat);
+  const cudaStream_t st = stream();
+  check(unlocked([&] {
+          return (q8 ? tcrv_cuda_repack_gemv_q8_0_q8_0 : tcrv_cuda_repack_gemv_q4_0_q8_0)(
+              static_cast<size_t>(nb * kQK), floats(out), bytes(w), bytes(x), static_cast<size_t>(nc), flags, st);
+        }),
+        "tcrv_cuda_repack_gemv");
+  return given_or_wrapped(a[4], std::move(made));
+}
+
+// bind(_check)
+TCRV_CALL(bind, 1) {
+  Py_INCREF(a[0]);
+  Py_XSETREF(g_check, a[0]);
+  Py_RETURN_NONE;
+}
+
+#define TCRV_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {TCRV_METHOD(add),          TCRV_METHOD(dequantize),       TCRV_METHOD(quantize),
+                         TCRV_METHOD(gemv),         TCRV_METHOD(gemv_group),       TCRV_METHOD(gemm),
+                         TCRV_METHOD(gemm_prepared), TCRV_METHOD(sibling_dot_rows), TCRV_METHOD(rms_norm),
+                         TCRV_METHOD(rope_apply),   TCRV_METHOD(vec_silu),         TCRV_METHOD(vec_scale_),
+                         TCRV_METHOD(repack_gemv),  TCRV_METHOD(bind),             {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_tcrv_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__tcrv_torch() { return PyModule_Create(&module_def); }
