@@ -22,7 +22,7 @@ TORCH_CALLS = os.path.join(HERE, "_tcrv_torch.so")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17", "-rdc=true",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC", "-shared", "--threads", "0",
 ]
 
 

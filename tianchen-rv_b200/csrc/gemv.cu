@@ -3,6 +3,7 @@
 // block count and also implements the strict (sequential) fold order.  Plus the debug kernel
 // that exposes the integer stage (per-block int32 sums).
 #include <atomic>
+#include "gemv_any.cuh"
 #include "gemv_mma.cuh"
 #include "gemv_mma_rows.cuh"
 #include "gemv_mma_strict.cuh"
@@ -196,6 +197,7 @@ int launch_stream(const GemvArgs &args, uint32_t nc, int grid, size_t smem, cuda
 inline bool multiple_of(const void *p, uintptr_t m) { return reinterpret_cast<uintptr_t>(p) % m == 0; }
 
 constexpr size_t kMmaMinCols = 4;
+constexpr int kAnyMinRows = 8;
 
 // Ring depth of the tensor-core GEMV for a row of nb blocks with `groups` 16-row groups per
 // slot, 0 if it does not fit.
@@ -577,6 +579,17 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
       return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sm_count(), stream);
   }
 
+  // rows the kernels above cannot take (a block count that is no multiple of 8, a base or stride
+  // off 16 bytes): the streaming kernel for any row.  Fewer rows than a CTA has warps leave most
+  // of its memory idle; they, odd addresses and more than 8 columns stay on the general kernel.
+  if (nr >= static_cast<size_t>(kAnyMinRows)) {
+    GemvAnyPlan plan;
+    constexpr int kFormat = kQ8W ? 5 : 4;
+    if (plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, strict, (flags & TCRV_CUDA_FLAG_STATIC_WEIGHTS) != 0,
+                               sm_count(), plan))
+      return strict ? launch_gemv_any<kFormat, true>(plan, stream) : launch_gemv_any<kFormat, false>(plan, stream);
+  }
+
   // generic path
   const size_t items = nr * nc;
   size_t blocks = (items + 7) / 8;
@@ -600,48 +613,10 @@ template int launch_gemv<true>(size_t, float *, const uint8_t *, const uint8_t *
 
 namespace {
 
-template <bool kQ8W>
-int launch_gemv_group_impl(const GemvGroupItem *items, size_t count, cudaStream_t stream) {
-  if (count < 2 || count > static_cast<size_t>(kGemvGroupMax))
-    return TCRV_CUDA_ERR_UNSUPPORTED;
-  const bool strict = (items[0].flags & TCRV_CUDA_FLAG_STRICT_ORDER) != 0;
-  constexpr unsigned kKnownFlags = TCRV_CUDA_FLAG_STRICT_ORDER | TCRV_CUDA_FLAG_STATIC_WEIGHTS;
-  GemvGroupArgs group = {};
-  group.count = static_cast<uint32_t>(count);
-  size_t smem = 0;
-  double cost[kGemvGroupMax], all_cost = 0.0;
-  uint32_t warps = 0;
-  int cap[kGemvGroupMax];
-  for (size_t i = 0; i < count; ++i) {
-    const GemvGroupItem &it = items[i];
-    const uint32_t nb = static_cast<uint32_t>(it.n / kQK);
-    // one column each, no tuning bits, the same order for all, operands the bulk copies accept
-    if (it.nc != 1 || it.nr == 0 || (it.flags & ~kKnownFlags) != 0 ||
-        ((it.flags & TCRV_CUDA_FLAG_STRICT_ORDER) != 0) != strict || it.n % kQK != 0 || nb == 0 || nb % 8 != 0 ||
-        !multiple_of(it.vx, 16) || it.bx % 16 != 0 || !multiple_of(it.vy, 2) || it.by % 2 != 0)
-      return TCRV_CUDA_ERR_UNSUPPORTED;
-    StreamPlan plan;
-    const bool ok = strict ? plan_stream_strict<kQ8W>(nb, it.s, it.vx, it.vy, it.by, it.nr, 1, it.bx, it.bs, it.flags, plan)
-                           : plan_stream_fast<kQ8W>(nb, it.s, it.vx, it.vy, it.by, it.nr, 1, it.bx, it.bs, it.flags, plan);
-    if (!ok)
-      return TCRV_CUDA_ERR_UNSUPPORTED;
-    group.problem[i] = plan.args;
-    cap[i] = plan.grid;
-    smem = plan.smem > smem ? plan.smem : smem;
-    warps = plan.args.nwarps > warps ? plan.args.nwarps : warps;
-    // What a problem costs an SM: its weight bytes, and more per byte where rows longer than
-    // 4.5 KB leave a CTA fewer warps and rows per slot (measured per-SM rates on 32000 x 4096
-    // against 4096 x 11008: 39 : 35 GB/s in the kernel's own order, 36 : 22 in the reference's).
-    const double per_byte = plan.args.row_bytes > 4608 ? (strict ? 1.5 : 1.1) : 1.0;
-    cost[i] = static_cast<double>(it.nr) * plan.args.row_bytes * per_byte;
-    all_cost += cost[i];
-  }
-  // One CTA per SM in all, dealt in proportion to that cost (every problem at least one, none
-  // more than it has slots of rows), so that all problems end at about the same time.
-  const uint32_t sms = static_cast<uint32_t>(sm_count());
-  if (count > sms)
-    return TCRV_CUDA_ERR_UNSUPPORTED;
-  uint32_t share[kGemvGroupMax], dealt = 0;
+// Deals `sms` CTAs out among the problems of a group in proportion to their cost (every problem at
+// least one, none more than it has slots of rows), so that all end at about the same time.
+void deal_ctas(const double *cost, double all_cost, const int *cap, size_t count, uint32_t sms, uint32_t *share) {
+  uint32_t dealt = 0;
   for (size_t i = 0; i < count; ++i) {
     uint32_t want = static_cast<uint32_t>(cost[i] / all_cost * sms);
     want = want < 1 ? 1 : want;
@@ -672,6 +647,98 @@ int launch_gemv_group_impl(const GemvGroupItem *items, size_t count, cudaStream_
       --dealt;
     }
   }
+}
+
+// The group on the streaming kernel for any row (one launch; same orders, same bits).
+template <bool kQ8W>
+int launch_gemv_any_group(const GemvGroupItem *items, size_t count, bool strict, cudaStream_t stream) {
+  constexpr int kFormat = kQ8W ? 5 : 4;
+  GemvAnyGroupArgs group = {};
+  group.count = static_cast<uint32_t>(count);
+  const uint32_t sms = static_cast<uint32_t>(sm_count());
+  if (count > sms)
+    return TCRV_CUDA_ERR_UNSUPPORTED;
+  size_t smem = 0;
+  double cost[kGemvGroupMax], all_cost = 0.0;
+  int cap[kGemvGroupMax];
+  uint32_t warps = 0, share[kGemvGroupMax];
+  for (size_t i = 0; i < count; ++i) {
+    const GemvGroupItem &it = items[i];
+    GemvAnyPlan plan;
+    if (!plan_gemv_any<kFormat>(it.n, it.s, it.vx, it.vy, it.by, it.nr, 1, it.bx, it.bs, strict,
+                                (it.flags & TCRV_CUDA_FLAG_STATIC_WEIGHTS) != 0, static_cast<int>(sms), plan))
+      return TCRV_CUDA_ERR_UNSUPPORTED;
+    group.problem[i] = plan.args;
+    cap[i] = plan.grid;
+    smem = plan.smem > smem ? plan.smem : smem;
+    warps = plan.args.nwarps > warps ? plan.args.nwarps : warps;
+    cost[i] = static_cast<double>(it.nr) * plan.args.row_bytes;
+    all_cost += cost[i];
+  }
+  deal_ctas(cost, all_cost, cap, count, sms, share);
+  for (size_t i = 0; i < count; ++i)
+    group.first[i + 1] = group.first[i] + share[i];
+  auto kernel = strict ? gemv_any_group_kernel<kFormat, true> : gemv_any_group_kernel<kFormat, false>;
+  static std::atomic<bool> configured[2][64];
+  const int st = any_configure(kernel, configured[strict ? 1 : 0]);
+  if (st != TCRV_CUDA_OK)
+    return st;
+  TCRV_CUDA_TRY(launch_pdl(kernel, static_cast<int>(group.first[count]), static_cast<int>(warps * 32), smem, stream, group));
+  TCRV_CUDA_TRY(cudaGetLastError());
+  return TCRV_CUDA_OK;
+}
+
+template <bool kQ8W>
+int launch_gemv_group_impl(const GemvGroupItem *items, size_t count, cudaStream_t stream) {
+  if (count < 2 || count > static_cast<size_t>(kGemvGroupMax))
+    return TCRV_CUDA_ERR_UNSUPPORTED;
+  const bool strict = (items[0].flags & TCRV_CUDA_FLAG_STRICT_ORDER) != 0;
+  constexpr unsigned kKnownFlags = TCRV_CUDA_FLAG_STRICT_ORDER | TCRV_CUDA_FLAG_STATIC_WEIGHTS;
+  GemvGroupArgs group = {};
+  group.count = static_cast<uint32_t>(count);
+  size_t smem = 0;
+  double cost[kGemvGroupMax], all_cost = 0.0;
+  uint32_t warps = 0;
+  int cap[kGemvGroupMax];
+  bool aligned = true;
+  for (size_t i = 0; i < count; ++i) {
+    const GemvGroupItem &it = items[i];
+    const uint32_t nb = static_cast<uint32_t>(it.n / kQK);
+    // one column each, no tuning bits, the same order for all
+    if (it.nc != 1 || it.nr == 0 || (it.flags & ~kKnownFlags) != 0 ||
+        ((it.flags & TCRV_CUDA_FLAG_STRICT_ORDER) != 0) != strict || it.n % kQK != 0)
+      return TCRV_CUDA_ERR_UNSUPPORTED;
+    aligned = aligned && nb != 0 && nb % 8 == 0 && multiple_of(it.vx, 16) && it.bx % 16 == 0;
+  }
+  if (!aligned)
+    return launch_gemv_any_group<kQ8W>(items, count, strict, stream);
+  for (size_t i = 0; i < count; ++i) {
+    const GemvGroupItem &it = items[i];
+    const uint32_t nb = static_cast<uint32_t>(it.n / kQK);
+    if (!multiple_of(it.vy, 2) || it.by % 2 != 0)
+      return TCRV_CUDA_ERR_UNSUPPORTED;
+    StreamPlan plan;
+    const bool ok = strict ? plan_stream_strict<kQ8W>(nb, it.s, it.vx, it.vy, it.by, it.nr, 1, it.bx, it.bs, it.flags, plan)
+                           : plan_stream_fast<kQ8W>(nb, it.s, it.vx, it.vy, it.by, it.nr, 1, it.bx, it.bs, it.flags, plan);
+    if (!ok)
+      return TCRV_CUDA_ERR_UNSUPPORTED;
+    group.problem[i] = plan.args;
+    cap[i] = plan.grid;
+    smem = plan.smem > smem ? plan.smem : smem;
+    warps = plan.args.nwarps > warps ? plan.args.nwarps : warps;
+    // What a problem costs an SM: its weight bytes, and more per byte where rows longer than
+    // 4.5 KB leave a CTA fewer warps and rows per slot (measured per-SM rates on 32000 x 4096
+    // against 4096 x 11008: 39 : 35 GB/s in the kernel's own order, 36 : 22 in the reference's).
+    const double per_byte = plan.args.row_bytes > 4608 ? (strict ? 1.5 : 1.1) : 1.0;
+    cost[i] = static_cast<double>(it.nr) * plan.args.row_bytes * per_byte;
+    all_cost += cost[i];
+  }
+  // One CTA per SM in all
+  const uint32_t sms = static_cast<uint32_t>(sm_count());
+  if (count > sms)
+    return TCRV_CUDA_ERR_UNSUPPORTED;
+  uint32_t share[kGemvGroupMax];
+  deal_ctas(cost, all_cost, cap, count, sms, share);
   group.first[0] = 0;
   for (size_t i = 0; i < count; ++i)
     group.first[i + 1] = group.first[i] + share[i];

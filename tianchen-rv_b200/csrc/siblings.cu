@@ -6,6 +6,7 @@
 //   Q4_1, Q5_1:  sumf = sumf + fma(d_x*d_y, (float)sumi, m_x*s_y)
 // (the contraction one C expression gets; lib/Conversion/RVV/RVVToEmitCBlockQuantLinear.cpp:
 // 6817-7263, 472-915, 916-1391).
+#include "gemv_any.cuh"
 #include "launchers.h"
 #include "strict_stream.cuh"
 #include "tcrv_common.cuh"
@@ -107,6 +108,9 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
         vx, vy, sums, bx, by, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
   } else if (const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx)) {
     return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sm_count(), stream);
+  } else if (GemvAnyPlan plan; nr >= 8 && plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true,
+                                                                 /*static_weights=*/false, sm_count(), plan)) {
+    return launch_gemv_any<kFormat, true>(plan, stream);  // rows of any block count on 2-byte boundaries
   } else {
     const size_t want = (nr * nc + 7) / 8;
     sibling_dot_kernel<kFormat><<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(
