@@ -141,10 +141,16 @@ __device__ __forceinline__ int any_sumi(const AnyBlock &b, const uint32_t (&y)[8
   return F::kBias != 0 ? raw - static_cast<int>(bias_sum) : raw;
 }
 
-// kRows rows of a slot against every column.
-template <int kFormat, int kCols, bool kStrict, int kRows>
-__device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *slot, const uint32_t (&off)[4], uint32_t r_first,
-                                         const uint8_t *xsm, uint32_t xcol_bytes, float *table, uint32_t row, int lane) {
+// Items of a lane that fit in registers for a whole kernel (one column): rows of up to 128 blocks.
+template <int kFormat>
+constexpr int kAnyXItems = AnyFormat<kFormat>::kPairs ? 2 : 4;
+
+// kRows rows of a slot against every column.  kMis: a row may start in the middle of a word.
+// kXReg: the lane's activation items are in `xr` (one column, at most kAnyXItems items a lane).
+template <int kFormat, int kCols, bool kStrict, bool kMis, bool kXReg, int kRows>
+__device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *slot, const uint32_t (&off)[4],
+                                         const AnyX<kFormat> *xr, const uint8_t *xsm, uint32_t xcol_bytes, float *table,
+                                         uint32_t row, int lane) {
   using F = StrictFormat<kFormat>;
   using A = AnyFormat<kFormat>;
   constexpr uint32_t U = A::kUnit, UW = A::kUnitWords;
@@ -154,8 +160,8 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
   uint32_t sh[kRows];
 #pragma unroll
   for (int r = 0; r < kRows; ++r) {
-    base[r] = reinterpret_cast<const uint32_t *>(slot + (off[r_first + r] & ~3u));
-    sh[r] = (off[r_first + r] & 2u) * 8u;
+    base[r] = reinterpret_cast<const uint32_t *>(slot + (kMis ? off[r] & ~3u : off[r]));
+    sh[r] = (off[r] & 2u) * 8u;
   }
   float acc[kRows][kCols];
 #pragma unroll
@@ -164,17 +170,23 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
     for (int c = 0; c < kCols; ++c)
       acc[r][c] = 0.0f;
   float *prod = table + ncols * kRows * pitch;  // kTwo: the second plane
-  for (uint32_t p = lane; p < units; p += 32) {
+  auto one_item = [&](uint32_t p, [[maybe_unused]] const AnyX<kFormat> *xp) {
     uint32_t w[kRows][UW];
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
-      uint32_t t[UW + 1];
+      if constexpr (kMis) {
+        uint32_t t[UW + 1];
 #pragma unroll
-      for (uint32_t k = 0; k <= UW; ++k)
-        t[k] = base[r][p * UW + k];
+        for (uint32_t k = 0; k <= UW; ++k)
+          t[k] = base[r][p * UW + k];
 #pragma unroll
-      for (uint32_t k = 0; k < UW; ++k)
-        w[r][k] = __funnelshift_r(t[k], t[k + 1], sh[r]);
+        for (uint32_t k = 0; k < UW; ++k)
+          w[r][k] = __funnelshift_r(t[k], t[k + 1], sh[r]);
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < UW; ++k)
+          w[r][k] = base[r][p * UW + k];
+      }
     }
     const bool second = U == 2 && 2 * p + 1 < nb;
 #pragma unroll
@@ -182,7 +194,10 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
       if (kCols > 1 && c >= static_cast<int>(ncols))
         break;
       AnyX<kFormat> x;
-      any_load_x<kFormat>(x, xsm + static_cast<size_t>(c) * xcol_bytes, units, nbp, p);
+      if constexpr (kXReg)
+        x = *xp;
+      else
+        any_load_x<kFormat>(x, xsm + static_cast<size_t>(c) * xcol_bytes, units, nbp, p);
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
         float term[U], pr[U];
@@ -221,6 +236,15 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
         }
       }
     }
+  };
+  if constexpr (kXReg) {
+#pragma unroll
+    for (int i = 0; i < kAnyXItems<kFormat>; ++i)
+      if (lane + 32u * i < units)
+        one_item(lane + 32u * i, xr + i);
+  } else {
+    for (uint32_t p = lane; p < units; p += 32)
+      one_item(p, nullptr);
   }
   if constexpr (!kStrict) {
 #pragma unroll
@@ -275,7 +299,7 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
 }
 
 // CTA `cta` of the `nctas` that share the problem.  The block may have more warps than a.nwarps.
-template <int kFormat, int kCols, bool kStrict>
+template <int kFormat, int kCols, bool kStrict, bool kMis, bool kXReg>
 __device__ __forceinline__ void gemv_any_body(const GemvAnyArgs &a, uint32_t cta, uint32_t nctas, uint8_t *smem) {
   using F = StrictFormat<kFormat>;
   constexpr uint32_t U = AnyFormat<kFormat>::kUnit;
@@ -380,6 +404,13 @@ __device__ __forceinline__ void gemv_any_body(const GemvAnyArgs &a, uint32_t cta
   if (spare)
     return;
 
+  AnyX<kFormat> xr[kXReg ? kAnyXItems<kFormat> : 1];
+  if constexpr (kXReg) {
+#pragma unroll
+    for (int i = 0; i < kAnyXItems<kFormat>; ++i)
+      if (lane + 32u * i < units)
+        any_load_x<kFormat>(xr[i], xsm, units, nbp, lane + 32u * i);
+  }
   float *table = reinterpret_cast<float *>(tables + static_cast<size_t>(warp) * a.table_bytes);
   for (uint32_t t = 0; t < mine; ++t) {
     const uint32_t bar = warp * kAnyRing + t % kAnyRing;
@@ -419,24 +450,24 @@ __device__ __forceinline__ void gemv_any_body(const GemvAnyArgs &a, uint32_t cta
     }
     if (rows == 4) {
       if constexpr (kCols == 1)
-        any_rows<kFormat, kCols, kStrict, 4>(a, slot, off, 0, xsm, xcol_bytes, table, row, lane);
+        any_rows<kFormat, kCols, kStrict, kMis, kXReg, 4>(a, slot, off, xr, xsm, xcol_bytes, table, row, lane);
     } else if (rows == 3) {
       if constexpr (kCols == 1)
-        any_rows<kFormat, kCols, kStrict, 3>(a, slot, off, 0, xsm, xcol_bytes, table, row, lane);
+        any_rows<kFormat, kCols, kStrict, kMis, kXReg, 3>(a, slot, off, xr, xsm, xcol_bytes, table, row, lane);
     } else if (rows == 2) {
       if constexpr (kCols <= 4)
-        any_rows<kFormat, kCols, kStrict, 2>(a, slot, off, 0, xsm, xcol_bytes, table, row, lane);
+        any_rows<kFormat, kCols, kStrict, kMis, kXReg, 2>(a, slot, off, xr, xsm, xcol_bytes, table, row, lane);
     } else {
-      any_rows<kFormat, kCols, kStrict, 1>(a, slot, off, 0, xsm, xcol_bytes, table, row, lane);
+      any_rows<kFormat, kCols, kStrict, kMis, kXReg, 1>(a, slot, off, xr, xsm, xcol_bytes, table, row, lane);
     }
     __syncwarp();
   }
 }
 
-template <int kFormat, int kCols, bool kStrict>
+template <int kFormat, int kCols, bool kStrict, bool kMis, bool kXReg>
 __global__ void __launch_bounds__(kAnyMaxWarps * 32, 1) gemv_any_kernel(const __grid_constant__ GemvAnyArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
-  gemv_any_body<kFormat, kCols, kStrict>(a, blockIdx.x, gridDim.x, smem);
+  gemv_any_body<kFormat, kCols, kStrict, kMis, kXReg>(a, blockIdx.x, gridDim.x, smem);
 }
 
 // Several independent one-column problems in one launch (see gemv_stream_group_kernel).
@@ -452,7 +483,12 @@ __global__ void __launch_bounds__(kAnyMaxWarps * 32, 1) gemv_any_group_kernel(co
   uint32_t i = 0;
   while (i + 1 < g.count && blockIdx.x >= g.first[i + 1])
     ++i;
-  gemv_any_body<kFormat, 1, kStrict>(g.problem[i], blockIdx.x - g.first[i], g.first[i + 1] - g.first[i], smem);
+  const GemvAnyArgs &a = g.problem[i];
+  const uint32_t cta = blockIdx.x - g.first[i], nctas = g.first[i + 1] - g.first[i];
+  if (any_units<kFormat>(a.nb) <= 32u * kAnyXItems<kFormat>)
+    gemv_any_body<kFormat, 1, kStrict, true, true>(a, cta, nctas, smem);
+  else
+    gemv_any_body<kFormat, 1, kStrict, true, false>(a, cta, nctas, smem);
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -525,28 +561,43 @@ int any_configure(Kernel kernel, std::atomic<bool> (&configured)[64]) {
   return TCRV_CUDA_OK;
 }
 
-template <int kFormat, int kCols, bool kStrict>
+template <int kFormat, int kCols, bool kStrict, bool kMis, bool kXReg>
 int launch_any_instance(const GemvAnyPlan &plan, cudaStream_t stream) {
   static std::atomic<bool> configured[64];
-  const int st = any_configure(gemv_any_kernel<kFormat, kCols, kStrict>, configured);
+  auto kernel = gemv_any_kernel<kFormat, kCols, kStrict, kMis, kXReg>;
+  const int st = any_configure(kernel, configured);
   if (st != TCRV_CUDA_OK)
     return st;
-  TCRV_CUDA_TRY(launch_pdl(gemv_any_kernel<kFormat, kCols, kStrict>, plan.grid, static_cast<int>(plan.args.nwarps * 32),
-                           plan.smem, stream, plan.args));
+  TCRV_CUDA_TRY(launch_pdl(kernel, plan.grid, static_cast<int>(plan.args.nwarps * 32), plan.smem, stream, plan.args));
   TCRV_CUDA_TRY(cudaGetLastError());
   return TCRV_CUDA_OK;
 }
 
 // (column counts are served by the next larger of 1, 2, 4, 8: the loops stop at the real count)
+template <int kFormat, bool kStrict, bool kMis>
+int launch_any_columns(const GemvAnyPlan &plan, cudaStream_t stream) {
+  if (plan.args.nc == 1) {
+    if (any_units<kFormat>(plan.args.nb) <= 32u * kAnyXItems<kFormat>)
+      return launch_any_instance<kFormat, 1, kStrict, kMis, true>(plan, stream);
+    return launch_any_instance<kFormat, 1, kStrict, kMis, false>(plan, stream);
+  }
+  if (plan.args.nc == 2)
+    return launch_any_instance<kFormat, 2, kStrict, kMis, false>(plan, stream);
+  if (plan.args.nc <= 4)
+    return launch_any_instance<kFormat, 4, kStrict, kMis, false>(plan, stream);
+  return launch_any_instance<kFormat, 8, kStrict, kMis, false>(plan, stream);
+}
+
 template <int kFormat, bool kStrict>
 int launch_gemv_any(const GemvAnyPlan &plan, cudaStream_t stream) {
-  if (plan.args.nc == 1)
-    return launch_any_instance<kFormat, 1, kStrict>(plan, stream);
-  if (plan.args.nc == 2)
-    return launch_any_instance<kFormat, 2, kStrict>(plan, stream);
-  if (plan.args.nc <= 4)
-    return launch_any_instance<kFormat, 4, kStrict>(plan, stream);
-  return launch_any_instance<kFormat, 8, kStrict>(plan, stream);
+  // The sibling formats have no other streaming kernel for one word-aligned row after another, so
+  // they get an instance without the re-alignment; Q4_0 and Q8_0 rows of that kind go elsewhere.
+  if constexpr (kFormat <= 3) {
+    const GemvAnyArgs &a = plan.args;
+    if (((reinterpret_cast<uintptr_t>(a.vx) | a.bx) & 3u) == 0)
+      return launch_any_columns<kFormat, kStrict, false>(plan, stream);
+  }
+  return launch_any_columns<kFormat, kStrict, true>(plan, stream);
 }
 
 }  // namespace tcrv

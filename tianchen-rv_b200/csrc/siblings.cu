@@ -93,6 +93,16 @@ __global__ void __launch_bounds__(256) sibling_dot_kernel(const uint8_t *__restr
   }
 }
 
+// Which of the two streaming kernels takes a call that both accept.  Measured (us, table per CTA /
+// table per warp): one column of Q5_0 against many short rows is the one family where the
+// former's 512 workers on one slot win, 10.6 / 11.7 on 11008 x 4096 and 23.5 / 25.8 on 32000 x 4096;
+// Q4_1 and Q5_1 there 8.5 / 8.4 and 11.0 / 10.7, four columns 22.1 / 18.3 (Q5_0), 4096 x 11008
+// 13.0 / 10.1 (Q4_1), 1024 x 1024 3.5 / 2.8, eight columns equal within 3 %.
+template <int kFormat>
+bool table_per_cta(uint32_t nb, size_t nr, size_t nc) {
+  return kFormat == 2 && nc == 1 && nb <= 128 && nr >= 8192;
+}
+
 template <int kFormat>
 int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8_t *vy, size_t by, size_t nr, size_t nc,
                size_t bx, size_t bs, cudaStream_t stream) {
@@ -106,11 +116,11 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
     const size_t want = (nr * nc * nb + 255) / 256;
     sibling_sums_kernel<kFormat><<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(
         vx, vy, sums, bx, by, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
-  } else if (const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx)) {
+  } else if (const uint32_t rps = table_per_cta<kFormat>(nb, nr, nc) ? strict_stream_rows<kFormat>(nb, nr, nc, vx, bx) : 0) {
     return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sm_count(), stream);
   } else if (GemvAnyPlan plan; nr >= 8 && plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true,
                                                                  /*static_weights=*/false, sm_count(), plan)) {
-    return launch_gemv_any<kFormat, true>(plan, stream);  // rows of any block count on 2-byte boundaries
+    return launch_gemv_any<kFormat, true>(plan, stream);
   } else {
     const size_t want = (nr * nc + 7) / 8;
     sibling_dot_kernel<kFormat><<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(
