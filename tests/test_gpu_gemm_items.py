@@ -1,0 +1,38 @@
+"""GPU parity, work items of the prefill GEMM: whole, half and narrow items at their edges (rows around
+128 and 256, columns around 32 and 64, block counts that end a stage early) equal the sequential oracle
+bit for bit, in both folds' layouts and with several destinations."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nr,k,nc", [
+    (127, 32, 31), (129, 96, 33), (255, 160, 63), (257, 224, 65), (4096, 416, 77),  # narrow items
+    (4864, 160, 512),   # 152 whole items: one round and four items cut into halves
+    (4737, 96, 481),    # the same with a second row tile that does not exist and ragged columns
+    (20480, 32, 128),   # 160 whole items of one block
+])
+def test_items_at_their_edges_are_bit_exact(cuda, pkg, O, nr, k, nc):
+    w = O.quantize_q4_0(O.fill_normal(nr * k, 51, 0, 0.02).reshape(nr, k))
+    x = O.quantize_q8_0(O.fill_normal(nc * k, 52).reshape(nc, k))
+    want = O.gemm(w, x, fold=O.FOLD_FMA, threads=8).view(np.uint32)
+    wd, xd = cuda.from_numpy(w).cuda(), cuda.from_numpy(x).cuda()
+    pw = pkg.PreparedWeights(wd)
+    assert np.array_equal(pkg.gemm(pw, xd).cpu().numpy().view(np.uint32), want)
+    # two destinations: the staging tile of the fused gather
+    L = pkg.lib()
+    ws = cuda.empty(L.tcrv_cuda_gemm_acts_workspace_bytes(k, nc), dtype=cuda.uint8, device="cuda")
+    bs = (nc + 3) // 4 * 4
+    outs = [cuda.full((nr, bs), -1.0, dtype=cuda.float32, device="cuda") for _ in range(2)]
+    dst = (ctypes.c_void_p * 2)(*[o.data_ptr() for o in outs])
+    st = L.tcrv_cuda_gemm_q4_0_q8_0_prepared_multi(k, dst, 2, pw.buffer.data_ptr(), xd.data_ptr(), xd.stride(0), nr, nc,
+                                                   bs, ws.data_ptr(), ws.numel(), 0,
+                                                   cuda.cuda.current_stream().cuda_stream)
+    assert st == 0
+    pkg.check_device_errors()
+    for o in outs:
+        res = o.cpu().numpy()
+        assert np.array_equal(np.ascontiguousarray(res[:, :nc]).view(np.uint32), want) and np.all(res[:, nc:] == -1.0)

@@ -19,8 +19,6 @@ namespace tcrv {
 
 namespace {
 
-constexpr bool kGemmF8 = true;
-
 constexpr size_t kAlign = 256;
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -290,7 +288,7 @@ int make_map_2d(CUtensorMap *map, CUtensorMapDataType type, size_t elem_bytes, c
 struct PlanarSizes {
   size_t nb, nbp, ncp, k;
   size_t w8, dw, x8, dxt;  // region sizes (aligned)
-  size_t x_plane;          // one activation plane; x8 holds one (int8) or two (e4m3 low, high)
+  size_t x_plane;          // one activation plane; x8 holds two (low, high)
 };
 
 PlanarSizes planar_sizes(size_t n, size_t nr, size_t nc) {
@@ -302,7 +300,7 @@ PlanarSizes planar_sizes(size_t n, size_t nr, size_t nc) {
   p.w8 = align_up(nr * n, kAlign);
   p.dw = align_up(nr * p.nbp * 4, kAlign);
   p.x_plane = align_up(nc * n, kAlign);
-  p.x8 = (kGemmF8 ? 2 : 1) * p.x_plane;
+  p.x8 = 2 * p.x_plane;
   p.dxt = align_up(p.nb * p.ncp * 4, kAlign);
   return p;
 }
@@ -313,38 +311,79 @@ inline int blocks_for(size_t items) {
   return static_cast<int>(b < cap ? (b ? b : 1) : cap);
 }
 
-// `repack`: fold with the scales multiplied first and store token-major (dst[0][col*bs + row]).
-int run_gemm(size_t n, float *const *dst, size_t ndst, const uint8_t *weights_planar, const uint8_t *acts_planar,
-             size_t nr, size_t nc, size_t bs, cudaStream_t stream, bool repack = false) {
-  const PlanarSizes p = planar_sizes(n, nr, nc);
+// Whether a launch deals out 128 x 32 items instead of 256 x 64 ones (whose last round is cut into
+// 128 x 64 halves where those fill no more than half of the SMs).  Rounds of each kind times what an
+// item takes, in hundredths of a 256 x 64 one: measured on 512 x 32000 x 4096, 36.6 us a round of whole
+// items, 19.5 of halves, 13.8 of narrow ones.  Narrow items win where the others leave SMs without
+// work: 77 x 4096 x 11008 44.0 against 55.6 us; 512 x 11008 x 4096 144 against 97.0 us.
+bool narrow_items(size_t nr, size_t nc, size_t ctas) {
+  const auto cdiv = [](size_t a, size_t b) { return (a + b - 1) / b; };
+  const size_t tiles = cdiv(nr, 256) * cdiv(nc, 64), rem = tiles % ctas;
+  const size_t wide = tiles / ctas * 100 + (rem == 0 ? 0 : 2 * rem <= ctas ? 54 : 100);
+  return cdiv(cdiv(nr, 128) * cdiv(nc, 32), ctas) * 38 < wide;
+}
+
+// One instantiation of the kernel: its tensor maps, its work items, its launch.
+template <bool kMulti, bool kRepack, bool kNarrow>
+int launch_gemm_kernel(const PlanarSizes &p, const uint8_t *weights_planar, const uint8_t *acts_planar, GemmArgs &args,
+                       cudaStream_t stream) {
+  using Plan = GemmPlan<kNarrow>;
   const int8_t *w8 = reinterpret_cast<const int8_t *>(weights_planar);
   const float *dw = reinterpret_cast<const float *>(weights_planar + p.w8);
   const int8_t *x8 = reinterpret_cast<const int8_t *>(acts_planar);
   const float *dxt = reinterpret_cast<const float *>(acts_planar + p.x8);
+  const size_t n = p.k, nr = args.nr, nc = args.nc;
 
   CUtensorMap map_w, map_x, map_xhi, map_dw, map_dx;
   int st = make_map_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w8, n, nr, n, kGemmStageBlocks * kQK, kGemmTileRows,
                        CU_TENSOR_MAP_SWIZZLE_128B);
-  // activations and their scales are fetched in boxes of 64 columns (two per full tile)
   if (st == TCRV_CUDA_OK)
-    st = make_map_2d(&map_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, x8, n, nc, n, kGemmStageBlocks * kQK, kGemmHalfCols,
+    st = make_map_2d(&map_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, x8, n, nc, n, kGemmStageBlocks * kQK, Plan::kBoxCols,
                      CU_TENSOR_MAP_SWIZZLE_128B);
   if (st == TCRV_CUDA_OK)
-    st = make_map_2d(&map_xhi, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, x8 + (kGemmF8 ? p.x_plane : 0), n, nc, n,
-                     kGemmStageBlocks * kQK, kGemmHalfCols, CU_TENSOR_MAP_SWIZZLE_128B);
+    st = make_map_2d(&map_xhi, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, x8 + p.x_plane, n, nc, n, kGemmStageBlocks * kQK,
+                     Plan::kBoxCols, CU_TENSOR_MAP_SWIZZLE_128B);
   if (st == TCRV_CUDA_OK)
     st = make_map_2d(&map_dw, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dw, p.nbp, nr, p.nbp * 4, kGemmStageBlocks,
                      kGemmTileRows, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (st == TCRV_CUDA_OK)
-    st = make_map_2d(&map_dx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dxt, p.ncp, p.nb, p.ncp * 4, kGemmHalfCols,
+    st = make_map_2d(&map_dx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dxt, p.ncp, p.nb, p.ncp * 4, Plan::kBoxCols,
                      kGemmStageBlocks, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (st != TCRV_CUDA_OK)
     return st;
 
+  args.tiles_m = static_cast<uint32_t>((nc + Plan::Full::kCols - 1) / Plan::Full::kCols);
+  const uint32_t tiles = static_cast<uint32_t>((nr + Plan::Full::kRows - 1) / Plan::Full::kRows) * args.tiles_m;
+  const uint32_t ctas = static_cast<uint32_t>(sm_count());
+  const uint32_t rem = tiles % ctas;
+  args.full_items = !kNarrow && 2 * rem <= ctas ? tiles - rem : tiles;
+  args.items = args.full_items + 2 * (tiles - args.full_items);
+  const int grid = static_cast<int>(args.items < ctas ? args.items : ctas);
+
+  constexpr size_t smem = GemmSmem<kMulti, kNarrow>::kBytes;
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  TCRV_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64)
+    return TCRV_CUDA_ERR_UNSUPPORTED;
+  if (!configured[dev]) {
+    TCRV_CUDA_TRY(cudaFuncSetAttribute(gemm_q4_0_q8_0_tc_kernel<kMulti, kRepack, kNarrow>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    configured[dev] = true;
+  }
+  TCRV_CUDA_TRY(launch_pdl(gemm_q4_0_q8_0_tc_kernel<kMulti, kRepack, kNarrow>, grid, kGemmThreads, smem, stream, map_w,
+                           map_x, map_xhi, map_dw, map_dx, args));
+  TCRV_CUDA_TRY(cudaGetLastError());
+  return TCRV_CUDA_OK;
+}
+
+// `repack`: fold with the scales multiplied first and store token-major (dst[0][col*bs + row]).
+int run_gemm(size_t n, float *const *dst, size_t ndst, const uint8_t *weights_planar, const uint8_t *acts_planar,
+             size_t nr, size_t nc, size_t bs, cudaStream_t stream, bool repack = false) {
+  const PlanarSizes p = planar_sizes(n, nr, nc);
   const bool multi = ndst > 1;
   if (repack && multi)
     return TCRV_CUDA_ERR_UNSUPPORTED;
-  const int sms = sm_count();
   GemmArgs args = {};
   for (size_t d = 0; d < ndst; ++d)
     args.dst[d] = dst[d];
@@ -353,51 +392,13 @@ int run_gemm(size_t n, float *const *dst, size_t ndst, const uint8_t *weights_pl
   args.nr = static_cast<uint32_t>(nr);
   args.nc = static_cast<uint32_t>(nc);
   args.nb = static_cast<uint32_t>(p.nb);
-  args.tiles_m = static_cast<uint32_t>((nc + kGemmTileCols - 1) / kGemmTileCols);
-  // Work items: whole tiles round-robin over the CTAs; a last round that would occupy at most
-  // half of them is cut into half-width items instead (see gemm_tc.cuh).
-  const uint32_t tiles = static_cast<uint32_t>((nr + kGemmTileRows - 1) / kGemmTileRows) * args.tiles_m;
-  const uint32_t ctas = static_cast<uint32_t>(sms);
-  const uint32_t rem = tiles % ctas;
-  if (rem != 0 && 2 * rem <= ctas) {
-    args.full_items = tiles - rem;
-    args.items = args.full_items + 2 * rem;
-  } else {
-    args.full_items = tiles;
-    args.items = tiles;
-  }
-  const int grid = static_cast<int>(args.items < ctas ? args.items : ctas);
-
-  const int variant = repack ? 2 : (multi ? 1 : 0);
-  static std::atomic<bool> configured[64][3];
-  int dev = 0;
-  TCRV_CUDA_TRY(cudaGetDevice(&dev));
-  constexpr size_t smem_single = GemmSmem<false, kGemmF8>::kBytes, smem_multi = GemmSmem<true, kGemmF8>::kBytes;
-  if (dev < 0 || dev >= 64)
-    return TCRV_CUDA_ERR_UNSUPPORTED;
-  if (!configured[dev][variant]) {
-    if (repack)
-      TCRV_CUDA_TRY(cudaFuncSetAttribute(gemm_q4_0_q8_0_tc_kernel<false, true, kGemmF8>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_single)));
-    else if (multi)
-      TCRV_CUDA_TRY(cudaFuncSetAttribute(gemm_q4_0_q8_0_tc_kernel<true, false, kGemmF8>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_multi)));
-    else
-      TCRV_CUDA_TRY(cudaFuncSetAttribute(gemm_q4_0_q8_0_tc_kernel<false, false, kGemmF8>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_single)));
-    configured[dev][variant] = true;
-  }
-  if (repack)
-    TCRV_CUDA_TRY(launch_pdl(gemm_q4_0_q8_0_tc_kernel<false, true, kGemmF8>, grid, kGemmThreads, smem_single, stream,
-                             map_w, map_x, map_xhi, map_dw, map_dx, args));
-  else if (multi)
-    TCRV_CUDA_TRY(launch_pdl(gemm_q4_0_q8_0_tc_kernel<true, false, kGemmF8>, grid, kGemmThreads, smem_multi, stream,
-                             map_w, map_x, map_xhi, map_dw, map_dx, args));
-  else
-    TCRV_CUDA_TRY(launch_pdl(gemm_q4_0_q8_0_tc_kernel<false, false, kGemmF8>, grid, kGemmThreads, smem_single, stream,
-                             map_w, map_x, map_xhi, map_dw, map_dx, args));
-  TCRV_CUDA_TRY(cudaGetLastError());
-  return TCRV_CUDA_OK;
+  if (multi)
+    return launch_gemm_kernel<true, false, false>(p, weights_planar, acts_planar, args, stream);
+  if (narrow_items(nr, nc, static_cast<size_t>(sm_count())))
+    return repack ? launch_gemm_kernel<false, true, true>(p, weights_planar, acts_planar, args, stream)
+                  : launch_gemm_kernel<false, false, true>(p, weights_planar, acts_planar, args, stream);
+  return repack ? launch_gemm_kernel<false, true, false>(p, weights_planar, acts_planar, args, stream)
+                : launch_gemm_kernel<false, false, false>(p, weights_planar, acts_planar, args, stream);
 }
 
 }  // namespace

@@ -4,23 +4,32 @@
 //   S_b[row,col]    = int32 dot of the 32 int8 weight values and 32 int8 activation values
 //
 // Every ggml block (32 elements of K) has its own pair of fp16 scales, so the contraction
-// cannot accumulate across blocks inside the tensor core: each block gets a fresh TMEM
-// accumulator tile (128 weight rows x up to 128 activation columns, K = 32), and the epilogue
-// warps fold that tile into fp32 register accumulators with the two scales before the block
-// after next arrives.  The fold runs in strict ascending block order per output element, in
+// cannot accumulate across blocks inside the tensor core: each block gets fresh TMEM
+// accumulator tiles (128 weight rows x up to 64 activation columns, K = 32), and the epilogue
+// warps fold them into fp32 register accumulators with the two scales.  The fold runs in strict ascending block order per output element, in
 // the fused form fma((float)S * d_w, d_x, acc).
 //
 // The fold on the CUDA cores, not the tensor pipe, bounds this kernel, so the tensor core is
-// asked for the form that is cheapest to fold.  Two operand encodings exist:
-//  * kF8 (default): the block sum arrives as an fp32 number.  Weights (nibble - 8, in
-//    [-8, 7]) are stored as e4m3, where every such integer is exact; an int8 activation q
-//    is split as q = 16*h + l with h = q >> 4 in [-8, 7] and l = q & 15 in [0, 15], and the
-//    two e4m3 planes 16*h and l are both exact.  Two tcgen05.mma kind::f8f6f4 per block (the
-//    second accumulating) give S exactly: every product is an integer below 2^11, every
-//    partial sum an integer below 2^17, far inside fp32's 24-bit significand.  The fold is
-//    then two packed fp32 operations per pair of outputs and nothing else.
-//  * int8 (kind::i8): one MMA per block into an int32 tile; the epilogue pays an integer add
-//    per element to turn it into a float (see scaled_pair()).
+// asked for the form that is cheapest to fold: the block sum arrives as an fp32 number.
+// Weights (nibble - 8, in [-8, 7]) are stored as e4m3, where every such integer is exact; an
+// int8 activation q is split as q = 16*h + l with h = q >> 4 in [-8, 7] and l = q & 15 in
+// [0, 15], and the two e4m3 planes 16*h and l are both exact.  Two tcgen05.mma kind::f8f6f4 per
+// block (the second accumulating) give S exactly: every product is an integer below 2^11, every
+// partial sum an integer below 2^17, far inside fp32's 24-bit significand.  The fold is
+// then two packed fp32 operations per pair of outputs and nothing else.  (int8 operands with
+// kind::i8 need one MMA and an integer add per element: 17 % slower.)
+//
+// Work items.  256 weight rows x 64 columns: the two row tiles share their columns, so one broadcast
+// load of activation scales serves two outputs of a thread (with 128 x 128 items those loads put 64 KB
+// per block through the shared-memory pipe beside the operands: 305 us for 512 x 32000 x 4096, 640
+// cycles per 128 x 128 x 32 of arithmetic that takes 276; they still cost 40 us of the 256).  8
+// epilogue warps with 64 accumulators a thread: fewer would not fill the FMA pipes, more leave no
+// registers for the second chunk buffer that hides the TMEM load and the barrier test (16 warps
+// without it: 318 us; 16 instead of 32 registers a chunk, scales fetched before the wait: 283 ->
+// 256 us).  512 x 11008 x 4096: 122.8 -> 97.0 us.
+// Whole items are dealt round-robin to the CTAs; a last round that would leave more than half of
+// them idle is cut into halves of 128 rows.  Few columns: items of 128 rows x 32 columns, 4 blocks to
+// a hand-over (gemm.cu chooses; 77 x 4096 x 11008: 89.9 -> 44.0 us, halves 55.6).
 //
 // A second fold (kRepack) serves the consumer of the 16-row interleaved layouts: the same
 // contraction with fma((float)S, d_w * d_x, acc) (the scales multiplied first, an exact
@@ -28,19 +37,14 @@
 //
 // Operands come from a planar ("prepared") layout written by the unpack kernels: 8-bit
 // matrices [rows][K] and fp32 scale matrices, all fetched with tiled TMA loads (128-byte
-// swizzle for the 8-bit tiles, no multicast).  Warp roles in a CTA of 18 warps:
-//   warps 0..15 epilogue: warp w reads TMEM lanes 32*(w%4).. (its weight rows) and a quarter
-//               of the columns of every accumulator tile
-//   warp 16     TMA producer (one lane)
-//   warp 17     TMEM allocation + MMA issue (one lane)
-// Pipelines: shared-memory stages of 4 blocks each (full/empty mbarriers) and two TMEM stages of
-// two accumulator tiles each, i.e. two consecutive blocks per hand-over (full/empty mbarriers),
-// so the tensor core runs up to four blocks ahead of the fold.  The epilogue warps wait on the
-// accumulator barriers only: a stage's scale tiles have landed when its first accumulator has.
-//
-// Work items: 128 x 128 tiles dealt round-robin to the CTAs; when the last round would leave
-// more than half of the CTAs idle its tiles are cut into two 128 x 64 items (same row order,
-// half the columns), which costs half a round instead of a whole one.
+// swizzle for the 8-bit tiles, no multicast).  Warp roles in a CTA of 10 warps:
+//   warps 0..7  epilogue: warp w reads TMEM lanes 32*(w%4).. (its weight rows) and half of the
+//               columns of every accumulator tile
+//   warp 8      TMA producer (one lane)
+//   warp 9      TMEM allocation + MMA issue (one elected lane)
+// Pipelines: shared-memory stages of 4 blocks each (full/empty mbarriers) and TMEM stages of
+// several blocks each (full/empty mbarriers).  The epilogue warps wait on the accumulator barriers
+// only: a stage's scale tiles have landed when its first accumulator has.
 //
 // Every wait is bounded; a failed wait raises the device error word and the CTA winds down.
 #pragma once
@@ -50,52 +54,69 @@
 
 namespace tcrv {
 
-constexpr int kGemmTileRows = 128;   // weight rows per tile  (MMA M, TMEM lanes)
-constexpr int kGemmTileCols = 128;   // activation columns per full tile (MMA N, TMEM columns)
-constexpr int kGemmHalfCols = 64;    // columns of a half item; also the column count of one activation TMA box
-constexpr int kGemmStageBlocks = 4;  // ggml blocks per shared-memory stage (128 bytes of K)
-// Blocks per accumulator hand-over.  Every hand-over costs an epilogue warp a barrier test and a
-// release (about 180 + 110 cycles in the instrumented kernel) whatever it carries, so a TMEM
-// stage holds the tiles of two consecutive blocks: measured 355 -> 331 us on N = 32000 and
-// 147 -> 133 us on N = 11008 against one block per hand-over (TCRV_GEMM_HANDOVER_BLOCKS=1).
-#ifndef TCRV_GEMM_HANDOVER_BLOCKS
-#define TCRV_GEMM_HANDOVER_BLOCKS 2
-#endif
-constexpr int kGemmHandover = TCRV_GEMM_HANDOVER_BLOCKS;  // 1 or 2
-static_assert(kGemmHandover == 1 || kGemmHandover == 2, "a stage of 4 blocks is handed over in ones or pairs");
-constexpr int kGemmTmemStages = 4 / kGemmHandover;        // accumulator stages in flight
-constexpr int kGemmTmemStageCols = kGemmTileCols * kGemmHandover;
-constexpr int kGemmTmemCols = kGemmTmemStages * kGemmTmemStageCols;  // 512: all of TMEM
-constexpr int kGemmEpilogueWarps = 16;                          // 4 lane quarters x 4 column groups
+constexpr int kGemmTileRows = 128;      // weight rows of one MMA (M, TMEM lanes)
+constexpr int kGemmStageBlocks = 4;     // ggml blocks per shared-memory stage (128 bytes of K)
+constexpr int kGemmTmemCols = 512;      // all of TMEM
+constexpr int kGemmEpilogueWarps = 8;  // 4 lane quarters x 2 column groups
 constexpr int kGemmThreads = (kGemmEpilogueWarps + 2) * 32;
-
-constexpr int kGemmABytes = kGemmTileRows * kGemmStageBlocks * kQK;       // 16384
-constexpr int kGemmBPlaneBytes = kGemmTileCols * kGemmStageBlocks * kQK;  // 16384
-constexpr int kGemmBHalfBytes = kGemmBPlaneBytes / 2;                     // one 64-column TMA box
-constexpr int kGemmDwBytes = kGemmTileRows * kGemmStageBlocks * 4;        // [128][4] fp32
-constexpr int kGemmDxBytes = kGemmStageBlocks * kGemmTileCols * 4;        // 2 x [4][64] fp32
-constexpr int kGemmDxHalfBytes = kGemmDxBytes / 2;
 constexpr int kGemmCtrlBytes = 1024;  // barriers, TMEM base, abort flag
 
-template <bool kF8>
-struct GemmStage {
-  static constexpr int kBBytes = kF8 ? 2 * kGemmBPlaneBytes : kGemmBPlaneBytes;  // e4m3: low plane, then high plane
-  static constexpr int kOffB = kGemmABytes;
-  static constexpr int kOffDw = kOffB + kBBytes;
-  static constexpr int kOffDx = kOffDw + kGemmDwBytes;
-  static constexpr int kBytes = kOffDx + kGemmDxBytes;  // 36864 (int8) / 53248 (e4m3); multiples of 1024
+// The shape of a work item: kRowTiles x 128 weight rows, kCols activation columns.
+template <int kRowTiles_, int kCols_>
+struct GemmShape {
+  static constexpr int kRowTiles = kRowTiles_, kCols = kCols_;
+  static constexpr int kRows = kRowTiles * kGemmTileRows;
+  static constexpr int kCpw = kCols / (kGemmEpilogueWarps / 4);  // columns of an epilogue warp
+  static constexpr int kBlockCols = kRowTiles * kCols;           // TMEM columns of one block's accumulators
+  // A chunk is what a thread loads from TMEM at a time, up to 16 registers: kChunkCols columns of its
+  // rows of one block, or all its columns of several blocks.
+  static constexpr int kChunkRegs = 16;
+  static constexpr int kChunkCols = kRowTiles * kCpw > kChunkRegs ? kChunkRegs / kRowTiles : kCpw;
+  static constexpr int kChunkBlocks = kChunkRegs / (kRowTiles * kChunkCols);
+  static constexpr int kBlockChunks = kCpw / kChunkCols;  // chunks of one block
+  // Blocks per accumulator hand-over.  A hand-over costs a barrier test, a release and a commit
+  // whatever it carries, so it carries what leaves two TMEM stages.
+  static constexpr int kHandover = 256 / kBlockCols < kGemmStageBlocks ? 256 / kBlockCols : kGemmStageBlocks;
+  static constexpr int kChunks = kGemmStageBlocks / kChunkBlocks * kBlockChunks;  // of a shared-memory stage
+  static constexpr int kHandoverChunks = kHandover / kChunkBlocks * kBlockChunks;
+  static_assert(kChunks % 2 == 0 && kChunks % kHandoverChunks == 0, "two chunk buffers, whole hand-overs");
 };
 
-// Several output copies: the finished tile is staged in shared memory as 128 rows of 512 bytes
-// (16 bytes of padding per row keep the staging stores conflict-free) and leaves through bulk
-// shared->global copies of whole rows.
-constexpr int kGemmOutRowBytes = kGemmTileCols * 4 + 16;
-constexpr int kGemmOutBytes = kGemmTileRows * kGemmOutRowBytes;  // 67584
+// What one launch works on: whole items, and halves of such items.
+template <bool kNarrow>
+struct GemmPlan {
+  using Full = GemmShape<kNarrow ? 1 : 2, kNarrow ? 32 : 64>;
+  using Half = GemmShape<1, kNarrow ? 32 : 64>;
+  static constexpr uint32_t kColParts = Full::kCols / Half::kCols;
+  static constexpr uint32_t kParts = Full::kRowTiles * kColParts;
+  static constexpr int kTmemStages = kNarrow ? 4 : 2;
+  static constexpr int kTmemStageCols = kGemmTmemCols / kTmemStages;
+  static_assert(Full::kBlockCols * Full::kHandover <= kTmemStageCols, "a hand-over fits a TMEM stage");
+  static_assert(Half::kBlockCols * Half::kHandover <= kTmemStageCols, "a hand-over fits a TMEM stage");
+  // one shared-memory stage; activations and their scales come in boxes of kBoxCols columns
+  static constexpr int kBoxCols = Half::kCols;
+  static constexpr int kATileBytes = kGemmTileRows * kGemmStageBlocks * kQK;  // 16384
+  static constexpr int kBoxBytes = kBoxCols * kGemmStageBlocks * kQK;
+  static constexpr int kPlaneBytes = Full::kCols * kGemmStageBlocks * kQK;    // one activation plane
+  static constexpr int kDwTileBytes = kGemmTileRows * kGemmStageBlocks * 4;   // [128][4] fp32
+  static constexpr int kDxBoxBytes = kGemmStageBlocks * kBoxCols * 4;         // [4][kBoxCols] fp32
+  static constexpr int kOffB = Full::kRowTiles * kATileBytes;                 // low plane, then high plane
+  static constexpr int kOffDw = kOffB + 2 * kPlaneBytes;
+  static constexpr int kOffDx = kOffDw + Full::kRowTiles * kDwTileBytes;
+  static constexpr int kStageBytes = (kOffDx + Full::kCols / kBoxCols * kDxBoxBytes + 1023) / 1024 * 1024;
+};
 
-template <bool kMulti, bool kF8>
+// Several output copies: a finished 128-row tile is staged in shared memory (16 bytes of padding
+// per row keep the staging stores conflict-free) and leaves through bulk shared->global copies of
+// whole rows.
+constexpr int kGemmOutRowBytes = 64 * 4 + 16;
+constexpr int kGemmOutBytes = kGemmTileRows * kGemmOutRowBytes;  // 34816
+
+template <bool kMulti, bool kNarrow>
 struct GemmSmem {
-  static constexpr int kStages = kF8 ? (kMulti ? 3 : 4) : (kMulti ? 4 : 5);
-  static constexpr size_t kBytes = kGemmCtrlBytes + 1024 + static_cast<size_t>(kStages) * GemmStage<kF8>::kBytes +
+  static constexpr int kStages = kNarrow ? 8 : kMulti ? 3 : 4;
+  static constexpr size_t kBytes = kGemmCtrlBytes + 1024 +
+                                   static_cast<size_t>(kStages) * GemmPlan<kNarrow>::kStageBytes +
                                    (kMulti ? kGemmOutBytes : 0);
 };
 
@@ -110,27 +131,25 @@ struct GemmArgs {
   uint32_t ndst;
   size_t bs;
   uint32_t nr, nc, nb;
-  uint32_t tiles_m;     // column tiles of 128
-  uint32_t full_items;  // items [0, full_items) are whole tiles; a multiple of the grid size unless all are
-  uint32_t items;       // items [full_items, items) are halves: tile full_items + j/2, half j&1
+  uint32_t tiles_m;     // column tiles
+  uint32_t full_items;  // items [0, full_items) are whole ones
+  uint32_t items;       // items [full_items, items) are halves: half j % 2 of whole item full_items + j / 2
 };
 
 struct GemmItem {
-  uint32_t n0, m0, width;
+  uint32_t n0, m0;
+  bool whole;
 };
 
+template <bool kNarrow>
 __device__ __forceinline__ GemmItem gemm_item(const GemmArgs &a, uint32_t idx) {
+  using Plan = GemmPlan<kNarrow>;
   GemmItem it;
-  if (idx < a.full_items) {
-    it.n0 = (idx / a.tiles_m) * kGemmTileRows;
-    it.m0 = (idx % a.tiles_m) * kGemmTileCols;
-    it.width = kGemmTileCols;
-  } else {
-    const uint32_t j = idx - a.full_items, tile = a.full_items + (j >> 1);
-    it.n0 = (tile / a.tiles_m) * kGemmTileRows;
-    it.m0 = (tile % a.tiles_m) * kGemmTileCols + (j & 1u) * kGemmHalfCols;
-    it.width = kGemmHalfCols;
-  }
+  it.whole = idx < a.full_items;
+  const uint32_t j = it.whole ? 0u : idx - a.full_items;
+  const uint32_t tile = it.whole ? idx : a.full_items + j / Plan::kParts, part = j % Plan::kParts;
+  it.n0 = (tile / a.tiles_m) * Plan::Full::kRows + part / Plan::kColParts * Plan::Half::kRows;
+  it.m0 = (tile % a.tiles_m) * Plan::Full::kCols + part % Plan::kColParts * Plan::Half::kCols;
   return it;
 }
 
@@ -148,11 +167,6 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
@@ -162,19 +176,6 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
 // 256-bit store of four packed fp32 pairs (address 32-byte aligned).
 __device__ __forceinline__ void st_global_v4_b64(float *p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
   asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
-}
-
-// int8 kind only: (float)S * d_w for two int32 block sums without an int->float conversion
-// instruction (the conversion unit, at 16 results per clock per SM, would bound the kernel):
-// adding 0x4B400000 to S as an INTEGER gives the bit pattern of the float 12582912 + S
-// exactly (|S| <= 32768 stays inside the binade whose ulp is 1), and
-// fma(12582912 + S, d_w, -12582912 * d_w) is the exact product S * d_w rounded once, i.e.
-// bit-identical to (float)S * d_w.  `c2` holds -12582912 * d_w (exact) in both halves.
-constexpr uint32_t kMagicBits = 0x4B400000u;
-constexpr float kMagic = 12582912.0f;
-
-__device__ __forceinline__ uint64_t biased_pair(uint32_t s_lo, uint32_t s_hi) {
-  return pack_f32x2(__uint_as_float(s_lo + kMagicBits), __uint_as_float(s_hi + kMagicBits));
 }
 
 struct PipeState {
@@ -200,43 +201,31 @@ __device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.
 __device__ __forceinline__ void bulk_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// One block's accumulator piece (this thread's row, CPW columns) folded into acc.
+// One block's part of a chunk (this thread's kRowTiles rows, kChunkCols columns of each) folded into
+// acc[.][col0 / 2 ..].
 //   plain:  acc = fma((float)S * d_w, d_x, acc)      repack: acc = fma((float)S, d_w * d_x, acc)
-// `dx` points at the CPW activation scales of this block in shared memory (16-byte aligned).
-template <int CPW, bool kRepack, bool kF8>
-__device__ __forceinline__ void fold_block(const uint32_t (&v)[CPW], uint64_t (&acc)[CPW / 2], float dw,
-                                           const uint8_t *dx) {
-  const uint64_t dw2 = pack_f32x2(dw, dw);
-  const ulonglong2 *dx2 = reinterpret_cast<const ulonglong2 *>(dx);
-  if constexpr (kF8) {
+// `dx2` holds the activation scales of this block and these columns; a scale that has been loaded
+// serves the rows of all row tiles.
+template <typename Shape, bool kRepack>
+__device__ __forceinline__ void fold_part(const uint32_t *v, uint64_t (&acc)[Shape::kRowTiles][Shape::kCpw / 2],
+                                          int col0, const float (&dw)[Shape::kRowTiles],
+                                          const ulonglong2 *dx2) {
 #pragma unroll
-    for (int j = 0; j < CPW / 4; ++j) {
-      const ulonglong2 d = dx2[j];
-      const uint64_t s0 = pack_f32x2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]));
-      const uint64_t s1 = pack_f32x2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-      if constexpr (kRepack) {
-        acc[2 * j] = fma_f32x2(s0, mul_f32x2(dw2, d.x), acc[2 * j]);
-        acc[2 * j + 1] = fma_f32x2(s1, mul_f32x2(dw2, d.y), acc[2 * j + 1]);
-      } else {
-        acc[2 * j] = fma_f32x2(mul_f32x2(s0, dw2), d.x, acc[2 * j]);
-        acc[2 * j + 1] = fma_f32x2(mul_f32x2(s1, dw2), d.y, acc[2 * j + 1]);
-      }
-    }
-  } else {
-    const float cneg = __fmul_rn(-kMagic, dw);  // exact: 2-bit x 11-bit significands
-    const uint64_t c2 = kRepack ? pack_f32x2(-kMagic, -kMagic) : pack_f32x2(cneg, cneg);
+  for (int j = 0; j < Shape::kChunkCols / 4; ++j) {
+    const ulonglong2 d = dx2[j];
+    const int at = col0 / 2 + 2 * j;
 #pragma unroll
-    for (int j = 0; j < CPW / 4; ++j) {
-      const ulonglong2 d = dx2[j];
-      const uint64_t b0 = biased_pair(v[4 * j], v[4 * j + 1]);
-      const uint64_t b1 = biased_pair(v[4 * j + 2], v[4 * j + 3]);
+    for (int r = 0; r < Shape::kRowTiles; ++r) {
+      const uint64_t dw2 = pack_f32x2(dw[r], dw[r]);
+      const uint32_t *s = v + r * Shape::kChunkCols + 4 * j;
+      const uint64_t s0 = pack_f32x2(__uint_as_float(s[0]), __uint_as_float(s[1]));
+      const uint64_t s1 = pack_f32x2(__uint_as_float(s[2]), __uint_as_float(s[3]));
       if constexpr (kRepack) {
-        // (float)S exactly: the biased value minus the bias (integers below 2^24)
-        acc[2 * j] = fma_f32x2(add_f32x2(b0, c2), mul_f32x2(dw2, d.x), acc[2 * j]);
-        acc[2 * j + 1] = fma_f32x2(add_f32x2(b1, c2), mul_f32x2(dw2, d.y), acc[2 * j + 1]);
+        acc[r][at] = fma_f32x2(s0, mul_f32x2(dw2, d.x), acc[r][at]);
+        acc[r][at + 1] = fma_f32x2(s1, mul_f32x2(dw2, d.y), acc[r][at + 1]);
       } else {
-        acc[2 * j] = fma_f32x2(fma_f32x2(b0, dw2, c2), d.x, acc[2 * j]);
-        acc[2 * j + 1] = fma_f32x2(fma_f32x2(b1, dw2, c2), d.y, acc[2 * j + 1]);
+        acc[r][at] = fma_f32x2(mul_f32x2(s0, dw2), d.x, acc[r][at]);
+        acc[r][at + 1] = fma_f32x2(mul_f32x2(s1, dw2), d.y, acc[r][at + 1]);
       }
     }
   }
@@ -252,7 +241,7 @@ struct GemmEpilogueCtx {
   PipeState ps, ts;
 };
 
-// Sync of the 16 epilogue warps on an mbarrier (bounded, unlike a named barrier).
+// Sync of the epilogue warps on an mbarrier (bounded, unlike a named barrier).
 __device__ __forceinline__ bool epilogue_sync(GemmEpilogueCtx &c, int lane) {
   __syncwarp();
   if (lane == 0)
@@ -262,158 +251,50 @@ __device__ __forceinline__ bool epilogue_sync(GemmEpilogueCtx &c, int lane) {
   return ok;
 }
 
-// One work item for one epilogue warp: fold all blocks, then store.  CPW = columns per warp
-// (a quarter of the item's width).  Returns false after a failed wait.
-template <int CPW, bool kMulti, bool kRepack, bool kF8>
-__device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilogueCtx &c, const GemmItem it, int warp,
-                                                   int lane) {
-  using Stage = GemmStage<kF8>;
-  constexpr int kStages = GemmSmem<kMulti, kF8>::kStages;
-  const int quarter = warp & 3, colgroup = warp >> 2;
-  const int row_local = quarter * 32 + lane;
-  const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
-  const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
-  // this warp's activation scales inside a stage's scale tile: full items hold two [4][64]
-  // boxes one after the other, half items one
-  const uint32_t dx_off = CPW == 32 ? static_cast<uint32_t>(colgroup >> 1) * kGemmDxHalfBytes + (colgroup & 1) * 128u
-                                    : static_cast<uint32_t>(colgroup) * 64u;
-  const uint32_t tmem_col = static_cast<uint32_t>(colgroup * CPW);
-  uint64_t acc[CPW / 2];
-#pragma unroll
-  for (int j = 0; j < CPW / 2; ++j)
-    acc[j] = 0ull;
-  for (uint32_t kb = 0; kb < nkb; ++kb) {
-    // The stage's scale tiles arrive with its operands (same transaction barrier), and the MMA
-    // thread issues a block's MMAs only after that barrier has completed; so when an
-    // accumulator barrier of this stage has completed, the scale tiles are in shared memory.
-    // The epilogue therefore does not wait on the stage's own barrier (one barrier test per
-    // warp and stage less: 332 -> 307 us on N = 32000) and reads no scale before its first
-    // accumulator wait of the stage.
-    const uint8_t *st = c.stages + static_cast<size_t>(c.ps.stage) * Stage::kBytes;
-    float dws[4];
-    const uint8_t *dx_base = st + Stage::kOffDx + dx_off;
-    const uint32_t steps = min(static_cast<uint32_t>(kGemmStageBlocks), a.nb - kb * kGemmStageBlocks);
-#pragma unroll
-    for (uint32_t kk = 0; kk < kGemmStageBlocks; kk += kGemmHandover) {
-      if (kk < steps) {
-        if (!mbar_wait_bounded(&c.tmem_full[c.ts.stage], c.ts.phase, c.abort_flag))
-          return false;
-        tcgen05_fence_after_thread_sync();
-        if (kk == 0) {
-          const float4 dw4 = reinterpret_cast<const float4 *>(st + Stage::kOffDw)[row_local];
-          dws[0] = dw4.x, dws[1] = dw4.y, dws[2] = dw4.z, dws[3] = dw4.w;
-        }
-        const uint32_t taddr = c.tmem_base + lane_field + c.ts.stage * kGemmTmemStageCols + tmem_col;
-        uint32_t v[CPW];
-        tmem_ld_32x32b<CPW>(taddr, v);
-        tmem_ld_wait();
-        if (kGemmHandover == 2 && kk + 1 < steps) {
-          // two blocks per hand-over: the stage goes back when the second tile has been read
-          fold_block<CPW, kRepack, kF8>(v, acc, dws[kk], dx_base + kk * (kGemmHalfCols * 4));
-          tmem_ld_32x32b<CPW>(taddr + kGemmTileCols, v);
-          tmem_ld_wait();
-        }
-        // the accumulator tiles are in registers: hand the TMEM stage back
-        tcgen05_fence_before_thread_sync();
-        __syncwarp();
-        if (lane == 0)
-          mbar_arrive(&c.tmem_empty[c.ts.stage]);
-        c.ts.advance(kGemmTmemStages);
-        const uint32_t last = (kGemmHandover == 2 && kk + 1 < steps) ? kk + 1 : kk;
-        fold_block<CPW, kRepack, kF8>(v, acc, dws[last], dx_base + last * (kGemmHalfCols * 4));
-      }
-    }
-    // this warp no longer needs the stage's scale tiles
-    __syncwarp();
-    if (lane == 0)
-      mbar_arrive(&c.smem_empty[c.ps.stage]);
-    c.ps.advance(kStages);
-  }
-
-  // ---- store: this thread owns CPW consecutive outputs of one weight row
-  const uint32_t row = it.n0 + row_local;
-  const uint32_t m0 = it.m0 + colgroup * CPW;
+// kCpw consecutive outputs of one weight row, columns m0.., to every destination (token-major: to
+// the one destination's column vectors).
+template <int kCpw, bool kRepack>
+__device__ __forceinline__ void store_outputs(const GemmArgs &a, const uint64_t (&acc)[kCpw / 2], uint32_t row,
+                                              uint32_t m0) {
+  if (row >= a.nr)
+    return;
   if constexpr (kRepack) {
-    // token-major: for one column the 32 lanes of the warp write 32 consecutive floats
-    if (row < a.nr) {
-      float *dst = a.dst[0] + row;
+    // for one column the 32 lanes of the warp write 32 consecutive floats
+    float *dst = a.dst[0] + row;
 #pragma unroll
-      for (int j = 0; j < CPW / 2; ++j) {
-        float lo, hi;
-        unpack_f32x2(acc[j], lo, hi);
-        if (m0 + 2 * j < a.nc)
-          dst[static_cast<size_t>(m0 + 2 * j) * a.bs] = lo;
-        if (m0 + 2 * j + 1 < a.nc)
-          dst[static_cast<size_t>(m0 + 2 * j + 1) * a.bs] = hi;
-      }
+    for (int j = 0; j < kCpw / 2; ++j) {
+      float lo, hi;
+      unpack_f32x2(acc[j], lo, hi);
+      if (m0 + 2 * j < a.nc)
+        dst[static_cast<size_t>(m0 + 2 * j) * a.bs] = lo;
+      if (m0 + 2 * j + 1 < a.nc)
+        dst[static_cast<size_t>(m0 + 2 * j + 1) * a.bs] = hi;
     }
-    return true;
+    return;
   }
-  if constexpr (kMulti) {
-    // whole item inside the matrix and every base 16-byte aligned: rows leave as bulk copies
-    bool bulk = (a.bs % 4 == 0) && (it.m0 + it.width <= a.nc);
-    for (uint32_t d = 0; d < a.ndst; ++d)
-      bulk = bulk && ((reinterpret_cast<uintptr_t>(a.dst[d]) & 15u) == 0);
-    if (bulk) {
-      // the previous item's copies must have read the staging tile before it is rewritten
-      bulk_store_wait_read();
-      if (!epilogue_sync(c, lane))
-        return false;
-      float4 *mine = reinterpret_cast<float4 *>(c.out_stage + static_cast<size_t>(row_local) * kGemmOutRowBytes +
-                                                static_cast<size_t>(colgroup) * CPW * 4);
+  bool vec = (a.bs % 4 == 0) && (m0 + kCpw <= a.nc);  // warp-uniform
+  for (uint32_t d = 0; d < a.ndst; ++d)
+    vec = vec && ((reinterpret_cast<uintptr_t>(a.dst[d]) & 15u) == 0);
+  const size_t off = static_cast<size_t>(row) * a.bs + m0;
+  for (uint32_t d = 0; d < a.ndst; ++d) {
+    float *dst = a.dst[d] + off;
+    if (vec && (a.bs % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.dst[d]) & 31u) == 0)) {
+      // 32-byte stores: every lane writes whole sectors of its row
 #pragma unroll
-      for (int j = 0; j < CPW / 4; ++j) {
+      for (int j = 0; j < kCpw / 8; ++j)
+        st_global_v4_b64(dst + 8 * j, acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+    } else if (vec) {
+#pragma unroll
+      for (int j = 0; j < kCpw / 4; ++j) {
         float4 o;
         unpack_f32x2(acc[2 * j], o.x, o.y);
         unpack_f32x2(acc[2 * j + 1], o.z, o.w);
-        mine[j] = o;
+        reinterpret_cast<float4 *>(dst)[j] = o;
       }
-      fence_proxy_async_smem();
-      if (!epilogue_sync(c, lane))
-        return false;
-      // thread t sends row t%128 to destinations t/128, t/128 + 4
-      const uint32_t t = static_cast<uint32_t>(warp * 32 + lane);
-      const uint32_t r = t & 127u, grow = it.n0 + r;
-      if (grow < a.nr) {
-        const uint8_t *src = c.out_stage + static_cast<size_t>(r) * kGemmOutRowBytes;
-        for (uint32_t d = t >> 7; d < a.ndst; d += 4)
-          bulk_store_s2g(a.dst[d] + static_cast<size_t>(grow) * a.bs + it.m0, src, it.width * 4u);
-      }
-      bulk_store_commit();
-      return true;
-    }
-  }
-  bool vec = (a.bs % 4 == 0) && (m0 + CPW <= a.nc);  // warp-uniform
-  for (uint32_t d = 0; d < a.ndst; ++d)
-    vec = vec && ((reinterpret_cast<uintptr_t>(a.dst[d]) & 15u) == 0);
-  if (vec) {
-    if (row < a.nr) {
-      const size_t off = static_cast<size_t>(row) * a.bs + m0;
-      for (uint32_t d = 0; d < a.ndst; ++d) {
-        float *dst = a.dst[d] + off;
-        if ((a.bs % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.dst[d]) & 31u) == 0)) {
-          // 32-byte stores: every lane writes whole sectors of its row
+    } else {
+      // ragged columns or unaligned bases: element by element
 #pragma unroll
-          for (int j = 0; j < CPW / 8; ++j)
-            st_global_v4_b64(dst + 8 * j, acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < CPW / 4; ++j) {
-            float4 o;
-            unpack_f32x2(acc[2 * j], o.x, o.y);
-            unpack_f32x2(acc[2 * j + 1], o.z, o.w);
-            reinterpret_cast<float4 *>(dst)[j] = o;
-          }
-        }
-      }
-    }
-  } else if (row < a.nr) {
-    // ragged columns or unaligned bases: this lane writes its row element by element
-    const size_t off = static_cast<size_t>(row) * a.bs + m0;
-    for (uint32_t d = 0; d < a.ndst; ++d) {
-      float *dst = a.dst[d] + off;
-#pragma unroll
-      for (int j = 0; j < CPW / 2; ++j) {
+      for (int j = 0; j < kCpw / 2; ++j) {
         float lo, hi;
         unpack_f32x2(acc[j], lo, hi);
         if (m0 + 2 * j < a.nc)
@@ -423,33 +304,253 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
       }
     }
   }
+}
+
+// One work item for one epilogue warp: fold all blocks, then store.  Returns false after a failed
+// wait.
+template <typename Plan, typename Shape, bool kMulti, bool kRepack, int kStages>
+__device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilogueCtx &c, const GemmItem it, int warp,
+                                                   int lane) {
+  constexpr int kCpw = Shape::kCpw, kRt = Shape::kRowTiles;
+  const int quarter = warp & 3, colgroup = warp >> 2;
+  const int row_local = quarter * 32 + lane;
+  const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
+  const uint32_t tmem_lane = c.tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + colgroup * kCpw;
+  uint64_t acc[kRt][kCpw / 2];
+#pragma unroll
+  for (int r = 0; r < kRt; ++r)
+#pragma unroll
+    for (int j = 0; j < kCpw / 2; ++j)
+      acc[r][j] = 0ull;
+  uint32_t v[2][Shape::kChunkRegs];
+  // chunk i of a shared-memory stage, from TMEM into a buffer; waits for the hand-over that the
+  // chunk opens
+  auto load_chunk = [&](uint32_t i, uint32_t buffer) -> bool {
+    if (i % Shape::kHandoverChunks == 0) {
+      if (!mbar_wait_bounded(&c.tmem_full[c.ts.stage], c.ts.phase, c.abort_flag))
+        return false;
+      tcgen05_fence_after_thread_sync();
+    }
+    const uint32_t h = i % Shape::kHandoverChunks / Shape::kBlockChunks * Shape::kChunkBlocks;  // block of the hand-over
+    const uint32_t taddr = tmem_lane + c.ts.stage * Plan::kTmemStageCols + h * Shape::kBlockCols +
+                           i % Shape::kBlockChunks * Shape::kChunkCols;
+#pragma unroll
+    for (int t = 0; t < Shape::kChunkBlocks * kRt; ++t)
+      tmem_ld_32x32b<Shape::kChunkCols>(taddr + t * Shape::kCols, v[buffer] + t * Shape::kChunkCols);
+    return true;
+  };
+  auto release_tmem = [&]() {  // the hand-over's last chunk is in registers: the TMEM stage goes back
+    tcgen05_fence_before_thread_sync();
+    __syncwarp();
+    if (lane == 0)
+      mbar_arrive(&c.tmem_empty[c.ts.stage]);
+    c.ts.advance(Plan::kTmemStages);
+  };
+  // The stage's scale tiles arrive with its operands (same transaction barrier), and the MMA
+  // warp issues a block's MMAs only after that barrier has completed; so when an
+  // accumulator barrier of this stage has completed, the scale tiles are in shared memory.
+  // The epilogue therefore does not wait on the stage's own barrier and reads no scale before
+  // its first accumulator wait of the stage.
+  const uint8_t *st = nullptr;
+  float dws[kGemmStageBlocks][kRt];
+  auto open_stage = [&]() {
+    st = c.stages + static_cast<size_t>(c.ps.stage) * Plan::kStageBytes;
+#pragma unroll
+    for (int r = 0; r < kRt; ++r) {
+      const float4 dw4 = reinterpret_cast<const float4 *>(st + Plan::kOffDw)[r * kGemmTileRows + row_local];
+      dws[0][r] = dw4.x, dws[1][r] = dw4.y, dws[2][r] = dw4.z, dws[3][r] = dw4.w;
+    }
+  };
+  auto close_stage = [&]() {  // this warp no longer needs the stage's scale tiles
+    __syncwarp();
+    if (lane == 0)
+      mbar_arrive(&c.smem_empty[c.ps.stage]);
+    c.ps.advance(kStages);
+  };
+  // the activation scales of chunk i into a buffer, from the stage `at`: column c of an item is column
+  // c % kBoxCols of box c / kBoxCols
+  constexpr int kScaleVecs = Shape::kChunkCols / 4;
+  ulonglong2 xd[2][Shape::kChunkBlocks * kScaleVecs];
+  auto load_scales = [&](const uint8_t *at, uint32_t i, uint32_t buffer) {
+    const uint32_t block = i / Shape::kBlockChunks * Shape::kChunkBlocks;
+    const uint32_t col = colgroup * kCpw + i % Shape::kBlockChunks * Shape::kChunkCols;
+    const uint8_t *dx = at + Plan::kOffDx + col / Plan::kBoxCols * Plan::kDxBoxBytes + col % Plan::kBoxCols * 4;
+#pragma unroll
+    for (uint32_t b = 0; b < Shape::kChunkBlocks; ++b)
+#pragma unroll
+      for (int j = 0; j < kScaleVecs; ++j)
+        xd[buffer][b * kScaleVecs + j] =
+            reinterpret_cast<const ulonglong2 *>(dx + (block + b) * (Plan::kBoxCols * 4))[j];
+  };
+  auto fold_chunk = [&](uint32_t i, uint32_t buffer, uint32_t steps) {
+    const uint32_t block = i / Shape::kBlockChunks * Shape::kChunkBlocks;
+#pragma unroll
+    for (uint32_t b = 0; b < Shape::kChunkBlocks; ++b)
+      if (b == 0 || block + b < steps)  // (blocks past the row's end hold an older block's numbers)
+        fold_part<Shape, kRepack>(v[buffer] + b * kRt * Shape::kChunkCols, acc,
+                                  i % Shape::kBlockChunks * Shape::kChunkCols, dws[block + b],
+                                  xd[buffer] + b * kScaleVecs);
+  };
+  // All stages but the last are whole.  Their chunks are software-pipelined: while one is folded the
+  // next is on its way from TMEM, across hand-overs and stages, so neither the barrier test nor the
+  // load's latency stands between two folds.
+  if (!load_chunk(0, 0))
+    return false;
+  for (uint32_t kb = 0; kb + 1 < nkb; ++kb) {
+    open_stage();
+#pragma unroll
+    for (uint32_t i = 0; i < Shape::kChunks; ++i) {
+      load_scales(st, i, i & 1);
+      tmem_ld_wait();
+      if ((i + 1) % Shape::kHandoverChunks == 0)
+        release_tmem();
+      if (!load_chunk((i + 1) % Shape::kChunks, (i + 1) & 1))
+        return false;
+      fold_chunk(i, i & 1, kGemmStageBlocks);
+    }
+    close_stage();
+  }
+  open_stage();
+  const uint32_t steps = a.nb - (nkb - 1) * kGemmStageBlocks;
+#pragma unroll
+  for (uint32_t i = 0; i < Shape::kChunks; ++i) {
+    if (i / Shape::kBlockChunks * Shape::kChunkBlocks < steps) {
+      if (i > 0 && !load_chunk(i, 0))
+        return false;
+      load_scales(st, i, 0);
+      tmem_ld_wait();
+      if ((i + 1) % Shape::kHandoverChunks == 0 || (i + 1) / Shape::kBlockChunks * Shape::kChunkBlocks >= steps)
+        release_tmem();
+      fold_chunk(i, 0, steps);
+    }
+  }
+  close_stage();
+
+  // ---- store: this thread owns kCpw consecutive outputs of kRt weight rows
+  if constexpr (kMulti) {
+    // whole item inside the matrix and every base 16-byte aligned: rows leave as bulk copies
+    bool bulk = (a.bs % 4 == 0) && (it.m0 + Shape::kCols <= a.nc);
+    for (uint32_t d = 0; d < a.ndst; ++d)
+      bulk = bulk && ((reinterpret_cast<uintptr_t>(a.dst[d]) & 15u) == 0);
+    if (bulk) {
+#pragma unroll
+      for (int r = 0; r < kRt; ++r) {
+        // the previous tile's copies must have read the staging tile before it is rewritten
+        bulk_store_wait_read();
+        if (!epilogue_sync(c, lane))
+          return false;
+        float4 *mine = reinterpret_cast<float4 *>(c.out_stage + static_cast<size_t>(row_local) * kGemmOutRowBytes +
+                                                  static_cast<size_t>(colgroup) * kCpw * 4);
+#pragma unroll
+        for (int j = 0; j < kCpw / 4; ++j) {
+          float4 o;
+          unpack_f32x2(acc[r][2 * j], o.x, o.y);
+          unpack_f32x2(acc[r][2 * j + 1], o.z, o.w);
+          mine[j] = o;
+        }
+        fence_proxy_async_smem();
+        if (!epilogue_sync(c, lane))
+          return false;
+        // thread t sends row t%128 to destinations t/128, t/128 + 2, ...
+        const uint32_t t = static_cast<uint32_t>(warp * 32 + lane);
+        const uint32_t lr = t & 127u, grow = it.n0 + r * kGemmTileRows + lr;
+        if (grow < a.nr) {
+          const uint8_t *src = c.out_stage + static_cast<size_t>(lr) * kGemmOutRowBytes;
+          for (uint32_t d = t >> 7; d < a.ndst; d += kGemmEpilogueWarps / 4)
+            bulk_store_s2g(a.dst[d] + static_cast<size_t>(grow) * a.bs + it.m0, src, Shape::kCols * 4u);
+        }
+        bulk_store_commit();
+      }
+      return true;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRt; ++r)
+    store_outputs<kCpw, kRepack>(a, acc[r], it.n0 + r * kGemmTileRows + row_local, it.m0 + colgroup * kCpw);
+  return true;
+}
+
+// One work item for the (converged) MMA warp.  Returns false after a failed wait.
+template <typename Plan, typename Shape, int kStages>
+__device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx &c, uint32_t stage_base_addr,
+                                              bool leader) {
+  constexpr uint32_t idesc = umma_idesc_e4m3(kGemmTileRows, Shape::kCols);
+  const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
+  for (uint32_t kb = 0; kb < nkb; ++kb) {
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_full[c.ps.stage], c.ps.phase, c.abort_flag)))
+      return false;
+    tcgen05_fence_after_thread_sync();
+    // Operand descriptors of the stage's first block; a block further along K is 32 bytes
+    // further inside the 128-byte swizzled rows, i.e. +2 in the descriptor's 16-byte
+    // address field.
+    const uint32_t a_addr = stage_base_addr + c.ps.stage * Plan::kStageBytes;
+    const uint64_t da0 = umma_desc_k_major_sw128(a_addr);
+    const uint64_t dl0 = umma_desc_k_major_sw128(a_addr + Plan::kOffB);
+    const uint64_t dh0 = umma_desc_k_major_sw128(a_addr + Plan::kOffB + Plan::kPlaneBytes);
+    const uint32_t steps = min(static_cast<uint32_t>(kGemmStageBlocks), a.nb - kb * kGemmStageBlocks);
+#pragma unroll
+    for (uint32_t kk = 0; kk < kGemmStageBlocks; kk += Shape::kHandover) {
+      if (kk < steps) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.tmem_empty[c.ts.stage], c.ts.phase ^ 1, c.abort_flag)))
+          return false;
+        tcgen05_fence_after_thread_sync();
+        constexpr uint64_t kStep = (kQK >> 4);  // 32 bytes in 16-byte units
+        if (leader) {
+#pragma unroll
+          for (uint32_t h = 0; h < Shape::kHandover; ++h) {
+            if (kk + h < steps) {
+              const uint64_t off = (kk + h) * kStep;
+#pragma unroll
+              for (uint32_t r = 0; r < Shape::kRowTiles; ++r) {
+                const uint32_t d_tmem = c.tmem_base + c.ts.stage * Plan::kTmemStageCols +
+                                        (h * Shape::kRowTiles + r) * Shape::kCols;
+                const uint64_t da = da0 + off + r * (Plan::kATileBytes >> 4);
+                umma_f8_first(d_tmem, da, dl0 + off, idesc);
+                umma_f8_again(d_tmem, da, dh0 + off, idesc);
+              }
+            }
+          }
+          umma_commit(&c.tmem_full[c.ts.stage]);
+        }
+        __syncwarp();
+        c.ts.advance(Plan::kTmemStages);
+      }
+    }
+    if (leader)
+      umma_commit(&c.smem_empty[c.ps.stage]);
+    __syncwarp();
+    c.ps.advance(kStages);
+  }
   return true;
 }
 
 // kMulti: the result goes to several output copies (peers) through a shared-memory staging tile.
 // kRepack (single destination only): scales multiplied first, token-major output.
-// kF8: e4m3 operand planes and fp32 accumulator tiles instead of int8 / int32.
-template <bool kMulti, bool kRepack, bool kF8>
+// kNarrow: items of 128 rows x 32 columns (few tokens) instead of 256 x 64 and halves of those.
+template <bool kMulti, bool kRepack, bool kNarrow>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_q4_0_q8_0_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                              const __grid_constant__ CUtensorMap map_xhi, const __grid_constant__ CUtensorMap map_dw,
                              const __grid_constant__ CUtensorMap map_dx, const __grid_constant__ GemmArgs a) {
-  using Stage = GemmStage<kF8>;
-  constexpr int kStages = GemmSmem<kMulti, kF8>::kStages;
+  using Plan = GemmPlan<kNarrow>;
+  using Full = typename Plan::Full;
+  using Half = typename Plan::Half;
+  constexpr int kStages = GemmSmem<kMulti, kNarrow>::kStages;
   extern __shared__ uint8_t smem_raw[];
   // control block first, then stages on a 1024-byte boundary (required by the 128B swizzle)
-  uint8_t *ctrl = smem_raw;
-  uint64_t *smem_full = reinterpret_cast<uint64_t *>(ctrl);
-  uint64_t *smem_empty = smem_full + kStages;
-  uint64_t *tmem_full = smem_empty + kStages;
-  uint64_t *tmem_empty = tmem_full + kGemmTmemStages;
-  uint64_t *drain_bar = tmem_empty + kGemmTmemStages;
-  uint64_t *store_bar = drain_bar + 1;
-  uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(store_bar + 1);
-  volatile uint32_t *abort_flag = tmem_base_slot + 1;
+  GemmEpilogueCtx c;
+  c.smem_full = reinterpret_cast<uint64_t *>(smem_raw);
+  c.smem_empty = c.smem_full + kStages;
+  c.tmem_full = c.smem_empty + kStages;
+  c.tmem_empty = c.tmem_full + Plan::kTmemStages;
+  uint64_t *drain_bar = c.tmem_empty + Plan::kTmemStages;
+  c.store_bar = drain_bar + 1;
+  uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(c.store_bar + 1);
+  c.abort_flag = tmem_base_slot + 1;
   const uint32_t stage_base_addr = (smem_addr(smem_raw) + kGemmCtrlBytes + 1023u) & ~1023u;
-  uint8_t *stages = smem_raw + (stage_base_addr - smem_addr(smem_raw));
-  uint8_t *out_stage = stages + static_cast<size_t>(kStages) * Stage::kBytes;  // 1024-byte aligned
+  c.stages = smem_raw + (stage_base_addr - smem_addr(smem_raw));
+  c.out_stage = c.stages + static_cast<size_t>(kStages) * Plan::kStageBytes;  // 1024-byte aligned
+  c.store_syncs = 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
@@ -457,16 +558,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(&smem_full[i], 1);
-      mbar_init(&smem_empty[i], 1 + kGemmEpilogueWarps);  // MMA commit + every epilogue warp
+      mbar_init(&c.smem_full[i], 1);
+      mbar_init(&c.smem_empty[i], 1 + kGemmEpilogueWarps);  // MMA commit + every epilogue warp
     }
-    for (int i = 0; i < kGemmTmemStages; ++i) {
-      mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], kGemmEpilogueWarps);
+    for (int i = 0; i < Plan::kTmemStages; ++i) {
+      mbar_init(&c.tmem_full[i], 1);
+      mbar_init(&c.tmem_empty[i], kGemmEpilogueWarps);
     }
     mbar_init(drain_bar, 1);
-    mbar_init(store_bar, kGemmEpilogueWarps);
-    *abort_flag = 0;
+    mbar_init(c.store_bar, kGemmEpilogueWarps);
+    *c.abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == kGemmEpilogueWarps + 1) {
@@ -476,155 +577,106 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   tcgen05_fence_before_thread_sync();
   __syncthreads();
   tcgen05_fence_after_thread_sync();
-  const uint32_t tmem_base = *tmem_base_slot;
+  c.tmem_base = *tmem_base_slot;
   // Programmatic dependent launch: everything above touched only this CTA's shared memory and
   // TMEM, so it may overlap the tail of the preceding kernel (the activation unpack); operands
   // are read and outputs written only after that kernel has completed.
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
+  bool ok = true;
   if (warp == kGemmEpilogueWarps) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
       prefetch_tensormap(&map_w);
       prefetch_tensormap(&map_x);
-      if (kF8)
-        prefetch_tensormap(&map_xhi);
+      prefetch_tensormap(&map_xhi);
       prefetch_tensormap(&map_dw);
       prefetch_tensormap(&map_dx);
       PipeState ps;
-      bool ok = true;
       uint32_t issued = 0;
       for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
-        const GemmItem it = gemm_item(a, idx);
-        if (it.m0 >= a.nc)
+        const GemmItem it = gemm_item<kNarrow>(a, idx);
+        if (it.n0 >= a.nr || it.m0 >= a.nc)
           continue;
         const int n0 = static_cast<int>(it.n0), m0 = static_cast<int>(it.m0);
-        const bool whole = it.width == kGemmTileCols;
-        const uint32_t halves = whole ? 2u : 1u;
-        const uint32_t tx = kGemmABytes + kGemmDwBytes + halves * ((kF8 ? 2 : 1) * kGemmBHalfBytes + kGemmDxHalfBytes);
+        const int row_tiles = it.whole ? Full::kRowTiles : Half::kRowTiles;
+        const int boxes = it.whole ? Full::kCols / Plan::kBoxCols : 1;
+        const uint32_t tx = row_tiles * (Plan::kATileBytes + Plan::kDwTileBytes) +
+                            boxes * (2 * Plan::kBoxBytes + Plan::kDxBoxBytes);
         for (uint32_t kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_bounded(&smem_empty[ps.stage], ps.phase ^ 1, abort_flag);
+          ok = mbar_wait_bounded(&c.smem_empty[ps.stage], ps.phase ^ 1, c.abort_flag);
           if (!ok)
             break;
-          uint8_t *st = stages + static_cast<size_t>(ps.stage) * Stage::kBytes;
-          uint64_t *bar = &smem_full[ps.stage];
+          uint8_t *st = c.stages + static_cast<size_t>(ps.stage) * Plan::kStageBytes;
+          uint64_t *bar = &c.smem_full[ps.stage];
           mbar_arrive_expect_tx(bar, tx);
           const int kbyte = static_cast<int>(kb) * kGemmStageBlocks * kQK;
           const int kblk = static_cast<int>(kb) * kGemmStageBlocks;
-          tma_load_2d(st, &map_w, kbyte, n0, bar);
-          tma_load_2d(st + Stage::kOffDw, &map_dw, kblk, n0, bar);
-          for (uint32_t h = 0; h < halves; ++h) {
-            const int mh = m0 + static_cast<int>(h) * kGemmHalfCols;
-            tma_load_2d(st + Stage::kOffB + h * kGemmBHalfBytes, &map_x, kbyte, mh, bar);
-            if (kF8)
-              tma_load_2d(st + Stage::kOffB + kGemmBPlaneBytes + h * kGemmBHalfBytes, &map_xhi, kbyte, mh, bar);
-            tma_load_2d(st + Stage::kOffDx + h * kGemmDxHalfBytes, &map_dx, mh, kblk, bar);
+          for (int r = 0; r < row_tiles; ++r) {
+            // (a second tile that starts past the last row reads as zeros)
+            tma_load_2d(st + r * Plan::kATileBytes, &map_w, kbyte, n0 + r * kGemmTileRows, bar);
+            tma_load_2d(st + Plan::kOffDw + r * Plan::kDwTileBytes, &map_dw, kblk, n0 + r * kGemmTileRows, bar);
+          }
+          for (int b = 0; b < boxes; ++b) {
+            const int mb = m0 + b * Plan::kBoxCols;
+            tma_load_2d(st + Plan::kOffB + b * Plan::kBoxBytes, &map_x, kbyte, mb, bar);
+            tma_load_2d(st + Plan::kOffB + Plan::kPlaneBytes + b * Plan::kBoxBytes, &map_xhi, kbyte, mb, bar);
+            tma_load_2d(st + Plan::kOffDx + b * Plan::kDxBoxBytes, &map_dx, mb, kblk, bar);
           }
           ps.advance(kStages);
           ++issued;
         }
       }
       if (!ok) {
-        *abort_flag = 1;
+        *c.abort_flag = 1;
         raise_device_error(kDevErrBarrierTimeout);
       }
-      if (*abort_flag != 0) {
+      if (*c.abort_flag != 0) {
         // winding down after a failed wait: let this CTA's own copies land before it exits
         const uint32_t first = issued > kStages ? issued - kStages : 0;
         for (uint32_t i = first; i < issued; ++i)
-          (void)mbar_wait_bounded(&smem_full[i % kStages], (i / kStages) & 1, nullptr);
+          (void)mbar_wait_bounded(&c.smem_full[i % kStages], (i / kStages) & 1, nullptr);
       }
     }
   } else if (warp == kGemmEpilogueWarps + 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
-      PipeState ps, ts;
-      bool ok = true;
-      for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
-        const GemmItem it = gemm_item(a, idx);
-        if (it.m0 >= a.nc)
-          continue;
-        const uint32_t idesc = kF8 ? umma_idesc_e4m3(kGemmTileRows, static_cast<int>(it.width))
-                                   : umma_idesc_s8(kGemmTileRows, static_cast<int>(it.width));
-        for (uint32_t kb = 0; kb < nkb && ok; ++kb) {
-          ok = mbar_wait_bounded(&smem_full[ps.stage], ps.phase, abort_flag);
-          if (!ok)
-            break;
-          tcgen05_fence_after_thread_sync();
-          // Operand descriptors of the stage's first block; a block further along K is 32 bytes
-          // further inside the 128-byte swizzled rows, i.e. +2 in the descriptor's 16-byte
-          // address field.  One thread feeds the tensor core, so its per-block work is kept to
-          // a wait, one addition per operand and the instructions themselves.
-          const uint32_t a_addr = stage_base_addr + ps.stage * Stage::kBytes;
-          const uint64_t da0 = umma_desc_k_major_sw128(a_addr);
-          const uint64_t db0 = umma_desc_k_major_sw128(a_addr + Stage::kOffB);
-          [[maybe_unused]] const uint64_t dh0 = umma_desc_k_major_sw128(a_addr + Stage::kOffB + kGemmBPlaneBytes);
-          const uint32_t steps = min(static_cast<uint32_t>(kGemmStageBlocks), a.nb - kb * kGemmStageBlocks);
-#pragma unroll
-          for (uint32_t kk = 0; kk < kGemmStageBlocks; kk += kGemmHandover) {
-            if (kk < steps && ok) {
-              ok = mbar_wait_bounded(&tmem_empty[ts.stage], ts.phase ^ 1, abort_flag);
-              if (ok) {
-                tcgen05_fence_after_thread_sync();
-                constexpr uint64_t kStep = (kQK >> 4);  // 32 bytes in 16-byte units
-#pragma unroll
-                for (uint32_t h = 0; h < static_cast<uint32_t>(kGemmHandover); ++h) {
-                  if (kk + h < steps) {
-                    const uint32_t d_tmem = tmem_base + ts.stage * kGemmTmemStageCols + h * kGemmTileCols;
-                    const uint64_t off = (kk + h) * kStep;
-                    if constexpr (kF8) {
-                      umma_f8_ss<false>(d_tmem, da0 + off, db0 + off, idesc);
-                      umma_f8_ss<true>(d_tmem, da0 + off, dh0 + off, idesc);
-                    } else {
-                      umma_s8_ss<false>(d_tmem, da0 + off, db0 + off, idesc);
-                    }
-                  }
-                }
-                umma_commit(&tmem_full[ts.stage]);
-                ts.advance(kGemmTmemStages);
-              }
-            }
-          }
-          if (ok)
-            umma_commit(&smem_empty[ps.stage]);
-          ps.advance(kStages);
-        }
-      }
-      if (!ok) {
-        *abort_flag = 1;
-        raise_device_error(kDevErrBarrierTimeout);
-      }
-      // every MMA issued above must have finished before TMEM is released
-      umma_commit(drain_bar);
-      (void)mbar_wait_bounded(drain_bar, 0, nullptr);
+    // The whole warp walks the loop and one elected lane issues.  Operand descriptors live in uniform
+    // registers; computed in code that the compiler knows to be converged they are there already,
+    // while a single-lane branch had to move six values per MMA across: 85 cycles per MMA and 340
+    // per commit, which bounded every shape's hand-overs.  (128 x 128 items without the fold: 204 ->
+    // 169 us on 512 x 32000 x 4096.)
+    const bool leader = elect_one();
+    for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
+      const GemmItem it = gemm_item<kNarrow>(a, idx);
+      if (it.n0 >= a.nr || it.m0 >= a.nc)
+        continue;
+      ok = it.whole ? gemm_mma_item<Plan, Full, kStages>(a, c, stage_base_addr, leader)
+                    : gemm_mma_item<Plan, Half, kStages>(a, c, stage_base_addr, leader);
     }
+    if (!ok && leader) {
+      *c.abort_flag = 1;
+      raise_device_error(kDevErrBarrierTimeout);
+    }
+    // every MMA issued above must have finished before TMEM is released
+    if (leader)
+      umma_commit(drain_bar);
+    __syncwarp();
+    (void)mbar_wait_bounded(drain_bar, 0, nullptr);
   } else {
     // ------------------------------ epilogue warps ------------------------------
-    GemmEpilogueCtx c;
-    c.stages = stages;
-    c.out_stage = out_stage;
-    c.smem_full = smem_full;
-    c.smem_empty = smem_empty;
-    c.tmem_full = tmem_full;
-    c.tmem_empty = tmem_empty;
-    c.store_bar = store_bar;
-    c.abort_flag = abort_flag;
-    c.tmem_base = tmem_base;
-    c.store_syncs = 0;
-    bool ok = true;
     for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
-      const GemmItem it = gemm_item(a, idx);
-      if (it.m0 >= a.nc)
+      const GemmItem it = gemm_item<kNarrow>(a, idx);
+      if (it.n0 >= a.nr || it.m0 >= a.nc)
         continue;
-      if (it.width == kGemmTileCols)
-        ok = gemm_epilogue_item<kGemmTileCols / 4, kMulti, kRepack, kF8>(a, c, it, warp, lane);
+      if (it.whole)
+        ok = gemm_epilogue_item<Plan, Full, kMulti, kRepack, kStages>(a, c, it, warp, lane);
       else
-        ok = gemm_epilogue_item<kGemmHalfCols / 4, kMulti, kRepack, kF8>(a, c, it, warp, lane);
+        ok = gemm_epilogue_item<Plan, Half, kMulti, kRepack, kStages>(a, c, it, warp, lane);
     }
     if (kMulti)
       bulk_store_wait_all();  // the staging tile must outlive the copies that read it
     if (!ok && lane == 0) {
-      *abort_flag = 1;
+      *c.abort_flag = 1;
       raise_device_error(kDevErrBarrierTimeout);
     }
   }
@@ -633,7 +685,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   if (warp == kGemmEpilogueWarps + 1) {
     tcgen05_fence_after_thread_sync();
-    tmem_dealloc(tmem_base, kGemmTmemCols);
+    tmem_dealloc(c.tmem_base, kGemmTmemCols);
   }
 }
 

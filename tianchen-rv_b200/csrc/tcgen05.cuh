@@ -58,26 +58,17 @@ __device__ __forceinline__ uint64_t umma_desc_k_major_sw128(uint32_t smem_byte_a
   return desc;
 }
 
-// ---- instruction descriptor for kind::i8: signed int8 A and B, both K-major, int32 D.
-__host__ __device__ constexpr uint32_t umma_idesc_s8(int m, int n) {
-  return (2u << 4)                                 // D format: S32
-         | (1u << 7)                               // A: signed 8-bit
-         | (1u << 10)                              // B: signed 8-bit
-         | (static_cast<uint32_t>(n >> 3) << 17)   // N / 8
-         | (static_cast<uint32_t>(m >> 4) << 24);  // M / 16
-}
-
-// D[tmem] = A[smem] * B[smem] (kAccumulate false) or D += A * B.  One thread issues.
-template <bool kAccumulate>
-__device__ __forceinline__ void umma_s8_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t leader;
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0)
-      : "memory");
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(leader));
+  return leader != 0;
 }
 
 // Arrive on an mbarrier once every tcgen05.mma issued so far by this thread has completed.
@@ -94,44 +85,54 @@ __host__ __device__ constexpr uint32_t umma_idesc_e4m3(int m, int n) {
          | (static_cast<uint32_t>(m >> 4) << 24);  // M / 16
 }
 
-template <bool kAccumulate>
-__device__ __forceinline__ void umma_f8_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+// Two MMAs with the same A: D = A * B keeps A in the tensor core's operand buffer, the next
+// D += A * B' takes it from there instead of reading shared memory again.
+__device__ __forceinline__ void umma_f8_first(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4.collector::a::fill [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(0)
       : "memory");
 }
 
-// 32 lanes x N consecutive 32-bit columns (N = 16 or 32): thread i of the warp receives lane
-// (base+i).
+__device__ __forceinline__ void umma_f8_again(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4.collector::a::lastuse [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(1)
+      : "memory");
+}
+
+// 32 lanes x N consecutive 32-bit columns (N = 8 or 16) into v[0..N): thread i of the warp
+// receives lane (base+i).
 template <int N>
-__device__ __forceinline__ void tmem_ld_32x32b(uint32_t taddr, uint32_t (&v)[N]);
+__device__ __forceinline__ void tmem_ld_32x32b(uint32_t taddr, uint32_t *v);
 
 template <>
-__device__ __forceinline__ void tmem_ld_32x32b<32>(uint32_t taddr, uint32_t (&v)[32]) {
+__device__ __forceinline__ void tmem_ld_32x32b<8>(uint32_t taddr, uint32_t *v) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7])
       : "r"(taddr)
       : "memory");
 }
 
 template <>
-__device__ __forceinline__ void tmem_ld_32x32b<16>(uint32_t taddr, uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_ld_32x32b<16>(uint32_t taddr, uint32_t *v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
       : "r"(taddr)
       : "memory");
 }
