@@ -90,14 +90,25 @@ void check(int status, const char *where) {
   throw PyError{};
 }
 
-// Runs a launch without the interpreter lock, as a ctypes call does.
+// The interpreter lock, given up as a ctypes call does and taken back however the scope is left:
+// torch throws from data_ptr() for a tensor without storage (vmap, fake tensors), and what the
+// handlers below do needs the lock.
+class Unlocked {
+ public:
+  Unlocked() : state_(PyEval_SaveThread()) {}
+  ~Unlocked() { PyEval_RestoreThread(state_); }
+  Unlocked(const Unlocked &) = delete;
+  Unlocked &operator=(const Unlocked &) = delete;
+
+ private:
+  PyThreadState *state_;
+};
+
+// Runs a launch without the interpreter lock.
 template <typename F>
 inline int unlocked(F &&launch) {
-  int status;
-  Py_BEGIN_ALLOW_THREADS
-  status = launch();
-  Py_END_ALLOW_THREADS
-  return status;
+  const Unlocked scope;
+  return launch();
 }
 
 inline int64_t blocks_of(int64_t row_bytes, int64_t block_bytes) {
