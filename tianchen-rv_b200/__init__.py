@@ -165,17 +165,16 @@ class _NativeCalls:
 
     def __getattr__(self, name):
         global _native
-        if not os.path.exists(_build.TORCH_CALLS):
+        path = _build.torch_calls_path()  # (imports torch: its libraries have to be loaded first)
+        if not os.path.exists(path):
             raise RuntimeError(
-                f"{_build.TORCH_CALLS} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`; "
+                f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`; "
                 "this provider has no CPU or PyTorch fallback"
             )
         import importlib.util
 
-        import torch  # noqa: F401 - its libraries have to be loaded first
-
         lib()
-        spec = importlib.util.spec_from_file_location("_tcrv_torch", _build.TORCH_CALLS)
+        spec = importlib.util.spec_from_file_location("_tcrv_torch", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         module.bind(_check)

@@ -2,8 +2,8 @@
 
 ``build_library()`` compiles ``csrc/*.cu`` into ``libtcrv_cuda.so`` next to this file with
 nvcc; it needs no GPU (nvcc cross-compiles).  ``build_torch_calls()`` compiles
-``csrc/torch_calls.cpp``, the package's native call path, into ``_tcrv_torch.so`` beside it with
-the host compiler.  Run as a script to force a rebuild.
+``csrc/torch_calls.cpp``, the package's native call path, into ``_tcrv_torch.<Python ABI>.torch-<version>.so``
+beside it with the host compiler.  Run as a script to force a rebuild.
 """
 from __future__ import annotations
 
@@ -12,12 +12,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtcrv_cuda.so")
-TORCH_CALLS = os.path.join(HERE, "_tcrv_torch.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -41,7 +41,8 @@ def _stale() -> bool:
     if not os.path.exists(LIB):
         return True
     built = os.path.getmtime(LIB)
-    deps = glob.glob(os.path.join(CSRC, "*")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    deps = [p for kind in ("*.cu", "*.cuh", "*.h") for p in glob.glob(os.path.join(CSRC, kind))]
+    deps += glob.glob(os.path.join(ROOT, "include", "*.h"))
     return any(os.path.getmtime(p) > built for p in deps)
 
 
@@ -56,16 +57,23 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
-def build_torch_calls(force: bool = False) -> str:
-    """The Python calls' native half; needs the C-ABI library (it links against it)."""
-    import sysconfig
-
+def torch_calls_path() -> str:
+    """Where the native call path is for this interpreter and this torch.  It is compiled against
+    CPython's and torch's C++ headers, so a build for others must not be loaded: the name tells them apart."""
     import torch
 
+    return os.path.join(HERE, f"_tcrv_torch.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
+
+
+def build_torch_calls(force: bool = False) -> str:
+    """The Python calls' native half; needs the C-ABI library (it links against it)."""
+    import torch
+
+    out = torch_calls_path()
     source = os.path.join(CSRC, "torch_calls.cpp")
-    deps = [source, os.path.join(ROOT, "include", "tcrv_cuda.h")]
-    if not force and os.path.exists(TORCH_CALLS) and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_CALLS) for d in deps):
-        return TORCH_CALLS
+    deps = [source, os.path.join(ROOT, "include", "tcrv_cuda.h"), os.path.abspath(__file__)]
+    if not force and os.path.exists(out) and all(os.path.getmtime(d) <= os.path.getmtime(out) for d in deps):
+        return out
     torch_dir = os.path.dirname(torch.__file__)
     torch_lib = os.path.join(torch_dir, "lib")
     cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
@@ -74,11 +82,11 @@ def build_torch_calls(force: bool = False) -> str:
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
         "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"],
         "-isystem", os.path.join(torch_dir, "include"), "-isystem", os.path.join(torch_dir, "include/torch/csrc/api/include"),
-        "-isystem", cuda_include, "-o", TORCH_CALLS, source,
+        "-isystem", cuda_include, "-o", out, source,
         "-L", HERE, "-ltcrv_cuda", "-L", torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}",
     ], check=True)
-    return TORCH_CALLS
+    return out
 
 
 if __name__ == "__main__":
