@@ -60,3 +60,13 @@ def test_another_torch_or_python_does_not_get_the_old_module(build, monkeypatch)
     monkeypatch.undo()
     monkeypatch.setattr(b.sysconfig, "get_config_var", lambda name: "cpython-399")
     assert os.path.basename(b.torch_calls_path()) != os.path.basename(old)
+
+
+def test_the_c_library_builds_where_there_is_no_torch(build, pkg, monkeypatch):
+    import importlib.util
+
+    b, csrc, now, ran = build
+    os.utime(csrc / "gemv.cu", (now + 120, now + 120))
+    monkeypatch.setattr(b, "build_torch_calls", lambda force=False: pytest.fail("needs torch"))
+    monkeypatch.setattr(importlib.util, "find_spec", lambda name: None)
+    assert pkg.build_library() == b.LIB and len(ran) == 1

@@ -155,8 +155,12 @@ def lib() -> ctypes.CDLL:
 
 
 def build_library(force: bool = False) -> str:
+    """The C-ABI library and, where torch is installed, the package's native call path."""
+    import importlib.util
+
     path = _build.build_library(force=force)
-    _build.build_torch_calls(force=force)
+    if importlib.util.find_spec("torch") is not None:
+        _build.build_torch_calls(force=force)
     return path
 
 

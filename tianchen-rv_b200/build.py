@@ -90,5 +90,8 @@ def build_torch_calls(force: bool = False) -> str:
 
 
 if __name__ == "__main__":
+    import importlib.util
+
     print(build_library(force=True, verbose="-v" in sys.argv))
-    print(build_torch_calls(force=True))
+    if importlib.util.find_spec("torch") is not None:  # the C library needs none
+        print(build_torch_calls(force=True))
