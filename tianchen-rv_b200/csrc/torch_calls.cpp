@@ -10,6 +10,7 @@
 
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "tcrv_cuda.h"
@@ -139,8 +140,8 @@ inline PyObject *given_or_wrapped(PyObject *given, at::Tensor &&made) {
       return name##_body(a); \
     } catch (const PyError &) { \
       return nullptr; \
-    } catch (const std::exception &e) { \
-      PyErr_SetString(PyExc_RuntimeError, e.what()); \
+    } catch (...) { /* as torch's own functions raise it: OutOfMemoryError, IndexError, ... */ \
+      torch::translate_exception_to_python(std::current_exception()); \
       return nullptr; \
     } \
   } \
