@@ -105,7 +105,7 @@ class Unlocked {
   PyThreadState *state_;
 };
 
-// Runs a launch without the interpreter lock.
+// Runs an allocation and a launch without the interpreter lock.
 template <typename F>
 inline int unlocked(F &&launch) {
   const Unlocked scope;
@@ -121,13 +121,35 @@ inline int64_t blocks_of(int64_t row_bytes, int64_t block_bytes) {
   return row_bytes / block_bytes;
 }
 
-inline PyObject *given_or_wrapped(PyObject *given, at::Tensor &&made) {
-  if (given != Py_None) {
+// The output of a call: the caller's, or one that is made without the interpreter lock, in front of
+// the launch (an allocation may have to wait for the device or flush torch's cache).
+struct Output {
+  PyObject *given;
+  at::Tensor tensor;
+
+  // `type` as dense() checks it
+  Output(PyObject *o, at::ScalarType type) : given(o) {
+    if (given != Py_None)
+      tensor = dense(given, type);
+  }
+  // any CUDA tensor
+  explicit Output(PyObject *o) : given(o) {
+    if (given != Py_None)
+      tensor = ::tensor(given);
+  }
+  void make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like) {
+    if (given == Py_None)
+      tensor = empty(shape, type, like);
+  }
+  float *floats() const { return ::floats(tensor); }
+  size_t stride() const { return static_cast<size_t>(tensor.stride(0)); }
+  PyObject *result() {
+    if (given == Py_None)
+      return THPVariable_Wrap(std::move(tensor));
     Py_INCREF(given);
     return given;
   }
-  return THPVariable_Wrap(std::move(made));
-}
+};
 
 #define TCRV_CALL(name, count) \
   PyObject *name##_body(PyObject *const *a); \
@@ -154,24 +176,18 @@ TCRV_CALL(add, 3) {
   if (type != at::kFloat && type != at::kInt)
     fail(PyExc_TypeError, "add supports float32 and int32");
   const at::Tensor &l = dense(a[0], type), &r = dense(a[1], type);
-  at::Tensor made;
-  if (a[2] == Py_None)
-    made = empty(l.sizes(), type, l);
-  void *out = a[2] == Py_None ? made.data_ptr() : dense(a[2], type).data_ptr();
+  Output out(a[2], type);
   const size_t n = static_cast<size_t>(l.numel());
   const cudaStream_t st = stream();
-  if (type == at::kFloat)
-    check(unlocked([&] {
-            return tcrv_cuda_add_f32(floats(l), floats(r), static_cast<float *>(out), n, st);
-          }),
-          "tcrv_cuda_add_f32");
-  else
-    check(unlocked([&] {
-            return tcrv_cuda_add_i32(static_cast<const int32_t *>(l.data_ptr()), static_cast<const int32_t *>(r.data_ptr()),
-                                     static_cast<int32_t *>(out), n, st);
-          }),
-          "tcrv_cuda_add_i32");
-  return given_or_wrapped(a[2], std::move(made));
+  check(unlocked([&] {
+          out.make(l.sizes(), type, l);
+          return type == at::kFloat
+                     ? tcrv_cuda_add_f32(floats(l), floats(r), out.floats(), n, st)
+                     : tcrv_cuda_add_i32(static_cast<const int32_t *>(l.data_ptr()), static_cast<const int32_t *>(r.data_ptr()),
+                                         static_cast<int32_t *>(out.tensor.data_ptr()), n, st);
+        }),
+        type == at::kFloat ? "tcrv_cuda_add_f32" : "tcrv_cuda_add_i32");
+  return out.result();
 }
 
 // dequantize(vx, out, block_bytes)
@@ -181,20 +197,18 @@ TCRV_CALL(dequantize, 3) {
   if (vx.dim() == 0)
     fail(PyExc_ValueError, "blocks come in rows");
   const int64_t nb = blocks_of(vx.size(-1), block);
-  at::Tensor made;
-  if (a[1] == Py_None) {
-    auto shape = vx.sizes().vec();
-    shape.back() = nb * kQK;
-    made = empty(shape, at::kFloat, vx);
-  }
-  const at::Tensor &out = a[1] == Py_None ? made : dense(a[1], at::kFloat);
-  const size_t n = static_cast<size_t>(out.numel());
+  auto shape = vx.sizes().vec();
+  shape.back() = nb * kQK;
+  Output out(a[1], at::kFloat);
   const cudaStream_t st = stream();
-  if (block == TCRV_Q8_0_BLOCK_BYTES)
-    check(unlocked([&] { return tcrv_cuda_dequantize_row_q8_0(bytes(vx), floats(out), n, st); }), "tcrv_cuda_dequantize_row_q8_0");
-  else
-    check(unlocked([&] { return tcrv_cuda_dequantize_row_q4_0(bytes(vx), floats(out), n, st); }), "tcrv_cuda_dequantize_row_q4_0");
-  return given_or_wrapped(a[1], std::move(made));
+  const bool q8 = block == TCRV_Q8_0_BLOCK_BYTES;
+  check(unlocked([&] {
+          out.make(shape, at::kFloat, vx);
+          return (q8 ? tcrv_cuda_dequantize_row_q8_0 : tcrv_cuda_dequantize_row_q4_0)(
+              bytes(vx), out.floats(), static_cast<size_t>(out.tensor.numel()), st);
+        }),
+        q8 ? "tcrv_cuda_dequantize_row_q8_0" : "tcrv_cuda_dequantize_row_q4_0");
+  return out.result();
 }
 
 // quantize(x, out, block_bytes)
@@ -204,20 +218,18 @@ TCRV_CALL(quantize, 3) {
   if (x.dim() == 0 || x.size(-1) % kQK != 0)
     fail(PyExc_ValueError, "last dimension must be a multiple of 32");
   dense(a[0], at::kFloat);
-  at::Tensor made;
-  if (a[1] == Py_None) {
-    auto shape = x.sizes().vec();
-    shape.back() = shape.back() / kQK * block;
-    made = empty(shape, at::kByte, x);
-  }
-  const at::Tensor &out = a[1] == Py_None ? made : dense(a[1], at::kByte);
+  auto shape = x.sizes().vec();
+  shape.back() = shape.back() / kQK * block;
+  Output out(a[1], at::kByte);
   const size_t n = static_cast<size_t>(x.numel());
   const cudaStream_t st = stream();
-  if (block == TCRV_Q8_0_BLOCK_BYTES)
-    check(unlocked([&] { return tcrv_cuda_quantize_row_q8_0(n, floats(x), bytes(out), st); }), "tcrv_cuda_quantize_row_q8_0");
-  else
-    check(unlocked([&] { return tcrv_cuda_quantize_row_q4_0(n, floats(x), bytes(out), st); }), "tcrv_cuda_quantize_row_q4_0");
-  return given_or_wrapped(a[1], std::move(made));
+  const bool q8 = block == TCRV_Q8_0_BLOCK_BYTES;
+  check(unlocked([&] {
+          out.make(shape, at::kByte, x);
+          return (q8 ? tcrv_cuda_quantize_row_q8_0 : tcrv_cuda_quantize_row_q4_0)(n, floats(x), bytes(out.tensor), st);
+        }),
+        q8 ? "tcrv_cuda_quantize_row_q8_0" : "tcrv_cuda_quantize_row_q4_0");
+  return out.result();
 }
 
 // gemv(w, x, q8_weights, flags, out)
@@ -231,19 +243,18 @@ TCRV_CALL(gemv, 5) {
   if (blocks_of(w.size(1), q8 ? TCRV_Q8_0_BLOCK_BYTES : TCRV_Q4_0_BLOCK_BYTES) != nb)
     fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
   const int64_t nr = w.size(0), nc = x.size(0);
-  at::Tensor made;
-  if (a[4] == Py_None)
-    made = empty({nr, nc}, at::kFloat, w);
-  const at::Tensor &out = a[4] == Py_None ? made : dense(a[4], at::kFloat);
+  Output out(a[4], at::kFloat);
   const size_t n = static_cast<size_t>(nb * kQK), bx = static_cast<size_t>(w.stride(0)),
-               by = static_cast<size_t>(x.stride(0)), bs = static_cast<size_t>(out.stride(0));
+               by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
   check(unlocked([&] {
+          out.make({nr, nc}, at::kFloat, w);
           return (q8 ? tcrv_cuda_gemv_q8_0_q8_0 : tcrv_cuda_gemv_q4_0_q8_0)(
-              n, floats(out), bytes(w), bytes(x), by, static_cast<size_t>(nr), static_cast<size_t>(nc), bx, bs, flags, st);
+              n, out.floats(), bytes(w), bytes(x), by, static_cast<size_t>(nr), static_cast<size_t>(nc), bx, out.stride(),
+              flags, st);
         }),
         q8 ? "tcrv_cuda_gemv_q8_0_q8_0" : "tcrv_cuda_gemv_q4_0_q8_0");
-  return given_or_wrapped(a[4], std::move(made));
+  return out.result();
 }
 
 // gemv_group(address of the calls, count, q8_weights, flags)
@@ -265,12 +276,18 @@ TCRV_CALL(gemv_group, 4) {
 // Device scratch of at least `need` bytes: the caller's tensor, or a new one.  (A new one may go
 // back to torch's allocator as soon as the launches are queued: its next user on this stream
 // runs behind them.)
-inline const at::Tensor &scratch(PyObject *given, at::Tensor &made, size_t need, const at::Tensor &like) {
-  if (given != Py_None)
-    return tensor(given);
-  made = empty({static_cast<int64_t>(need < 256 ? 256 : need)}, at::kByte, like);
-  return made;
-}
+struct Scratch {
+  at::Tensor tensor;
+  explicit Scratch(PyObject *given) {
+    if (given != Py_None)
+      tensor = ::tensor(given);
+  }
+  void make(size_t need, const at::Tensor &like) {
+    if (!tensor.defined())
+      tensor = empty({static_cast<int64_t>(need < 256 ? 256 : need)}, at::kByte, like);
+  }
+  size_t size() const { return static_cast<size_t>(tensor.numel()); }
+};
 
 // gemm(w, x, out, workspace)
 TCRV_CALL(gemm, 4) {
@@ -281,19 +298,18 @@ TCRV_CALL(gemm, 4) {
   if (blocks_of(w.size(1), TCRV_Q4_0_BLOCK_BYTES) != nb)
     fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
   const size_t n = static_cast<size_t>(nb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
-  at::Tensor made, made_ws;
-  if (a[2] == Py_None)
-    made = empty({w.size(0), x.size(0)}, at::kFloat, w);
-  const at::Tensor &out = a[2] == Py_None ? made : dense(a[2], at::kFloat);
-  const at::Tensor &ws = scratch(a[3], made_ws, tcrv_cuda_gemm_workspace_bytes(n, nr, nc), w);
-  const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0)), bs = static_cast<size_t>(out.stride(0));
+  Output out(a[2], at::kFloat);
+  Scratch ws(a[3]);
+  const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
   check(unlocked([&] {
-          return tcrv_cuda_gemm_q4_0_q8_0(n, floats(out), bytes(w), bytes(x), by, nr, nc, bx, bs, ws.data_ptr(),
-                                          static_cast<size_t>(ws.numel()), 0, st);
+          out.make({w.size(0), x.size(0)}, at::kFloat, w);
+          ws.make(tcrv_cuda_gemm_workspace_bytes(n, nr, nc), w);
+          return tcrv_cuda_gemm_q4_0_q8_0(n, out.floats(), bytes(w), bytes(x), by, nr, nc, bx, out.stride(),
+                                          ws.tensor.data_ptr(), ws.size(), 0, st);
         }),
         "tcrv_cuda_gemm_q4_0_q8_0");
-  return given_or_wrapped(a[2], std::move(made));
+  return out.result();
 }
 
 // gemm_prepared(buffer, n, nr, x, out, workspace)
@@ -305,19 +321,18 @@ TCRV_CALL(gemm_prepared, 6) {
   if (static_cast<size_t>(blocks_of(x.size(1), TCRV_Q8_0_BLOCK_BYTES) * kQK) != n)
     fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
   const size_t nc = static_cast<size_t>(x.size(0));
-  at::Tensor made, made_ws;
-  if (a[4] == Py_None)
-    made = empty({static_cast<int64_t>(nr), x.size(0)}, at::kFloat, x);
-  const at::Tensor &out = a[4] == Py_None ? made : dense(a[4], at::kFloat);
-  const at::Tensor &ws = scratch(a[5], made_ws, tcrv_cuda_gemm_acts_workspace_bytes(n, nc), x);
-  const size_t by = static_cast<size_t>(x.stride(0)), bs = static_cast<size_t>(out.stride(0));
+  Output out(a[4], at::kFloat);
+  Scratch ws(a[5]);
+  const size_t by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
   check(unlocked([&] {
-          return tcrv_cuda_gemm_q4_0_q8_0_prepared(n, floats(out), buffer.data_ptr(), bytes(x), by, nr, nc, bs, ws.data_ptr(),
-                                                   static_cast<size_t>(ws.numel()), 0, st);
+          out.make({static_cast<int64_t>(nr), x.size(0)}, at::kFloat, x);
+          ws.make(tcrv_cuda_gemm_acts_workspace_bytes(n, nc), x);
+          return tcrv_cuda_gemm_q4_0_q8_0_prepared(n, out.floats(), buffer.data_ptr(), bytes(x), by, nr, nc, out.stride(),
+                                                   ws.tensor.data_ptr(), ws.size(), 0, st);
         }),
         "tcrv_cuda_gemm_q4_0_q8_0_prepared");
-  return given_or_wrapped(a[4], std::move(made));
+  return out.result();
 }
 
 // sibling_dot_rows(format, weight block bytes, activation block bytes, w, x, out)
@@ -328,17 +343,15 @@ TCRV_CALL(sibling_dot_rows, 6) {
   if (w.dim() != 2 || x.dim() != 2 || w.size(1) % wb != 0 || x.size(1) % ab != 0 || w.size(1) / wb != x.size(1) / ab)
     fail(PyExc_ValueError, "row bytes do not match the format's block sizes");
   const size_t n = static_cast<size_t>(w.size(1) / wb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
-  at::Tensor made;
-  if (a[5] == Py_None)
-    made = empty({w.size(0), x.size(0)}, at::kFloat, w);
-  const at::Tensor &out = a[5] == Py_None ? made : dense(a[5], at::kFloat);
+  Output out(a[5], at::kFloat);
   const cudaStream_t st = stream();
   check(unlocked([&] {
-          return tcrv_cuda_sibling_dot_rows(format, n, floats(out), bytes(w), bytes(x), static_cast<size_t>(x.stride(0)), nr, nc,
-                                            static_cast<size_t>(w.stride(0)), static_cast<size_t>(out.stride(0)), st);
+          out.make({w.size(0), x.size(0)}, at::kFloat, w);
+          return tcrv_cuda_sibling_dot_rows(format, n, out.floats(), bytes(w), bytes(x), static_cast<size_t>(x.stride(0)), nr,
+                                            nc, static_cast<size_t>(w.stride(0)), out.stride(), st);
         }),
         "tcrv_cuda_sibling_dot_rows");
-  return given_or_wrapped(a[5], std::move(made));
+  return out.result();
 }
 
 inline const at::Tensor &row_matrix(PyObject *o) {
@@ -354,49 +367,45 @@ TCRV_CALL(rms_norm, 4) {
   const at::Tensor &x = row_matrix(a[0]);
   const float eps = static_cast<float>(real(a[1]));
   const unsigned flags = static_cast<unsigned>(integer(a[3]));
-  at::Tensor made;
-  if (a[2] == Py_None)
-    made = empty({x.size(0), x.size(1)}, at::kFloat, x);
-  const at::Tensor &out = a[2] == Py_None ? made : tensor(a[2]);
+  Output out(a[2]);
   const cudaStream_t st = stream();
   check(unlocked([&] {
-          return tcrv_cuda_rms_norm_f32_flags(static_cast<size_t>(x.size(1)), floats(x), floats(out), eps,
+          out.make({x.size(0), x.size(1)}, at::kFloat, x);
+          return tcrv_cuda_rms_norm_f32_flags(static_cast<size_t>(x.size(1)), floats(x), out.floats(), eps,
                                               static_cast<size_t>(x.size(0)), static_cast<size_t>(x.stride(0)),
-                                              static_cast<size_t>(out.stride(0)), flags, st);
+                                              out.stride(), flags, st);
         }),
         "tcrv_cuda_rms_norm_f32_flags");
-  return given_or_wrapped(a[2], std::move(made));
+  return out.result();
 }
 
 // rope_apply(x, cache, out)
 TCRV_CALL(rope_apply, 3) {
   const at::Tensor &x = row_matrix(a[0]);
   const at::Tensor &cache = dense(a[1], at::kFloat);
-  at::Tensor made;
-  if (a[2] == Py_None)
-    made = empty({x.size(0), x.size(1)}, at::kFloat, x);
-  const at::Tensor &out = a[2] == Py_None ? made : tensor(a[2]);
+  Output out(a[2]);
   const cudaStream_t st = stream();
   check(unlocked([&] {
-          return tcrv_cuda_rope_apply_f32(static_cast<size_t>(x.size(1)), floats(x), floats(out), floats(cache),
+          out.make({x.size(0), x.size(1)}, at::kFloat, x);
+          return tcrv_cuda_rope_apply_f32(static_cast<size_t>(x.size(1)), floats(x), out.floats(), floats(cache),
                                           static_cast<size_t>(x.size(0)), static_cast<size_t>(x.stride(0)),
-                                          static_cast<size_t>(out.stride(0)), st);
+                                          out.stride(), st);
         }),
         "tcrv_cuda_rope_apply_f32");
-  return given_or_wrapped(a[2], std::move(made));
+  return out.result();
 }
 
 // vec_silu(x, out)
 TCRV_CALL(vec_silu, 2) {
   const at::Tensor &x = dense(a[0], at::kFloat);
-  at::Tensor made;
-  if (a[1] == Py_None)
-    made = empty(x.sizes(), at::kFloat, x);
-  const at::Tensor &out = a[1] == Py_None ? made : dense(a[1], at::kFloat);
+  Output out(a[1], at::kFloat);
   const cudaStream_t st = stream();
-  check(unlocked([&] { return tcrv_cuda_vec_silu_f32(static_cast<size_t>(x.numel()), floats(x), floats(out), st); }),
+  check(unlocked([&] {
+          out.make(x.sizes(), at::kFloat, x);
+          return tcrv_cuda_vec_silu_f32(static_cast<size_t>(x.numel()), floats(x), out.floats(), st);
+        }),
         "tcrv_cuda_vec_silu_f32");
-  return given_or_wrapped(a[1], std::move(made));
+  return out.result();
 }
 
 // vec_scale_(y, v)
@@ -421,17 +430,15 @@ TCRV_CALL(repack_gemv, 6) {
     fail(PyExc_ValueError, "weights, activation and nc do not describe the same shape");
   dense(a[0], at::kByte);
   dense(a[1], at::kByte);
-  at::Tensor made;
-  if (a[4] == Py_None)
-    made = empty({nc}, at::kFloat, w);
-  const at::Tensor &out = a[4] == Py_None ? made : dense(a[4], at::kFloat);
+  Output out(a[4], at::kFloat);
   const cudaStream_t st = stream();
   check(unlocked([&] {
+          out.make({nc}, at::kFloat, w);
           return (q8 ? tcrv_cuda_repack_gemv_q8_0_q8_0 : tcrv_cuda_repack_gemv_q4_0_q8_0)(
-              static_cast<size_t>(nb * kQK), floats(out), bytes(w), bytes(x), static_cast<size_t>(nc), flags, st);
+              static_cast<size_t>(nb * kQK), out.floats(), bytes(w), bytes(x), static_cast<size_t>(nc), flags, st);
         }),
         "tcrv_cuda_repack_gemv");
-  return given_or_wrapped(a[4], std::move(made));
+  return out.result();
 }
 
 // bind(_check)
