@@ -2,6 +2,8 @@
 cannot take."""
 import pytest
 
+import sibling_data as sd
+
 pytestmark = pytest.mark.gpu
 
 
@@ -29,3 +31,67 @@ def test_errors_of_torch_keep_their_class(cuda, pkg):
     x = cuda.zeros(1, 34 * 4, dtype=cuda.uint8, device="cuda")
     with pytest.raises(IndexError):  # an output without dimensions has no row stride
         pkg.gemv(w, x, out=cuda.zeros((), device="cuda"))
+
+
+@pytest.fixture(scope="module")
+def operands(cuda, pkg):
+    """Small operands of every call: 48 weight rows of 4 blocks, 3 columns, 8 rows of 128 floats."""
+    f = cuda.randn(48, 128, device="cuda")
+    x = cuda.randn(8, 128, device="cuda")
+    wq, xq = pkg.quantize_q4_0(f), pkg.quantize_q8_0(x[:3].contiguous())
+    sw, sx = sd.make(2, 48, 3, 4, 5)
+    return {"f": f, "x": x, "wq": wq, "xq": xq, "pw": pkg.PreparedWeights(wq), "w16": cuda.zeros(3 * 4 * 288, dtype=cuda.uint8, device="cuda"),
+            "sw": cuda.from_numpy(sw).cuda(), "sx": cuda.from_numpy(sx).cuda(), "cache": pkg.rope_cache(128, 1.0, 0.9)}
+
+
+# every call with an output: the call, the output's type, the fewest elements that it can take
+OUTPUTS = {
+    "add": (lambda p, o, out: p.add(o["x"], o["x"], out=out), "float32", 1024),
+    "dequantize_q4_0": (lambda p, o, out: p.dequantize_q4_0(o["wq"], out=out), "float32", None),
+    "quantize_q8_0": (lambda p, o, out: p.quantize_q8_0(o["x"], out=out), "uint8", 8 * 136),
+    "quantize_q4_0": (lambda p, o, out: p.quantize_q4_0(o["x"], out=out), "uint8", 8 * 72),
+    "gemv": (lambda p, o, out: p.gemv(o["wq"], o["xq"], out=out.view(-1, 3)), "float32", 144),
+    "gemv_group_calls": (lambda p, o, out: p.gemv_group_calls([(o["wq"], o["xq"], out.view(-1, 3))]), "float32", 144),
+    "gemm": (lambda p, o, out: p.gemm(o["wq"], o["xq"], out=out.view(-1, 3)), "float32", 144),
+    "gemm_prepared": (lambda p, o, out: p.gemm(o["pw"], o["xq"], out=out.view(-1, 3)), "float32", 144),
+    "sibling_dot_rows": (lambda p, o, out: p.sibling_dot_rows(2, o["sw"], o["sx"], out=out.view(-1, 3)), "float32", 144),
+    "rms_norm": (lambda p, o, out: p.rms_norm(o["x"], 1e-5, out=out.view(-1, 128)), "float32", 1024),
+    "rope_apply": (lambda p, o, out: p.rope_apply(o["x"], o["cache"], out=out.view(-1, 128)), "float32", 1024),
+    "vec_silu": (lambda p, o, out: p.vec_silu(o["x"], out=out), "float32", 1024),
+    "repack_gemv": (lambda p, o, out: p.repack_gemv(o["w16"], o["xq"][0], 48, out=out), "float32", 48),
+}
+
+
+@pytest.mark.parametrize("name", sorted(OUTPUTS))
+def test_an_output_that_is_too_small_is_refused(cuda, pkg, operands, name):
+    call, dtype, least = OUTPUTS[name]
+    if least is None:  # as many elements as the output has: more than the blocks hold
+        big = cuda.empty(48 * 128 + 32, dtype=cuda.float32, device="cuda")
+        with pytest.raises(ValueError):
+            call(pkg, operands, big)
+        call(pkg, operands, big[:64])
+        return
+    row = 3 if least == 144 else 128 if name in ("rms_norm", "rope_apply") else 1  # elements of a row of `out`
+    room = cuda.empty(least, dtype=getattr(cuda, dtype), device="cuda")
+    with pytest.raises(ValueError):
+        call(pkg, operands, room[:least - row])
+    call(pkg, operands, room)
+    pkg.check_device_errors()
+
+
+def test_inputs_that_end_early_are_refused(cuda, pkg, operands):
+    with pytest.raises(ValueError):
+        pkg.add(operands["x"], operands["x"][:7])
+    with pytest.raises(ValueError):
+        pkg.rope_apply(operands["x"], operands["cache"][:126])
+
+
+@pytest.mark.parametrize("call", [lambda p, o, out: p.rms_norm(o["x"], 1e-5, out=out),
+                                  lambda p, o, out: p.rope_apply(o["x"], o["cache"], out=out)])
+def test_row_outputs_are_float32_with_contiguous_rows(cuda, pkg, operands, call):
+    with pytest.raises(TypeError):
+        call(pkg, operands, cuda.empty(8, 128, dtype=cuda.int32, device="cuda"))
+    with pytest.raises(ValueError):
+        call(pkg, operands, cuda.empty(8, 256, device="cuda")[:, ::2])
+    call(pkg, operands, cuda.empty(8, 256, device="cuda")[:, 3:131])  # a row stride is fine
+    pkg.check_device_errors()

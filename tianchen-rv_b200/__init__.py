@@ -315,7 +315,10 @@ def gemv_group_calls(problems, q8_weights: bool = False):
     calls = []
     for w, x, out in problems:
         n, nr, nc, bx, by, torch = _matrix_args(w, x, wblock)
-        calls.append(GemvCall(n, _dev(out, torch.float32), w.data_ptr(), x.data_ptr(), by, nr, nc, bx, out.stride(0)))
+        s = _dev(out, torch.float32)
+        if nr > 0 and nc > 0 and (nr - 1) * out.stride(0) + nc > out.numel():
+            raise ValueError("the output is too small for the result")
+        calls.append(GemvCall(n, s, w.data_ptr(), x.data_ptr(), by, nr, nc, bx, out.stride(0)))
     return (GemvCall * len(calls))(*calls)
 
 

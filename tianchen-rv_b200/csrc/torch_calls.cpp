@@ -121,6 +121,16 @@ inline int64_t blocks_of(int64_t row_bytes, int64_t block_bytes) {
   return row_bytes / block_bytes;
 }
 
+// Elements from a tensor's first to its last one in memory.
+inline int64_t extent(const at::Tensor &t) {
+  if (t.numel() == 0)
+    return 0;
+  int64_t n = 1;
+  for (int64_t d = 0; d < t.dim(); ++d)
+    n += (t.size(d) - 1) * t.stride(d);
+  return n;
+}
+
 // The output of a call: the caller's, or one that is made without the interpreter lock, in front of
 // the launch (an allocation may have to wait for the device or flush torch's cache).
 struct Output {
@@ -132,10 +142,25 @@ struct Output {
     if (given != Py_None)
       tensor = dense(given, type);
   }
-  // any CUDA tensor
+  // rows with a stride: a float32 CUDA tensor whose last dimension is contiguous
   explicit Output(PyObject *o) : given(o) {
-    if (given != Py_None)
-      tensor = ::tensor(given);
+    if (given == Py_None)
+      return;
+    tensor = ::tensor(given);
+    if (tensor.scalar_type() != at::kFloat)
+      fail(PyExc_TypeError, "expected dtype torch.float32 for the output");
+    if (tensor.dim() > 0 && tensor.size(-1) > 1 && tensor.stride(-1) != 1)
+      fail(PyExc_ValueError, "the output's rows must be contiguous");
+  }
+  // A caller's tensor must hold what the launch writes: `count` elements from its first one on,
+  void require(int64_t count) const {
+    if (given != Py_None && count > extent(tensor))
+      fail(PyExc_ValueError, "the output is too small for the result");
+  }
+  // or `rows` rows of `cols` elements, its row stride apart.
+  void require_rows(int64_t rows, int64_t cols) const {
+    if (given != Py_None && rows > 0 && cols > 0)
+      require((rows - 1) * tensor.stride(0) + cols);
   }
   void make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like) {
     if (given == Py_None)
@@ -177,6 +202,9 @@ TCRV_CALL(add, 3) {
     fail(PyExc_TypeError, "add supports float32 and int32");
   const at::Tensor &l = dense(a[0], type), &r = dense(a[1], type);
   Output out(a[2], type);
+  out.require(l.numel());
+  if (r.numel() < l.numel())
+    fail(PyExc_ValueError, "operands differ in size");
   const size_t n = static_cast<size_t>(l.numel());
   const cudaStream_t st = stream();
   check(unlocked([&] {
@@ -200,6 +228,8 @@ TCRV_CALL(dequantize, 3) {
   auto shape = vx.sizes().vec();
   shape.back() = nb * kQK;
   Output out(a[1], at::kFloat);
+  if (out.given != Py_None && out.tensor.numel() > vx.numel() / block * kQK)
+    fail(PyExc_ValueError, "the output asks for more elements than the blocks hold");
   const cudaStream_t st = stream();
   const bool q8 = block == TCRV_Q8_0_BLOCK_BYTES;
   check(unlocked([&] {
@@ -221,6 +251,7 @@ TCRV_CALL(quantize, 3) {
   auto shape = x.sizes().vec();
   shape.back() = shape.back() / kQK * block;
   Output out(a[1], at::kByte);
+  out.require(x.numel() / kQK * block);
   const size_t n = static_cast<size_t>(x.numel());
   const cudaStream_t st = stream();
   const bool q8 = block == TCRV_Q8_0_BLOCK_BYTES;
@@ -244,6 +275,7 @@ TCRV_CALL(gemv, 5) {
     fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
   const int64_t nr = w.size(0), nc = x.size(0);
   Output out(a[4], at::kFloat);
+  out.require_rows(nr, nc);
   const size_t n = static_cast<size_t>(nb * kQK), bx = static_cast<size_t>(w.stride(0)),
                by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
@@ -299,6 +331,7 @@ TCRV_CALL(gemm, 4) {
     fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
   const size_t n = static_cast<size_t>(nb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
   Output out(a[2], at::kFloat);
+  out.require_rows(w.size(0), x.size(0));
   Scratch ws(a[3]);
   const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
@@ -322,6 +355,7 @@ TCRV_CALL(gemm_prepared, 6) {
     fail(PyExc_ValueError, "weights and activations disagree on the number of blocks per row");
   const size_t nc = static_cast<size_t>(x.size(0));
   Output out(a[4], at::kFloat);
+  out.require_rows(static_cast<int64_t>(nr), x.size(0));
   Scratch ws(a[5]);
   const size_t by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
@@ -344,6 +378,7 @@ TCRV_CALL(sibling_dot_rows, 6) {
     fail(PyExc_ValueError, "row bytes do not match the format's block sizes");
   const size_t n = static_cast<size_t>(w.size(1) / wb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
   Output out(a[5], at::kFloat);
+  out.require_rows(w.size(0), x.size(0));
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make({w.size(0), x.size(0)}, at::kFloat, w);
@@ -368,6 +403,7 @@ TCRV_CALL(rms_norm, 4) {
   const float eps = static_cast<float>(real(a[1]));
   const unsigned flags = static_cast<unsigned>(integer(a[3]));
   Output out(a[2]);
+  out.require_rows(x.size(0), x.size(1));
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make({x.size(0), x.size(1)}, at::kFloat, x);
@@ -383,7 +419,10 @@ TCRV_CALL(rms_norm, 4) {
 TCRV_CALL(rope_apply, 3) {
   const at::Tensor &x = row_matrix(a[0]);
   const at::Tensor &cache = dense(a[1], at::kFloat);
+  if (cache.numel() < x.size(1))
+    fail(PyExc_ValueError, "the angle cache is too small");
   Output out(a[2]);
+  out.require_rows(x.size(0), x.size(1));
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make({x.size(0), x.size(1)}, at::kFloat, x);
@@ -399,6 +438,7 @@ TCRV_CALL(rope_apply, 3) {
 TCRV_CALL(vec_silu, 2) {
   const at::Tensor &x = dense(a[0], at::kFloat);
   Output out(a[1], at::kFloat);
+  out.require(x.numel());
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make(x.sizes(), at::kFloat, x);
@@ -431,6 +471,7 @@ TCRV_CALL(repack_gemv, 6) {
   dense(a[0], at::kByte);
   dense(a[1], at::kByte);
   Output out(a[4], at::kFloat);
+  out.require(nc);
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make({nc}, at::kFloat, w);
