@@ -95,3 +95,29 @@ def test_row_outputs_are_float32_with_contiguous_rows(cuda, pkg, operands, call)
         call(pkg, operands, cuda.empty(8, 256, device="cuda")[:, ::2])
     call(pkg, operands, cuda.empty(8, 256, device="cuda")[:, 3:131])  # a row stride is fine
     pkg.check_device_errors()
+
+
+def test_operands_in_page_locked_memory_are_read_where_they_lie(cuda, pkg, operands):
+    o = operands
+    wq, xq = o["wq"].cpu().pin_memory(), o["xq"].cpu().pin_memory()
+    out = cuda.full((48, 3), -1.0, device="cuda")
+    assert cuda.equal(pkg.gemv(o["wq"], xq), pkg.gemv(o["wq"], o["xq"]))
+    want = pkg.gemm(o["wq"], o["xq"])
+    assert cuda.equal(pkg.gemm(o["wq"], xq), want)
+    assert cuda.equal(pkg.gemm(wq, xq, out=out), want)
+    assert cuda.equal(pkg.gemm(o["pw"], xq, out=out.fill_(-1.0)), want)
+    rows = cuda.zeros(8, 128).pin_memory()
+    normed, rotated = pkg.rms_norm(o["x"], 1e-5), pkg.rope_apply(o["x"], o["cache"])
+    pkg.rms_norm(o["x"], 1e-5, out=rows)
+    cuda.cuda.synchronize()
+    assert cuda.equal(rows, normed.cpu())
+    pkg.rope_apply(o["x"], o["cache"], out=rows)
+    cuda.cuda.synchronize()
+    assert cuda.equal(rows, rotated.cpu())
+    # a result without a place of its own needs an operand on the device to lie beside; pageable memory is refused
+    for call in (lambda: pkg.gemv(wq, xq), lambda: pkg.gemm(wq, xq), lambda: pkg.gemm(o["pw"], xq),
+                 lambda: pkg.gemv(o["wq"], o["xq"].cpu()), lambda: pkg.gemm(o["wq"].cpu(), o["xq"]),
+                 lambda: pkg.rms_norm(o["x"], 1e-5, out=cuda.zeros(8, 128))):
+        with pytest.raises(TypeError):
+            call()
+    pkg.check_device_errors()

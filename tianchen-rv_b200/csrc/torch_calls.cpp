@@ -38,6 +38,14 @@ inline const at::Tensor &tensor(PyObject *o) {
   return t;
 }
 
+// What a kernel can read and write where it lies: a CUDA tensor, or one in page-locked host memory
+// (mapped at the same address).  The GEMV and GEMM operands and the strided outputs may be either.
+inline const at::Tensor &mapped(PyObject *o) {
+  if (THPVariable_Check(o) && !THPVariable_Unpack(o).is_cuda() && THPVariable_Unpack(o).is_pinned())
+    return THPVariable_Unpack(o);
+  return tensor(o);
+}
+
 // A contiguous CUDA tensor of the given type.
 inline const at::Tensor &dense(PyObject *o, at::ScalarType type) {
   const at::Tensor &t = tensor(o);
@@ -142,11 +150,11 @@ struct Output {
     if (given != Py_None)
       tensor = dense(given, type);
   }
-  // rows with a stride: a float32 CUDA tensor whose last dimension is contiguous
+  // rows with a stride: a float32 tensor, in device or page-locked memory, whose last dimension is contiguous
   explicit Output(PyObject *o) : given(o) {
     if (given == Py_None)
       return;
-    tensor = ::tensor(given);
+    tensor = mapped(given);
     if (tensor.scalar_type() != at::kFloat)
       fail(PyExc_TypeError, "expected dtype torch.float32 for the output");
     if (tensor.dim() > 0 && tensor.size(-1) > 1 && tensor.stride(-1) != 1)
@@ -161,6 +169,11 @@ struct Output {
   void require_rows(int64_t rows, int64_t cols) const {
     if (given != Py_None && rows > 0 && cols > 0)
       require((rows - 1) * tensor.stride(0) + cols);
+  }
+  // An output that is made lies beside `like`, which has to be a CUDA tensor then.
+  void beside(PyObject *like) const {
+    if (given == Py_None)
+      ::tensor(like);
   }
   void make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like) {
     if (given == Py_None)
@@ -267,7 +280,7 @@ TCRV_CALL(quantize, 3) {
 TCRV_CALL(gemv, 5) {
   const bool q8 = truth(a[2]);
   const unsigned flags = static_cast<unsigned>(integer(a[3]));
-  const at::Tensor &w = tensor(a[0]), &x = tensor(a[1]);
+  const at::Tensor &w = mapped(a[0]), &x = mapped(a[1]);
   if (w.dim() != 2 || x.dim() != 2)
     fail(PyExc_ValueError, "weights are (rows, row_bytes), activations are (columns, column_bytes)");
   const int64_t nb = blocks_of(x.size(1), TCRV_Q8_0_BLOCK_BYTES);
@@ -276,6 +289,7 @@ TCRV_CALL(gemv, 5) {
   const int64_t nr = w.size(0), nc = x.size(0);
   Output out(a[4], at::kFloat);
   out.require_rows(nr, nc);
+  out.beside(a[0]);
   const size_t n = static_cast<size_t>(nb * kQK), bx = static_cast<size_t>(w.stride(0)),
                by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
@@ -312,7 +326,7 @@ struct Scratch {
   at::Tensor tensor;
   explicit Scratch(PyObject *given) {
     if (given != Py_None)
-      tensor = ::tensor(given);
+      tensor = mapped(given);
   }
   void make(size_t need, const at::Tensor &like) {
     if (!tensor.defined())
@@ -323,7 +337,7 @@ struct Scratch {
 
 // gemm(w, x, out, workspace)
 TCRV_CALL(gemm, 4) {
-  const at::Tensor &w = tensor(a[0]), &x = tensor(a[1]);
+  const at::Tensor &w = mapped(a[0]), &x = mapped(a[1]);
   if (w.dim() != 2 || x.dim() != 2)
     fail(PyExc_ValueError, "weights are (rows, row_bytes), activations are (columns, column_bytes)");
   const int64_t nb = blocks_of(x.size(1), TCRV_Q8_0_BLOCK_BYTES);
@@ -332,12 +346,13 @@ TCRV_CALL(gemm, 4) {
   const size_t n = static_cast<size_t>(nb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
   Output out(a[2], at::kFloat);
   out.require_rows(w.size(0), x.size(0));
+  out.beside(a[0]);
   Scratch ws(a[3]);
   const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make({w.size(0), x.size(0)}, at::kFloat, w);
-          ws.make(tcrv_cuda_gemm_workspace_bytes(n, nr, nc), w);
+          ws.make(tcrv_cuda_gemm_workspace_bytes(n, nr, nc), out.tensor);
           return tcrv_cuda_gemm_q4_0_q8_0(n, out.floats(), bytes(w), bytes(x), by, nr, nc, bx, out.stride(),
                                           ws.tensor.data_ptr(), ws.size(), 0, st);
         }),
@@ -347,7 +362,7 @@ TCRV_CALL(gemm, 4) {
 
 // gemm_prepared(buffer, n, nr, x, out, workspace)
 TCRV_CALL(gemm_prepared, 6) {
-  const at::Tensor &buffer = tensor(a[0]), &x = tensor(a[3]);
+  const at::Tensor &buffer = tensor(a[0]), &x = mapped(a[3]);
   const size_t n = static_cast<size_t>(integer(a[1])), nr = static_cast<size_t>(integer(a[2]));
   if (x.dim() != 2)
     fail(PyExc_ValueError, "activations are (columns, column_bytes)");
@@ -356,12 +371,13 @@ TCRV_CALL(gemm_prepared, 6) {
   const size_t nc = static_cast<size_t>(x.size(0));
   Output out(a[4], at::kFloat);
   out.require_rows(static_cast<int64_t>(nr), x.size(0));
+  out.beside(a[3]);
   Scratch ws(a[5]);
   const size_t by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
   check(unlocked([&] {
           out.make({static_cast<int64_t>(nr), x.size(0)}, at::kFloat, x);
-          ws.make(tcrv_cuda_gemm_acts_workspace_bytes(n, nc), x);
+          ws.make(tcrv_cuda_gemm_acts_workspace_bytes(n, nc), out.tensor);
           return tcrv_cuda_gemm_q4_0_q8_0_prepared(n, out.floats(), buffer.data_ptr(), bytes(x), by, nr, nc, out.stride(),
                                                    ws.tensor.data_ptr(), ws.size(), 0, st);
         }),
