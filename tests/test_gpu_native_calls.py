@@ -121,3 +121,15 @@ def test_operands_in_page_locked_memory_are_read_where_they_lie(cuda, pkg, opera
         with pytest.raises(TypeError):
             call()
     pkg.check_device_errors()
+
+
+def test_a_package_under_a_second_name_raises_its_own_errors(cuda, pkg, operands):
+    import importlib
+
+    other = importlib.import_module("tianchen-rv_b200")
+    assert other is not pkg and other.TcrvCudaError is not pkg.TcrvCudaError
+    narrow = cuda.empty(144, device="cuda")  # one dimension: a row stride of 1 for rows of 3 floats
+    for p in (pkg, other, pkg):
+        with pytest.raises(p.TcrvCudaError) as e:
+            p.gemv(operands["wq"], operands["xq"], out=narrow)
+        assert e.value.status == -1

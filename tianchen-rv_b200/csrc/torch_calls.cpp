@@ -18,7 +18,13 @@
 namespace {
 
 constexpr int64_t kQK = TCRV_QK;
-PyObject *g_check = nullptr;  // the package's _check(status, where)
+
+// What a module object keeps: the _check(status, where) of the package that loaded it.  (One package
+// directory can be imported under several names; each raises its own TcrvCudaError.)
+struct ModuleState {
+  PyObject *check;
+};
+inline ModuleState &state(PyObject *module) { return *static_cast<ModuleState *>(PyModule_GetState(module)); }
 
 struct PyError {};  // a Python exception is set
 
@@ -88,10 +94,10 @@ inline bool truth(PyObject *o) {
   return v != 0;
 }
 
-void check(int status, const char *where) {
+void check(PyObject *module, int status, const char *where) {
   if (status == TCRV_CUDA_OK)
     return;
-  PyObject *r = PyObject_CallFunction(g_check, "is", status, where);
+  PyObject *r = PyObject_CallFunction(state(module).check, "is", status, where);
   if (r != nullptr) {
     Py_DECREF(r);
     PyErr_SetString(PyExc_RuntimeError, where);
@@ -190,14 +196,14 @@ struct Output {
 };
 
 #define TCRV_CALL(name, count) \
-  PyObject *name##_body(PyObject *const *a); \
-  PyObject *name(PyObject *, PyObject *const *a, Py_ssize_t n) { \
+  PyObject *name##_body(PyObject *module, PyObject *const *a); \
+  PyObject *name(PyObject *module, PyObject *const *a, Py_ssize_t n) { \
     if (n != (count)) { \
       PyErr_SetString(PyExc_TypeError, #name ": wrong number of arguments"); \
       return nullptr; \
     } \
     try { \
-      return name##_body(a); \
+      return name##_body(module, a); \
     } catch (const PyError &) { \
       return nullptr; \
     } catch (...) { /* as torch's own functions raise it: OutOfMemoryError, IndexError, ... */ \
@@ -205,7 +211,7 @@ struct Output {
       return nullptr; \
     } \
   } \
-  PyObject *name##_body(PyObject *const *a)
+  PyObject *name##_body([[maybe_unused]] PyObject *module, PyObject *const *a)
 
 // add(lhs, rhs, out)
 TCRV_CALL(add, 3) {
@@ -220,7 +226,7 @@ TCRV_CALL(add, 3) {
     fail(PyExc_ValueError, "operands differ in size");
   const size_t n = static_cast<size_t>(l.numel());
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make(l.sizes(), type, l);
           return type == at::kFloat
                      ? tcrv_cuda_add_f32(floats(l), floats(r), out.floats(), n, st)
@@ -245,7 +251,7 @@ TCRV_CALL(dequantize, 3) {
     fail(PyExc_ValueError, "the output asks for more elements than the blocks hold");
   const cudaStream_t st = stream();
   const bool q8 = block == TCRV_Q8_0_BLOCK_BYTES;
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make(shape, at::kFloat, vx);
           return (q8 ? tcrv_cuda_dequantize_row_q8_0 : tcrv_cuda_dequantize_row_q4_0)(
               bytes(vx), out.floats(), static_cast<size_t>(out.tensor.numel()), st);
@@ -268,7 +274,7 @@ TCRV_CALL(quantize, 3) {
   const size_t n = static_cast<size_t>(x.numel());
   const cudaStream_t st = stream();
   const bool q8 = block == TCRV_Q8_0_BLOCK_BYTES;
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make(shape, at::kByte, x);
           return (q8 ? tcrv_cuda_quantize_row_q8_0 : tcrv_cuda_quantize_row_q4_0)(n, floats(x), bytes(out.tensor), st);
         }),
@@ -293,7 +299,7 @@ TCRV_CALL(gemv, 5) {
   const size_t n = static_cast<size_t>(nb * kQK), bx = static_cast<size_t>(w.stride(0)),
                by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({nr, nc}, at::kFloat, w);
           return (q8 ? tcrv_cuda_gemv_q8_0_q8_0 : tcrv_cuda_gemv_q4_0_q8_0)(
               n, out.floats(), bytes(w), bytes(x), by, static_cast<size_t>(nr), static_cast<size_t>(nc), bx, out.stride(),
@@ -312,7 +318,7 @@ TCRV_CALL(gemv_group, 4) {
   const bool q8 = truth(a[2]);
   const unsigned flags = static_cast<unsigned>(integer(a[3]));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           return (q8 ? tcrv_cuda_gemv_group_q8_0_q8_0 : tcrv_cuda_gemv_group_q4_0_q8_0)(calls, count, flags, st);
         }),
         q8 ? "tcrv_cuda_gemv_group_q8_0_q8_0" : "tcrv_cuda_gemv_group_q4_0_q8_0");
@@ -350,7 +356,7 @@ TCRV_CALL(gemm, 4) {
   Scratch ws(a[3]);
   const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({w.size(0), x.size(0)}, at::kFloat, w);
           ws.make(tcrv_cuda_gemm_workspace_bytes(n, nr, nc), out.tensor);
           return tcrv_cuda_gemm_q4_0_q8_0(n, out.floats(), bytes(w), bytes(x), by, nr, nc, bx, out.stride(),
@@ -375,7 +381,7 @@ TCRV_CALL(gemm_prepared, 6) {
   Scratch ws(a[5]);
   const size_t by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({static_cast<int64_t>(nr), x.size(0)}, at::kFloat, x);
           ws.make(tcrv_cuda_gemm_acts_workspace_bytes(n, nc), out.tensor);
           return tcrv_cuda_gemm_q4_0_q8_0_prepared(n, out.floats(), buffer.data_ptr(), bytes(x), by, nr, nc, out.stride(),
@@ -396,7 +402,7 @@ TCRV_CALL(sibling_dot_rows, 6) {
   Output out(a[5], at::kFloat);
   out.require_rows(w.size(0), x.size(0));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({w.size(0), x.size(0)}, at::kFloat, w);
           return tcrv_cuda_sibling_dot_rows(format, n, out.floats(), bytes(w), bytes(x), static_cast<size_t>(x.stride(0)), nr,
                                             nc, static_cast<size_t>(w.stride(0)), out.stride(), st);
@@ -421,7 +427,7 @@ TCRV_CALL(rms_norm, 4) {
   Output out(a[2]);
   out.require_rows(x.size(0), x.size(1));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({x.size(0), x.size(1)}, at::kFloat, x);
           return tcrv_cuda_rms_norm_f32_flags(static_cast<size_t>(x.size(1)), floats(x), out.floats(), eps,
                                               static_cast<size_t>(x.size(0)), static_cast<size_t>(x.stride(0)),
@@ -440,7 +446,7 @@ TCRV_CALL(rope_apply, 3) {
   Output out(a[2]);
   out.require_rows(x.size(0), x.size(1));
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({x.size(0), x.size(1)}, at::kFloat, x);
           return tcrv_cuda_rope_apply_f32(static_cast<size_t>(x.size(1)), floats(x), out.floats(), floats(cache),
                                           static_cast<size_t>(x.size(0)), static_cast<size_t>(x.stride(0)),
@@ -456,7 +462,7 @@ TCRV_CALL(vec_silu, 2) {
   Output out(a[1], at::kFloat);
   out.require(x.numel());
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make(x.sizes(), at::kFloat, x);
           return tcrv_cuda_vec_silu_f32(static_cast<size_t>(x.numel()), floats(x), out.floats(), st);
         }),
@@ -469,7 +475,7 @@ TCRV_CALL(vec_scale_, 2) {
   const at::Tensor &y = dense(a[0], at::kFloat);
   const float v = static_cast<float>(real(a[1]));
   const cudaStream_t st = stream();
-  check(unlocked([&] { return tcrv_cuda_vec_scale_f32(static_cast<size_t>(y.numel()), floats(y), v, st); }),
+  check(module, unlocked([&] { return tcrv_cuda_vec_scale_f32(static_cast<size_t>(y.numel()), floats(y), v, st); }),
         "tcrv_cuda_vec_scale_f32");
   Py_INCREF(a[0]);
   return a[0];
@@ -489,7 +495,7 @@ TCRV_CALL(repack_gemv, 6) {
   Output out(a[4], at::kFloat);
   out.require(nc);
   const cudaStream_t st = stream();
-  check(unlocked([&] {
+  check(module, unlocked([&] {
           out.make({nc}, at::kFloat, w);
           return (q8 ? tcrv_cuda_repack_gemv_q8_0_q8_0 : tcrv_cuda_repack_gemv_q4_0_q8_0)(
               static_cast<size_t>(nb * kQK), out.floats(), bytes(w), bytes(x), static_cast<size_t>(nc), flags, st);
@@ -501,7 +507,7 @@ TCRV_CALL(repack_gemv, 6) {
 // bind(_check)
 TCRV_CALL(bind, 1) {
   Py_INCREF(a[0]);
-  Py_XSETREF(g_check, a[0]);
+  Py_XSETREF(state(module).check, a[0]);
   Py_RETURN_NONE;
 }
 
@@ -511,8 +517,19 @@ PyMethodDef methods[] = {TCRV_METHOD(add),          TCRV_METHOD(dequantize),    
                          TCRV_METHOD(gemm_prepared), TCRV_METHOD(sibling_dot_rows), TCRV_METHOD(rms_norm),
                          TCRV_METHOD(rope_apply),   TCRV_METHOD(vec_silu),         TCRV_METHOD(vec_scale_),
                          TCRV_METHOD(repack_gemv),  TCRV_METHOD(bind),             {nullptr, nullptr, 0, nullptr}};
-PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_tcrv_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+int traverse(PyObject *module, visitproc visit, void *arg) {
+  Py_VISIT(state(module).check);
+  return 0;
+}
+int clear(PyObject *module) {
+  Py_CLEAR(state(module).check);
+  return 0;
+}
+void release(void *module) { clear(static_cast<PyObject *>(module)); }
+
+PyModuleDef_Slot slots[] = {{0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_tcrv_torch", nullptr, sizeof(ModuleState), methods, slots, traverse, clear, release};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__tcrv_torch() { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__tcrv_torch() { return PyModuleDef_Init(&module_def); }
