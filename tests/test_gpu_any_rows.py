@@ -4,6 +4,7 @@ column count; all bit-exact against the oracle (lane-pair order or the sequentia
 import numpy as np
 import pytest
 
+import graph_time
 import sibling_data as sd
 from test_gpu_gemv import dev, make, restated
 
@@ -24,7 +25,9 @@ def place(torch, w, lead, pad):
 @pytest.mark.parametrize("q8w", [False, True])
 @pytest.mark.parametrize("nr,nb,nc,lead,pad", [(64, 1, 1, 0, 0), (257, 3, 2, 2, 0), (300, 63, 1, 14, 0), (300, 65, 3, 0, 2),
                                                (4000, 91, 1, 0, 0), (2500, 66, 1, 6, 0), (97, 130, 8, 0, 14),
-                                               (97, 129, 5, 4, 0), (8, 341, 1, 2, 0), (40, 343, 6, 0, 0)])
+                                               (97, 129, 5, 4, 0), (8, 341, 1, 2, 0), (40, 343, 6, 0, 0),
+                                               # shared memory for one or two of the sixteen rings
+                                               (8, 1001, 4, 0, 0), (33, 563, 8, 2, 0), (300, 1501, 2, 0, 2)])
 def test_any_rows_match_the_oracle(cuda, pkg, O, q8w, nr, nb, nc, lead, pad):
     k = nb * 32
     w, x = make(O, nr, k, nc, q8w, 40 + nr + nb)
@@ -70,3 +73,20 @@ def test_a_group_with_such_rows_has_the_bits_of_the_single_calls(cuda, pkg, O, q
     for (_, _, out), ref in zip(problems, want):
         assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32))
     pkg.check_device_errors()
+
+
+def gemv_times(cuda, pkg, q8w, nr, nb, nc, flags):
+    """us of a call on the streaming kernel's route and on the general kernel (activations at an odd address)."""
+    row = nb * (34 if q8w else 18)
+    w = cuda.randint(0, 60, (nr * row,), dtype=cuda.uint8, device="cuda")
+    x = cuda.randint(0, 60, (nc * nb * 34 + 1,), dtype=cuda.uint8, device="cuda")
+    out = cuda.empty(nr * nc, device="cuda")
+    fn = pkg.lib().tcrv_cuda_gemv_q8_0_q8_0 if q8w else pkg.lib().tcrv_cuda_gemv_q4_0_q8_0
+    return [graph_time.us(cuda, lambda st: fn(nb * 32, out.data_ptr(), w.data_ptr(), x.data_ptr() + odd, nb * 34, nr, nc, row, nc,
+                                              flags, st)) for odd in (0, 1)]
+
+
+@pytest.mark.parametrize("q8w,nr,nb,nc,flags", [(False, 8, 1001, 4, 0), (False, 64, 1001, 4, 1), (True, 16, 343, 8, 1)])
+def test_few_rings_are_no_slower_than_the_general_kernel(cuda, pkg, q8w, nr, nb, nc, flags):
+    streaming, general = gemv_times(cuda, pkg, q8w, nr, nb, nc, flags)
+    assert streaming < 1.15 * general, f"{streaming:.2f} us against {general:.2f}"

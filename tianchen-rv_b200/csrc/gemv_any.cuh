@@ -568,7 +568,10 @@ int launch_any_instance(const GemvAnyPlan &plan, cudaStream_t stream) {
   const int st = any_configure(kernel, configured);
   if (st != TCRV_CUDA_OK)
     return st;
-  TCRV_CUDA_TRY(launch_pdl(kernel, plan.grid, static_cast<int>(plan.args.nwarps * 32), plan.smem, stream, plan.args));
+  // All 16 warps whatever a.nwarps is: where long rows or many columns leave shared memory for one or
+  // two rings, the spare warps still stage the activations (8 rows x 1001 blocks x 4 columns of Q4_0:
+  // 51.5 us with the one warp that has a ring, 12.1 us; the general kernel takes 34).
+  TCRV_CUDA_TRY(launch_pdl(kernel, plan.grid, kAnyMaxWarps * 32, plan.smem, stream, plan.args));
   TCRV_CUDA_TRY(cudaGetLastError());
   return TCRV_CUDA_OK;
 }
