@@ -86,7 +86,8 @@ def gemv_times(cuda, pkg, q8w, nr, nb, nc, flags):
                                               flags, st)) for odd in (0, 1)]
 
 
-@pytest.mark.parametrize("q8w,nr,nb,nc,flags", [(False, 8, 1001, 4, 0), (False, 64, 1001, 4, 1), (True, 16, 343, 8, 1)])
-def test_few_rings_are_no_slower_than_the_general_kernel(cuda, pkg, q8w, nr, nb, nc, flags):
+@pytest.mark.parametrize("q8w,nr,nb,nc,flags", [(False, 8, 1001, 4, 0), (False, 64, 1001, 4, 1), (True, 16, 343, 8, 1),  # few rings
+                                                  (False, 148, 5, 8, 1), (True, 300, 5, 1, 1), (False, 300, 1, 1, 0)])  # tiny
+def test_few_rings_and_tiny_matrices_are_no_slower_than_the_general_kernel(cuda, pkg, q8w, nr, nb, nc, flags):
     streaming, general = gemv_times(cuda, pkg, q8w, nr, nb, nc, flags)
     assert streaming < 1.15 * general, f"{streaming:.2f} us against {general:.2f}"

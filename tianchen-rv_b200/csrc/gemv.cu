@@ -580,9 +580,11 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
   }
 
   // rows the kernels above cannot take (a block count that is no multiple of 8, a base or stride
-  // off 16 bytes): the streaming kernel for any row.  Fewer rows than a CTA has warps leave most
-  // of its memory idle; they, odd addresses and more than 8 columns stay on the general kernel.
-  if (nr >= static_cast<size_t>(kAnyMinRows)) {
+  // off 16 bytes): the streaming kernel for any row.  Tiny matrices, odd addresses and more than 8
+  // columns stay on the general kernel; so do fewer than 8 rows, where the line could lie lower (one
+  // row in the strict order, us on the general kernel and on this one: 5 blocks 2.4 / 2.7, 33 blocks
+  // 2.9 / 2.7, 343 blocks 10.6 / 4.3).
+  if (nr >= static_cast<size_t>(kAnyMinRows) && !any_tiny(nb, nr, nc, strict, sm_count())) {
     GemvAnyPlan plan;
     constexpr int kFormat = kQ8W ? 5 : 4;
     if (plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, strict, (flags & TCRV_CUDA_FLAG_STATIC_WEIGHTS) != 0,

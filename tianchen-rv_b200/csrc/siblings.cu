@@ -118,8 +118,9 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
         vx, vy, sums, bx, by, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
   } else if (const uint32_t rps = table_per_cta<kFormat>(nb, nr, nc) ? strict_stream_rows<kFormat>(nb, nr, nc, vx, bx) : 0) {
     return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sm_count(), stream);
-  } else if (GemvAnyPlan plan; nr >= 8 && plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true,
-                                                                 /*static_weights=*/false, sm_count(), plan)) {
+  } else if (GemvAnyPlan plan; nr >= 8 && !any_tiny(nb, nr, nc, /*strict=*/true, sm_count()) &&
+                               plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true,
+                                                      /*static_weights=*/false, sm_count(), plan)) {
     return launch_gemv_any<kFormat, true>(plan, stream);
   } else {
     const size_t want = (nr * nc + 7) / 8;
