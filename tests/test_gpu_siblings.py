@@ -3,6 +3,7 @@ oracle: per-block int32 sums and fp32 rows, both bit-exact (strict ascending fol
 import numpy as np
 import pytest
 
+import graph_time
 import sibling_data as sd
 
 pytestmark = pytest.mark.gpu
@@ -51,8 +52,9 @@ def test_sibling_vec_dot_entries_padded_and_unaligned(cuda, pkg, O, fmt, entry):
 @pytest.mark.parametrize("fmt", [1, 2, 3])
 @pytest.mark.parametrize("nr,nb,pad", [(2000, 128, 0), (777, 8, 0), (130, 40, 48), (4099, 64, 16)])
 def test_sibling_streaming_rows_bit_exact(cuda, pkg, O, fmt, nr, nb, pad):
-    # One column against many 16-byte aligned rows takes the streaming kernel: contiguous rows,
-    # rows with a stride, ragged last slots, and an activation column at an odd address.
+    # One column against many 16-byte aligned rows takes a streaming kernel: contiguous rows, rows with
+    # a stride, ragged last slots; the one with a table per warp, and at an odd address of the
+    # activation column the one with a table per CTA.
     w, x = sd.make(fmt, nr, 1, nb, 900 + fmt + nr)
     wb = w.shape[1]
     padded = np.zeros((nr, wb + pad), dtype=np.uint8)
@@ -74,4 +76,20 @@ def test_sibling_streaming_rows_bit_exact(cuda, pkg, O, fmt, nr, nb, pad):
     flat = cuda.zeros(x.shape[1] + 1, dtype=cuda.uint8, device="cuda")
     flat[1:] = xd[0]
     assert np.array_equal(run(flat.data_ptr() + 1)[rows].view(np.uint32), want.view(np.uint32))
+    pkg.check_device_errors()
+
+
+@pytest.mark.parametrize("fmt,nr,nb,nc", [(1, 4096, 128, 1), (2, 4096, 344, 2), (3, 11008, 128, 8), (1, 32000, 8, 6), (2, 32000, 16, 3),
+                                          (3, 5120, 448, 4), (3, 4096, 344, 6)])
+def test_sibling_calls_take_the_faster_streaming_kernel(cuda, pkg, fmt, nr, nb, nc):
+    # activations at an odd address leave only the table per CTA: a call at an even one is no slower, and
+    # one at an odd address streams as well (the general kernel takes 2.4 to 9 times as long)
+    wb, ab = sd.STRIDES[fmt]
+    w = cuda.randint(0, 60, (nr * nb * wb,), dtype=cuda.uint8, device="cuda")
+    x = cuda.randint(0, 60, (nc * nb * ab + 1,), dtype=cuda.uint8, device="cuda")
+    out = cuda.empty(nr * nc, device="cuda")
+    fn = pkg.lib().tcrv_cuda_sibling_dot_rows
+    even, odd = (graph_time.us(cuda, lambda st: fn(fmt, nb * 32, out.data_ptr(), w.data_ptr(), x.data_ptr() + o, nb * ab, nr, nc,
+                                                   nb * wb, nc, st)) for o in (0, 1))
+    assert even < 1.1 * odd and odd < 1.6 * even, f"{even:.2f} us at an even address, {odd:.2f} at an odd one"
     pkg.check_device_errors()

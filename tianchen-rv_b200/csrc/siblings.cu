@@ -93,14 +93,30 @@ __global__ void __launch_bounds__(256) sibling_dot_kernel(const uint8_t *__restr
   }
 }
 
-// Which of the two streaming kernels takes a call that both accept.  Measured (us, table per CTA /
-// table per warp): one column of Q5_0 against many short rows is the one family where the
-// former's 512 workers on one slot win, 10.6 / 11.7 on 11008 x 4096 and 23.5 / 25.8 on 32000 x 4096;
-// Q4_1 and Q5_1 there 8.5 / 8.4 and 11.0 / 10.7, four columns 22.1 / 18.3 (Q5_0), 4096 x 11008
-// 13.0 / 10.1 (Q4_1), 1024 x 1024 3.5 / 2.8, eight columns equal within 3 %.
+// Which of the two streaming kernels takes a call that both accept: strict_stream.cuh (a term table per
+// CTA, 512 workers on one slot) or gemv_any.cuh (a table per warp, a row is one warp's work).  The
+// latter wins wherever its lanes and warps have work.  They have not, with more than one slot to a
+// warp, where rows have few items (half of the lanes idle), where it folds one row at a time (more
+// than 4 columns), and where shared memory leaves it few rings.  Measured, us, table per CTA / per warp:
+//   1 column     Q5_0 11008 x 4096 10.6 / 11.7; Q4_1, Q5_1 there 8.5 / 8.4, 10.9 / 10.7; Q5_1 32000 x 256 7.0 / 8.8
+//   2..4         Q5_0 32000 x 512, 3 columns 11.4 / 17.1, x 1280, 2 columns 16.3 / 18.6, 4 columns 23.6 / 21.4;
+//                Q5_1 11008 x 4096, 4 columns 21.2 / 17.1; Q5_1 5120 x 14336, 4 columns (5 rings) 42.5 / 47.9, 3 columns
+//                (6 rings) 40.1 / 37.9
+//   5..8         Q5_1 32000 rows, 5 columns, K 1024 19.0 / 24.6, K 1536 27.5 / 33.0, 8 columns, K 2048 40.7 / 42.5;
+//                4096 x 11008, 6 columns (5 rings) 31.7 / 42.5; 11008 x 4096, 8 columns 30.2 / 28.4
 template <int kFormat>
-bool table_per_cta(uint32_t nb, size_t nr, size_t nc) {
-  return kFormat == 2 && nc == 1 && nb <= 128 && nr >= 8192;
+bool table_per_cta(const GemvAnyPlan &plan, uint32_t nb, size_t nr, size_t nc, int sms) {
+  if (nc == 1 && kFormat == 2 && nb <= 128 && nr >= 8192)
+    return true;
+  const GemvAnyArgs &a = plan.args;
+  if (nr <= static_cast<size_t>(sms) * a.nwarps * a.rps)
+    return false;
+  const uint32_t units = any_units<kFormat>(nb);
+  if (nc == 1)
+    return units <= 8;
+  if (nc <= 4)
+    return (units <= 24 && units * nc <= 64) || a.nwarps <= 5;
+  return nb * nc <= 340 || a.nwarps <= 6;
 }
 
 template <int kFormat>
@@ -116,13 +132,17 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
     const size_t want = (nr * nc * nb + 255) / 256;
     sibling_sums_kernel<kFormat><<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(
         vx, vy, sums, bx, by, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
-  } else if (const uint32_t rps = table_per_cta<kFormat>(nb, nr, nc) ? strict_stream_rows<kFormat>(nb, nr, nc, vx, bx) : 0) {
-    return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sm_count(), stream);
-  } else if (GemvAnyPlan plan; nr >= 8 && !any_tiny(nb, nr, nc, /*strict=*/true, sm_count()) &&
-                               plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true,
-                                                      /*static_weights=*/false, sm_count(), plan)) {
-    return launch_gemv_any<kFormat, true>(plan, stream);
   } else {
+    const int sms = sm_count();
+    const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx);  // 0: not for that kernel
+    GemvAnyPlan plan;
+    const bool any = nr >= 8 && (rps != 0 || !any_tiny(nb, nr, nc, /*strict=*/true, sms)) &&
+                     plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true, /*static_weights=*/false, sms, plan);
+    // (activations at odd addresses are not for the table per warp)
+    if (rps != 0 && (!any || table_per_cta<kFormat>(plan, nb, nr, nc, sms)))
+      return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sms, stream);
+    if (any)
+      return launch_gemv_any<kFormat, true>(plan, stream);
     const size_t want = (nr * nc + 7) / 8;
     sibling_dot_kernel<kFormat><<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(
         vx, vy, s, bx, by, bs, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
