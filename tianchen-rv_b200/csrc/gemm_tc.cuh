@@ -17,7 +17,8 @@
 // block (the second accumulating) give S exactly: every product is an integer below 2^11, every
 // partial sum an integer below 2^17, far inside fp32's 24-bit significand.  The fold is
 // then two packed fp32 operations per pair of outputs and nothing else.  (int8 operands with
-// kind::i8 need one MMA and an integer add per element: 17 % slower.)
+// kind::i8 need one MMA and an integer add per element.  That was 17 % slower on 128 x 128 items whose
+// MMAs a single-lane branch issued; it has not been measured on the items below.)
 //
 // Work items.  256 weight rows x 64 columns: the two row tiles share their columns, so one broadcast
 // load of activation scales serves two outputs of a thread (with 128 x 128 items those loads put 64 KB
@@ -68,17 +69,17 @@ struct GemmShape {
   static constexpr int kRows = kRowTiles * kGemmTileRows;
   static constexpr int kCpw = kCols / (kGemmEpilogueWarps / 4);  // columns of an epilogue warp
   static constexpr int kBlockCols = kRowTiles * kCols;           // TMEM columns of one block's accumulators
-  // A chunk is what a thread loads from TMEM at a time, up to 16 registers: kChunkCols columns of its
-  // rows of one block, or all its columns of several blocks.
+  // A chunk is what a thread loads from TMEM at a time, 16 registers: kChunkCols columns of its rows of
+  // one block.
   static constexpr int kChunkRegs = 16;
-  static constexpr int kChunkCols = kRowTiles * kCpw > kChunkRegs ? kChunkRegs / kRowTiles : kCpw;
-  static constexpr int kChunkBlocks = kChunkRegs / (kRowTiles * kChunkCols);
+  static constexpr int kChunkCols = kChunkRegs / kRowTiles;
+  static_assert(kCpw % kChunkCols == 0, "a block is whole chunks");
   static constexpr int kBlockChunks = kCpw / kChunkCols;  // chunks of one block
   // Blocks per accumulator hand-over.  A hand-over costs a barrier test, a release and a commit
   // whatever it carries, so it carries what leaves two TMEM stages.
   static constexpr int kHandover = 256 / kBlockCols < kGemmStageBlocks ? 256 / kBlockCols : kGemmStageBlocks;
-  static constexpr int kChunks = kGemmStageBlocks / kChunkBlocks * kBlockChunks;  // of a shared-memory stage
-  static constexpr int kHandoverChunks = kHandover / kChunkBlocks * kBlockChunks;
+  static constexpr int kChunks = kGemmStageBlocks * kBlockChunks;  // of a shared-memory stage
+  static constexpr int kHandoverChunks = kHandover * kBlockChunks;
   static_assert(kChunks % 2 == 0 && kChunks % kHandoverChunks == 0, "two chunk buffers, whole hand-overs");
 };
 
@@ -201,7 +202,7 @@ __device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.
 __device__ __forceinline__ void bulk_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// One block's part of a chunk (this thread's kRowTiles rows, kChunkCols columns of each) folded into
+// A chunk (this thread's kRowTiles rows of one block, kChunkCols columns of each) folded into
 // acc[.][col0 / 2 ..].
 //   plain:  acc = fma((float)S * d_w, d_x, acc)      repack: acc = fma((float)S, d_w * d_x, acc)
 // `dx2` holds the activation scales of this block and these columns; a scale that has been loaded
@@ -331,12 +332,12 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
         return false;
       tcgen05_fence_after_thread_sync();
     }
-    const uint32_t h = i % Shape::kHandoverChunks / Shape::kBlockChunks * Shape::kChunkBlocks;  // block of the hand-over
+    const uint32_t h = i % Shape::kHandoverChunks / Shape::kBlockChunks;  // block of the hand-over
     const uint32_t taddr = tmem_lane + c.ts.stage * Plan::kTmemStageCols + h * Shape::kBlockCols +
                            i % Shape::kBlockChunks * Shape::kChunkCols;
 #pragma unroll
-    for (int t = 0; t < Shape::kChunkBlocks * kRt; ++t)
-      tmem_ld_32x32b<Shape::kChunkCols>(taddr + t * Shape::kCols, v[buffer] + t * Shape::kChunkCols);
+    for (int r = 0; r < kRt; ++r)
+      tmem_ld_32x32b<Shape::kChunkCols>(taddr + r * Shape::kCols, v[buffer] + r * Shape::kChunkCols);
     return true;
   };
   auto release_tmem = [&]() {  // the hand-over's last chunk is in registers: the TMEM stage goes back
@@ -370,26 +371,18 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
   // the activation scales of chunk i into a buffer, from the stage `at`: column c of an item is column
   // c % kBoxCols of box c / kBoxCols
   constexpr int kScaleVecs = Shape::kChunkCols / 4;
-  ulonglong2 xd[2][Shape::kChunkBlocks * kScaleVecs];
+  ulonglong2 xd[2][kScaleVecs];
   auto load_scales = [&](const uint8_t *at, uint32_t i, uint32_t buffer) {
-    const uint32_t block = i / Shape::kBlockChunks * Shape::kChunkBlocks;
+    const uint32_t block = i / Shape::kBlockChunks;
     const uint32_t col = colgroup * kCpw + i % Shape::kBlockChunks * Shape::kChunkCols;
     const uint8_t *dx = at + Plan::kOffDx + col / Plan::kBoxCols * Plan::kDxBoxBytes + col % Plan::kBoxCols * 4;
 #pragma unroll
-    for (uint32_t b = 0; b < Shape::kChunkBlocks; ++b)
-#pragma unroll
-      for (int j = 0; j < kScaleVecs; ++j)
-        xd[buffer][b * kScaleVecs + j] =
-            reinterpret_cast<const ulonglong2 *>(dx + (block + b) * (Plan::kBoxCols * 4))[j];
+    for (int j = 0; j < kScaleVecs; ++j)
+      xd[buffer][j] = reinterpret_cast<const ulonglong2 *>(dx + block * (Plan::kBoxCols * 4))[j];
   };
-  auto fold_chunk = [&](uint32_t i, uint32_t buffer, uint32_t steps) {
-    const uint32_t block = i / Shape::kBlockChunks * Shape::kChunkBlocks;
-#pragma unroll
-    for (uint32_t b = 0; b < Shape::kChunkBlocks; ++b)
-      if (b == 0 || block + b < steps)  // (blocks past the row's end hold an older block's numbers)
-        fold_part<Shape, kRepack>(v[buffer] + b * kRt * Shape::kChunkCols, acc,
-                                  i % Shape::kBlockChunks * Shape::kChunkCols, dws[block + b],
-                                  xd[buffer] + b * kScaleVecs);
+  auto fold_chunk = [&](uint32_t i, uint32_t buffer) {
+    fold_part<Shape, kRepack>(v[buffer], acc, i % Shape::kBlockChunks * Shape::kChunkCols, dws[i / Shape::kBlockChunks],
+                              xd[buffer]);
   };
   // All stages but the last are whole.  Their chunks are software-pipelined: while one is folded the
   // next is on its way from TMEM, across hand-overs and stages, so neither the barrier test nor the
@@ -406,7 +399,7 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
         release_tmem();
       if (!load_chunk((i + 1) % Shape::kChunks, (i + 1) & 1))
         return false;
-      fold_chunk(i, i & 1, kGemmStageBlocks);
+      fold_chunk(i, i & 1);
     }
     close_stage();
   }
@@ -414,14 +407,14 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
   const uint32_t steps = a.nb - (nkb - 1) * kGemmStageBlocks;
 #pragma unroll
   for (uint32_t i = 0; i < Shape::kChunks; ++i) {
-    if (i / Shape::kBlockChunks * Shape::kChunkBlocks < steps) {
+    if (i / Shape::kBlockChunks < steps) {
       if (i > 0 && !load_chunk(i, 0))
         return false;
       load_scales(st, i, 0);
       tmem_ld_wait();
-      if ((i + 1) % Shape::kHandoverChunks == 0 || (i + 1) / Shape::kBlockChunks * Shape::kChunkBlocks >= steps)
+      if ((i + 1) % Shape::kHandoverChunks == 0 || (i + 1) / Shape::kBlockChunks >= steps)
         release_tmem();
-      fold_chunk(i, 0, steps);
+      fold_chunk(i, 0);
     }
   }
   close_stage();
