@@ -27,7 +27,13 @@ def place(torch, w, lead, pad):
                                                (4000, 91, 1, 0, 0), (2500, 66, 1, 6, 0), (97, 130, 8, 0, 14),
                                                (97, 129, 5, 4, 0), (8, 341, 1, 2, 0), (40, 343, 6, 0, 0),
                                                # shared memory for one or two of the sixteen rings
-                                               (8, 1001, 4, 0, 0), (33, 563, 8, 2, 0), (300, 1501, 2, 0, 2)])
+                                               (8, 1001, 4, 0, 0), (33, 563, 8, 2, 0), (300, 1501, 2, 0, 2),
+                                               # the smallest rows that do not stay on the general kernel
+                                               (2500, 1, 1, 0, 0), (1250, 3, 2, 2, 0), (3000, 5, 1, 0, 4),
+                                               # slots of 3 and 4 rows, then three slots to a warp and more
+                                               # (a ring slot is used again), in equal and unequal parts
+                                               (7500, 91, 1, 0, 0), (20001, 65, 1, 2, 0), (32000, 91, 1, 0, 0),
+                                               (9000, 35, 3, 0, 2), (20000, 33, 8, 6, 0)])
 def test_any_rows_match_the_oracle(cuda, pkg, O, q8w, nr, nb, nc, lead, pad):
     k = nb * 32
     w, x = make(O, nr, k, nc, q8w, 40 + nr + nb)
@@ -48,7 +54,8 @@ def test_any_rows_match_the_oracle(cuda, pkg, O, q8w, nr, nb, nc, lead, pad):
 
 @pytest.mark.parametrize("fmt", [1, 2, 3])
 @pytest.mark.parametrize("nr,nb,nc,lead,pad", [(64, 1, 1, 0, 0), (300, 33, 2, 2, 0), (2500, 91, 1, 0, 0), (130, 127, 4, 8, 2),
-                                               (70, 346, 8, 0, 0)])
+                                               (70, 346, 8, 0, 0), (2500, 1, 1, 0, 0), (7500, 61, 1, 0, 0),
+                                               (20001, 67, 1, 4, 0), (9000, 35, 3, 0, 2), (12000, 17, 6, 2, 0)])
 def test_any_sibling_rows_match_the_oracle(cuda, pkg, O, fmt, nr, nb, nc, lead, pad):
     w, x = sd.make(fmt, nr, nc, nb, 500 + fmt + nb)
     buf, xd = place(cuda, w, lead, pad), dev(cuda, x)
@@ -64,7 +71,8 @@ def test_any_sibling_rows_match_the_oracle(cuda, pkg, O, fmt, nr, nb, nc, lead, 
 def test_a_group_with_such_rows_has_the_bits_of_the_single_calls(cuda, pkg, O, q8w, strict):
     flags = pkg.FLAG_STRICT_ORDER if strict else 0
     problems, want = [], []
-    for i, (nr, nb) in enumerate([(1000, 91), (300, 64), (64, 3), (2000, 90)]):
+    # rows of more than 128 blocks (activations not in registers) and several slots to a warp among them
+    for i, (nr, nb) in enumerate([(1000, 91), (300, 64), (64, 3), (2000, 90), (700, 131), (9000, 33)]):
         w, x = make(O, nr, nb * 32, 1, q8w, 80 + i)
         wd, xd = dev(cuda, w), dev(cuda, x)
         problems.append((wd, xd, cuda.empty((nr, 1), dtype=cuda.float32, device="cuda")))

@@ -1,6 +1,6 @@
 """GPU parity, work items of the prefill GEMM: whole, half and narrow items at their edges (rows around
 128 and 256, columns around 32 and 64, block counts that end a stage early) equal the sequential oracle
-bit for bit, in both folds' layouts and with several destinations."""
+bit for bit, with both folds and with several destinations."""
 import ctypes
 
 import numpy as np
@@ -36,3 +36,15 @@ def test_items_at_their_edges_are_bit_exact(cuda, pkg, O, nr, k, nc):
     for o in outs:
         res = o.cpu().numpy()
         assert np.array_equal(np.ascontiguousarray(res[:, :nc]).view(np.uint32), want) and np.all(res[:, nc:] == -1.0)
+
+
+# (tokens, weight rows, K): whole items with halves in the last round, a row tile that does not exist with
+# ragged columns, items of one block
+@pytest.mark.parametrize("tokens,rows,k", [(512, 4864, 160), (484, 4752, 96), (128, 20480, 32)])
+def test_whole_items_of_the_repacked_gemm_are_bit_exact(cuda, pkg, O, tokens, rows, k):
+    w = O.quantize_q4_0(O.fill_normal(rows * k, 53, 0, 0.02).reshape(rows, k))
+    x = O.quantize_q8_0(O.fill_normal(tokens * k, 54).reshape(tokens, k))
+    wx, xx = O.rows_to_q4_0x16(w), O.rows_to_q8_0x4(x)
+    got = pkg.repack_gemm(cuda.from_numpy(wx).cuda(), cuda.from_numpy(xx).cuda(), k, tokens, rows).cpu().numpy()
+    pkg.check_device_errors()
+    assert np.array_equal(got.view(np.uint32), O.repack_gemm(wx, xx, k, tokens, rows).view(np.uint32))

@@ -79,6 +79,21 @@ def test_sibling_streaming_rows_bit_exact(cuda, pkg, O, fmt, nr, nb, pad):
     pkg.check_device_errors()
 
 
+# the calls that the table per CTA takes at any address: ragged slots, rows with a stride
+@pytest.mark.parametrize("fmt,nr,nb,nc,pad", [(2, 8192, 128, 1, 0), (2, 11009, 64, 1, 16), (3, 20003, 8, 1, 0), (1, 6001, 16, 4, 0),
+                                              (2, 9001, 24, 2, 32), (3, 8195, 40, 8, 0), (1, 2049, 344, 7, 16)])
+def test_sibling_table_per_cta_bit_exact(cuda, pkg, O, fmt, nr, nb, nc, pad):
+    w, x = sd.make(fmt, nr, nc, nb, 950 + fmt + nb)
+    padded = np.zeros((nr, w.shape[1] + pad), dtype=np.uint8)
+    padded[:, :w.shape[1]] = w
+    wd, xd = dev(cuda, padded), dev(cuda, x)
+    out = cuda.full((nr, nc), float("nan"), dtype=cuda.float32, device="cuda")
+    assert pkg.lib().tcrv_cuda_sibling_dot_rows(fmt, nb * 32, out.data_ptr(), wd.data_ptr(), xd.data_ptr(), xd.stride(0), nr, nc,
+                                                padded.shape[1], nc, cuda.cuda.current_stream().cuda_stream) == 0
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), O.sibling_dot_rows(fmt, w, x).view(np.uint32))
+    pkg.check_device_errors()
+
+
 @pytest.mark.parametrize("fmt,nr,nb,nc", [(1, 4096, 128, 1), (2, 4096, 344, 2), (3, 11008, 128, 8), (1, 32000, 8, 6), (2, 32000, 16, 3),
                                           (3, 5120, 448, 4), (3, 4096, 344, 6)])
 def test_sibling_calls_take_the_faster_streaming_kernel(cuda, pkg, fmt, nr, nb, nc):
