@@ -133,3 +133,52 @@ def test_a_package_under_a_second_name_raises_its_own_errors(cuda, pkg, operands
         with pytest.raises(p.TcrvCudaError) as e:
             p.gemv(operands["wq"], operands["xq"], out=narrow)
         assert e.value.status == -1
+
+
+# (what is wrong, the call, the error): every check that a call makes before it launches
+REFUSED = [
+    ("not a tensor", lambda p, c, o: p.vec_silu([1.0]), TypeError),
+    ("host memory", lambda p, c, o: p.vec_silu(o["x"].cpu()), TypeError),
+    ("element type", lambda p, c, o: p.vec_silu(o["x"].double()), TypeError),
+    ("element type of the output", lambda p, c, o: p.gemv(o["wq"], o["xq"], out=c.empty(48, 3, dtype=c.int32, device="cuda")), TypeError),
+    ("strided input", lambda p, c, o: p.vec_silu(o["x"][:, ::2]), ValueError),
+    ("strided output", lambda p, c, o: p.gemv(o["wq"], o["xq"], out=c.empty(48, 6, device="cuda")[:, ::2]), ValueError),
+    ("types of the addends", lambda p, c, o: p.add(o["x"], o["x"].int()), TypeError),
+    ("a type without a sum", lambda p, c, o: p.add(o["x"].half(), o["x"].half()), TypeError),
+    ("bytes that are no whole blocks", lambda p, c, o: p.dequantize_q8_0(o["xq"][:, :35].contiguous()), ValueError),
+    ("blocks without rows", lambda p, c, o: p.dequantize_q8_0(o["xq"][0, 0]), ValueError),
+    ("floats that are no whole blocks", lambda p, c, o: p.quantize_q8_0(o["x"][:, :33].contiguous()), ValueError),
+    ("weights of one dimension", lambda p, c, o: p.gemv(o["wq"][0], o["xq"]), ValueError),
+    ("row lengths", lambda p, c, o: p.gemv(o["wq"][:, :54], o["xq"]), ValueError),
+    ("weight format", lambda p, c, o: p.gemv(o["wq"], o["xq"], q8_weights=True), ValueError),
+    ("row lengths", lambda p, c, o: p.gemm(o["wq"][:, :54], o["xq"]), ValueError),
+    ("activations of one dimension", lambda p, c, o: p.gemm(o["wq"], o["xq"][0]), ValueError),
+    ("prepared row lengths", lambda p, c, o: p.gemm(o["pw"], o["xq"][:, :102]), ValueError),
+    ("activations of one dimension", lambda p, c, o: p.gemm(o["pw"], o["xq"][0]), ValueError),
+    ("row lengths", lambda p, c, o: p.sibling_dot_rows(2, o["sw"], o["sx"][:, :102].contiguous()), ValueError),
+    ("rows that are not contiguous", lambda p, c, o: p.rms_norm(o["x"].t(), 1e-5), ValueError),
+    ("rows of another type", lambda p, c, o: p.rope_apply(o["x"].double(), o["cache"]), ValueError),
+    ("type of the angles", lambda p, c, o: p.rope_apply(o["x"], o["cache"].double()), TypeError),
+    ("rows of the interleaved layout", lambda p, c, o: p.repack_gemv(o["w16"], o["xq"][0], 47), ValueError),
+    ("scale that is no number", lambda p, c, o: p.vec_scale_(o["x"].clone(), "2"), TypeError),
+    ("flags that are no number", lambda p, c, o: p.gemv(o["wq"], o["xq"], flags="strict"), TypeError),
+]
+
+
+@pytest.mark.parametrize("what,call,error", REFUSED, ids=[f"{i}: {r[0]}" for i, r in enumerate(REFUSED)])
+def test_operands_that_do_not_fit_are_refused(cuda, pkg, operands, what, call, error):
+    with pytest.raises(error):
+        call(pkg, cuda, operands)
+
+
+def test_statuses_of_the_c_entries_become_errors(cuda, pkg, operands):
+    o = operands
+    small = cuda.empty(256, dtype=cuda.uint8, device="cuda")
+    for call, status in [(lambda: pkg.gemm(o["wq"], o["xq"], workspace=small), -5), (lambda: pkg.gemm(o["pw"], o["xq"], workspace=small), -5),
+                         (lambda: pkg.rms_norm(o["x"], 1e-5, flags=64), -1), (lambda: pkg.rope_apply(o["x"][:, :127], o["cache"]), -1)]:
+        with pytest.raises(pkg.TcrvCudaError) as e:
+            call()
+        assert e.value.status == status
+    # (a native function has a fixed number of arguments)
+    with pytest.raises(TypeError):
+        pkg._native.vec_silu(o["x"])
