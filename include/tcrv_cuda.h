@@ -41,12 +41,12 @@ typedef enum {
 /* flags for the GEMV / GEMM entry points */
 #define TCRV_CUDA_FLAG_NONE 0u
 /* fold every row's blocks in strict ascending order (bit-identical to the sequential
- * scalar kernel with the fused fold).  Up to 8 columns against at least 64 rows whose base and
- * stride are multiples of 16 bytes (block count a multiple of 8) run on a streaming kernel that
- * keeps that order (many threads compute the per-block terms, a few fold them block after
- * block; 3..8 columns on rows of up to 4096 elements use the tensor cores for the terms): about
- * two thirds of the bandwidth of the default orders; anything else on a general warp-per-output
- * kernel */
+ * scalar kernel with the fused fold).  Up to 8 columns against at least 8 rows at even addresses
+ * run on streaming kernels that keep that order (many threads compute the per-block terms, a few
+ * fold them block after block; 3..8 columns on rows of up to 4096 elements whose base and stride
+ * are multiples of 16 bytes use the tensor cores for the terms): about two thirds of the bandwidth
+ * of the default orders.  Fewer rows, tiny matrices, odd addresses and more columns run on a
+ * general warp-per-output kernel */
 #define TCRV_CUDA_FLAG_STRICT_ORDER 1u
 /* the weight buffer was not written by the work that immediately precedes this call on the
  * stream (model weights are static): the decode GEMV may then start streaming weights while
@@ -122,8 +122,9 @@ int tcrv_cuda_vec_dot_q8_0_q8_0(size_t n, float *s, const uint8_t *vx, const uin
  *   TCRV_CUDA_FLAG_STRICT_ORDER: every output is the sequential fold over blocks 0, 1, 2, ...
  *     (TCRV_CUDA_ORDER_STRICT), on streaming kernels that pass the block terms through a table
  *     in shared memory (one column: 0.71 of the HBM peak on 32000 x 4096);
- *   operands that rule out 16-byte bulk copies: sequential or lane-pair order on the generic
- *     kernel.
+ *   rows off 16-byte boundaries (a block count that is no multiple of 8, for instance): sequential
+ *     or lane-pair order for every column count, streamed if all addresses and strides are even and
+ *     there are at least 8 rows, otherwise (and for tiny matrices) on the generic kernel.
  * The GEMM folds every output element in strict ascending block order.  All use the fused
  * form fma((float)sumi * d_x, d_y, sumf). */
 #define TCRV_CUDA_ORDER_STRICT 0
@@ -200,11 +201,12 @@ int tcrv_cuda_gemm_q4_0_q8_0_prepared(size_t n, float *s, const void *prepared_w
  *   Q4_1, Q5_1:  sumf = sumf + fma(d_x*d_y, (float)sumi, m_x*s_y),
  * i.e. bit-identical to the sequential fold.  `dot_rows` is the matrix form
  * (s[row*bs + col], strides as in tcrv_cuda_gemv_*); the vec_dot entries are the reference's
- * one-row kernels (ABI order n, s, vx, vy).  Up to 8 columns against at least 64 rows whose
- * base and stride are multiples of 16 bytes, with a block count that is a multiple of 8, run on
- * the streaming kernel of TCRV_CUDA_FLAG_STRICT_ORDER (bulk copies, a table of block terms
- * folded row by row in ascending order); everything else on a general warp-per-output
- * kernel.  Both perform the same operations in the same order. */
+ * one-row kernels (ABI order n, s, vx, vy).  Up to 8 columns against at least 8 rows at even
+ * addresses run on streaming kernels (bulk copies, block terms in a table per warp or per CTA
+ * folded row by row in ascending order); activations at odd addresses do so against at least 64
+ * rows whose base and stride are multiples of 16 bytes, with a block count that is a multiple of
+ * 8; everything else runs on a general warp-per-output kernel.  All perform the same operations
+ * in the same order. */
 #define TCRV_CUDA_FORMAT_Q4_1_Q8_1 1
 #define TCRV_CUDA_FORMAT_Q5_0_Q8_0 2
 #define TCRV_CUDA_FORMAT_Q5_1_Q8_1 3

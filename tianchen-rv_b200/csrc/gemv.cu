@@ -1,7 +1,8 @@
-// GEMV launchers: the streaming kernel (gemv_stream.cuh) when the operands allow 16-byte
-// bulk copies, otherwise a generic warp-per-row kernel that accepts any alignment and any
-// block count and also implements the strict (sequential) fold order.  Plus the debug kernel
-// that exposes the integer stage (per-block int32 sums).
+// GEMV launchers: the streaming kernels for rows on 16-byte boundaries (gemv_stream.cuh, the
+// tensor-core forms gemv_mma*.cuh, strict_stream.cuh), the one for rows of any block count at even
+// addresses (gemv_any.cuh), and a generic warp-per-row kernel that accepts any alignment and also
+// implements the strict (sequential) fold order.  Plus the debug kernel that exposes the integer
+// stage (per-block int32 sums).
 #include <atomic>
 #include "gemv_any.cuh"
 #include "gemv_mma.cuh"

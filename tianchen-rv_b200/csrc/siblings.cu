@@ -1,7 +1,9 @@
 // Block dots of the sibling ggml formats the reference also compiles: Q4_1 x Q8_1, Q5_0 x Q8_0
-// and Q5_1 x Q8_1.  One warp per (weight row, activation column); every lane computes one block
-// of a group of 32 (byte-granular loads: no alignment assumptions), then the 32 terms are folded
-// one after another in ascending block order, so the result is the sequential fold bit for bit.
+// and Q5_1 x Q8_1.  The launchers choose between two streaming kernels, gemv_any.cuh (a table of block
+// terms per warp) and strict_stream.cuh (one per CTA), and the general kernel below: one warp per
+// (weight row, activation column); every lane computes one block of a group of 32 (byte-granular
+// loads: no alignment assumptions), then the 32 terms are folded one after another.  All fold in
+// ascending block order, so the result is the sequential fold bit for bit.
 //   Q5_0:        sumf = fma(d_x*d_y, (float)sumi, sumf)
 //   Q4_1, Q5_1:  sumf = sumf + fma(d_x*d_y, (float)sumi, m_x*s_y)
 // (the contraction one C expression gets; lib/Conversion/RVV/RVVToEmitCBlockQuantLinear.cpp:

@@ -21,6 +21,10 @@
 // with one column and a block count that divides the worker count, a thread meets the same
 // block in every row and keeps its activation words in registers.
 //
+// It serves Q4_0 / Q8_0 rows on 16-byte boundaries that are too long for the tensor-core form, and the
+// sibling formats where its 512 workers on one slot beat the table per warp of gemv_any.cuh
+// (siblings.cu has the rule) or where the activations lie at an odd address.
+//
 // Folds (reference: lib/Conversion/RVV/RVVToEmitCBlockQuantLinear.cpp:322-356, 7538-7573,
 // 472-915, 916-1391, 6817-7263):
 //   Q4_0 x Q8_0:    sumf = fma((float)sumi * d_w, d_x, sumf)       table: (float)sumi * d_w
