@@ -68,11 +68,15 @@ def test_any_sibling_rows_match_the_oracle(cuda, pkg, O, fmt, nr, nb, nc, lead, 
 
 @pytest.mark.parametrize("q8w", [False, True])
 @pytest.mark.parametrize("strict", [False, True])
-def test_a_group_with_such_rows_has_the_bits_of_the_single_calls(cuda, pkg, O, q8w, strict):
+@pytest.mark.parametrize("shapes", [
+    # rows of more than 128 blocks (activations not in registers) and several slots to a warp among them
+    [(1000, 91), (300, 64), (64, 3), (2000, 90), (700, 131), (9000, 33)],
+    [(33, 1001), (300, 1401)],  # shared memory for two to five rings
+])
+def test_a_group_with_such_rows_has_the_bits_of_the_single_calls(cuda, pkg, O, q8w, strict, shapes):
     flags = pkg.FLAG_STRICT_ORDER if strict else 0
     problems, want = [], []
-    # rows of more than 128 blocks (activations not in registers) and several slots to a warp among them
-    for i, (nr, nb) in enumerate([(1000, 91), (300, 64), (64, 3), (2000, 90), (700, 131), (9000, 33)]):
+    for i, (nr, nb) in enumerate(shapes):
         w, x = make(O, nr, nb * 32, 1, q8w, 80 + i)
         wd, xd = dev(cuda, w), dev(cuda, x)
         problems.append((wd, xd, cuda.empty((nr, 1), dtype=cuda.float32, device="cuda")))

@@ -664,7 +664,7 @@ int launch_gemv_any_group(const GemvGroupItem *items, size_t count, bool strict,
   size_t smem = 0;
   double cost[kGemvGroupMax], all_cost = 0.0;
   int cap[kGemvGroupMax];
-  uint32_t warps = 0, share[kGemvGroupMax];
+  uint32_t share[kGemvGroupMax];
   for (size_t i = 0; i < count; ++i) {
     const GemvGroupItem &it = items[i];
     GemvAnyPlan plan;
@@ -674,7 +674,6 @@ int launch_gemv_any_group(const GemvGroupItem *items, size_t count, bool strict,
     group.problem[i] = plan.args;
     cap[i] = plan.grid;
     smem = plan.smem > smem ? plan.smem : smem;
-    warps = plan.args.nwarps > warps ? plan.args.nwarps : warps;
     cost[i] = static_cast<double>(it.nr) * plan.args.row_bytes;
     all_cost += cost[i];
   }
@@ -686,7 +685,8 @@ int launch_gemv_any_group(const GemvGroupItem *items, size_t count, bool strict,
   const int st = any_configure(kernel, configured[strict ? 1 : 0]);
   if (st != TCRV_CUDA_OK)
     return st;
-  TCRV_CUDA_TRY(launch_pdl(kernel, static_cast<int>(group.first[count]), static_cast<int>(warps * 32), smem, stream, group));
+  // (16 warps, as for a single problem: those without a ring help to stage the activations)
+  TCRV_CUDA_TRY(launch_pdl(kernel, static_cast<int>(group.first[count]), kAnyMaxWarps * 32, smem, stream, group));
   TCRV_CUDA_TRY(cudaGetLastError());
   return TCRV_CUDA_OK;
 }
