@@ -47,9 +47,12 @@ inline const at::Tensor &tensor(PyObject *o) {
 // What a kernel can read and write where it lies: a CUDA tensor, or one in page-locked host memory
 // (mapped at the same address).  The GEMV and GEMM operands and the strided outputs may be either.
 inline const at::Tensor &mapped(PyObject *o) {
-  if (THPVariable_Check(o) && !THPVariable_Unpack(o).is_cuda() && THPVariable_Unpack(o).is_pinned())
-    return THPVariable_Unpack(o);
-  return tensor(o);
+  if (THPVariable_Check(o)) {
+    const at::Tensor &t = THPVariable_Unpack(o);
+    if (t.is_cuda() || t.is_pinned())
+      return t;
+  }
+  return tensor(o);  // (refuses it)
 }
 
 // A contiguous CUDA tensor of the given type.
@@ -177,9 +180,9 @@ struct Output {
       require((rows - 1) * tensor.stride(0) + cols);
   }
   // An output that is made lies beside `like`, which has to be a CUDA tensor then.
-  void beside(PyObject *like) const {
-    if (given == Py_None)
-      ::tensor(like);
+  void beside(const at::Tensor &like) const {
+    if (given == Py_None && !like.is_cuda())
+      fail(PyExc_TypeError, "operands must be CUDA torch tensors (device pointers cross the C ABI)");
   }
   void make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like) {
     if (given == Py_None)
@@ -295,7 +298,7 @@ TCRV_CALL(gemv, 5) {
   const int64_t nr = w.size(0), nc = x.size(0);
   Output out(a[4], at::kFloat);
   out.require_rows(nr, nc);
-  out.beside(a[0]);
+  out.beside(w);
   const size_t n = static_cast<size_t>(nb * kQK), bx = static_cast<size_t>(w.stride(0)),
                by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
@@ -352,7 +355,7 @@ TCRV_CALL(gemm, 4) {
   const size_t n = static_cast<size_t>(nb * kQK), nr = static_cast<size_t>(w.size(0)), nc = static_cast<size_t>(x.size(0));
   Output out(a[2], at::kFloat);
   out.require_rows(w.size(0), x.size(0));
-  out.beside(a[0]);
+  out.beside(w);
   Scratch ws(a[3]);
   const size_t bx = static_cast<size_t>(w.stride(0)), by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
@@ -377,7 +380,7 @@ TCRV_CALL(gemm_prepared, 6) {
   const size_t nc = static_cast<size_t>(x.size(0));
   Output out(a[4], at::kFloat);
   out.require_rows(static_cast<int64_t>(nr), x.size(0));
-  out.beside(a[3]);
+  out.beside(x);
   Scratch ws(a[5]);
   const size_t by = static_cast<size_t>(x.stride(0));
   const cudaStream_t st = stream();
