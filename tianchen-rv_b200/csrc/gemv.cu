@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const uint8_t *__rest
                                                            size_t bx, size_t by, size_t bs, uint32_t nr, uint32_t nc,
                                                            uint32_t nb) {
   constexpr int WB = WeightFormat<kQ8W>::kBlockBytes;
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const size_t warp = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const size_t nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -599,12 +600,9 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
   const size_t cap = static_cast<size_t>(sm_count()) * 8;
   if (blocks > cap)
     blocks = cap;
-  if (strict)
-    gemv_generic_kernel<kQ8W, true><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        vx, vy, s, bx, by, bs, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
-  else
-    gemv_generic_kernel<kQ8W, false><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        vx, vy, s, bx, by, bs, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
+  auto kernel = strict ? gemv_generic_kernel<kQ8W, true> : gemv_generic_kernel<kQ8W, false>;
+  TCRV_CUDA_TRY(launch_pdl(kernel, static_cast<int>(blocks), 256, 0, stream, vx, vy, s, bx, by, bs,
+                           static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb));
   TCRV_CUDA_TRY(cudaGetLastError());
   return TCRV_CUDA_OK;
 }

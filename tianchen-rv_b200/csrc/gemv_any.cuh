@@ -549,13 +549,14 @@ bool plan_gemv_any(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, siz
   return true;
 }
 
-// Matrices that are done before this kernel is set up: rows of half a warp's pass and no more than two
-// rounds of warps on the general kernel, which asks for no shared memory.  us, general / this one:
-// strict order 148 x 5 blocks, 8 columns 2.5 / 3.4, 600 x 9 2.5 / 3.1, 1200 x 9 2.9 / 3.0, 600 x 9 x 4
-// 3.3 / 3.3, 200 x 17 2.9 / 2.9, 200 x 33 3.6 / 3.0; the kernel's own order 300 x 1 2.4 / 2.9,
-// 300 x 5 2.9 / 2.9, 300 x 17 3.1 / 2.9; Q5_0 148 x 9 x 4 2.6 / 3.2, 600 x 17 2.9 / 3.4, 600 x 33 3.7 / 3.4.
+// Matrices that are done before this kernel is set up: rows of half a warp's pass, and no more than two
+// rounds of warps on the general kernel, which asks for no shared memory.  (With fewer outputs than half
+// of the SMs only a few CTAs of this kernel start.)  us, general / this one: strict Q4_0 148 x 5 blocks
+// 2.0 / 3.1, 600 x 9 2.2 / 3.0, 1200 x 9 2.6 / 3.1, 2400 x 9 2.9 / 3.3; strict Q5_0 148 x 9 2.0 / 3.1, 1200 x 9
+// 2.5 / 3.2; lane pairs 300 x 1 2.0 / 2.9, 300 x 5 2.4 / 2.9, 40 x 3 2.4 / 2.2.
 inline bool any_tiny(uint32_t nb, size_t nr, size_t nc, bool strict, int sms) {
-  return nb <= (strict ? 16u : 4u) && nr * nc <= 16u * static_cast<size_t>(sms);
+  const size_t outputs = nr * nc;
+  return nb <= (strict ? 16u : 4u) && 2 * outputs >= static_cast<size_t>(sms) && outputs <= 16u * static_cast<size_t>(sms);
 }
 
 template <typename Kernel>

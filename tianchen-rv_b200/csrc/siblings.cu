@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(256) sibling_dot_kernel(const uint8_t *__restr
                                                           float *__restrict__ s, size_t bx, size_t by, size_t bs,
                                                           uint32_t nr, uint32_t nc, uint32_t nb) {
   using F = Sibling<kFormat>;
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const size_t warp = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const size_t nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -146,8 +147,8 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
     if (any)
       return launch_gemv_any<kFormat, true>(plan, stream);
     const size_t want = (nr * nc + 7) / 8;
-    sibling_dot_kernel<kFormat><<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(
-        vx, vy, s, bx, by, bs, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
+    TCRV_CUDA_TRY(launch_pdl(sibling_dot_kernel<kFormat>, static_cast<int>(want < cap ? want : cap), 256, 0, stream, vx, vy, s,
+                             bx, by, bs, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb));
   }
   TCRV_CUDA_TRY(cudaGetLastError());
   return TCRV_CUDA_OK;
