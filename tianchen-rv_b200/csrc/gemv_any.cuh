@@ -549,14 +549,16 @@ bool plan_gemv_any(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, siz
   return true;
 }
 
-// Matrices that are done before this kernel is set up: rows of half a warp's pass, and no more than two
-// rounds of warps on the general kernel, which asks for no shared memory.  (With fewer outputs than half
-// of the SMs only a few CTAs of this kernel start.)  us, general / this one: strict Q4_0 148 x 5 blocks
-// 2.0 / 3.1, 600 x 9 2.2 / 3.0, 1200 x 9 2.6 / 3.1, 2400 x 9 2.9 / 3.3; strict Q5_0 148 x 9 2.0 / 3.1, 1200 x 9
-// 2.5 / 3.2; lane pairs 300 x 1 2.0 / 2.9, 300 x 5 2.4 / 2.9, 40 x 3 2.4 / 2.2.
+// Matrices that are done before this kernel is set up stay on the general kernels, which ask for no shared
+// memory: in the strict order rows of one pass of a warp there and no more than one round of its warps, in
+// the lane-pair order rows of half as many blocks, and outputs for at least half of the SMs (with fewer only
+// a few CTAs of this kernel start).  us, general / this one:
+//   strict Q4_0   148 x 5 blocks 2.0 / 3.1, 600 x 25 2.6 / 3.2, 1200 x 9 2.6 / 3.1, 1200 x 25 3.5 / 3.3, 600 x 33 3.4 / 3.2
+//   strict Q5_0   148 x 9 2.0 / 3.1, 600 x 25 2.7 / 3.3, 1200 x 25 3.5 / 3.4, 600 x 33 3.5 / 3.3
+//   lane pairs    300 x 5 2.4 / 2.9, 600 x 12 2.7 / 2.8, 300 x 17 2.9 / 2.9, 1200 x 5 3.0 / 2.9, 40 x 5 2.4 / 2.1
 inline bool any_tiny(uint32_t nb, size_t nr, size_t nc, bool strict, int sms) {
-  const size_t outputs = nr * nc;
-  return nb <= (strict ? 16u : 4u) && 2 * outputs >= static_cast<size_t>(sms) && outputs <= 16u * static_cast<size_t>(sms);
+  const size_t outputs = nr * nc, n = static_cast<size_t>(sms);
+  return strict ? nb <= 32 && outputs <= 8 * n : nb <= 16 && 2 * outputs >= n && outputs <= 4 * n;
 }
 
 template <typename Kernel>
