@@ -1,7 +1,7 @@
 """Build recipe for the provider's native code (sm_100a only, in-tree outputs).
 
-``build_library()`` compiles ``csrc/*.cu`` into ``libtcrv_cuda.so`` next to this file with
-nvcc; it needs no GPU (nvcc cross-compiles).  ``build_torch_calls()`` compiles
+``build_library()`` has the Makefile compile ``csrc/*.cu`` into ``libtcrv_cuda.so`` next to this file
+with nvcc; it needs no GPU (nvcc cross-compiles).  ``build_torch_calls()`` compiles
 ``csrc/torch_calls.cpp``, the package's native call path, into ``_tcrv_torch.<Python ABI>.torch-<version>.so``
 beside it with the host compiler.  Run as a script to force a rebuild.
 """
@@ -19,22 +19,11 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtcrv_cuda.so")
 
-NVCC_FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a",
-    "-lineinfo", "-O3", "-std=c++17", "-rdc=true",
-    "-Xcompiler", "-fPIC", "-shared", "--threads", "0",
-]
-
-
 def _nvcc() -> str:
     exe = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(exe):
         raise RuntimeError("nvcc not found: the provider's CUDA library cannot be built")
     return exe
-
-
-def sources() -> list[str]:
-    return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
 def _stale() -> bool:
@@ -49,10 +38,14 @@ def _stale() -> bool:
 def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return LIB
-    cmd = [_nvcc(), *NVCC_FLAGS, "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-o", LIB, *sources()]
+    cmd = ["make", "-C", HERE, f"-j{os.cpu_count()}", f"NVCC={_nvcc()}", os.path.basename(LIB)]
+    if force:
+        cmd.insert(1, "-B")
     if verbose:
-        cmd.insert(1, "-Xptxas=-v")
+        cmd.append("NVCCEXTRA=-Xptxas=-v")
         print(" ".join(cmd), file=sys.stderr)
+    else:
+        cmd.insert(1, "-s")
     subprocess.run(cmd, check=True)
     return LIB
 

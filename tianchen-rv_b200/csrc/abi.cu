@@ -38,6 +38,25 @@ int sm_count() {
   return cached[dev];
 }
 
+int device_error_words(DeviceErrorWords *out) {
+  static std::atomic<int *> word[64];
+  static std::atomic<int **> mirror[64];
+  int dev = 0;
+  TCRV_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64)
+    return TCRV_CUDA_ERR_UNSUPPORTED;
+  if (mirror[dev].load() == nullptr) {  // host threads may race to fill these with the same values
+    void *w = nullptr, *m = nullptr;
+    TCRV_CUDA_TRY(cudaGetSymbolAddress(&w, g_device_error));
+    TCRV_CUDA_TRY(cudaGetSymbolAddress(&m, g_host_error_mirror));
+    word[dev] = static_cast<int *>(w);
+    mirror[dev] = static_cast<int **>(m);
+  }
+  out->word = word[dev];
+  out->mirror = mirror[dev];
+  return TCRV_CUDA_OK;
+}
+
 namespace {
 
 inline cudaStream_t as_stream(tcrv_cuda_stream s) { return static_cast<cudaStream_t>(s); }

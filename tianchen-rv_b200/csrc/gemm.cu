@@ -392,6 +392,9 @@ int run_gemm(size_t n, float *const *dst, size_t ndst, const uint8_t *weights_pl
   args.nr = static_cast<uint32_t>(nr);
   args.nc = static_cast<uint32_t>(nc);
   args.nb = static_cast<uint32_t>(p.nb);
+  const int st = device_error_words(&args.errors);
+  if (st != TCRV_CUDA_OK)
+    return st;
   if (multi)
     return launch_gemm_kernel<true, false, false>(p, weights_planar, acts_planar, args, stream);
   if (narrow_items(nr, nc, static_cast<size_t>(sm_count())))

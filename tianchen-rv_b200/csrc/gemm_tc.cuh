@@ -38,15 +38,22 @@
 //
 // Operands come from a planar ("prepared") layout written by the unpack kernels: 8-bit
 // matrices [rows][K] and fp32 scale matrices, all fetched with tiled TMA loads (128-byte
-// swizzle for the 8-bit tiles, no multicast).  Warp roles in a CTA of 10 warps:
+// swizzle for the 8-bit tiles, no multicast).  Warp roles in a CTA of 12 warps:
 //   warps 0..7  epilogue: warp w reads TMEM lanes 32*(w%4).. (its weight rows) and half of the
 //               columns of every accumulator tile
-//   warp 8      TMA producer (one lane)
-//   warp 9      TMEM allocation + MMA issue (one elected lane)
+//   warp 8      TMA producer (one elected lane)
+//   warps 9, 10 MMA issue (one elected lane each), by turns; warp 9 allocates TMEM
 // Pipelines: shared-memory stages of 4 blocks each (full/empty mbarriers) and TMEM stages of
 // several blocks each (full/empty mbarriers).  The epilogue warps wait on the accumulator barriers
 // only: a stage's scale tiles have landed when its first accumulator has.
 //
+// What bounds it: per 256 x 64 block of outputs the fold's 128 packed operations a warp pair take about
+// 320 cycles of a scheduler's FMA pipe (a packed FMA of three different register pairs takes 3 cycles, not
+// 2), and the scale loads' 256 and the MMA operands' 128 cycles share the shared-memory pipe: without
+// the scale loads 210, without MMAs 206 of 230 us (512 x 32000 x 4096, operands in L2).  With one MMA warp,
+// 16-register chunks and a single-lane producer it was 250; 512 x 11008 x 4096 92.7 -> 88.2 us, 77 x 4096 x
+// 11008 41.6 -> 32.5 us (there the producer's 780 cycles per stage were the limit).  32-register chunks need
+// more than the 168 registers a thread starts with; without setmaxnreg, 16-register chunks: 244 us.
 // Every wait is bounded; a failed wait raises the device error word and the CTA winds down.
 #pragma once
 
@@ -59,7 +66,12 @@ constexpr int kGemmTileRows = 128;      // weight rows of one MMA (M, TMEM lanes
 constexpr int kGemmStageBlocks = 4;     // ggml blocks per shared-memory stage (128 bytes of K)
 constexpr int kGemmTmemCols = 512;      // all of TMEM
 constexpr int kGemmEpilogueWarps = 8;  // 4 lane quarters x 2 column groups
-constexpr int kGemmThreads = (kGemmEpilogueWarps + 2) * 32;
+constexpr int kGemmMmaWarps = 2;
+constexpr int kGemmThreads = (kGemmEpilogueWarps + 4) * 32;  // TMA, MMA and one warp that fills the third warpgroup
+// The block starts with 384 x 168 registers; the third warpgroup keeps 128 x 40 of them and the epilogue's
+// two take 256 x 216 (60416 of 64512 in all).
+constexpr int kGemmEpilogueRegs = 216, kGemmOtherRegs = 40;
+static_assert(8 * kGemmEpilogueWarps * kGemmEpilogueRegs + 32 * kGemmOtherRegs <= 8 * 12 * 168, "the launch's registers");
 constexpr int kGemmCtrlBytes = 1024;  // barriers, TMEM base, abort flag
 
 // The shape of a work item: kRowTiles x 128 weight rows, kCols activation columns.
@@ -69,17 +81,20 @@ struct GemmShape {
   static constexpr int kRows = kRowTiles * kGemmTileRows;
   static constexpr int kCpw = kCols / (kGemmEpilogueWarps / 4);  // columns of an epilogue warp
   static constexpr int kBlockCols = kRowTiles * kCols;           // TMEM columns of one block's accumulators
-  // A chunk is what a thread loads from TMEM at a time, 16 registers: kChunkCols columns of its rows of
-  // one block.
-  static constexpr int kChunkRegs = 16;
-  static constexpr int kChunkCols = kChunkRegs / kRowTiles;
-  static_assert(kCpw % kChunkCols == 0, "a block is whole chunks");
-  static constexpr int kBlockChunks = kCpw / kChunkCols;  // chunks of one block
+  // A chunk is what a thread loads from TMEM at a time, 32 registers: kChunkCols columns of its rows of
+  // kChunkBlocks blocks.
+  static constexpr int kChunkRegs = 32;
+  static constexpr int kChunkCols = kCpw < kChunkRegs / kRowTiles ? kCpw : kChunkRegs / kRowTiles;
+  static constexpr int kChunkBlocks = kChunkRegs / (kRowTiles * kChunkCols);
+  static constexpr int kBlockChunks = kCpw / kChunkCols;  // chunks of one block, where it has several
+  static_assert(kCpw % kChunkCols == 0 && (kChunkBlocks == 1 || kBlockChunks == 1), "part of a block or whole blocks");
+  __host__ __device__ static constexpr uint32_t chunk_block(uint32_t i) { return i / kBlockChunks * kChunkBlocks; }
+  __host__ __device__ static constexpr uint32_t chunk_col(uint32_t i) { return i % kBlockChunks * kChunkCols; }
   // Blocks per accumulator hand-over.  A hand-over costs a barrier test, a release and a commit
   // whatever it carries, so it carries what leaves two TMEM stages.
   static constexpr int kHandover = 256 / kBlockCols < kGemmStageBlocks ? 256 / kBlockCols : kGemmStageBlocks;
-  static constexpr int kChunks = kGemmStageBlocks * kBlockChunks;  // of a shared-memory stage
-  static constexpr int kHandoverChunks = kHandover * kBlockChunks;
+  static constexpr int kChunks = kGemmStageBlocks * kBlockChunks / kChunkBlocks;  // of a shared-memory stage
+  static constexpr int kHandoverChunks = kHandover * kBlockChunks / kChunkBlocks;
   static_assert(kChunks % 2 == 0 && kChunks % kHandoverChunks == 0, "two chunk buffers, whole hand-overs");
 };
 
@@ -135,6 +150,7 @@ struct GemmArgs {
   uint32_t tiles_m;     // column tiles
   uint32_t full_items;  // items [0, full_items) are whole ones
   uint32_t items;       // items [full_items, items) are halves: half j % 2 of whole item full_items + j / 2
+  DeviceErrorWords errors;
 };
 
 struct GemmItem {
@@ -239,6 +255,7 @@ struct GemmEpilogueCtx {
   volatile uint32_t *abort_flag;
   uint32_t tmem_base;
   uint32_t store_syncs;  // syncs of the epilogue warps done so far (parity of the next one)
+  uint32_t mma_warp;     // an MMA warp fills the TMEM stages of its parity
   PipeState ps, ts;
 };
 
@@ -317,6 +334,7 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
   const int row_local = quarter * 32 + lane;
   const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
   const uint32_t tmem_lane = c.tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + colgroup * kCpw;
+  constexpr int kScaleVecs = Shape::kChunkCols / 4;  // activation scales of one block of a chunk
   uint64_t acc[kRt][kCpw / 2];
 #pragma unroll
   for (int r = 0; r < kRt; ++r)
@@ -324,100 +342,123 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
     for (int j = 0; j < kCpw / 2; ++j)
       acc[r][j] = 0ull;
   uint32_t v[2][Shape::kChunkRegs];
-  // chunk i of a shared-memory stage, from TMEM into a buffer; waits for the hand-over that the
-  // chunk opens
-  auto load_chunk = [&](uint32_t i, uint32_t buffer) -> bool {
-    if (i % Shape::kHandoverChunks == 0) {
-      if (!mbar_wait_bounded(&c.tmem_full[c.ts.stage], c.ts.phase, c.abort_flag))
-        return false;
-      tcgen05_fence_after_thread_sync();
-    }
-    const uint32_t h = i % Shape::kHandoverChunks / Shape::kBlockChunks;  // block of the hand-over
-    const uint32_t taddr = tmem_lane + c.ts.stage * Plan::kTmemStageCols + h * Shape::kBlockCols +
-                           i % Shape::kBlockChunks * Shape::kChunkCols;
-#pragma unroll
-    for (int r = 0; r < kRt; ++r)
-      tmem_ld_32x32b<Shape::kChunkCols>(taddr + r * Shape::kCols, v[buffer] + r * Shape::kChunkCols);
+  ulonglong2 xd[2][Shape::kChunkBlocks * kScaleVecs];
+  float4 dw[kRt];
+  const uint8_t *st = nullptr;
+  uint32_t tmem_at = 0;
+  bool ready = false;
+  // Whether the next hand-over is there already, asked one chunk before the answer is needed.
+  auto peek_handover = [&]() {
+    PipeState next = c.ts;
+    next.advance(Plan::kTmemStages);
+    ready = mbar_test(&c.tmem_full[next.stage], next.phase);
+  };
+  auto open_handover = [&]() -> bool {
+    if (!ready && !mbar_wait_bounded(&c.tmem_full[c.ts.stage], c.ts.phase, c.abort_flag))
+      return false;
+    tcgen05_fence_after_thread_sync();
+    tmem_at = tmem_lane + c.ts.stage * Plan::kTmemStageCols;
     return true;
   };
-  auto release_tmem = [&]() {  // the hand-over's last chunk is in registers: the TMEM stage goes back
+  auto release_handover = [&]() {  // its last chunk is in registers: the TMEM stage goes back
     tcgen05_fence_before_thread_sync();
     __syncwarp();
-    if (lane == 0)
-      mbar_arrive(&c.tmem_empty[c.ts.stage]);
+    mbar_arrive_if(&c.tmem_empty[c.ts.stage], lane == 0);
     c.ts.advance(Plan::kTmemStages);
   };
-  // The stage's scale tiles arrive with its operands (same transaction barrier), and the MMA
-  // warp issues a block's MMAs only after that barrier has completed; so when an
-  // accumulator barrier of this stage has completed, the scale tiles are in shared memory.
-  // The epilogue therefore does not wait on the stage's own barrier and reads no scale before
-  // its first accumulator wait of the stage.
-  const uint8_t *st = nullptr;
-  float dws[kGemmStageBlocks][kRt];
+  // The stage's scale tiles arrive with its operands (same transaction barrier), and an MMA warp
+  // issues a block's MMAs only after that barrier has completed; so when an accumulator barrier of
+  // this stage has completed, the scale tiles are in shared memory.  The epilogue therefore does not
+  // wait on the stage's own barrier and reads no scale before its first accumulator wait of the stage.
+  float4 dw_next[kRt];
   auto open_stage = [&]() {
     st = c.stages + static_cast<size_t>(c.ps.stage) * Plan::kStageBytes;
 #pragma unroll
-    for (int r = 0; r < kRt; ++r) {
-      const float4 dw4 = reinterpret_cast<const float4 *>(st + Plan::kOffDw)[r * kGemmTileRows + row_local];
-      dws[0][r] = dw4.x, dws[1][r] = dw4.y, dws[2][r] = dw4.z, dws[3][r] = dw4.w;
-    }
+    for (int r = 0; r < kRt; ++r)
+      dw_next[r] = reinterpret_cast<const float4 *>(st + Plan::kOffDw)[r * kGemmTileRows + row_local];
   };
-  auto close_stage = [&]() {  // this warp no longer needs the stage's scale tiles
+  // All accumulators of the stage have been waited for, so its MMAs have read its operands, and this
+  // warp has requested its last scales (reads that an arrive is ordered behind).
+  auto close_stage = [&]() {
     __syncwarp();
-    if (lane == 0)
-      mbar_arrive(&c.smem_empty[c.ps.stage]);
+    mbar_arrive_if(&c.smem_empty[c.ps.stage], lane == 0);
     c.ps.advance(kStages);
   };
-  // the activation scales of chunk i into a buffer, from the stage `at`: column c of an item is column
-  // c % kBoxCols of box c / kBoxCols
-  constexpr int kScaleVecs = Shape::kChunkCols / 4;
-  ulonglong2 xd[2][kScaleVecs];
-  auto load_scales = [&](const uint8_t *at, uint32_t i, uint32_t buffer) {
-    const uint32_t block = i / Shape::kBlockChunks;
-    const uint32_t col = colgroup * kCpw + i % Shape::kBlockChunks * Shape::kChunkCols;
-    const uint8_t *dx = at + Plan::kOffDx + col / Plan::kBoxCols * Plan::kDxBoxBytes + col % Plan::kBoxCols * 4;
+  // chunk i of the stage, from TMEM into a buffer
+  auto load_chunk = [&](uint32_t i, uint32_t buffer) {
 #pragma unroll
-    for (int j = 0; j < kScaleVecs; ++j)
-      xd[buffer][j] = reinterpret_cast<const ulonglong2 *>(dx + block * (Plan::kBoxCols * 4))[j];
+    for (int b = 0; b < Shape::kChunkBlocks; ++b) {
+      const uint32_t at =
+          (Shape::chunk_block(i) + b) % Shape::kHandover * Shape::kBlockCols + Shape::chunk_col(i);
+#pragma unroll
+      for (int r = 0; r < kRt; ++r)
+        tmem_ld_32x32b<Shape::kChunkCols>(tmem_at + at + r * Shape::kCols, v[buffer] + (b * kRt + r) * Shape::kChunkCols);
+    }
+  };
+  // the activation scales of chunk i into a buffer: column c of an item is column c % kBoxCols of box
+  // c / kBoxCols
+  auto load_scales = [&](uint32_t i, uint32_t buffer) {
+    const uint32_t col = colgroup * kCpw + Shape::chunk_col(i);
+    const uint8_t *dx = st + Plan::kOffDx + col / Plan::kBoxCols * Plan::kDxBoxBytes + col % Plan::kBoxCols * 4;
+#pragma unroll
+    for (int b = 0; b < Shape::kChunkBlocks; ++b)
+#pragma unroll
+      for (int j = 0; j < kScaleVecs; ++j)
+        xd[buffer][b * kScaleVecs + j] =
+            reinterpret_cast<const ulonglong2 *>(dx + (Shape::chunk_block(i) + b) * (Plan::kBoxCols * 4))[j];
   };
   auto fold_chunk = [&](uint32_t i, uint32_t buffer) {
-    fold_part<Shape, kRepack>(v[buffer], acc, i % Shape::kBlockChunks * Shape::kChunkCols, dws[i / Shape::kBlockChunks],
-                              xd[buffer]);
+#pragma unroll
+    for (int b = 0; b < Shape::kChunkBlocks; ++b) {
+      const uint32_t block = Shape::chunk_block(i) + b;
+      float d[kRt];
+#pragma unroll
+      for (int r = 0; r < kRt; ++r)
+        d[r] = block == 0 ? dw[r].x : block == 1 ? dw[r].y : block == 2 ? dw[r].z : dw[r].w;
+      fold_part<Shape, kRepack>(v[buffer] + b * kRt * Shape::kChunkCols, acc, Shape::chunk_col(i), d,
+                                xd[buffer] + b * kScaleVecs);
+    }
   };
-  // All stages but the last are whole.  Their chunks are software-pipelined: while one is folded the
-  // next is on its way from TMEM, across hand-overs and stages, so neither the barrier test nor the
-  // load's latency stands between two folds.
-  if (!load_chunk(0, 0))
+  // The chunks are software-pipelined: while one is folded the next, and its scales, are on their
+  // way, across hand-overs and stages, so neither the barrier test nor the loads' latency stands
+  // between two folds.  A stage is always folded whole: blocks past the last one were read as zeros and
+  // add +0 (an accumulator is never -0: it starts as +0 and x + -x is +0).
+  if (!open_handover())
     return false;
-  for (uint32_t kb = 0; kb + 1 < nkb; ++kb) {
-    open_stage();
+  open_stage();
+  load_chunk(0, 0);
+  load_scales(0, 0);
+  for (uint32_t kb = 0; kb < nkb; ++kb) {
+#pragma unroll
+    for (int r = 0; r < kRt; ++r)
+      dw[r] = dw_next[r];
 #pragma unroll
     for (uint32_t i = 0; i < Shape::kChunks; ++i) {
-      load_scales(st, i, i & 1);
+      const bool last_of_handover = (i + 1) % Shape::kHandoverChunks == 0;
+      if (last_of_handover)
+        peek_handover();
+      if (i + 1 < Shape::kChunks)
+        load_scales(i + 1, (i + 1) & 1);
       tmem_ld_wait();
-      if ((i + 1) % Shape::kHandoverChunks == 0)
-        release_tmem();
-      if (!load_chunk((i + 1) % Shape::kChunks, (i + 1) & 1))
-        return false;
+      if (last_of_handover)
+        release_handover();
+      if (i + 1 < Shape::kChunks) {
+        if (last_of_handover && !open_handover())
+          return false;
+        load_chunk(i + 1, (i + 1) & 1);
+      } else {
+        close_stage();
+        if (kb + 1 < nkb) {
+          if (!open_handover())
+            return false;
+          open_stage();
+          load_chunk(0, 0);
+          load_scales(0, 0);
+        }
+      }
       fold_chunk(i, i & 1);
     }
-    close_stage();
   }
-  open_stage();
-  const uint32_t steps = a.nb - (nkb - 1) * kGemmStageBlocks;
-#pragma unroll
-  for (uint32_t i = 0; i < Shape::kChunks; ++i) {
-    if (i / Shape::kBlockChunks < steps) {
-      if (i > 0 && !load_chunk(i, 0))
-        return false;
-      load_scales(st, i, 0);
-      tmem_ld_wait();
-      if ((i + 1) % Shape::kHandoverChunks == 0 || (i + 1) / Shape::kBlockChunks >= steps)
-        release_tmem();
-      fold_chunk(i, 0);
-    }
-  }
-  close_stage();
 
   // ---- store: this thread owns kCpw consecutive outputs of kRt weight rows
   if constexpr (kMulti) {
@@ -463,7 +504,7 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
   return true;
 }
 
-// One work item for the (converged) MMA warp.  Returns false after a failed wait.
+// One work item for a (converged) MMA warp.  Returns false after a failed wait.
 template <typename Plan, typename Shape, int kStages>
 __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx &c, uint32_t stage_base_addr,
                                               bool leader) {
@@ -472,7 +513,6 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
   for (uint32_t kb = 0; kb < nkb; ++kb) {
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_full[c.ps.stage], c.ps.phase, c.abort_flag)))
       return false;
-    tcgen05_fence_after_thread_sync();
     // Operand descriptors of the stage's first block; a block further along K is 32 bytes
     // further inside the 128-byte swizzled rows, i.e. +2 in the descriptor's 16-byte
     // address field.
@@ -480,10 +520,9 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
     const uint64_t da0 = umma_desc_k_major_sw128(a_addr);
     const uint64_t dl0 = umma_desc_k_major_sw128(a_addr + Plan::kOffB);
     const uint64_t dh0 = umma_desc_k_major_sw128(a_addr + Plan::kOffB + Plan::kPlaneBytes);
-    const uint32_t steps = min(static_cast<uint32_t>(kGemmStageBlocks), a.nb - kb * kGemmStageBlocks);
 #pragma unroll
     for (uint32_t kk = 0; kk < kGemmStageBlocks; kk += Shape::kHandover) {
-      if (kk < steps) {
+      if (c.ts.stage % kGemmMmaWarps == c.mma_warp) {
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.tmem_empty[c.ts.stage], c.ts.phase ^ 1, c.abort_flag)))
           return false;
         tcgen05_fence_after_thread_sync();
@@ -491,27 +530,22 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
         if (leader) {
 #pragma unroll
           for (uint32_t h = 0; h < Shape::kHandover; ++h) {
-            if (kk + h < steps) {
-              const uint64_t off = (kk + h) * kStep;
+            const uint64_t off = (kk + h) * kStep;
 #pragma unroll
-              for (uint32_t r = 0; r < Shape::kRowTiles; ++r) {
-                const uint32_t d_tmem = c.tmem_base + c.ts.stage * Plan::kTmemStageCols +
-                                        (h * Shape::kRowTiles + r) * Shape::kCols;
-                const uint64_t da = da0 + off + r * (Plan::kATileBytes >> 4);
-                umma_f8_first(d_tmem, da, dl0 + off, idesc);
-                umma_f8_again(d_tmem, da, dh0 + off, idesc);
-              }
+            for (uint32_t r = 0; r < Shape::kRowTiles; ++r) {
+              const uint32_t d_tmem = c.tmem_base + c.ts.stage * Plan::kTmemStageCols +
+                                      (h * Shape::kRowTiles + r) * Shape::kCols;
+              const uint64_t da = da0 + off + r * (Plan::kATileBytes >> 4);
+              umma_f8_first(d_tmem, da, dl0 + off, idesc);
+              umma_f8_again(d_tmem, da, dh0 + off, idesc);
             }
           }
           umma_commit(&c.tmem_full[c.ts.stage]);
         }
         __syncwarp();
-        c.ts.advance(Plan::kTmemStages);
       }
+      c.ts.advance(Plan::kTmemStages);
     }
-    if (leader)
-      umma_commit(&c.smem_empty[c.ps.stage]);
-    __syncwarp();
     c.ps.advance(kStages);
   }
   return true;
@@ -545,20 +579,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   c.out_stage = c.stages + static_cast<size_t>(kStages) * Plan::kStageBytes;  // 1024-byte aligned
   c.store_syncs = 0;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (shuffled, so that the compiler knows them to be the same for the whole warp)
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&c.smem_full[i], 1);
-      mbar_init(&c.smem_empty[i], 1 + kGemmEpilogueWarps);  // MMA commit + every epilogue warp
+      mbar_init(&c.smem_empty[i], kGemmEpilogueWarps);
     }
     for (int i = 0; i < Plan::kTmemStages; ++i) {
       mbar_init(&c.tmem_full[i], 1);
       mbar_init(&c.tmem_empty[i], kGemmEpilogueWarps);
     }
-    mbar_init(drain_bar, 1);
+    mbar_init(drain_bar, kGemmMmaWarps);
     mbar_init(c.store_bar, kGemmEpilogueWarps);
     *c.abort_flag = 0;
     mbar_fence_init();
@@ -570,21 +605,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   tcgen05_fence_before_thread_sync();
   __syncthreads();
   tcgen05_fence_after_thread_sync();
-  c.tmem_base = *tmem_base_slot;
+  c.tmem_base = __shfl_sync(0xffffffffu, *tmem_base_slot, 0);
   // Programmatic dependent launch: everything above touched only this CTA's shared memory and
   // TMEM, so it may overlap the tail of the preceding kernel (the activation unpack); operands
   // are read and outputs written only after that kernel has completed.
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   bool ok = true;
-  if (warp == kGemmEpilogueWarps) {
-    // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      prefetch_tensormap(&map_w);
-      prefetch_tensormap(&map_x);
-      prefetch_tensormap(&map_xhi);
-      prefetch_tensormap(&map_dw);
-      prefetch_tensormap(&map_dx);
+  if (warp >= kGemmEpilogueWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kGemmOtherRegs));
+    // In these roles the whole warp walks the loop and one elected lane issues.  Coordinates and operand
+    // descriptors live in uniform registers; computed in code that the compiler knows to be converged
+    // they are there already, while a single-lane branch had to move them across: 85 cycles per MMA,
+    // 340 per commit and 780 for the five copies of a 128 x 32 stage.
+    const bool leader = elect_one();
+    if (warp == kGemmEpilogueWarps) {
+      // ------------------------------ TMA producer ------------------------------
+      if (leader) {
+        prefetch_tensormap(&map_w);
+        prefetch_tensormap(&map_x);
+        prefetch_tensormap(&map_xhi);
+        prefetch_tensormap(&map_dw);
+        prefetch_tensormap(&map_dx);
+      }
+      __syncwarp();
       PipeState ps;
       uint32_t issued = 0;
       for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
@@ -597,65 +641,67 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const uint32_t tx = row_tiles * (Plan::kATileBytes + Plan::kDwTileBytes) +
                             boxes * (2 * Plan::kBoxBytes + Plan::kDxBoxBytes);
         for (uint32_t kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait_bounded(&c.smem_empty[ps.stage], ps.phase ^ 1, c.abort_flag);
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_empty[ps.stage], ps.phase ^ 1, c.abort_flag));
           if (!ok)
             break;
-          uint8_t *st = c.stages + static_cast<size_t>(ps.stage) * Plan::kStageBytes;
-          uint64_t *bar = &c.smem_full[ps.stage];
-          mbar_arrive_expect_tx(bar, tx);
-          const int kbyte = static_cast<int>(kb) * kGemmStageBlocks * kQK;
-          const int kblk = static_cast<int>(kb) * kGemmStageBlocks;
-          for (int r = 0; r < row_tiles; ++r) {
-            // (a second tile that starts past the last row reads as zeros)
-            tma_load_2d(st + r * Plan::kATileBytes, &map_w, kbyte, n0 + r * kGemmTileRows, bar);
-            tma_load_2d(st + Plan::kOffDw + r * Plan::kDwTileBytes, &map_dw, kblk, n0 + r * kGemmTileRows, bar);
+          if (leader) {
+            uint8_t *st = c.stages + static_cast<size_t>(ps.stage) * Plan::kStageBytes;
+            uint64_t *bar = &c.smem_full[ps.stage];
+            mbar_arrive_expect_tx(bar, tx);
+            const int kbyte = static_cast<int>(kb) * kGemmStageBlocks * kQK;
+            const int kblk = static_cast<int>(kb) * kGemmStageBlocks;
+            for (int r = 0; r < row_tiles; ++r) {
+              // (a second tile that starts past the last row reads as zeros)
+              tma_load_2d(st + r * Plan::kATileBytes, &map_w, kbyte, n0 + r * kGemmTileRows, bar);
+              tma_load_2d(st + Plan::kOffDw + r * Plan::kDwTileBytes, &map_dw, kblk, n0 + r * kGemmTileRows, bar);
+            }
+            for (int b = 0; b < boxes; ++b) {
+              const int mb = m0 + b * Plan::kBoxCols;
+              tma_load_2d(st + Plan::kOffB + b * Plan::kBoxBytes, &map_x, kbyte, mb, bar);
+              tma_load_2d(st + Plan::kOffB + Plan::kPlaneBytes + b * Plan::kBoxBytes, &map_xhi, kbyte, mb, bar);
+              tma_load_2d(st + Plan::kOffDx + b * Plan::kDxBoxBytes, &map_dx, mb, kblk, bar);
+            }
           }
-          for (int b = 0; b < boxes; ++b) {
-            const int mb = m0 + b * Plan::kBoxCols;
-            tma_load_2d(st + Plan::kOffB + b * Plan::kBoxBytes, &map_x, kbyte, mb, bar);
-            tma_load_2d(st + Plan::kOffB + Plan::kPlaneBytes + b * Plan::kBoxBytes, &map_xhi, kbyte, mb, bar);
-            tma_load_2d(st + Plan::kOffDx + b * Plan::kDxBoxBytes, &map_dx, mb, kblk, bar);
-          }
+          __syncwarp();
           ps.advance(kStages);
           ++issued;
         }
       }
-      if (!ok) {
+      if (!ok && leader) {
         *c.abort_flag = 1;
-        raise_device_error(kDevErrBarrierTimeout);
+        raise_device_error(a.errors, kDevErrBarrierTimeout);
       }
+      __syncwarp();
       if (*c.abort_flag != 0) {
         // winding down after a failed wait: let this CTA's own copies land before it exits
         const uint32_t first = issued > kStages ? issued - kStages : 0;
         for (uint32_t i = first; i < issued; ++i)
           (void)mbar_wait_bounded(&c.smem_full[i % kStages], (i / kStages) & 1, nullptr);
       }
+    } else if (warp <= kGemmEpilogueWarps + kGemmMmaWarps) {
+      // ------------------------------ MMA issuers ------------------------------
+      // Two warps take turns at the TMEM stages: one warp's wait, wait, issue and commit for a hand-over
+      // (640 cycles) is longer than what eight MMAs take (240 to 300).
+      c.mma_warp = static_cast<uint32_t>(warp - kGemmEpilogueWarps - 1);
+      for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
+        const GemmItem it = gemm_item<kNarrow>(a, idx);
+        if (it.n0 >= a.nr || it.m0 >= a.nc)
+          continue;
+        ok = it.whole ? gemm_mma_item<Plan, Full, kStages>(a, c, stage_base_addr, leader)
+                      : gemm_mma_item<Plan, Half, kStages>(a, c, stage_base_addr, leader);
+      }
+      if (!ok && leader) {
+        *c.abort_flag = 1;
+        raise_device_error(a.errors, kDevErrBarrierTimeout);
+      }
+      // every MMA issued above must have finished before TMEM is released
+      if (leader)
+        umma_commit(drain_bar);
+      __syncwarp();
+      (void)mbar_wait_bounded(drain_bar, 0, nullptr);
     }
-  } else if (warp == kGemmEpilogueWarps + 1) {
-    // ------------------------------ MMA issuer ------------------------------
-    // The whole warp walks the loop and one elected lane issues.  Operand descriptors live in uniform
-    // registers; computed in code that the compiler knows to be converged they are there already,
-    // while a single-lane branch had to move six values per MMA across: 85 cycles per MMA and 340
-    // per commit, which bounded every shape's hand-overs.  (128 x 128 items without the fold: 204 ->
-    // 169 us on 512 x 32000 x 4096.)
-    const bool leader = elect_one();
-    for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
-      const GemmItem it = gemm_item<kNarrow>(a, idx);
-      if (it.n0 >= a.nr || it.m0 >= a.nc)
-        continue;
-      ok = it.whole ? gemm_mma_item<Plan, Full, kStages>(a, c, stage_base_addr, leader)
-                    : gemm_mma_item<Plan, Half, kStages>(a, c, stage_base_addr, leader);
-    }
-    if (!ok && leader) {
-      *c.abort_flag = 1;
-      raise_device_error(kDevErrBarrierTimeout);
-    }
-    // every MMA issued above must have finished before TMEM is released
-    if (leader)
-      umma_commit(drain_bar);
-    __syncwarp();
-    (void)mbar_wait_bounded(drain_bar, 0, nullptr);
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kGemmEpilogueRegs));
     // ------------------------------ epilogue warps ------------------------------
     for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
       const GemmItem it = gemm_item<kNarrow>(a, idx);
@@ -670,7 +716,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       bulk_store_wait_all();  // the staging tile must outlive the copies that read it
     if (!ok && lane == 0) {
       *c.abort_flag = 1;
-      raise_device_error(kDevErrBarrierTimeout);
+      raise_device_error(a.errors, kDevErrBarrierTimeout);
     }
   }
 

@@ -109,21 +109,10 @@ __device__ __forceinline__ void umma_f8_again(uint32_t tmem_d, uint64_t desc_a, 
       : "memory");
 }
 
-// 32 lanes x N consecutive 32-bit columns (N = 8 or 16) into v[0..N): thread i of the warp
+// 32 lanes x N consecutive 32-bit columns (N = 16 or 32) into v[0..N): thread i of the warp
 // receives lane (base+i).
 template <int N>
 __device__ __forceinline__ void tmem_ld_32x32b(uint32_t taddr, uint32_t *v);
-
-template <>
-__device__ __forceinline__ void tmem_ld_32x32b<8>(uint32_t taddr, uint32_t *v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7])
-      : "r"(taddr)
-      : "memory");
-}
 
 template <>
 __device__ __forceinline__ void tmem_ld_32x32b<16>(uint32_t taddr, uint32_t *v) {
@@ -133,6 +122,22 @@ __device__ __forceinline__ void tmem_ld_32x32b<16>(uint32_t taddr, uint32_t *v) 
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
         "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
         "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+template <>
+__device__ __forceinline__ void tmem_ld_32x32b<32>(uint32_t taddr, uint32_t *v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, "
+      "%8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, "
+      "%24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr)
       : "memory");
 }

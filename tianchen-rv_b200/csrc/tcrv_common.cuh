@@ -16,23 +16,36 @@ constexpr int kQ8Block = TCRV_Q8_0_BLOCK_BYTES;
 constexpr int kNumSMsB200 = 148;
 
 // Device-side error word: kernels with bounded waits OR a code into it when a wait
-// expires.  Read and cleared by tcrv_cuda_check_device_errors().
-extern __device__ int g_device_error;
-// Optional mirror of the error word in mapped host memory (set by the host-pointer layer, null
-// otherwise): a failed wait also stores its code there, so a synchronous caller learns of it
-// from the stream synchronisation it does anyway instead of a device-to-host copy per call.
-extern __device__ int *g_host_error_mirror;
+// expires.  Read and cleared by tcrv_cuda_check_device_errors().  An optional mirror of it in mapped
+// host memory (set by the host-pointer layer, null otherwise) gets the code too, so a synchronous
+// caller learns of a failed wait from the stream synchronisation it does anyway instead of a
+// device-to-host copy per call.
+struct DeviceErrorWords {
+  int *word;
+  int **mirror;
+};
 constexpr int kDevErrBarrierTimeout = 1;
 
 // What a kernel calls when one of its bounded waits expires.
-__device__ __forceinline__ void raise_device_error(int code) {
-  atomicOr(&g_device_error, code);
-  int *mirror = g_host_error_mirror;
+__device__ __forceinline__ void raise_device_error(const DeviceErrorWords &w, int code) {
+  atomicOr(w.word, code);
+  int *mirror = *w.mirror;
   if (mirror != nullptr) {
     *reinterpret_cast<volatile int *>(mirror) = code;
     __threadfence_system();
   }
 }
+
+#ifdef __CUDACC_RDC__
+extern __device__ int g_device_error;
+extern __device__ int *g_host_error_mirror;
+__device__ __forceinline__ void raise_device_error(int code) {
+  raise_device_error(DeviceErrorWords{&g_device_error, &g_host_error_mirror}, code);
+}
+#endif
+// The words' addresses on the current device, for kernels that are compiled without relocatable device
+// code (gemm.cu) and get them as an argument.
+int device_error_words(DeviceErrorWords *out);
 
 // Records a failing CUDA runtime call for tcrv_cuda_last_error_text().
 int record_cuda_error(cudaError_t err, const char *what);
