@@ -201,76 +201,45 @@ inline bool multiple_of(const void *p, uintptr_t m) { return reinterpret_cast<ui
 constexpr size_t kMmaMinCols = 4;
 constexpr int kAnyMinRows = 8;
 
-// Ring depth of the tensor-core GEMV for a row of nb blocks with `groups` 16-row groups per
-// slot, 0 if it does not fit.
+// Whether the chunk-wise tensor-core kernel takes these rows.  Its order (16-way K split) is what such calls
+// promise (gemv_fold_order), so the line stays where it was first drawn, by what fitted into shared memory:
+// 12288 elements of Q4_0, 5888 of Q8_0.  (A lane's 32-bit offsets reach over the 16 rows of a group.)
 template <bool kQ8W>
-size_t mma_slots(uint32_t nb, int groups) {
-  const size_t fixed = kMmaBarrierBytes + kMmaPartialBytes + static_cast<size_t>(nb) * kMmaXBytesPerBlock;
-  const size_t slot = static_cast<size_t>(kMmaRows * groups) * kMmaChunkBlocks * WeightFormat<kQ8W>::kBlockBytes;
-  if (fixed + 2 * kMmaWarps * slot > kMaxDynamicSmem)
-    return 0;
-  size_t spw = (kMaxDynamicSmem - fixed) / (kMmaWarps * slot);
-  return spw > kMmaMaxSlots ? kMmaMaxSlots : spw;
-}
-
-// Groups per slot: two when at least two such slots per warp fit, else one; 0 = no fit at all.
-template <bool kQ8W>
-int mma_groups(uint32_t nb) {
-  if (mma_slots<kQ8W>(nb, 2) >= 2)
-    return 2;
-  return mma_slots<kQ8W>(nb, 1) >= 2 ? 1 : 0;
+bool mma_chunks_take(uint32_t nb, size_t bx) {
+  constexpr uint32_t kMaxBlocks = kQ8W ? 184 : 384;
+  static_assert(kMmaMaxBlocks<kQ8W> >= kMaxBlocks, "chunks of a warp");
+  return nb <= kMaxBlocks && bx < (size_t{1} << 27);
 }
 
 template <bool kQ8W>
 int launch_mma(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t by, size_t nr, size_t nc, size_t bx,
-               size_t bs, unsigned flags, int slot_groups, cudaStream_t stream) {
-  constexpr int WB = WeightFormat<kQ8W>::kBlockBytes;
-  const int kMmaSlotRows = kMmaRows * slot_groups;
-  const uint32_t nb = static_cast<uint32_t>(n / kQK);
-  const size_t spw = mma_slots<kQ8W>(nb, slot_groups);
-  CUtensorMap map;
-  const int st = encode_tensor_map_2d_u16(&map, vx, static_cast<uint64_t>(nb) * WB / 2, nr, bx,
-                                          kMmaChunkBlocks * WB / 2, kMmaSlotRows);
-  if (st != TCRV_CUDA_OK)
-    return st;
+               size_t bs, unsigned flags, cudaStream_t stream) {
   GemvMmaArgs args;
+  args.vx = vx;
   args.vy = vy;
   args.s = s;
+  args.bx = bx;
   args.by = by;
   args.bs = bs;
   args.nr = static_cast<uint32_t>(nr);
   args.nc = static_cast<uint32_t>(nc);
-  args.nb = nb;
-  args.slots = static_cast<uint32_t>(spw);
+  args.nb = static_cast<uint32_t>(n / kQK);
   args.static_weights = (flags & TCRV_CUDA_FLAG_STATIC_WEIGHTS) ? 1u : 0u;
-  const size_t smem = kMmaBarrierBytes + kMmaPartialBytes + static_cast<size_t>(nb) * kMmaXBytesPerBlock +
-                      spw * kMmaWarps * kMmaSlotRows * kMmaChunkBlocks * WB;
-  // rows of at most 16 chunks: one chunk per warp, activation fragments live in registers
-  const bool xregs = nb <= static_cast<uint32_t>(kMmaWarps * kMmaChunkBlocks);
-  auto kernel = slot_groups == 2 ? (xregs ? gemv_mma_kernel<kQ8W, true, 2> : gemv_mma_kernel<kQ8W, false, 2>)
-                                 : (xregs ? gemv_mma_kernel<kQ8W, true, 1> : gemv_mma_kernel<kQ8W, false, 1>);
-  static std::atomic<bool> configured[64][4];
+  args.x_aligned = multiple_of(vy, 16) && (nc == 1 || by % 16 == 0) ? 1u : 0u;
+  static_assert(kMmaSmemBytes<kQ8W> <= kMaxDynamicSmem, "two ring positions per warp");
+  static std::atomic<bool> configured[64];
   int dev = 0;
   TCRV_CUDA_TRY(cudaGetDevice(&dev));
-  const int variant = (xregs ? 1 : 0) + (slot_groups == 2 ? 2 : 0);
-  if (dev < 64 && !configured[dev][variant]) {
-    TCRV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(kMaxDynamicSmem)));
-    configured[dev][variant] = true;
+  if (dev < 64 && !configured[dev]) {
+    TCRV_CUDA_TRY(cudaFuncSetAttribute(gemv_mma_kernel<kQ8W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kMmaSmemBytes<kQ8W>));
+    configured[dev] = true;
   }
-  const size_t groups = (nr + kMmaSlotRows - 1) / kMmaSlotRows;
-  const int sms = sm_count();
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(groups < static_cast<size_t>(sms) ? groups : sms));
-  cfg.blockDim = dim3(kMmaThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  TCRV_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map, args));
+  // as many groups for every CTA as the most loaded one has to take: no more CTAs than that fetch the columns
+  const size_t groups = (nr + kMmaRows - 1) / kMmaRows, sms = static_cast<size_t>(sm_count());
+  const size_t share = (groups + sms - 1) / sms;
+  TCRV_CUDA_TRY(launch_pdl(gemv_mma_kernel<kQ8W>, static_cast<int>((groups + share - 1) / share), kMmaThreads,
+                           kMmaSmemBytes<kQ8W>, stream, args));
   return TCRV_CUDA_OK;
 }
 
@@ -522,7 +491,8 @@ int gemv_fold_order(size_t n, size_t nc, const void *vx, size_t bx, const void *
     return TCRV_CUDA_ORDER_STRICT;
   const bool bulk = nb > 0 && nb % 8 == 0 && nc <= kGemvMaxCols && multiple_of(vx, 16) && bx % 16 == 0 &&
                     multiple_of(vy, 2) && by % 2 == 0;
-  if (bulk && (nc >= kMmaMinCols || (flags & 0x4000u) != 0) && (flags & 0x1000u) == 0 && mma_groups<kQ8W>(nb) > 0)
+  if (bulk && (nc >= kMmaMinCols || (flags & 0x4000u) != 0) && (flags & 0x1000u) == 0 &&
+      (mma_rows_ring<kQ8W>(nb) >= 2 || mma_chunks_take<kQ8W>(nb, bx)))
     return TCRV_CUDA_ORDER_KSPLIT16;
   return TCRV_CUDA_ORDER_LANE_PAIRS;
 }
@@ -557,12 +527,11 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
     // Many activation columns: the tensor-core kernel (measured faster from about 4 columns
     // on; flags bit 12 keeps the dp4a kernel, bit 14 takes this one for any column count: tuning).
     if ((nc >= kMmaMinCols || (flags & 0x4000u) != 0) && (flags & 0x1000u) == 0) {
-      // rows of up to 4096 elements come in as whole rows (flags bit 13 keeps the tiled form: tuning)
+      // rows of up to 4096 elements come in as whole rows (flags bit 13 keeps the chunk-wise form: tuning)
       if ((flags & 0x2000u) == 0 && mma_rows_ring<kQ8W>(nb) >= 2)
         return launch_mma_rows<kQ8W>(n, s, vx, vy, by, nr, nc, bx, bs, flags, stream);
-      const int slot_groups = mma_groups<kQ8W>(nb);
-      if (slot_groups > 0)
-        return launch_mma<kQ8W>(n, s, vx, vy, by, nr, nc, bx, bs, flags, slot_groups, stream);
+      if (mma_chunks_take<kQ8W>(nb, bx))
+        return launch_mma<kQ8W>(n, s, vx, vy, by, nr, nc, bx, bs, flags, stream);
     }
     StreamPlan plan;
     if (plan_stream_fast<kQ8W>(nb, s, vx, vy, by, nr, nc, bx, bs, flags, plan))

@@ -61,17 +61,6 @@ struct GemvRowsArgs {
   uint32_t x_aligned;       // vy and by are multiples of 16: the columns can be fetched in 16-byte pieces
 };
 
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ unsigned short lds_u16(uint32_t addr) {
-  unsigned short v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return v;
-}
-
 // The producer warp of the whole-row kernels: lane p brings row pair p of every 16-row unit
 // (units first_unit .. first_unit + nunits - 1 of the matrix) into ring position h % ring as soon
 // as all 16 consumer warps have handed the position back.  On a failed wait it raises the
@@ -120,9 +109,7 @@ __device__ __forceinline__ void rows_producer(const GemvRowsArgs &a, uint8_t *un
 
 // Activation fragments of one MMA warp for its K chunk (blocks 8 * warp .. 8 * warp + 7): for
 // thread (g = lane / 4, t = lane % 4) the two quant words of column g (`b0`, `b1`: the MMA's B
-// operand), the scale of column g (`dcol`) and -8 * sum(q) of columns 2t and 2t+1 (`sx`: the
-// MMA's C operand for Q4_0, summed over the quad that holds column g and fetched from the quads
-// of columns 2t, 2t+1).  Columns beyond a.nc are zero.  With 16-byte aligned columns the warp's
+// operand) and the scale of column g (`dcol`, see mma_act_scale).  Columns beyond a.nc are zero.  With 16-byte aligned columns the warp's
 // share of them (272 contiguous bytes of each) is first copied to `stage` (2176 bytes of shared
 // memory, this warp's own) in 16-byte pieces, all requested at once: picking the 2-byte aligned
 // words out of global memory directly took 48 small loads per thread in several dependent
@@ -130,9 +117,9 @@ __device__ __forceinline__ void rows_producer(const GemvRowsArgs &a, uint8_t *un
 struct RowsXFragments {
   uint32_t b0[kMmaChunkBlocks], b1[kMmaChunkBlocks];
   float dcol[kMmaChunkBlocks];
-  int2 sx[kMmaChunkBlocks];
 };
 
+template <bool kQ8W>
 __device__ __forceinline__ void rows_load_x_fragments(const GemvRowsArgs &a, uint32_t warp, int lane, uint8_t *stage,
                                                       RowsXFragments &x) {
   const int g = lane >> 2, t = lane & 3;
@@ -161,7 +148,7 @@ __device__ __forceinline__ void rows_load_x_fragments(const GemvRowsArgs &a, uin
       const uint32_t blk = mine + bi * kQ8Block + 2 + 4 * t;
       x.b0[bi] = static_cast<uint32_t>(lds_u16(blk)) | (static_cast<uint32_t>(lds_u16(blk + 2)) << 16);
       x.b1[bi] = static_cast<uint32_t>(lds_u16(blk + 16)) | (static_cast<uint32_t>(lds_u16(blk + 18)) << 16);
-      x.dcol[bi] = half_bits_to_float(lds_u16(mine + bi * kQ8Block));
+      x.dcol[bi] = mma_act_scale<kQ8W>(half_bits_to_float(lds_u16(mine + bi * kQ8Block)));
     }
   } else {
 #pragma unroll
@@ -170,46 +157,9 @@ __device__ __forceinline__ void rows_load_x_fragments(const GemvRowsArgs &a, uin
       const unsigned short *h = reinterpret_cast<const unsigned short *>(a.vy + g * a.by + off);
       x.b0[bi] = col_ok ? static_cast<uint32_t>(h[1 + 2 * t]) | (static_cast<uint32_t>(h[2 + 2 * t]) << 16) : 0u;
       x.b1[bi] = col_ok ? static_cast<uint32_t>(h[9 + 2 * t]) | (static_cast<uint32_t>(h[10 + 2 * t]) << 16) : 0u;
-      x.dcol[bi] = col_ok ? half_bits_to_float(h[0]) : 0.0f;
+      x.dcol[bi] = col_ok ? mma_act_scale<kQ8W>(half_bits_to_float(h[0])) : 0.0f;
     }
   }
-#pragma unroll
-  for (int bi = 0; bi < kMmaChunkBlocks; ++bi) {
-    int sum = __dp4a(static_cast<int>(x.b0[bi]), 0x01010101, __dp4a(static_cast<int>(x.b1[bi]), 0x01010101, 0));
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    x.sx[bi].x = -8 * __shfl_sync(0xffffffffu, sum, 8 * t);
-    x.sx[bi].y = -8 * __shfl_sync(0xffffffffu, sum, 8 * t + 4);
-  }
-}
-
-// The MMA's A operand for block `bi` of a chunk: rows at shared-window addresses `row_lo` and
-// `row_hi` (the chunk's first byte in each), thread column t; also the two rows' block scales.
-// Bytes 2.. of a block are 4-byte aligned for odd bi and off by two for even bi (bi is a
-// constant after unrolling).  Q4_0 nibbles come out unsigned.
-template <bool kQ8W>
-__device__ __forceinline__ void rows_load_a_fragment(uint32_t row_lo, uint32_t row_hi, int bi, int t,
-                                                     uint32_t (&afrag)[4], float &dw_lo, float &dw_hi) {
-  constexpr int WB = WeightFormat<kQ8W>::kBlockBytes;
-  auto load_row = [&](uint32_t row, uint32_t &k_lo, uint32_t &k_hi, float &dw) {
-    const uint32_t blk = row + bi * WB;
-    dw = half_bits_to_float(lds_u16(blk));
-    auto word_at = [&](int byte_off) -> uint32_t {  // the 4 bytes at blk + 2 + byte_off
-      if ((bi & 1) != 0)
-        return lds_u32(blk + 2 + byte_off);
-      return __funnelshift_r(lds_u32(blk + byte_off), lds_u32(blk + byte_off + 4), 16);
-    };
-    if constexpr (kQ8W) {
-      k_lo = word_at(4 * t);
-      k_hi = word_at(16 + 4 * t);
-    } else {
-      const uint32_t qw = word_at(4 * t);
-      k_lo = qw & 0x0f0f0f0fu;
-      k_hi = (qw >> 4) & 0x0f0f0f0fu;
-    }
-  };
-  load_row(row_lo, afrag[0], afrag[2], dw_lo);
-  load_row(row_hi, afrag[1], afrag[3], dw_hi);
 }
 
 template <bool kQ8W, int kGroups>
@@ -271,7 +221,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_mma_rows_kernel(const Ge
   uint64_t xdx[kMmaChunkBlocks];
   const bool active = warp < nchunks;
   if (active) {
-    rows_load_x_fragments(a, warp, lane, reinterpret_cast<uint8_t *>(partial) + warp * kRowsStageWarpBytes, xf);
+    rows_load_x_fragments<kQ8W>(a, warp, lane, reinterpret_cast<uint8_t *>(partial) + warp * kRowsStageWarpBytes, xf);
 #pragma unroll
     for (int bi = 0; bi < kMmaChunkBlocks; ++bi)
       xdx[bi] = mma_pack2(__shfl_sync(0xffffffffu, xf.dcol[bi], 8 * t), __shfl_sync(0xffffffffu, xf.dcol[bi], 8 * t + 4));
@@ -308,13 +258,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_mma_rows_kernel(const Ge
           const uint32_t row_hi = row_lo + a.row_bytes;
           uint32_t afrag[4];
           float dw_lo, dw_hi;
-          rows_load_a_fragment<kQ8W>(row_lo, row_hi, bi, t, afrag, dw_lo, dw_hi);
-          int c[4];
-          // Q4_0: the nibbles enter unsigned; -8 * sum(x) of each column rides in as the MMA's C input
-          if constexpr (kQ8W)
-            mma_m16n8k32_s8(c, afrag, xf.b0[bi], xf.b1[bi], 0, 0);
-          else
-            mma_m16n8k32_s8(c, afrag, xf.b0[bi], xf.b1[bi], xf.sx[bi].x, xf.sx[bi].y);
+          mma_load_a_fragment<kQ8W>(row_lo, row_hi, bi, t, afrag, dw_lo, dw_hi);
+          float c[4];
+          mma_m16n8k32_s8(c, afrag, xf.b0[bi], xf.b1[bi]);
           acc_lo[q] = mma_fold2<kQ8W>(acc_lo[q], c[0], c[1], dw_lo, xdx[bi]);
           acc_hi[q] = mma_fold2<kQ8W>(acc_hi[q], c[2], c[3], dw_hi, xdx[bi]);
         }

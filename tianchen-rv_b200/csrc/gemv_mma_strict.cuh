@@ -9,7 +9,7 @@
 // reference's fold - and drops the 16 x 8 terms of the block into a shared-memory table
 // term[row][block][column].  Four folding warps then run the second half as the reference does:
 // thread <-> (row, column), block after block,
-//   Q4_0:  acc = fma(term, d_x, acc),            term = (float)sumi * d_w
+//   Q4_0:  acc = fma(term, d_x / 16, acc),       term = 16 * ((float)sumi * d_w)
 //   Q8_0:  acc = fma(term, d_w * d_x, acc),      term = (float)sumi
 // so every output has the bits of the sequential fold (lib/Conversion/RVV/
 // RVVToEmitCBlockQuantLinear.cpp:322-356, 7538-7573).  One table, handed over in two halves of
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kStrictMmaThreads, 1) gemv_mma_strict_kernel(c
   RowsXFragments xf;
   const bool active = warp < nchunks;
   if (active) {
-    rows_load_x_fragments(a, warp, lane, reinterpret_cast<uint8_t *>(table) + warp * kRowsStageWarpBytes, xf);
+    rows_load_x_fragments<kQ8W>(a, warp, lane, reinterpret_cast<uint8_t *>(table) + warp * kRowsStageWarpBytes, xf);
     if (t == 0) {  // one lane per column
 #pragma unroll
       for (int bi = 0; bi < kMmaChunkBlocks; ++bi)
@@ -174,35 +174,18 @@ __global__ void __launch_bounds__(kStrictMmaThreads, 1) gemv_mma_strict_kernel(c
       for (int bi = 0; bi < kMmaChunkBlocks; ++bi) {
         uint32_t afrag[4];
         float dw_lo, dw_hi;
-        rows_load_a_fragment<kQ8W>(row_lo, row_hi, bi, t, afrag, dw_lo, dw_hi);
-        int c[4];
-        // Q4_0: the nibbles enter unsigned; -8 * sum(x) of each column rides in as the MMA's C input
-        if constexpr (kQ8W)
-          mma_m16n8k32_s8(c, afrag, xf.b0[bi], xf.b1[bi], 0, 0);
-        else
-          mma_m16n8k32_s8(c, afrag, xf.b0[bi], xf.b1[bi], xf.sx[bi].x, xf.sx[bi].y);
-        // (float)sumi without a conversion instruction (see gemv_mma.cuh), then the order-free
-        // half of the fold: Q4_0 scales by d_w (one rounding), Q8_0 keeps the exact integer
-        const uint64_t b_lo = mma_pack2(__uint_as_float(static_cast<uint32_t>(c[0]) + kMmaMagicBits),
-                                        __uint_as_float(static_cast<uint32_t>(c[1]) + kMmaMagicBits));
-        const uint64_t b_hi = mma_pack2(__uint_as_float(static_cast<uint32_t>(c[2]) + kMmaMagicBits),
-                                        __uint_as_float(static_cast<uint32_t>(c[3]) + kMmaMagicBits));
-        uint64_t t_lo, t_hi;
+        mma_load_a_fragment<kQ8W>(row_lo, row_hi, bi, t, afrag, dw_lo, dw_hi);
+        float c[4];
+        mma_m16n8k32_s8(c, afrag, xf.b0[bi], xf.b1[bi]);
+        // the order-free half of the fold: Q4_0 scales by d_w (one rounding), Q8_0 keeps the exact integer
         if constexpr (kQ8W) {
-          const uint64_t neg = mma_pack2(-kMmaMagic, -kMmaMagic);
-          t_lo = mma_add2(b_lo, neg);
-          t_hi = mma_add2(b_hi, neg);
           if (t == 0) {
             dwt[static_cast<size_t>(g) * pitch + warp * kMmaChunkBlocks + bi] = dw_lo;
             dwt[static_cast<size_t>(g + 8) * pitch + warp * kMmaChunkBlocks + bi] = dw_hi;
           }
-        } else {
-          const float n_lo = __fmul_rn(-kMmaMagic, dw_lo), n_hi = __fmul_rn(-kMmaMagic, dw_hi);
-          t_lo = mma_fma2(b_lo, mma_pack2(dw_lo, dw_lo), mma_pack2(n_lo, n_lo));
-          t_hi = mma_fma2(b_hi, mma_pack2(dw_hi, dw_hi), mma_pack2(n_hi, n_hi));
         }
-        *reinterpret_cast<uint64_t *>(out_lo + bi * kRowsCols) = t_lo;
-        *reinterpret_cast<uint64_t *>(out_hi + bi * kRowsCols) = t_hi;
+        *reinterpret_cast<uint64_t *>(out_lo + bi * kRowsCols) = mma_terms2<kQ8W>(c[0], c[1], dw_lo);
+        *reinterpret_cast<uint64_t *>(out_hi + bi * kRowsCols) = mma_terms2<kQ8W>(c[2], c[3], dw_hi);
       }
     }
     // every lane has read its words of the unit and written its terms

@@ -93,7 +93,4 @@ int launch_gemm_prepared_multi(size_t n, float *const *dst, size_t ndst, const u
 namespace tcrv {
 // Host-pointer layer: clears the current device's mapped mirror of the device error word.
 void host_error_mirror_reset();
-// Tiled TMA descriptor over a matrix of 16-bit elements (rows `row_stride_bytes` apart), no swizzle.
-int encode_tensor_map_2d_u16(CUtensorMap *map, const void *base, uint64_t inner_elems, uint64_t outer,
-                             uint64_t row_stride_bytes, uint32_t box_inner_elems, uint32_t box_outer);
 }  // namespace tcrv
