@@ -97,29 +97,28 @@ __global__ void __launch_bounds__(256) sibling_dot_kernel(const uint8_t *__restr
 }
 
 // Which of the two streaming kernels takes a call that both accept: strict_stream.cuh (a term table per
-// CTA, 512 workers on one slot) or gemv_any.cuh (a table per warp, a row is one warp's work).  The
-// latter wins wherever its lanes and warps have work.  They have not, with more than one slot to a
-// warp, where rows have few items (half of the lanes idle), where it folds one row at a time (more
-// than 4 columns), and where shared memory leaves it few rings.  Measured, us, table per CTA / per warp:
-//   1 column     Q5_0 11008 x 4096 10.6 / 11.7; Q4_1, Q5_1 there 8.5 / 8.4, 10.9 / 10.7; Q5_1 32000 x 256 7.0 / 8.8
-//   2..4         Q5_0 32000 x 512, 3 columns 11.4 / 17.1, x 1280, 2 columns 16.3 / 18.6, 4 columns 23.6 / 21.4;
-//                Q5_1 11008 x 4096, 4 columns 21.2 / 17.1; Q5_1 5120 x 14336, 4 columns (5 rings) 42.5 / 47.9, 3 columns
-//                (6 rings) 40.1 / 37.9
-//   5..8         Q5_1 32000 rows, 5 columns, K 1024 19.0 / 24.6, K 1536 27.5 / 33.0, 8 columns, K 2048 40.7 / 42.5;
-//                4096 x 11008, 6 columns (5 rings) 31.7 / 42.5; 11008 x 4096, 8 columns 30.2 / 28.4
+// CTA, 512 workers on one slot) or gemv_any.cuh (a table per warp, a row is one warp's work).  One column
+// is the former's unless there are few rows.  With several, the latter wins wherever its lanes and warps
+// have work; they have not, with more than one slot to a warp, where rows have few items (half of the
+// lanes idle), where it folds one row at a time (more than 4 columns), and where shared memory leaves it
+// few rings.  Measured, us, table per CTA / per warp:
+//   1 column     Q5_0 11008 x 4096 10.7 / 12.0, 4096 x 11008 14.3 / 16.6, 20000 x 512 5.1 / 7.7; Q4_1 4096 x 4096 3.8 / 4.3,
+//                4096 x 11008 11.3 / 10.8; Q5_1 32000 x 4096 21.3 / 21.0, 2048 x 8192 6.1 / 6.4
+//   2            Q5_0 32000 x 1024 10.7 / 16.6, 4096 x 4096 6.9 / 6.6, 16000 x 6400 29.1 / 33.4; Q4_1 8192 x 2048 5.5 / 5.9, 11008 x
+//                4096 12.4 / 11.5, 2048 x 8192 7.1 / 6.1, 4096 x 11008 14.0 / 15.7
+//   4            Q5_1 20000 x 512 6.6 / 9.9, 32000 x 1024 14.2 / 14.5, 8192 x 2048 8.5 / 7.6, 11008 x 4096 18.7 / 16.7, 2048 x 8192
+//                9.9 / 11.6, 4096 x 11008 20.6 / 25.1
+//   5..8         as the kernels were before one fold was shortened: Q5_1 32000 x 1024, 5 columns 19.0 / 24.6, 8 columns,
+//                K 2048 40.7 / 42.5; 4096 x 11008, 6 columns (5 rings) 31.7 (now 26.2) / 42.5; 11008 x 4096, 8 columns 30.2 / 28.4
 template <int kFormat>
 bool table_per_cta(const GemvAnyPlan &plan, uint32_t nb, size_t nr, size_t nc, int sms) {
-  if (nc == 1 && kFormat == 2 && nb <= 128 && nr >= 8192)
-    return true;
-  const GemvAnyArgs &a = plan.args;
-  if (nr <= static_cast<size_t>(sms) * a.nwarps * a.rps)
-    return false;
-  const uint32_t units = any_units<kFormat>(nb);
   if (nc == 1)
-    return units <= 8;
+    return nr >= 2048;
+  const GemvAnyArgs &a = plan.args;
+  const bool slots_to_spare = nr > static_cast<size_t>(sms) * a.nwarps * a.rps;
   if (nc <= 4)
-    return (units <= 24 && units * nc <= 64) || a.nwarps <= 5;
-  return nb * nc <= 340 || a.nwarps <= 6;
+    return (slots_to_spare && nb * nc <= 128) || (nb * nc >= 400 && nr * nc >= 8192);
+  return slots_to_spare && (nb * nc <= 340 || a.nwarps <= 6);
 }
 
 template <int kFormat>

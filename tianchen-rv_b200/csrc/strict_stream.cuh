@@ -14,12 +14,19 @@
 //     strides are conflict-free or nearly so) into a shared-memory table term[column][row][block];
 //   * 4 folding warps fold the table, thread <-> (row, column), block after block in ascending
 //     order with exactly the operations of the general kernels, so an output has the sequential
-//     fold's bits.  They run one slot behind the workers (two tables); the first of them also
+//     fold's bits.  They run one slot behind the workers (two tables); the last of them also
 //     requests the copies: a slot's buffer is free for the slot after next as soon as its
 //     table is complete.
 // The columns are converted once per CTA into word planes (word w of every block side by side);
 // with one column and a block count that divides the worker count, a thread meets the same
 // block in every row and keeps its activation words in registers.
+//
+// What bounds it: a slot's fold is one dependent operation per block, 4 cycles at best, whatever the number of
+// rows, so slots are as large as two of them fit, and the fold has its loads a batch ahead (strict_chain.cuh).
+// us before / after that, a launch that overlaps the one before, copies requested by the folding warp with
+// the fewest chains, and fewer instructions per term: Q5_0 11008 x 4096, 1 column 12.0 / 10.6, 32000 x 4096 23.4 /
+// 20.9; strict Q4_0 4096 x 11008, 4 columns 29.0 / 20.2, Q8_0 4096 x 8192, 3 columns 21.9 / 16.4; Q5_1 4096 x 11008, 6 columns
+// 31.7 / 26.2.  (More and smaller slots: Q5_0 11008 x 4096 with four of 16 rows 11.9.)
 //
 // It serves Q4_0 / Q8_0 rows on 16-byte boundaries that are too long for the tensor-core form, and the
 // sibling formats where its 512 workers on one slot beat the table per warp of gemv_any.cuh
@@ -36,6 +43,7 @@
 #include <atomic>
 
 #include "async_copy.cuh"
+#include "strict_chain.cuh"
 #include "tcrv_common.cuh"
 
 namespace tcrv {
@@ -122,6 +130,61 @@ __device__ __forceinline__ int strict_sumi_words(const uint32_t (&q)[8], uint32_
   }
 }
 
+// The streaming kernels' form of it: the float of the block's sum.  The chain of dot products starts from
+// `start`, the bits of the float 12582912 = 1.5 * 2^23 less the offset's part, so the result's bits are those
+// of 12582912 + sum (every sum is at most 2^19 in magnitude) and one exact subtraction makes the number.
+constexpr uint32_t kStrictMagicBits = 0x4B400000u;
+template <int kFormat>
+__device__ __forceinline__ uint32_t strict_start(int ysum) {
+  return kStrictMagicBits - static_cast<uint32_t>(StrictFormat<kFormat>::kBias * ysum);
+}
+
+__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {  // unsigned x signed bytes
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+// kOne: a word of weights meets one column only.  Then the high nibbles are left where they are (16 times
+// the code, one shift at the end instead of four), and the fifth bits are not merged into the codes but
+// dotted on their own: bit 8i + k of `qh` belongs to element 8i + k, so (qh >> k) & 0x01010101 meets
+// yb[k], the activations k, 8 + k, 16 + k, 24 + k.  24 instead of 32 instructions per block; with several
+// columns the merged codes are made once for all of them.
+template <int kFormat, bool kOne>
+__device__ __forceinline__ float strict_dot(const uint32_t (&q)[8], uint32_t qh, const uint32_t (&y)[8],
+                                            [[maybe_unused]] const uint32_t (&yb)[8], uint32_t start) {
+  using F = StrictFormat<kFormat>;
+  int sum = static_cast<int>(start);
+  if constexpr (F::kNibbles && kOne) {
+    int high = 0, bits = 0;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      sum = __dp4a(static_cast<int>(q[w] & 0x0f0f0f0fu), static_cast<int>(y[w]), sum);
+      high = dp4a_us(q[w] & 0xf0f0f0f0u, y[4 + w], high);
+    }
+    if constexpr (F::kQh != 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        bits = __dp4a(static_cast<int>((qh >> k) & 0x01010101u), static_cast<int>(yb[k]), bits);
+    }
+    sum += (high >> 4) + 16 * bits;
+  } else {
+    sum += strict_sumi_words<kFormat>(q, qh, y, 0);
+  }
+  return __fadd_rn(__int_as_float(sum), -12582912.0f);
+}
+
+// yb (see above) of the activation words y: two transpositions of 4 x 4 bytes.
+__device__ __forceinline__ void strict_bit_planes(const uint32_t (&y)[8], uint32_t (&yb)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t a = __byte_perm(y[h], y[2 + h], 0x5140), b = __byte_perm(y[4 + h], y[6 + h], 0x5140);
+    const uint32_t c = __byte_perm(y[h], y[2 + h], 0x7362), d = __byte_perm(y[4 + h], y[6 + h], 0x7362);
+    yb[4 * h + 0] = __byte_perm(a, b, 0x5410), yb[4 * h + 1] = __byte_perm(a, b, 0x7632);
+    yb[4 * h + 2] = __byte_perm(c, d, 0x5410), yb[4 * h + 3] = __byte_perm(c, d, 0x7632);
+  }
+}
+
 constexpr int kStrictWorkers = 512;
 constexpr int kStrictFoldWarps = 4;
 constexpr int kStrictThreads = kStrictWorkers + 32 * kStrictFoldWarps;
@@ -138,12 +201,20 @@ struct StrictStreamArgs {
 };
 
 // shared-memory pieces: word planes, scale and (Q8_1) sum of every column; the term tables
-__host__ __device__ inline size_t strict_x_bytes(uint32_t nb, uint32_t nc) { return static_cast<size_t>(nc) * nb * 10 * 4; }
-__host__ __device__ inline size_t strict_table_floats(uint32_t nb, uint32_t nc, uint32_t rps, bool two) {
-  return static_cast<size_t>(nc) * rps * (nb + 1) * (two ? 2 : 1);
+// (and, for one column against five-bit codes, the words that meet the fifth bits)
+__host__ __device__ inline size_t strict_x_bytes(uint32_t nb, uint32_t nc, bool bits) {
+  return (static_cast<size_t>(nc) * 10 + (bits && nc == 1 ? 8 : 0)) * nb * 4;
 }
-__host__ __device__ inline size_t strict_slots_offset(uint32_t nb, uint32_t nc, uint32_t rps, bool two) {
-  return (128 + strict_x_bytes(nb, nc) + 2 * strict_table_floats(nb, nc, rps, two) * 4 + 127) / 128 * 128;
+// (a row's pitch: 16 bytes times an odd number, so that the folding lanes' 16-byte loads are free of conflicts)
+__host__ __device__ inline uint32_t strict_pitch(uint32_t nb) { return nb + 4; }
+__host__ __device__ inline size_t strict_table_floats(uint32_t nb, uint32_t nc, uint32_t rps, bool two) {
+  return static_cast<size_t>(nc) * rps * strict_pitch(nb) * (two ? 2 : 1);
+}
+template <int kFormat>
+__host__ __device__ inline size_t strict_slots_offset(uint32_t nb, uint32_t nc, uint32_t rps) {
+  using F = StrictFormat<kFormat>;
+  return (128 + strict_x_bytes(nb, nc, F::kQh != 0) +
+          2 * strict_table_floats(nb, nc, rps, F::kFold == kFoldProduct) * 4 + 127) / 128 * 128;
 }
 
 // kOneCol: a.nc == 1, known at compile time (the common decode case: no column loops).
@@ -151,13 +222,14 @@ template <int kFormat, bool kOneCol>
 __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const StrictStreamArgs a) {
   using F = StrictFormat<kFormat>;
   constexpr bool kTwo = F::kFold == kFoldProduct;  // (float)sumi and the scale product kept apart
+  constexpr bool kBits = kOneCol && F::kQh != 0;    // the fifth bits are dotted on their own
   constexpr int kQWords = F::kNibbles ? 4 : 8;
   // Blocks of 18, 22 or 34 bytes start on a word boundary and in the middle of a word
   // alternately: a work item is then a PAIR of blocks (36, 44 or 68 bytes, whole words), and which
   // fields need re-aligning is known at compile time.  Blocks of 20 or 24 bytes are items of
-  // their own.  Everything kept per block (activation planes, scales, table rows) is laid out by
-  // item: the first blocks of all items, then the second blocks, so that consecutive threads
-  // touch consecutive words.
+  // their own.  The activation planes are laid out by item: the first blocks of all items, then the
+  // second blocks, so that consecutive threads touch consecutive words.  The scales and the table's
+  // rows, which the fold reads four blocks at a time, are in the blocks' order.
   constexpr bool kPairs = F::kW % 4 != 0;
   constexpr uint32_t kUnit = kPairs ? 2 : 1;         // blocks per work item
   constexpr uint32_t kUnitWords = kUnit * F::kW / 4;  // 5, 6 / 9, 11, 17
@@ -174,10 +246,12 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
   uint32_t *xq = reinterpret_cast<uint32_t *>(smem + 128);  // [nc][8][nb]
   float *xd = reinterpret_cast<float *>(xq + static_cast<size_t>(nc) * 8 * nb);  // [nc][nb]
   float *xs = xd + static_cast<size_t>(nc) * nb;                                  // [nc][nb] (Q8_1: s = d * sum(q))
-  float *table = xs + static_cast<size_t>(nc) * nb;  // [2][kTwo ? 2 : 1][nc][rps][nb + 1]
-  const size_t plane = static_cast<size_t>(nc) * rps * (nb + 1);  // one table of one buffer
+  uint32_t *xb = reinterpret_cast<uint32_t *>(xs + static_cast<size_t>(nc) * nb);  // kBits: [8][nb]
+  const uint32_t pitch = strict_pitch(nb);
+  float *table = reinterpret_cast<float *>(xb + (kBits ? 8 : 0) * nb);  // [2][kTwo ? 2 : 1][nc][rps][pitch]
+  const size_t plane = static_cast<size_t>(nc) * rps * pitch;  // one table of one buffer
   const size_t table_floats = plane * (kTwo ? 2 : 1);
-  uint8_t *slots = smem + strict_slots_offset(nb, nc, rps, kTwo);
+  uint8_t *slots = smem + strict_slots_offset<kFormat>(nb, nc, rps);
   const size_t slot_bytes = static_cast<size_t>(rps) * a.row_bytes;
 
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -195,6 +269,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
     mbar_fence_init();
   }
   __syncthreads();
+  pdl_enter();  // (everything above is this CTA's own)
   auto fail = [&]() {
     if (lane == 0 && *abort_flag == 0)
       raise_device_error(kDevErrBarrierTimeout);
@@ -202,7 +277,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
   };
 
   if (warp >= kStrictWorkers / 32) {
-    // ---- folding warps; the first also requests the copies.  Lane 0 announces a slot's bytes,
+    // ---- folding warps; the last, which has the fewest chains, also requests the copies.  Lane 0 announces a slot's bytes,
     // then lanes 0..7 copy an eighth of its rows each.
     const uint32_t fw = warp - kStrictWorkers / 32;
     auto issue = [&](uint32_t j) {
@@ -224,7 +299,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
       }
     };
     uint32_t issued = 0;
-    if (fw == 0)
+    if (fw == kStrictFoldWarps - 1)
       for (; issued < min(2u, nslots); ++issued)
         issue(issued);
     uint32_t j = 0;
@@ -236,44 +311,24 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
         break;
       }
       // the workers have read the slot's rows: its buffer takes the slot after next
-      if (fw == 0 && issued < nslots) {
+      if (fw == kStrictFoldWarps - 1 && issued < nslots) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         issue(issued++);
       }
       // chain = (row, column); this lane takes chains fw * 32 + lane, + 128, ...
       for (uint32_t c = fw * 32 + lane; c < rows * nc; c += 32 * kStrictFoldWarps) {
         const uint32_t r = c / nc, col = c - r * nc;
-        const float *t = ta + (static_cast<size_t>(col) * rps + r) * (nb + 1);
-        float acc = 0.0f;
-        // ascending block order: item k holds blocks kUnit * k + h at positions h * units + k
-        if constexpr (F::kFold == kFoldMin) {
-#pragma unroll 8
-          for (uint32_t k = 0; k < units; ++k)
-#pragma unroll
-            for (uint32_t h = 0; h < kUnit; ++h)
-              acc = __fadd_rn(acc, t[h * units + k]);
-        } else if constexpr (F::kFold == kFoldProduct) {
-          const float *p = t + plane;  // d_w * d_x
-#pragma unroll 8
-          for (uint32_t k = 0; k < units; ++k)
-#pragma unroll
-            for (uint32_t h = 0; h < kUnit; ++h)
-              acc = __fmaf_rn(t[h * units + k], p[h * units + k], acc);
-        } else {
-          const float *dx = xd + static_cast<size_t>(col) * nb;
-#pragma unroll 8
-          for (uint32_t k = 0; k < units; ++k)
-#pragma unroll
-            for (uint32_t h = 0; h < kUnit; ++h)
-              acc = __fmaf_rn(t[h * units + k], dx[h * units + k], acc);
-        }
+        const float *t = ta + (static_cast<size_t>(col) * rps + r) * pitch;
+        const float *m = kTwo ? t + plane : xd + static_cast<size_t>(col) * nb;  // d_w * d_x, or d_x
+        const float acc = strict_chain<F::kFold == kFoldMin, 4>(reinterpret_cast<const float4 *>(t),
+                                                             reinterpret_cast<const float4 *>(m), nb / 4);
         a.s[static_cast<size_t>(row0 + r) * a.bs + col] = acc;
       }
       __syncwarp();
       if (lane == 0)
         mbar_arrive(&tempty[j & 1u]);
     }
-    if (fw == 0 && j < nslots && lane == 0) {
+    if (fw == kStrictFoldWarps - 1 && j < nslots && lane == 0) {
       // leaving early: copies already requested must land before the CTA's memory goes away
       for (uint32_t u = issued >= 2 ? issued - 2 : 0; u < issued; ++u)
         (void)mbar_wait_bounded(&full[u & 1u], (u >> 1) & 1u);
@@ -290,25 +345,32 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
       return y_even ? static_cast<uint32_t>(*reinterpret_cast<const unsigned short *>(yb + off)) : load_u16(yb + off);
     };
     const uint32_t at = pos(ib);
-    xd[col * nb + at] = half_bits_to_float(static_cast<unsigned short>(half_at(0)));
+    xd[col * nb + ib] = half_bits_to_float(static_cast<unsigned short>(half_at(0)));
     uint32_t yw[8];
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
       yw[w] = half_at(F::kAq + 4 * w) | (half_at(F::kAq + 4 * w + 2) << 16);
       xq[(static_cast<size_t>(col) * 8 + w) * nb + at] = yw[w];
     }
-    // the third plane: Q8_1's s = d * sum(q) for the formats with a minimum, the plain integer
-    // sum(q) (as bits) for the formats whose weight codes carry an offset
+    // the third plane: Q8_1's s = d * sum(q) for the formats with a minimum, else where the block's sum
+    // starts (strict_start, as bits)
     if constexpr (F::kFold == kFoldMin)
       xs[col * nb + at] = half_bits_to_float(static_cast<unsigned short>(half_at(2)));
     else
-      xs[col * nb + at] = __int_as_float(strict_ysum(yw));
+      xs[col * nb + at] = __uint_as_float(strict_start<kFormat>(F::kBias != 0 ? strict_ysum(yw) : 0));
+    if constexpr (kBits) {
+      uint32_t yb8[8];
+      strict_bit_planes(yw, yb8);
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+        xb[w * nb + at] = yb8[w];
+    }
   }
   asm volatile("bar.sync 1, %0;" ::"r"(kStrictWorkers) : "memory");  // the workers only
 
   // one column and an item index that is the same in every row: the activation blocks live in registers
   const bool fixed = kOneCol && kStrictWorkers % units == 0;
-  uint32_t yfix[kUnit][8];
+  uint32_t yfix[kUnit][8], bfix[kUnit][8] = {};
   float dfix[kUnit], sfix[kUnit];
   if (fixed) {
 #pragma unroll
@@ -317,10 +379,17 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
 #pragma unroll
       for (int w = 0; w < 8; ++w)
         yfix[h][w] = xq[w * nb + at];
-      dfix[h] = xd[at], sfix[h] = xs[at];
+      if constexpr (kBits) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+          bfix[h][w] = xb[w * nb + at];
+      }
+      dfix[h] = xd[kUnit * (tid % units) + h], sfix[h] = xs[at];
     }
   }
 
+  const uint32_t first_row = tid / units, first_item = tid % units;
+  const uint32_t step_rows = kStrictWorkers / units, step_items = kStrictWorkers % units;
   for (uint32_t j = 0; j < nslots; ++j) {
     const uint32_t row0 = r0 + j * rps, rows = min(rps, r1 - row0);
     float *ta = table + (j & 1u) * table_floats;
@@ -330,28 +399,34 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
       return;
     }
     const uint32_t *wslot = reinterpret_cast<const uint32_t *>(slots + (j & 1u) * slot_bytes);
-    // terms of one block (row r of the slot, kept at position `at`, the h-th block of its item) for every column
-    auto emit = [&](uint32_t r, uint32_t at, uint32_t h, uint32_t dbits, uint32_t mbits, const uint32_t (&q)[8],
+    // terms of one block (row r of the slot, the h-th block of item iu) for every column
+    auto emit = [&](uint32_t r, uint32_t iu, uint32_t h, uint32_t dbits, uint32_t mbits, const uint32_t (&q)[8],
                     uint32_t qh) {
+      const uint32_t at = h * units + iu, ib = kUnit * iu + h;
       const float dw = half_bits_to_float(static_cast<unsigned short>(dbits));
       [[maybe_unused]] const float mw = half_bits_to_float(static_cast<unsigned short>(mbits));
       for (uint32_t col = 0; col < nc; ++col) {
-        uint32_t y[8];
+        uint32_t y[8], yb8[8] = {};
         float dy;
         float sy;
         if (fixed) {
 #pragma unroll
           for (int w = 0; w < 8; ++w)
-            y[w] = yfix[h][w];
+            y[w] = yfix[h][w], yb8[w] = bfix[h][w];
           dy = dfix[h], sy = sfix[h];
         } else {
 #pragma unroll
           for (int w = 0; w < 8; ++w)
             y[w] = xq[(static_cast<size_t>(col) * 8 + w) * nb + at];
-          dy = xd[col * nb + at], sy = xs[col * nb + at];
+          if constexpr (kBits) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+              yb8[w] = xb[w * nb + at];
+          }
+          dy = xd[col * nb + ib], sy = xs[col * nb + at];
         }
-        const float fs = __int2float_rn(strict_sumi_words<kFormat>(q, qh, y, __float_as_int(sy)));
-        float *t = ta + (static_cast<size_t>(col) * rps + r) * (nb + 1) + at;
+        const float fs = strict_dot<kFormat, kOneCol>(q, qh, y, yb8, F::kFold == kFoldMin ? kStrictMagicBits : __float_as_uint(sy));
+        float *t = ta + (static_cast<size_t>(col) * rps + r) * pitch + ib;
         if constexpr (F::kFold == kFoldMin) {
           *t = __fmaf_rn(__fmul_rn(dw, dy), fs, __fmul_rn(mw, sy));
         } else if constexpr (F::kFold == kFoldProduct) {
@@ -362,8 +437,14 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
         }
       }
     };
-    for (uint32_t e = tid; e < rows * units; e += kStrictWorkers) {
-      const uint32_t r = e / units, iu = e - r * units;
+    // item iu of row r, 512 items further every time
+    uint32_t r = first_row, iu = first_item;
+    for (; r < rows; r += step_rows, iu += step_items) {
+      if (iu >= units) {
+        iu -= units;
+        if (++r >= rows)
+          break;
+      }
       const uint32_t *w = wslot + static_cast<size_t>(r) * (a.row_bytes / 4) + iu * kUnitWords;
       uint32_t pw[kUnitWords];
 #pragma unroll
@@ -392,7 +473,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
           q[k] = pw[(F::kW + F::kWq + 4 * k) / 4];
         if constexpr (F::kQh != 0)
           qh = pw[(F::kW + F::kQh) / 4];
-        emit(r, units + iu, 1, pw[F::kW / 4] >> 16, 0, q, qh);
+        emit(r, iu, 1, pw[F::kW / 4] >> 16, 0, q, qh);
       }
     }
     // this warp's share of the table is written and its reads of the slot are done
@@ -410,9 +491,8 @@ uint32_t strict_stream_rows(uint32_t nb, size_t nr, size_t nc, const uint8_t *vx
       reinterpret_cast<uintptr_t>(vx) % 16 != 0 || bx % 16 != 0)
     return 0;
   const size_t row_bytes = static_cast<size_t>(nb) * F::kW;
-  const bool two = F::kFold == kFoldProduct;
   for (uint32_t rps = kStrictMaxRows; rps >= 4; rps -= 4) {
-    const size_t need = strict_slots_offset(nb, static_cast<uint32_t>(nc), rps, two) + 2 * rps * row_bytes;
+    const size_t need = strict_slots_offset<kFormat>(nb, static_cast<uint32_t>(nc), rps) + 2 * rps * row_bytes;
     if (need <= kStrictSmemCap)
       return rps;
   }
@@ -438,7 +518,7 @@ int launch_strict_stream(size_t n, float *s, const uint8_t *vx, const uint8_t *v
   args.row_bytes = nb * F::kW;
   args.rps = rps;
   args.contiguous = bx == static_cast<size_t>(nb) * F::kW ? 1u : 0u;
-  const size_t smem = strict_slots_offset(nb, args.nc, rps, F::kFold == kFoldProduct) +
+  const size_t smem = strict_slots_offset<kFormat>(nb, args.nc, rps) +
                       2 * static_cast<size_t>(rps) * args.row_bytes;
   static std::atomic<bool> configured[64];
   int dev = 0;
@@ -452,11 +532,8 @@ int launch_strict_stream(size_t n, float *s, const uint8_t *vx, const uint8_t *v
   }
   const size_t slots = (nr + rps - 1) / rps;
   const size_t grid = slots < static_cast<size_t>(sms) ? slots : static_cast<size_t>(sms);
-  if (nc == 1)
-    strict_stream_kernel<kFormat, true><<<static_cast<int>(grid), kStrictThreads, smem, stream>>>(args);
-  else
-    strict_stream_kernel<kFormat, false><<<static_cast<int>(grid), kStrictThreads, smem, stream>>>(args);
-  TCRV_CUDA_TRY(cudaGetLastError());
+  TCRV_CUDA_TRY(launch_pdl(nc == 1 ? strict_stream_kernel<kFormat, true> : strict_stream_kernel<kFormat, false>,
+                           static_cast<int>(grid), kStrictThreads, smem, stream, args));
   return TCRV_CUDA_OK;
 }
 
