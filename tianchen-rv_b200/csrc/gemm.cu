@@ -8,6 +8,7 @@
 //   activations  8-bit [nc][K] twice     an int8 q as two e4m3 planes: q & 15 and q - (q & 15), q = sum of both
 //   act. scale   fp32 [nb][ncp]          transposed; ncp = columns rounded up to 4
 #include <atomic>
+#include <type_traits>
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -311,20 +312,23 @@ inline int blocks_for(size_t items) {
   return static_cast<int>(b < cap ? (b ? b : 1) : cap);
 }
 
-// Whether a launch deals out 128 x 32 items instead of 256 x 64 ones (whose last round is cut into
-// 128 x 64 halves where those fill no more than half of the SMs).  Rounds of each kind times what an
-// item takes, in hundredths of a 256 x 64 one: measured on 512 x 32000 x 4096, 36.6 us a round of whole
-// items, 19.5 of halves, 13.8 of narrow ones.  Narrow items win where the others leave SMs without
-// work: 77 x 4096 x 11008 44.0 against 55.6 us; 512 x 11008 x 4096 144 against 97.0 us.
-bool narrow_items(size_t nr, size_t nc, size_t ctas) {
+// Which items a launch deals out: 256 x 64 ones (0; their last round is cut into 128 x 64 halves where those
+// fill no more than half of the SMs), 128 x 32 (32) or 128 x 16 (16).  Rounds of each kind times what an item
+// takes, in hundredths of a 256 x 64 one: with 128 blocks to a row a round takes 33 us whole, 20 in halves, 11.2 and
+// 7.4 to 8.3 narrow.  Narrow items win where the others leave SMs without work.  us, 256 x 64 / 128 x 32 / 128 x 16:
+// 77 x 4096 x 11008 59.4 / 35.5 / 43.8, 40 x 4096 x 4096 22.7 / 13.9 / 10.7, 33 x 20000 x 1024 19.1 / 18.5 / 14.8, 200 x 4096 x
+// 4096 23.8 / 26.1 / 26.3, 512 x 11008 x 4096 90.7 / 115 / 143.
+int narrow_items(size_t nr, size_t nc, size_t ctas) {
   const auto cdiv = [](size_t a, size_t b) { return (a + b - 1) / b; };
   const size_t tiles = cdiv(nr, 256) * cdiv(nc, 64), rem = tiles % ctas;
-  const size_t wide = tiles / ctas * 100 + (rem == 0 ? 0 : 2 * rem <= ctas ? 54 : 100);
-  return cdiv(cdiv(nr, 128) * cdiv(nc, 32), ctas) * 38 < wide;
+  const size_t wide = tiles / ctas * 100 + (rem == 0 ? 0 : 2 * rem <= ctas ? 60 : 100);
+  const size_t by32 = cdiv(cdiv(nr, 128) * cdiv(nc, 32), ctas) * 34;
+  const size_t by16 = cdiv(cdiv(nr, 128) * cdiv(nc, 16), ctas) * 24;
+  return by16 < by32 && by16 < wide ? 16 : by32 < wide ? 32 : 0;
 }
 
 // One instantiation of the kernel: its tensor maps, its work items, its launch.
-template <bool kMulti, bool kRepack, bool kNarrow>
+template <bool kMulti, bool kRepack, int kNarrow>
 int launch_gemm_kernel(const PlanarSizes &p, const uint8_t *weights_planar, const uint8_t *acts_planar, GemmArgs &args,
                        cudaStream_t stream) {
   using Plan = GemmPlan<kNarrow>;
@@ -356,7 +360,7 @@ int launch_gemm_kernel(const PlanarSizes &p, const uint8_t *weights_planar, cons
   const uint32_t tiles = static_cast<uint32_t>((nr + Plan::Full::kRows - 1) / Plan::Full::kRows) * args.tiles_m;
   const uint32_t ctas = static_cast<uint32_t>(sm_count());
   const uint32_t rem = tiles % ctas;
-  args.full_items = !kNarrow && 2 * rem <= ctas ? tiles - rem : tiles;
+  args.full_items = kNarrow == 0 && 2 * rem <= ctas ? tiles - rem : tiles;
   args.items = args.full_items + 2 * (tiles - args.full_items);
   const int grid = static_cast<int>(args.items < ctas ? args.items : ctas);
 
@@ -395,13 +399,18 @@ int run_gemm(size_t n, float *const *dst, size_t ndst, const uint8_t *weights_pl
   const int st = device_error_words(&args.errors);
   if (st != TCRV_CUDA_OK)
     return st;
+  const auto launch = [&](auto narrow) {
+    constexpr int kNarrow = decltype(narrow)::value;
+    return repack ? launch_gemm_kernel<false, true, kNarrow>(p, weights_planar, acts_planar, args, stream)
+                  : launch_gemm_kernel<false, false, kNarrow>(p, weights_planar, acts_planar, args, stream);
+  };
   if (multi)
-    return launch_gemm_kernel<true, false, false>(p, weights_planar, acts_planar, args, stream);
-  if (narrow_items(nr, nc, static_cast<size_t>(sm_count())))
-    return repack ? launch_gemm_kernel<false, true, true>(p, weights_planar, acts_planar, args, stream)
-                  : launch_gemm_kernel<false, false, true>(p, weights_planar, acts_planar, args, stream);
-  return repack ? launch_gemm_kernel<false, true, false>(p, weights_planar, acts_planar, args, stream)
-                : launch_gemm_kernel<false, false, false>(p, weights_planar, acts_planar, args, stream);
+    return launch_gemm_kernel<true, false, 0>(p, weights_planar, acts_planar, args, stream);
+  switch (narrow_items(nr, nc, static_cast<size_t>(sm_count()))) {
+    case 16: return launch(std::integral_constant<int, 16>());
+    case 32: return launch(std::integral_constant<int, 32>());
+    default: return launch(std::integral_constant<int, 0>());
+  }
 }
 
 }  // namespace

@@ -24,13 +24,11 @@
 // load of activation scales serves two outputs of a thread (with 128 x 128 items those loads put 64 KB
 // per block through the shared-memory pipe beside the operands: 305 us for 512 x 32000 x 4096, 640
 // cycles per 128 x 128 x 32 of arithmetic that takes 276; they still cost 40 us of the 256).  8
-// epilogue warps with 64 accumulators a thread: fewer would not fill the FMA pipes, more leave no
-// registers for the second chunk buffer that hides the TMEM load and the barrier test (16 warps
-// without it: 318 us; 16 instead of 32 registers a chunk, scales fetched before the wait: 283 ->
-// 256 us).  512 x 11008 x 4096: 122.8 -> 97.0 us.
+// epilogue warps with 64 accumulators a thread: with 16 a hand-over's fixed cost is paid twice as often and
+// registers run out (252 us and more instead of 231), with 4 nothing covers a warp's waits (267).
 // Whole items are dealt round-robin to the CTAs; a last round that would leave more than half of
-// them idle is cut into halves of 128 rows.  Few columns: items of 128 rows x 32 columns, 4 blocks to
-// a hand-over (gemm.cu chooses; 77 x 4096 x 11008: 89.9 -> 44.0 us, halves 55.6).
+// them idle is cut into halves of 128 rows.  Few columns or rows: items of 128 rows x 32 or 16 columns, 4
+// blocks to a hand-over (gemm.cu chooses).
 //
 // A second fold (kRepack) serves the consumer of the 16-row interleaved layouts: the same
 // contraction with fma((float)S, d_w * d_x, acc) (the scales multiplied first, an exact
@@ -81,9 +79,9 @@ struct GemmShape {
   static constexpr int kRows = kRowTiles * kGemmTileRows;
   static constexpr int kCpw = kCols / (kGemmEpilogueWarps / 4);  // columns of an epilogue warp
   static constexpr int kBlockCols = kRowTiles * kCols;           // TMEM columns of one block's accumulators
-  // A chunk is what a thread loads from TMEM at a time, 32 registers: kChunkCols columns of its rows of
-  // kChunkBlocks blocks.
-  static constexpr int kChunkRegs = 32;
+  // A chunk is what a thread loads from TMEM at a time, 32 registers (16 where a stage is no more than that):
+  // kChunkCols columns of its rows of kChunkBlocks blocks.
+  static constexpr int kChunkRegs = kRowTiles * kCpw * kGemmStageBlocks > 32 ? 32 : 16;
   static constexpr int kChunkCols = kCpw < kChunkRegs / kRowTiles ? kCpw : kChunkRegs / kRowTiles;
   static constexpr int kChunkBlocks = kChunkRegs / (kRowTiles * kChunkCols);
   static constexpr int kBlockChunks = kCpw / kChunkCols;  // chunks of one block, where it has several
@@ -98,14 +96,15 @@ struct GemmShape {
   static_assert(kChunks % 2 == 0 && kChunks % kHandoverChunks == 0, "two chunk buffers, whole hand-overs");
 };
 
-// What one launch works on: whole items, and halves of such items.
-template <bool kNarrow>
+// What one launch works on: whole items of 256 x 64 and halves of those (kNarrow 0), or items of 128 rows x
+// kNarrow columns.
+template <int kNarrow>
 struct GemmPlan {
-  using Full = GemmShape<kNarrow ? 1 : 2, kNarrow ? 32 : 64>;
-  using Half = GemmShape<1, kNarrow ? 32 : 64>;
+  using Full = GemmShape<kNarrow != 0 ? 1 : 2, kNarrow != 0 ? kNarrow : 64>;
+  using Half = GemmShape<1, kNarrow != 0 ? kNarrow : 64>;
   static constexpr uint32_t kColParts = Full::kCols / Half::kCols;
   static constexpr uint32_t kParts = Full::kRowTiles * kColParts;
-  static constexpr int kTmemStages = kNarrow ? 4 : 2;
+  static constexpr int kTmemStages = kNarrow != 0 ? 4 : 2;
   static constexpr int kTmemStageCols = kGemmTmemCols / kTmemStages;
   static_assert(Full::kBlockCols * Full::kHandover <= kTmemStageCols, "a hand-over fits a TMEM stage");
   static_assert(Half::kBlockCols * Half::kHandover <= kTmemStageCols, "a hand-over fits a TMEM stage");
@@ -128,9 +127,9 @@ struct GemmPlan {
 constexpr int kGemmOutRowBytes = 64 * 4 + 16;
 constexpr int kGemmOutBytes = kGemmTileRows * kGemmOutRowBytes;  // 34816
 
-template <bool kMulti, bool kNarrow>
+template <bool kMulti, int kNarrow>
 struct GemmSmem {
-  static constexpr int kStages = kNarrow ? 8 : kMulti ? 3 : 4;
+  static constexpr int kStages = kNarrow != 0 ? 8 : kMulti ? 3 : 4;
   static constexpr size_t kBytes = kGemmCtrlBytes + 1024 +
                                    static_cast<size_t>(kStages) * GemmPlan<kNarrow>::kStageBytes +
                                    (kMulti ? kGemmOutBytes : 0);
@@ -158,7 +157,7 @@ struct GemmItem {
   bool whole;
 };
 
-template <bool kNarrow>
+template <int kNarrow>
 __device__ __forceinline__ GemmItem gemm_item(const GemmArgs &a, uint32_t idx) {
   using Plan = GemmPlan<kNarrow>;
   GemmItem it;
@@ -553,8 +552,8 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
 
 // kMulti: the result goes to several output copies (peers) through a shared-memory staging tile.
 // kRepack (single destination only): scales multiplied first, token-major output.
-// kNarrow: items of 128 rows x 32 columns (few tokens) instead of 256 x 64 and halves of those.
-template <bool kMulti, bool kRepack, bool kNarrow>
+// kNarrow: see GemmPlan.
+template <bool kMulti, bool kRepack, int kNarrow>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_q4_0_q8_0_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                              const __grid_constant__ CUtensorMap map_xhi, const __grid_constant__ CUtensorMap map_dw,

@@ -109,10 +109,20 @@ __device__ __forceinline__ void umma_f8_again(uint32_t tmem_d, uint64_t desc_a, 
       : "memory");
 }
 
-// 32 lanes x N consecutive 32-bit columns (N = 16 or 32) into v[0..N): thread i of the warp
+// 32 lanes x N consecutive 32-bit columns (N = 8, 16 or 32) into v[0..N): thread i of the warp
 // receives lane (base+i).
 template <int N>
 __device__ __forceinline__ void tmem_ld_32x32b(uint32_t taddr, uint32_t *v);
+
+template <>
+__device__ __forceinline__ void tmem_ld_32x32b<8>(uint32_t taddr, uint32_t *v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "r"(taddr)
+      : "memory");
+}
 
 template <>
 __device__ __forceinline__ void tmem_ld_32x32b<16>(uint32_t taddr, uint32_t *v) {
