@@ -165,6 +165,50 @@ __global__ void __launch_bounds__(256) unpack_q4_0_kernel(const uint8_t *__restr
   }
 }
 
+// Columns on 16-byte boundaries: a CTA takes 8 columns x 32 blocks.  They come in with 16-byte loads; a
+// thread then converts one block (a warp: 32 blocks of a column, whole lines of both planes) and the scales
+// leave as sectors of 8 columns.  Bound by latency, load to store, at the sizes of a prompt.
+constexpr int kUnpackCols = 8, kUnpackColBlocks = 32;
+__global__ void __launch_bounds__(256) unpack_q8_0_tiles_kernel(const uint8_t *__restrict__ vy, size_t by, uint32_t nc,
+                                                                uint32_t nb, uint32_t ncp, int8_t *__restrict__ x8,
+                                                                size_t plane, float *__restrict__ dxt) {
+  constexpr uint32_t kColBytes = kUnpackColBlocks * kQ8Block;  // 1088
+  __shared__ __align__(16) uint8_t tile[kUnpackCols * kColBytes];
+  __shared__ float scales[kUnpackColBlocks][kUnpackCols + 1];
+  pdl_enter();
+  const uint32_t c0 = blockIdx.y * kUnpackCols, b0 = blockIdx.x * kUnpackColBlocks;
+  const uint32_t blocks = min(static_cast<uint32_t>(kUnpackColBlocks), nb - b0);
+  const uint32_t bytes = blocks * kQ8Block, pieces = bytes / 16;  // of a column; what is left of it is half words
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, col = c0 + warp;
+  if (col < nc) {
+    const uint8_t *src = vy + static_cast<size_t>(col) * by + static_cast<size_t>(b0) * kQ8Block;
+    uint8_t *dst = tile + warp * kColBytes;
+#pragma unroll
+    for (uint32_t k = 0; k < (kColBytes / 16 + 31) / 32; ++k)
+      if (k * 32 + lane < pieces)
+        reinterpret_cast<uint4 *>(dst)[k * 32 + lane] = __ldg(reinterpret_cast<const uint4 *>(src) + k * 32 + lane);
+    if (pieces * 8 + lane < bytes / 2)
+      reinterpret_cast<unsigned short *>(dst)[pieces * 8 + lane] = reinterpret_cast<const unsigned short *>(src)[pieces * 8 + lane];
+    __syncwarp();
+    if (lane < blocks) {
+      const unsigned short *h = reinterpret_cast<const unsigned short *>(dst + lane * kQ8Block);
+      uint32_t q[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        q[j] = static_cast<uint32_t>(h[1 + 2 * j]) | (static_cast<uint32_t>(h[2 + 2 * j]) << 16);
+      store_act_block(x8 + (static_cast<size_t>(col) * nb + b0 + lane) * kQK, plane, q);
+      scales[lane][warp] = half_bits_to_float(h[0]);
+    }
+  } else {
+    scales[lane][warp] = 0.0f;  // columns' padding (see store_act_scale)
+  }
+  __syncthreads();
+  const uint32_t block = threadIdx.x / kUnpackCols, c = threadIdx.x % kUnpackCols;
+  if (block < blocks && c0 + c < ncp)
+    dxt[static_cast<size_t>(b0 + block) * ncp + c0 + c] = scales[block][c];
+}
+
+// Any alignment.  One thread per (column, block).
 __global__ void __launch_bounds__(256) unpack_q8_0_kernel(const uint8_t *__restrict__ vy, size_t by, uint32_t nc,
                                                           uint32_t nb, uint32_t ncp, int8_t *__restrict__ x8,
                                                           size_t plane, float *__restrict__ dxt, bool aligned2) {
@@ -449,6 +493,14 @@ int launch_gemm_prepare_acts_q8_0(size_t n, const uint8_t *vy, size_t by, size_t
   const PlanarSizes p = planar_sizes(n, 0, nc);
   if (nc == 0 || p.nb == 0)
     return TCRV_CUDA_OK;
+  const size_t col_tiles = (nc + kUnpackCols - 1) / kUnpackCols;
+  if (reinterpret_cast<uintptr_t>(vy) % 16 == 0 && (by % 16 == 0 || nc == 1) && col_tiles <= 65535) {
+    const dim3 grid(static_cast<unsigned>((p.nb + kUnpackColBlocks - 1) / kUnpackColBlocks), static_cast<unsigned>(col_tiles));
+    TCRV_CUDA_TRY(launch_pdl(unpack_q8_0_tiles_kernel, grid, 256, 0, stream, vy, by, static_cast<uint32_t>(nc),
+                             static_cast<uint32_t>(p.nb), static_cast<uint32_t>(p.ncp), reinterpret_cast<int8_t *>(prepared),
+                             p.x_plane, reinterpret_cast<float *>(prepared + p.x8)));
+    return TCRV_CUDA_OK;
+  }
   const bool aligned2 = (reinterpret_cast<uintptr_t>(vy) % 2 == 0) && (by % 2 == 0);
   TCRV_CUDA_TRY(launch_pdl(unpack_q8_0_kernel, blocks_for(nc * p.nb), 256, 0, stream, vy, by, static_cast<uint32_t>(nc),
                            static_cast<uint32_t>(p.nb), static_cast<uint32_t>(p.ncp),

@@ -79,9 +79,10 @@ struct GemmShape {
   static constexpr int kRows = kRowTiles * kGemmTileRows;
   static constexpr int kCpw = kCols / (kGemmEpilogueWarps / 4);  // columns of an epilogue warp
   static constexpr int kBlockCols = kRowTiles * kCols;           // TMEM columns of one block's accumulators
-  // A chunk is what a thread loads from TMEM at a time, 32 registers (16 where a stage is no more than that):
+  // A chunk is what a thread loads from TMEM at a time, 32 registers (16 in halves and where a stage is no more than that):
   // kChunkCols columns of its rows of kChunkBlocks blocks.
-  static constexpr int kChunkRegs = kRowTiles * kCpw * kGemmStageBlocks > 32 ? 32 : 16;
+  static constexpr bool kHalf = kRowTiles == 1 && kCols == 64;
+  static constexpr int kChunkRegs = kRowTiles * kCpw * kGemmStageBlocks > 32 && !kHalf ? 32 : 16;
   static constexpr int kChunkCols = kCpw < kChunkRegs / kRowTiles ? kCpw : kChunkRegs / kRowTiles;
   static constexpr int kChunkBlocks = kChunkRegs / (kRowTiles * kChunkCols);
   static constexpr int kBlockChunks = kCpw / kChunkCols;  // chunks of one block, where it has several
@@ -422,6 +423,9 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
   // way, across hand-overs and stages, so neither the barrier test nor the loads' latency stands
   // between two folds.  A stage is always folded whole: blocks past the last one were read as zeros and
   // add +0 (an accumulator is never -0: it starts as +0 and x + -x is +0).
+  // (A scale serves one row in a half item: twice the registers per chunk, and fetched with their own chunk
+  // they leave more for the rest.  200 x 4096 x 4096 23.1 -> 21.8 us, 150 x 4096 x 11008 60.1 -> 56.1.)
+  constexpr bool kLate = Shape::kHalf;
   if (!open_handover())
     return false;
   open_stage();
@@ -436,7 +440,9 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
       const bool last_of_handover = (i + 1) % Shape::kHandoverChunks == 0;
       if (last_of_handover)
         peek_handover();
-      if (i + 1 < Shape::kChunks)
+      if (kLate)
+        load_scales(i, i & 1);
+      else if (i + 1 < Shape::kChunks)
         load_scales(i + 1, (i + 1) & 1);
       tmem_ld_wait();
       if (last_of_handover)
@@ -452,7 +458,8 @@ __device__ __forceinline__ bool gemm_epilogue_item(const GemmArgs &a, GemmEpilog
             return false;
           open_stage();
           load_chunk(0, 0);
-          load_scales(0, 0);
+          if (!kLate)
+            load_scales(0, 0);
         }
       }
       fold_chunk(i, i & 1);

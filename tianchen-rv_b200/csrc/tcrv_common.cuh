@@ -74,10 +74,10 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t stream,
                               Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(static_cast<unsigned>(block));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
