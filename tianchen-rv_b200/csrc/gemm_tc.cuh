@@ -517,8 +517,6 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
   constexpr uint32_t idesc = umma_idesc_e4m3(kGemmTileRows, Shape::kCols);
   const uint32_t nkb = (a.nb + kGemmStageBlocks - 1) / kGemmStageBlocks;
   for (uint32_t kb = 0; kb < nkb; ++kb) {
-    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_full[c.ps.stage], c.ps.phase, c.abort_flag)))
-      return false;
     // Operand descriptors of the stage's first block; a block further along K is 32 bytes
     // further inside the 128-byte swizzled rows, i.e. +2 in the descriptor's 16-byte
     // address field.
@@ -529,6 +527,10 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
 #pragma unroll
     for (uint32_t kk = 0; kk < kGemmStageBlocks; kk += Shape::kHandover) {
       if (c.ts.stage % kGemmMmaWarps == c.mma_warp) {
+        // Only the operands that this warp issues from are waited for: the epilogue hands a stage back when
+        // its accumulators have come, so it holds a stage for the warp that makes those and for no other.
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_full[c.ps.stage], c.ps.phase, c.abort_flag)))
+          return false;
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.tmem_empty[c.ts.stage], c.ts.phase ^ 1, c.abort_flag)))
           return false;
         tcgen05_fence_after_thread_sync();
