@@ -50,8 +50,8 @@ inline void tcgen05_fence_after_thread_sync() {}
 inline uint64_t umma_desc_k_major_sw128(uint32_t) { return 0; }
 inline bool elect_one() { return true; }
 constexpr uint32_t umma_idesc_e4m3(int, int) { return 0; }
-template <typename... A> inline void umma_f8_first(A...) {}
-template <typename... A> inline void umma_f8_again(A...) {}
+template <typename... A> inline void umma_f8_first(A...) { std::printf("fill\n"); }
+template <typename... A> inline void umma_f8_again(A...) { std::printf("use\n"); }
 template <int N> inline void tmem_ld_32x32b(uint32_t, uint32_t *v) { for (int i = 0; i < N; ++i) v[i] = 0; }
 inline void tmem_ld_wait() {}
 }  // namespace tcrv
@@ -87,7 +87,9 @@ void roles(uint32_t nb, int count, char **items) {
     c.smem_empty = reinterpret_cast<uint64_t *>(8 * 100);
     c.tmem_full = reinterpret_cast<uint64_t *>(8 * 200);
     c.tmem_empty = reinterpret_cast<uint64_t *>(8 * 300);
+    c.turn = reinterpret_cast<uint64_t *>(8 * 400);
     c.mma_warp = role;
+    c.turn_phase = role ^ 1;
     for (int i = 0; i < count; ++i) {
       const GemmItem it = {0, 0, items[i][0] == 'w'};
       if (role < 0 && it.whole)
@@ -132,7 +134,7 @@ def record(program, multi, narrow, nb, items):
     out = subprocess.run([program, str(multi), str(narrow), str(nb), *items], check=True, capture_output=True, text=True).stdout
     stages, roles = 0, {}
     for line in out.splitlines():
-        what, number, parity = (line.split() + ["0"])[:3]
+        what, number, parity = (line.split() + ["0", "0"])[:3]
         if what == "stages":
             stages = int(number)
         elif what == "role":
@@ -145,6 +147,7 @@ def record(program, multi, narrow, nb, items):
 def play(roles, late):
     """Every role runs as far as it can before `late` makes one step; the roles that never finish."""
     phase, at = {}, dict.fromkeys(roles, 0)  # completed phases of a barrier; next step of a role
+    filled = [None]  # whose A operand is in the tensor core's buffer
 
     def step(role):
         if at[role] == len(roles[role]):
@@ -152,6 +155,10 @@ def play(roles, late):
         what, bar, parity = roles[role][at[role]]
         if what == "arrive":
             phase[bar] = phase.get(bar, 0) + 1
+        elif what == "fill":
+            filled[0] = role
+        elif what == "use":
+            assert filled[0] == role, "another warp's MMA came between the two that share an operand"
         elif phase.get(bar, 0) % 2 == parity:
             return False
         at[role] += 1

@@ -106,6 +106,7 @@ struct GemmPlan {
   static constexpr uint32_t kColParts = Full::kCols / Half::kCols;
   static constexpr uint32_t kParts = Full::kRowTiles * kColParts;
   static constexpr int kTmemStages = kNarrow != 0 ? 4 : 2;
+  static_assert(kTmemStages % kGemmMmaWarps == 0, "the MMA warps take turns");
   static constexpr int kTmemStageCols = kGemmTmemCols / kTmemStages;
   static_assert(Full::kBlockCols * Full::kHandover <= kTmemStageCols, "a hand-over fits a TMEM stage");
   static_assert(Half::kBlockCols * Half::kHandover <= kTmemStageCols, "a hand-over fits a TMEM stage");
@@ -251,11 +252,12 @@ __device__ __forceinline__ void fold_part(const uint32_t *v, uint64_t (&acc)[Sha
 struct GemmEpilogueCtx {
   uint8_t *stages;
   uint8_t *out_stage;
-  uint64_t *smem_full, *smem_empty, *tmem_full, *tmem_empty, *store_bar;
+  uint64_t *smem_full, *smem_empty, *tmem_full, *tmem_empty, *store_bar, *turn;
   volatile uint32_t *abort_flag;
   uint32_t tmem_base;
   uint32_t store_syncs;  // syncs of the epilogue warps done so far (parity of the next one)
   uint32_t mma_warp;     // an MMA warp fills the TMEM stages of its parity
+  uint32_t turn_phase;   // parity of its next turn
   PipeState ps, ts;
 };
 
@@ -531,6 +533,11 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
         // its accumulators have come, so it holds a stage for the warp that makes those and for no other.
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_full[c.ps.stage], c.ps.phase, c.abort_flag)))
           return false;
+        // An MMA that takes A from the operand buffer has to follow the one that put it there: no MMA of the
+        // other warp may come between, so the hand-overs' MMAs are issued one after another.
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.turn[c.mma_warp], c.turn_phase, c.abort_flag)))
+          return false;
+        c.turn_phase ^= 1;
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.tmem_empty[c.ts.stage], c.ts.phase ^ 1, c.abort_flag)))
           return false;
         tcgen05_fence_after_thread_sync();
@@ -549,6 +556,8 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
             }
           }
           umma_commit(&c.tmem_full[c.ts.stage]);
+          tcgen05_fence_before_thread_sync();
+          mbar_arrive(&c.turn[c.mma_warp ^ 1]);
         }
         __syncwarp();
       }
@@ -580,7 +589,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   c.tmem_empty = c.tmem_full + Plan::kTmemStages;
   uint64_t *drain_bar = c.tmem_empty + Plan::kTmemStages;
   c.store_bar = drain_bar + 1;
-  uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(c.store_bar + 1);
+  c.turn = c.store_bar + 1;
+  uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(c.turn + kGemmMmaWarps);
   c.abort_flag = tmem_base_slot + 1;
   const uint32_t stage_base_addr = (smem_addr(smem_raw) + kGemmCtrlBytes + 1023u) & ~1023u;
   c.stages = smem_raw + (stage_base_addr - smem_addr(smem_raw));
@@ -603,6 +613,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     mbar_init(drain_bar, kGemmMmaWarps);
     mbar_init(c.store_bar, kGemmEpilogueWarps);
+    for (int i = 0; i < kGemmMmaWarps; ++i)
+      mbar_init(&c.turn[i], 1);
     *c.abort_flag = 0;
     mbar_fence_init();
   }
@@ -691,6 +703,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // Two warps take turns at the TMEM stages: one warp's wait, wait, issue and commit for a hand-over
       // (640 cycles) is longer than what eight MMAs take (240 to 300).
       c.mma_warp = static_cast<uint32_t>(warp - kGemmEpilogueWarps - 1);
+      c.turn_phase = c.mma_warp ^ 1;  // the first turn is warp 9's
       for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
         const GemmItem it = gemm_item<kNarrow>(a, idx);
         if (it.n0 >= a.nr || it.m0 >= a.nc)
