@@ -29,3 +29,17 @@ def test_long_rows_several_columns(cuda, pkg, O, q8w, nr, k, nc, pad, shift):
     assert np.array_equal(np.ascontiguousarray(got[:nr, :nc]).view(np.uint32),
                           O.gemv_ksplit_order(w, x, q8w).view(np.uint32))
     assert np.all(got[nr] == -1.0) and np.all(got[:, nc] == -1.0)
+
+
+@pytest.mark.parametrize("q8w,nr,k,nc,stride", [(False, 18, 4352, 5, 1 << 27), (True, 17, 4352, 4, (1 << 28) + 16)])
+def test_rows_far_apart_keep_the_order_of_near_ones(cuda, pkg, O, q8w, nr, k, nc, stride):
+    w = (O.quantize_q8_0 if q8w else O.quantize_q4_0)(O.fill_normal(nr * k, 63, 0, 0.02).reshape(nr, k))
+    x = O.quantize_q8_0(O.fill_normal(nc * k, 64).reshape(nc, k))
+    room = cuda.empty((nr - 1) * stride + w.shape[1], dtype=cuda.uint8, device="cuda")  # 2.3 and 4.3 GB
+    wd = room.as_strided(w.shape, (stride, 1))
+    wd.copy_(cuda.from_numpy(w))
+    xd = cuda.from_numpy(x).cuda()
+    assert pkg.gemv_fold_order(wd, xd, q8_weights=q8w) == 2
+    got = pkg.gemv(wd, xd, q8_weights=q8w)
+    pkg.check_device_errors()
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), O.gemv_ksplit_order(w, x, q8w).view(np.uint32))

@@ -203,12 +203,12 @@ constexpr int kAnyMinRows = 8;
 
 // Whether the chunk-wise tensor-core kernel takes these rows.  Its order (16-way K split) is what such calls
 // promise (gemv_fold_order), so the line stays where it was first drawn, by what fitted into shared memory:
-// 12288 elements of Q4_0, 5888 of Q8_0.  (A lane's 32-bit offsets reach over the 16 rows of a group.)
+// 12288 elements of Q4_0, 5888 of Q8_0.
 template <bool kQ8W>
-bool mma_chunks_take(uint32_t nb, size_t bx) {
+bool mma_chunks_take(uint32_t nb) {
   constexpr uint32_t kMaxBlocks = kQ8W ? 184 : 384;
   static_assert(kMmaMaxBlocks<kQ8W> >= kMaxBlocks, "chunks of a warp");
-  return nb <= kMaxBlocks && bx < (size_t{1} << 27);
+  return nb <= kMaxBlocks;
 }
 
 template <bool kQ8W>
@@ -227,18 +227,19 @@ int launch_mma(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t 
   args.static_weights = (flags & TCRV_CUDA_FLAG_STATIC_WEIGHTS) ? 1u : 0u;
   args.x_aligned = multiple_of(vy, 16) && (nc == 1 || by % 16 == 0) ? 1u : 0u;
   static_assert(kMmaSmemBytes<kQ8W> <= kMaxDynamicSmem, "two ring positions per warp");
-  static std::atomic<bool> configured[64];
+  const bool far = bx >= kMmaFarStride;
+  const auto kernel = far ? gemv_mma_kernel<kQ8W, true> : gemv_mma_kernel<kQ8W, false>;
+  static std::atomic<bool> configured[64][2];
   int dev = 0;
   TCRV_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 64 && !configured[dev]) {
-    TCRV_CUDA_TRY(cudaFuncSetAttribute(gemv_mma_kernel<kQ8W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kMmaSmemBytes<kQ8W>));
-    configured[dev] = true;
+  if (dev < 64 && !configured[dev][far]) {
+    TCRV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemBytes<kQ8W>));
+    configured[dev][far] = true;
   }
   // as many groups for every CTA as the most loaded one has to take: no more CTAs than that fetch the columns
   const size_t groups = (nr + kMmaRows - 1) / kMmaRows, sms = static_cast<size_t>(sm_count());
   const size_t share = (groups + sms - 1) / sms;
-  TCRV_CUDA_TRY(launch_pdl(gemv_mma_kernel<kQ8W>, static_cast<int>((groups + share - 1) / share), kMmaThreads,
+  TCRV_CUDA_TRY(launch_pdl(kernel, static_cast<int>((groups + share - 1) / share), kMmaThreads,
                            kMmaSmemBytes<kQ8W>, stream, args));
   return TCRV_CUDA_OK;
 }
@@ -492,7 +493,7 @@ int gemv_fold_order(size_t n, size_t nc, const void *vx, size_t bx, const void *
   const bool bulk = nb > 0 && nb % 8 == 0 && nc <= kGemvMaxCols && multiple_of(vx, 16) && bx % 16 == 0 &&
                     multiple_of(vy, 2) && by % 2 == 0;
   if (bulk && (nc >= kMmaMinCols || (flags & 0x4000u) != 0) && (flags & 0x1000u) == 0 &&
-      (mma_rows_ring<kQ8W>(nb) >= 2 || mma_chunks_take<kQ8W>(nb, bx)))
+      (mma_rows_ring<kQ8W>(nb) >= 2 || mma_chunks_take<kQ8W>(nb)))
     return TCRV_CUDA_ORDER_KSPLIT16;
   return TCRV_CUDA_ORDER_LANE_PAIRS;
 }
@@ -530,7 +531,7 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
       // rows of up to 4096 elements come in as whole rows (flags bit 13 keeps the chunk-wise form: tuning)
       if ((flags & 0x2000u) == 0 && mma_rows_ring<kQ8W>(nb) >= 2)
         return launch_mma_rows<kQ8W>(n, s, vx, vy, by, nr, nc, bx, bs, flags, stream);
-      if (mma_chunks_take<kQ8W>(nb, bx))
+      if (mma_chunks_take<kQ8W>(nb))
         return launch_mma<kQ8W>(n, s, vx, vy, by, nr, nc, bx, bs, flags, stream);
     }
     StreamPlan plan;
