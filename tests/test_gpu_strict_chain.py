@@ -26,3 +26,40 @@ def test_long_rows_in_the_reference_order(cuda, pkg, O, q8w, nb, nc):
     got = pkg.gemv(cuda.from_numpy(w).cuda(), cuda.from_numpy(x).cuda(), q8_weights=q8w, flags=pkg.FLAG_STRICT_ORDER).cpu().numpy()
     pkg.check_device_errors()
     assert np.array_equal(got.view(np.uint32), O.gemm(w, x, q8_weights=q8w, fold=O.FOLD_FMA).view(np.uint32))
+
+
+# Five-bit codes against one column: items that divide the workers of the table per CTA and items that do not
+# (activations at an odd address leave only that kernel), and rows of many blocks, with either table.
+@pytest.mark.parametrize("fmt,nr,nb,odd", [(2, 4099, 40, 1), (3, 2500, 128, 1), (2, 70, 824, 1), (3, 600, 872, 1), (2, 70, 1920, 0), (3, 20, 2000, 0)])
+def test_fifth_bits_against_one_column(cuda, pkg, O, fmt, nr, nb, odd):
+    w, x = sd.make(fmt, nr, 1, nb, 990 + fmt + nb)
+    wd = cuda.from_numpy(w).cuda()
+    xd = cuda.zeros(x.shape[1] + odd, dtype=cuda.uint8, device="cuda")[odd:]
+    xd.copy_(cuda.from_numpy(x[0]))
+    out = cuda.full((nr, 1), float("nan"), dtype=cuda.float32, device="cuda")
+    assert pkg.lib().tcrv_cuda_sibling_dot_rows(fmt, nb * 32, out.data_ptr(), wd.data_ptr(), xd.data_ptr(), x.shape[1], nr, 1,
+                                                w.shape[1], 1, cuda.cuda.current_stream().cuda_stream) == 0
+    pkg.check_device_errors()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), O.sibling_dot_rows(fmt, w, x).view(np.uint32))
+
+
+def us_per_call(cuda, pkg, fmt, nr, nb, nc):
+    """Time of a call; formats as in strict_stream.cuh (4: Q4_0 in the strict order)."""
+    import graph_time
+
+    wb, ab = {1: (20, 36), 2: (22, 34), 3: (24, 36), 4: (18, 34)}[fmt]
+    w = cuda.randint(0, 60, (nr * nb * wb,), dtype=cuda.uint8, device="cuda")
+    x = cuda.randint(0, 60, (nc * nb * ab,), dtype=cuda.uint8, device="cuda")
+    out = cuda.empty(nr * nc, device="cuda")
+    args = (nb * 32, out.data_ptr(), w.data_ptr(), x.data_ptr(), nb * ab, nr, nc, nb * wb, nc)
+    L = pkg.lib()
+    if fmt == 4:
+        return graph_time.us(cuda, lambda st: L.tcrv_cuda_gemv_q4_0_q8_0(*args, pkg.FLAG_STRICT_ORDER, st))
+    return graph_time.us(cuda, lambda st: L.tcrv_cuda_sibling_dot_rows(fmt, *args, st))
+
+
+@pytest.mark.parametrize("nr,nb", [(64, 1920), (2048, 1536)])
+def test_fifth_bits_do_not_keep_long_rows_off_the_streaming_kernels(cuda, pkg, nr, nb):
+    # (Q4_1 has no fifth bits: with bit planes in shared memory these took 5.6 and 2.0 times as long as it does; now 1.08 and 1.06)
+    four, five = us_per_call(cuda, pkg, 1, nr, nb, 1), us_per_call(cuda, pkg, 2, nr, nb, 1)
+    assert five < 1.6 * four, f"{five:.2f} us with fifth bits, {four:.2f} without"

@@ -59,11 +59,10 @@ __host__ __device__ inline uint32_t any_units(uint32_t nb) {
 }
 __host__ __device__ inline uint32_t any_padded(uint32_t nb) { return (nb + 3) / 4 * 4; }
 // a column: kUnit * 2 planes of 16 bytes per item, then scale and integer sum (or s) per block
-// (where the block's sum starts, or s); for one column against five-bit codes also the words that meet the fifth bits
+// (where the block's sum starts, or s)
 template <int kFormat>
-__host__ __device__ inline uint32_t any_xcol_bytes(uint32_t nb, bool one) {
-  const uint32_t planes = any_units<kFormat>(nb) * AnyFormat<kFormat>::kUnit * 32u;
-  return planes + any_padded(nb) * 8u + (one && StrictFormat<kFormat>::kQh != 0 ? planes : 0u);
+__host__ __device__ inline uint32_t any_xcol_bytes(uint32_t nb) {
+  return any_units<kFormat>(nb) * AnyFormat<kFormat>::kUnit * 32u + any_padded(nb) * 8u;
 }
 template <int kFormat>
 __host__ __device__ inline uint32_t any_table_bytes(uint32_t nb, uint32_t rps, uint32_t cols) {
@@ -148,7 +147,6 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
   using F = StrictFormat<kFormat>;
   using A = AnyFormat<kFormat>;
   constexpr uint32_t U = A::kUnit, UW = A::kUnitWords;
-  constexpr bool kBits = kCols == 1 && F::kQh != 0;  // the fifth bits are dotted on their own
   const uint32_t nb = a.nb, units = any_units<kFormat>(nb), nbp = any_padded(nb), pitch = nbp + 4u;
   const uint32_t ncols = kCols == 1 ? 1u : a.nc;
   const uint32_t *base[kRows];
@@ -193,16 +191,6 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
         x = *xp;
       else
         any_load_x<kFormat>(x, xsm + static_cast<size_t>(c) * xcol_bytes, units, nbp, p);
-      uint32_t xb[U][8] = {};
-      if constexpr (kBits) {
-        const uint4 *planes = reinterpret_cast<const uint4 *>(xsm + units * U * 32u + nbp * 8u);
-#pragma unroll
-        for (uint32_t h = 0; h < U; ++h) {
-          const uint4 lo = planes[(2 * h) * units + p], hi = planes[(2 * h + 1) * units + p];
-          xb[h][0] = lo.x, xb[h][1] = lo.y, xb[h][2] = lo.z, xb[h][3] = lo.w;
-          xb[h][4] = hi.x, xb[h][5] = hi.y, xb[h][6] = hi.z, xb[h][7] = hi.w;
-        }
-      }
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
         float term[U], pr[U];
@@ -211,7 +199,9 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
           AnyBlock b;
           any_block<kFormat>(w[r], h, b);
           const float dw = half_bits_to_float(b.d);
-          const float fs = strict_dot<kFormat, kCols == 1>(b.q, b.qh, x.y[h], xb[h],
+          // (five-bit codes are merged for one column too: the words that their fifth bits would meet cost a
+          // third of the rings on long rows, us: Q5_0 2048 x 49152 66 -> 126, or the kernel: 64 x 61440 14 -> 75)
+          const float fs = strict_dot<kFormat, kCols == 1 && F::kQh == 0>(b.q, b.qh, x.y[h], x.y[h],
                                                            F::kFold == kFoldMin ? kStrictMagicBits : x.s[h]);
           pr[h] = 0.0f;
           if constexpr (!kStrict) {
@@ -312,7 +302,7 @@ __device__ __forceinline__ void gemv_any_body(const GemvAnyArgs &a, uint32_t cta
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);
   uint8_t *xsm = smem + kAnyBarrierBytes;
   const uint32_t nb = a.nb, units = any_units<kFormat>(nb), nbp = any_padded(nb);
-  const uint32_t xcol_bytes = any_xcol_bytes<kFormat>(nb, kCols == 1);
+  const uint32_t xcol_bytes = any_xcol_bytes<kFormat>(nb);
   const uint32_t ncols = kCols == 1 ? 1u : a.nc;
   uint8_t *tables = xsm + static_cast<size_t>(ncols) * xcol_bytes;
   uint8_t *slots = tables + static_cast<size_t>(a.nwarps) * a.table_bytes;
@@ -402,13 +392,6 @@ __device__ __forceinline__ void gemv_any_body(const GemvAnyArgs &a, uint32_t cta
       uint4 *planes = reinterpret_cast<uint4 *>(xcol);
       planes[(2 * h) * units + p] = make_uint4(q[0], q[1], q[2], q[3]);
       planes[(2 * h + 1) * units + p] = make_uint4(q[4], q[5], q[6], q[7]);
-      if constexpr (kCols == 1 && F::kQh != 0) {
-        uint32_t b[8];
-        strict_bit_planes(q, b);
-        planes = reinterpret_cast<uint4 *>(xcol + units * U * 32u + nbp * 8u);
-        planes[(2 * h) * units + p] = make_uint4(b[0], b[1], b[2], b[3]);
-        planes[(2 * h + 1) * units + p] = make_uint4(b[4], b[5], b[6], b[7]);
-      }
     }
     reinterpret_cast<float *>(xcol + units * U * 32u)[ib] = d;
     reinterpret_cast<uint32_t *>(xcol + units * U * 32u + nbp * 4u)[ib] = third;
@@ -530,7 +513,7 @@ bool plan_gemv_any(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, siz
   const uint32_t cols = static_cast<uint32_t>(nc);
   // (a lane reads whole items, one word ahead: up to 60 bytes past the end of a row)
   const size_t pitch = (row_bytes + 15) / 16 * 16 + 64;
-  const size_t fixed = kAnyBarrierBytes + nc * static_cast<size_t>(any_xcol_bytes<kFormat>(nb, nc == 1));
+  const size_t fixed = kAnyBarrierBytes + nc * static_cast<size_t>(any_xcol_bytes<kFormat>(nb));
   // rows per slot as in gemv_stream.cuh: four chains side by side on short rows and one column,
   // two up to 4 columns, one beyond (registers); fewer when the slots do not fit
   size_t rps = nc == 1 ? (row_bytes <= 4096 ? 4 : 2) : (nc <= 4 ? 2 : 1);

@@ -201,10 +201,7 @@ struct StrictStreamArgs {
 };
 
 // shared-memory pieces: word planes, scale and (Q8_1) sum of every column; the term tables
-// (and, for one column against five-bit codes, the words that meet the fifth bits)
-__host__ __device__ inline size_t strict_x_bytes(uint32_t nb, uint32_t nc, bool bits) {
-  return (static_cast<size_t>(nc) * 10 + (bits && nc == 1 ? 8 : 0)) * nb * 4;
-}
+__host__ __device__ inline size_t strict_x_bytes(uint32_t nb, uint32_t nc) { return static_cast<size_t>(nc) * nb * 10 * 4; }
 // (a row's pitch: 16 bytes times an odd number, so that the folding lanes' 16-byte loads are free of conflicts)
 __host__ __device__ inline uint32_t strict_pitch(uint32_t nb) { return nb + 4; }
 __host__ __device__ inline size_t strict_table_floats(uint32_t nb, uint32_t nc, uint32_t rps, bool two) {
@@ -213,11 +210,26 @@ __host__ __device__ inline size_t strict_table_floats(uint32_t nb, uint32_t nc, 
 template <int kFormat>
 __host__ __device__ inline size_t strict_slots_offset(uint32_t nb, uint32_t nc, uint32_t rps) {
   using F = StrictFormat<kFormat>;
-  return (128 + strict_x_bytes(nb, nc, F::kQh != 0) +
+  return (128 + strict_x_bytes(nb, nc) +
           2 * strict_table_floats(nb, nc, rps, F::kFold == kFoldProduct) * 4 + 127) / 128 * 128;
 }
 
-// kOneCol: a.nc == 1, known at compile time (the common decode case: no column loops).
+// Work items of a row of nb blocks (see kPairs below), and whether they divide the workers: a worker then meets
+// the same blocks of the column in every row.
+template <int kFormat>
+__host__ __device__ inline uint32_t strict_units(uint32_t nb) {
+  return StrictFormat<kFormat>::kW % 4 != 0 ? nb / 2 : nb;
+}
+template <int kFormat>
+__host__ __device__ inline bool strict_fixed(uint32_t nb) {
+  return kStrictWorkers % strict_units<kFormat>(nb) == 0;
+}
+
+// kOneCol: a.nc == 1, known at compile time (the common decode case: no column loops).  Five-bit codes take it
+// where strict_fixed() holds: the words that meet their fifth bits are kept in registers only.  (Beside the
+// activations in shared memory they cost 32 bytes a block, that is rows of a slot, and a load each time: 11008
+// rows, us with them there / with the codes merged: Q5_0 K 9472 23.7 / 22.8, K 13568 35.8 / 31.5; in registers, K 4096
+// 10.0 / 12.0.)
 template <int kFormat, bool kOneCol>
 __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const StrictStreamArgs a) {
   using F = StrictFormat<kFormat>;
@@ -246,9 +258,8 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
   uint32_t *xq = reinterpret_cast<uint32_t *>(smem + 128);  // [nc][8][nb]
   float *xd = reinterpret_cast<float *>(xq + static_cast<size_t>(nc) * 8 * nb);  // [nc][nb]
   float *xs = xd + static_cast<size_t>(nc) * nb;                                  // [nc][nb] (Q8_1: s = d * sum(q))
-  uint32_t *xb = reinterpret_cast<uint32_t *>(xs + static_cast<size_t>(nc) * nb);  // kBits: [8][nb]
   const uint32_t pitch = strict_pitch(nb);
-  float *table = reinterpret_cast<float *>(xb + (kBits ? 8 : 0) * nb);  // [2][kTwo ? 2 : 1][nc][rps][pitch]
+  float *table = xs + static_cast<size_t>(nc) * nb;  // [2][kTwo ? 2 : 1][nc][rps][pitch]
   const size_t plane = static_cast<size_t>(nc) * rps * pitch;  // one table of one buffer
   const size_t table_floats = plane * (kTwo ? 2 : 1);
   uint8_t *slots = smem + strict_slots_offset<kFormat>(nb, nc, rps);
@@ -358,18 +369,11 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
       xs[col * nb + at] = half_bits_to_float(static_cast<unsigned short>(half_at(2)));
     else
       xs[col * nb + at] = __uint_as_float(strict_start<kFormat>(F::kBias != 0 ? strict_ysum(yw) : 0));
-    if constexpr (kBits) {
-      uint32_t yb8[8];
-      strict_bit_planes(yw, yb8);
-#pragma unroll
-      for (int w = 0; w < 8; ++w)
-        xb[w * nb + at] = yb8[w];
-    }
   }
   asm volatile("bar.sync 1, %0;" ::"r"(kStrictWorkers) : "memory");  // the workers only
 
   // one column and an item index that is the same in every row: the activation blocks live in registers
-  const bool fixed = kOneCol && kStrictWorkers % units == 0;
+  const bool fixed = kOneCol && (kBits || strict_fixed<kFormat>(nb));
   uint32_t yfix[kUnit][8], bfix[kUnit][8] = {};
   float dfix[kUnit], sfix[kUnit];
   if (fixed) {
@@ -379,11 +383,8 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
 #pragma unroll
       for (int w = 0; w < 8; ++w)
         yfix[h][w] = xq[w * nb + at];
-      if constexpr (kBits) {
-#pragma unroll
-        for (int w = 0; w < 8; ++w)
-          bfix[h][w] = xb[w * nb + at];
-      }
+      if constexpr (kBits)
+        strict_bit_planes(yfix[h], bfix[h]);
       dfix[h] = xd[kUnit * (tid % units) + h], sfix[h] = xs[at];
     }
   }
@@ -418,11 +419,6 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
 #pragma unroll
           for (int w = 0; w < 8; ++w)
             y[w] = xq[(static_cast<size_t>(col) * 8 + w) * nb + at];
-          if constexpr (kBits) {
-#pragma unroll
-            for (int w = 0; w < 8; ++w)
-              yb8[w] = xb[w * nb + at];
-          }
           dy = xd[col * nb + ib], sy = xs[col * nb + at];
         }
         const float fs = strict_dot<kFormat, kOneCol>(q, qh, y, yb8, F::kFold == kFoldMin ? kStrictMagicBits : __float_as_uint(sy));
@@ -532,7 +528,8 @@ int launch_strict_stream(size_t n, float *s, const uint8_t *vx, const uint8_t *v
   }
   const size_t slots = (nr + rps - 1) / rps;
   const size_t grid = slots < static_cast<size_t>(sms) ? slots : static_cast<size_t>(sms);
-  TCRV_CUDA_TRY(launch_pdl(nc == 1 ? strict_stream_kernel<kFormat, true> : strict_stream_kernel<kFormat, false>,
+  const bool one = nc == 1 && (F::kQh == 0 || strict_fixed<kFormat>(nb));
+  TCRV_CUDA_TRY(launch_pdl(one ? strict_stream_kernel<kFormat, true> : strict_stream_kernel<kFormat, false>,
                            static_cast<int>(grid), kStrictThreads, smem, stream, args));
   return TCRV_CUDA_OK;
 }
