@@ -63,3 +63,25 @@ def test_fifth_bits_do_not_keep_long_rows_off_the_streaming_kernels(cuda, pkg, n
     # (Q4_1 has no fifth bits: with bit planes in shared memory these took 5.6 and 2.0 times as long as it does; now 1.08 and 1.06)
     four, five = us_per_call(cuda, pkg, 1, nr, nb, 1), us_per_call(cuda, pkg, 2, nr, nb, 1)
     assert five < 1.6 * four, f"{five:.2f} us with fifth bits, {four:.2f} without"
+
+
+# slots of three and more rows that are no multiple of four, rows for which there is hardly room, fewer rows than a
+# slot holds (activations at an odd address leave only this kernel)
+@pytest.mark.parametrize("fmt,nr,nb,nc", [(2, 1300, 392, 4), (1, 1250, 392, 6), (2, 900, 256, 7), (3, 2100, 96, 3), (2, 149, 896, 1), (3, 150, 64, 2)])
+def test_slots_of_any_number_of_rows(cuda, pkg, O, fmt, nr, nb, nc):
+    w, x = sd.make(fmt, nr, nc, nb, 1010 + fmt + nb)
+    wd = cuda.from_numpy(w).cuda()
+    xd = cuda.zeros((nc, x.shape[1] + 1), dtype=cuda.uint8, device="cuda")[:, 1:]
+    xd.copy_(cuda.from_numpy(x))
+    out = cuda.full((nr, nc), float("nan"), dtype=cuda.float32, device="cuda")
+    assert pkg.lib().tcrv_cuda_sibling_dot_rows(fmt, nb * 32, out.data_ptr(), wd.data_ptr(), xd.data_ptr(), xd.stride(0), nr, nc,
+                                                w.shape[1], nc, cuda.cuda.current_stream().cuda_stream) == 0
+    pkg.check_device_errors()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), O.sibling_dot_rows(fmt, w, x).view(np.uint32))
+
+
+@pytest.mark.parametrize("fmt,nr,nb,more,nc", [(4, 11008, 144, 152, 8), (4, 11008, 192, 200, 8), (1, 11008, 344, 392, 6)])
+def test_a_little_longer_rows_take_a_little_longer(cuda, pkg, fmt, nr, nb, more, nc):
+    # (lengths at which a slot lost four of its rows or the kernel the call: up to 1.4 times as long)
+    few, many = us_per_call(cuda, pkg, fmt, nr, nb, nc), us_per_call(cuda, pkg, fmt, nr, more, nc)
+    assert many < 1.2 * few * more / nb, f"{few:.2f} us for {nb} blocks, {many:.2f} for {more}"

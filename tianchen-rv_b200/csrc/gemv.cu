@@ -547,7 +547,7 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
       if (const size_t ring = mma_strict_ring<kQ8W>(nb, nr, nc, vx, bx))
         return launch_mma_strict<kQ8W>(n, s, vx, vy, by, nr, nc, bx, bs, flags, ring, stream);
     constexpr int kFormat = kQ8W ? 5 : 4;
-    if (const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx))
+    if (const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx, sm_count()))
       return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sm_count(), stream);
   }
 

@@ -136,7 +136,7 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
         vx, vy, sums, bx, by, static_cast<uint32_t>(nr), static_cast<uint32_t>(nc), nb);
   } else {
     const int sms = sm_count();
-    const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx);  // 0: not for that kernel
+    const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx, sms);  // 0: not for that kernel
     GemvAnyPlan plan;
     const bool any = nr >= 8 && (rps != 0 || !any_tiny(nb, nr, nc, /*strict=*/true, sms)) &&
                      plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true, /*static_weights=*/false, sms, plan);
