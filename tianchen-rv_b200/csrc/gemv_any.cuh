@@ -202,7 +202,7 @@ __device__ __forceinline__ void any_rows(const GemvAnyArgs &a, const uint8_t *sl
           // (five-bit codes are merged for one column too: the words that their fifth bits would meet cost a
           // third of the rings on long rows, us: Q5_0 2048 x 49152 66 -> 126, or the kernel: 64 x 61440 14 -> 75)
           const float fs = strict_dot<kFormat, kCols == 1 && F::kQh == 0>(b.q, b.qh, x.y[h], x.y[h],
-                                                           F::kFold == kFoldMin ? kStrictMagicBits : x.s[h]);
+                                                           F::kBias == 0 ? kStrictMagicBits : x.s[h]);
           pr[h] = 0.0f;
           if constexpr (!kStrict) {
             const float next = kFormat == 5 ? __fmaf_rn(fs, __fmul_rn(dw, x.d[h]), acc[r][c])

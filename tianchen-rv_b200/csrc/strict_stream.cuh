@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_stream_kernel(const 
             y[w] = xq[(static_cast<size_t>(col) * 8 + w) * nb + at];
           dy = xd[col * nb + ib], sy = xs[col * nb + at];
         }
-        const float fs = strict_dot<kFormat, kOneCol>(q, qh, y, yb8, F::kFold == kFoldMin ? kStrictMagicBits : __float_as_uint(sy));
+        const float fs = strict_dot<kFormat, kOneCol>(q, qh, y, yb8, F::kBias == 0 ? kStrictMagicBits : __float_as_uint(sy));
         float *t = ta + col * col_floats + r * pitch + ib;
         if constexpr (F::kFold == kFoldMin) {
           *t = __fmaf_rn(__fmul_rn(dw, dy), fs, __fmul_rn(mw, sy));
