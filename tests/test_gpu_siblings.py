@@ -108,3 +108,32 @@ def test_sibling_calls_take_the_faster_streaming_kernel(cuda, pkg, fmt, nr, nb, 
                                                    nb * wb, nc, st)) for o in (0, 1))
     assert even < 1.1 * odd and odd < 1.6 * even, f"{even:.2f} us at an even address, {odd:.2f} at an odd one"
     pkg.check_device_errors()
+
+
+# calls on both sides of the lines between the two streaming kernels, the shapes whose route was wrong among them
+@pytest.mark.parametrize("fmt,nr,nb,nc", [(1, 11008, 128, 4), (3, 11008, 128, 4), (1, 4096, 128, 3), (2, 1536, 128, 8), (1, 4096, 344, 1), (2, 512, 256, 1),
+                                          (1, 2048, 128, 1), (3, 32000, 128, 1), (2, 11008, 200, 2), (3, 11008, 344, 4), (3, 11008, 128, 8), (2, 512, 128, 8)])
+def test_the_rule_takes_the_faster_of_both(cuda, pkg, fmt, nr, nb, nc):
+    # weights off 16-byte boundaries leave only the table per warp, activations at an odd address only the one per CTA
+    wb, ab = sd.STRIDES[fmt]
+    w = cuda.randint(0, 60, (nr * nb * wb + 4,), dtype=cuda.uint8, device="cuda")
+    x = cuda.randint(0, 60, (nc * nb * ab + 1,), dtype=cuda.uint8, device="cuda")
+    out = cuda.empty(nr * nc, device="cuda")
+    fn = pkg.lib().tcrv_cuda_sibling_dot_rows
+    rule, warp, cta = (graph_time.us(cuda, lambda st: fn(fmt, nb * 32, out.data_ptr(), w.data_ptr() + wo, x.data_ptr() + xo, nb * ab, nr, nc,
+                                                         nb * wb, nc, st)) for wo, xo in ((0, 0), (4, 0), (0, 1)))
+    assert rule < 1.09 * min(warp, cta), f"{rule:.2f} us by the rule, {warp:.2f} with the table per warp, {cta:.2f} per CTA"
+    pkg.check_device_errors()
+
+
+@pytest.mark.parametrize("nr", [300, 1000, 4096])
+def test_one_ring_is_not_for_many_rows(cuda, pkg, nr):
+    # rows of 1920 blocks leave a ring to one warp only; weights at an odd address leave only the general kernel
+    w = cuda.randint(0, 60, (nr * 1920 * 24 + 1,), dtype=cuda.uint8, device="cuda")
+    x = cuda.randint(0, 60, (1920 * 36,), dtype=cuda.uint8, device="cuda")
+    out = cuda.empty(nr, device="cuda")
+    fn = pkg.lib().tcrv_cuda_sibling_dot_rows
+    rule, general = (graph_time.us(cuda, lambda st: fn(3, 61440, out.data_ptr(), w.data_ptr() + o, x.data_ptr(), 1920 * 36, nr, 1, 1920 * 24, 1, st))
+                     for o in (0, 1))
+    assert rule < 1.1 * general, f"{rule:.1f} us by the rule, {general:.1f} on the general kernel"
+    pkg.check_device_errors()

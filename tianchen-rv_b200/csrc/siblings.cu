@@ -97,28 +97,38 @@ __global__ void __launch_bounds__(256) sibling_dot_kernel(const uint8_t *__restr
 }
 
 // Which of the two streaming kernels takes a call that both accept: strict_stream.cuh (a term table per
-// CTA, 512 workers on one slot) or gemv_any.cuh (a table per warp, a row is one warp's work).  One column
-// is the former's unless there are few rows.  With several, the latter wins wherever its lanes and warps
-// have work; they have not, with more than one slot to a warp, where rows have few items (half of the
-// lanes idle), where it folds one row at a time (more than 4 columns), and where shared memory leaves it
-// few rings.  Measured, us, table per CTA / per warp:
-//   1 column     Q5_0 11008 x 4096 10.7 / 12.0, 4096 x 11008 14.3 / 16.6, 20000 x 512 5.1 / 7.7; Q4_1 4096 x 4096 3.8 / 4.3,
-//                4096 x 11008 11.3 / 10.8; Q5_1 32000 x 4096 21.3 / 21.0, 2048 x 8192 6.1 / 6.4
-//   2            Q5_0 32000 x 1024 10.7 / 16.6, 4096 x 4096 6.9 / 6.6, 16000 x 6400 29.1 / 33.4; Q4_1 8192 x 2048 5.5 / 5.9, 11008 x
-//                4096 12.4 / 11.5, 2048 x 8192 7.1 / 6.1, 4096 x 11008 14.0 / 15.7
-//   4            Q5_1 20000 x 512 6.6 / 9.9, 32000 x 1024 14.2 / 14.5, 8192 x 2048 8.5 / 7.6, 11008 x 4096 18.7 / 16.7, 2048 x 8192
-//                9.9 / 11.6, 4096 x 11008 20.6 / 25.1
-//   5..8         as the kernels were before one fold was shortened: Q5_1 32000 x 1024, 5 columns 19.0 / 24.6, 8 columns,
-//                K 2048 40.7 / 42.5; 4096 x 11008, 6 columns (5 rings) 31.7 (now 26.2) / 42.5; 11008 x 4096, 8 columns 30.2 / 28.4
+// CTA, 512 workers on one slot) or gemv_any.cuh (a table per warp, a row is one warp's work).  One column is the
+// former's.  With several the latter wins where each of its warps has its rows in one slot and enough of them
+// have work, and with up to 4 columns at middling row lengths, where its lanes are full and two rows share the
+// columns' loads (not for Q5_0 below 4 columns: its table has two planes).  Both kernels timed on 2304 calls, 3
+// formats x 1..8 columns x 512..32000 rows x K 256..28672, weights from HBM: the rule is 0.4 % over the better
+// one on average, 19 % at worst, always the former 0.7 %, always the latter 21 %.  us, table per CTA / per warp:
+//   1 column   Q5_0 11008 x 4096 9.0 / 12.3, 512 x 8192 3.6 / 5.4; Q4_1 11008 x 4096 8.2 / 9.1, 4096 x 11008 10.8 / 11.0; Q5_1 32000 x
+//              4096 20.0 / 23.1
+//   2          Q4_1 4096 x 4096 6.4 / 6.0, 11008 x 4096 12.2 / 11.6, 4096 x 11008 13.5 / 15.6; Q5_0 11008 x 4096 13.9 / 14.7; Q5_1 11008 x
+//              6400 20.0 / 22.9; Q5_0 1024 x 4096 (a slot to a warp) 3.9 / 3.7
+//   3, 4       Q4_1 4096 x 4096, 3 columns 7.7 / 6.4; 11008 x 4096, 4 columns Q4_1 15.6 / 14.0, Q5_0 19.7 / 18.4, Q5_1 17.9 / 16.9; Q5_1
+//              11008 x 1024 6.7 / 7.0, 11008 x 6400 26.6 / 30.3; Q4_1 11008 x 4608 18.2 / 17.5; Q5_0 32000 x 512, 3 columns 9.3 / 16.8
+//   5..8       Q5_1 11008 x 4096, 8 columns 26.7 / 28.0, 4096 x 11008, 6 columns 25.6 / 41.9; a slot to a warp: Q5_0 1536 x 4096, 8
+//              columns 8.3 / 7.5, but 512 rows 4.7 / 6.5 (Q5_1)
 template <int kFormat>
 bool table_per_cta(const GemvAnyPlan &plan, uint32_t nb, size_t nr, size_t nc, int sms) {
   if (nc == 1)
-    return nr >= 2048;
+    return true;
   const GemvAnyArgs &a = plan.args;
-  const bool slots_to_spare = nr > static_cast<size_t>(sms) * a.nwarps * a.rps;
-  if (nc <= 4)
-    return (slots_to_spare && nb * nc <= 128) || (nb * nc >= 400 && nr * nc >= 8192);
-  return slots_to_spare && (nb * nc <= 340 || a.nwarps <= 6);
+  const size_t blocks = nb * nc, n = static_cast<size_t>(sms);
+  if (nr <= n * a.nwarps * a.rps)
+    return nr < 5 * n || blocks < 256;
+  if (nc > 4 || (kFormat == 2 && nc < 4))
+    return true;
+  return nr < 20 * n || nb > 160 || blocks < 256 || blocks > 600;
+}
+
+// One column against rows so long that shared memory has a ring for one warp only: past seven rows for it the
+// general kernel, which reads them in place, is no slower (us, that one / this: 1000 x 61440 Q4_1 113 / 75, Q5_0 130 / 80,
+// Q5_1 103 / 84; 1184 rows 69 / 85, 77 / 91, 72 / 96; 4096 rows 191 / 287, 226 / 307, 213 / 325).
+inline bool one_ring_too_many_rows(const GemvAnyPlan &plan, size_t nr, size_t nc, int sms) {
+  return nc == 1 && plan.args.nwarps == 1 && nr > 7 * static_cast<size_t>(sms);
 }
 
 template <int kFormat>
@@ -139,7 +149,8 @@ int launch_one(size_t n, float *s, int32_t *sums, const uint8_t *vx, const uint8
     const uint32_t rps = strict_stream_rows<kFormat>(nb, nr, nc, vx, bx, sms);  // 0: not for that kernel
     GemvAnyPlan plan;
     const bool any = nr >= 8 && (rps != 0 || !any_tiny(nb, nr, nc, /*strict=*/true, sms)) &&
-                     plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true, /*static_weights=*/false, sms, plan);
+                     plan_gemv_any<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, /*strict=*/true, /*static_weights=*/false, sms, plan) &&
+                     !one_ring_too_many_rows(plan, nr, nc, sms);
     // (activations at odd addresses are not for the table per warp)
     if (rps != 0 && (!any || table_per_cta<kFormat>(plan, nb, nr, nc, sms)))
       return launch_strict_stream<kFormat>(n, s, vx, vy, by, nr, nc, bx, bs, rps, sms, stream);
