@@ -1,5 +1,9 @@
 """What the build takes for up to date (no compiler runs here)."""
 import os
+import shutil
+import subprocess
+import threading
+import time
 
 import pytest
 
@@ -70,3 +74,85 @@ def test_the_c_library_builds_where_there_is_no_torch(build, pkg, monkeypatch):
     monkeypatch.setattr(b, "build_torch_calls", lambda force=False: pytest.fail("needs torch"))
     monkeypatch.setattr(importlib.util, "find_spec", lambda name: None)
     assert pkg.build_library() == b.LIB and len(ran) == 1
+
+
+def test_a_changed_makefile_rebuilds_the_library(build):
+    # (the compiler's flags are there)
+    b, csrc, now, ran = build
+    makefile = csrc.parent / "Makefile"
+    makefile.write_text("")
+    os.utime(makefile, (now, now))
+    b.build_library()
+    assert ran == []
+    os.utime(makefile, (now + 120, now + 120))
+    b.build_library()
+    assert len(ran) == 1
+
+
+def test_processes_build_one_after_another(build, monkeypatch):
+    b, _, now, ran = build
+    os.remove(b.LIB)
+    inside = []
+
+    def slow_make(cmd, **kw):
+        inside.append(len(inside))
+        time.sleep(0.2)
+        open(b.LIB, "w").close()
+        os.utime(b.LIB, (now + 60, now + 60))
+        ran.append(cmd)
+
+    monkeypatch.setattr(b.subprocess, "run", slow_make)
+    threads = [threading.Thread(target=b.build_library) for _ in range(3)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert len(ran) == 1  # the others found it built
+
+
+@pytest.fixture
+def tree(pkg, tmp_path):
+    """The Makefile on a made-up tree, and a call that runs it with a compiler that only notes what it was asked
+    to make: make(*arguments) -> the names of the files."""
+    tmp_path = tmp_path / "package"
+    for name in ("csrc/gemm.cu", "csrc/gemv.cu", "examples/gpu/decode_loop.cpp", "../include/tcrv_emitc_host.h"):
+        (tmp_path / name).parent.mkdir(parents=True, exist_ok=True)
+        (tmp_path / name).write_text("")
+    shutil.copy(os.path.join(os.path.dirname(pkg._build.__file__), "Makefile"), tmp_path)
+    asked = tmp_path / "asked"
+    for name in ("nvcc", "other"):
+        (tmp_path / name).write_text(f"""#!/bin/sh
+while [ $# -gt 0 ]; do [ "$1" = -o ] && {{ touch "$2"; basename "$2" >> {asked}; }}; shift; done
+""")
+        os.chmod(tmp_path / name, 0o755)
+
+    def make(*args):
+        asked.write_text("")
+        subprocess.run(["make", "-s", "-C", tmp_path, *args], check=True)
+        return sorted(asked.read_text().split())
+
+    return tmp_path, make
+
+
+def test_objects_follow_the_makefile_the_compiler_and_its_flags(tree):
+    path, make = tree
+    everything = ["gemm.o", "gemv.o", "libtcrv_cuda.so"]
+    nvcc = f"NVCC={path}/nvcc"
+    assert make("library", nvcc) == everything and (path / "libtcrv_cuda.so").exists()
+    os.remove(path / "libtcrv_cuda.so")
+    assert make("library", nvcc) == [] and (path / "libtcrv_cuda.so").exists()
+    for age, pattern in ((400, "include/*"), (400, "package/csrc/*"), (400, "package/Makefile"), (300, "package/build/obj/flags"),
+                         (200, "package/build/obj/*.o"), (100, "package/build/obj/*.so")):
+        for f in path.parent.glob(pattern):
+            os.utime(f, (time.time() - age,) * 2)
+    assert make("library", nvcc) == []
+    os.utime(path / "csrc/gemv.cu")
+    assert make("library", nvcc) == ["gemv.o", "libtcrv_cuda.so"]
+    os.utime(path / "Makefile")
+    assert make("library", nvcc) == everything and make("library", nvcc) == []
+    assert make("library", nvcc, "NVCCFLAGS=-O1") == everything
+    assert make("library", f"NVCC={path}/other", "NVCCFLAGS=-O1") == everything
+
+
+def test_the_step_loop_links_the_library_that_is_there(tree):
+    path, make = tree
+    (path / "libtcrv_cuda.so").write_text("")
+    assert make("decode_loop", f"NVCC={path}/nvcc", f"CXX={path}/other") == ["libtcrv_decode_loop.so"]

@@ -7,6 +7,8 @@ beside it with the host compiler.  Run as a script to force a rebuild.
 """
 from __future__ import annotations
 
+import contextlib
+import fcntl
 import glob
 import os
 import shutil
@@ -18,6 +20,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtcrv_cuda.so")
+
 
 def _nvcc() -> str:
     exe = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
@@ -31,14 +34,23 @@ def _stale() -> bool:
         return True
     built = os.path.getmtime(LIB)
     deps = [p for kind in ("*.cu", "*.cuh", "*.h") for p in glob.glob(os.path.join(CSRC, kind))]
-    deps += glob.glob(os.path.join(ROOT, "include", "*.h"))
+    deps += glob.glob(os.path.join(ROOT, "include", "*.h")) + glob.glob(os.path.join(HERE, "Makefile"))
     return any(os.path.getmtime(p) > built for p in deps)
+
+
+@contextlib.contextmanager
+def _one_builder():
+    """Processes that build at the same time share the objects: one after another."""
+    os.makedirs(os.path.join(HERE, "build"), exist_ok=True)
+    with open(os.path.join(HERE, "build", "lock"), "w") as f:
+        fcntl.flock(f, fcntl.LOCK_EX)
+        yield
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return LIB
-    cmd = ["make", "-C", HERE, f"-j{os.cpu_count()}", f"NVCC={_nvcc()}", os.path.basename(LIB)]
+    cmd = ["make", "-C", HERE, f"-j{os.cpu_count()}", f"NVCC={_nvcc()}", "library"]
     if force:
         cmd.insert(1, "-B")
     if verbose:
@@ -46,7 +58,9 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         print(" ".join(cmd), file=sys.stderr)
     else:
         cmd.insert(1, "-s")
-    subprocess.run(cmd, check=True)
+    with _one_builder():
+        if force or _stale():  # (another process may have built it meanwhile)
+            subprocess.run(cmd, check=True)
     return LIB
 
 
