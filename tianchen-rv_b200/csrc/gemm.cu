@@ -414,13 +414,17 @@ int launch_gemm_kernel(const PlanarSizes &p, const uint8_t *weights_planar, cons
   TCRV_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64)
     return TCRV_CUDA_ERR_UNSUPPORTED;
+  const auto kernel = gemm_q4_0_q8_0_tc_kernel<kMulti, kRepack, kNarrow>;
   if (!configured[dev]) {
-    TCRV_CUDA_TRY(cudaFuncSetAttribute(gemm_q4_0_q8_0_tc_kernel<kMulti, kRepack, kNarrow>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // a block that starts with fewer registers than its warps ask for would wait for them for ever
+    cudaFuncAttributes attributes;
+    TCRV_CUDA_TRY(cudaFuncGetAttributes(&attributes, kernel));
+    if (attributes.numRegs * kGemmThreads < kGemmSplitRegs)
+      return TCRV_CUDA_ERR_UNSUPPORTED;
+    TCRV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     configured[dev] = true;
   }
-  TCRV_CUDA_TRY(launch_pdl(gemm_q4_0_q8_0_tc_kernel<kMulti, kRepack, kNarrow>, grid, kGemmThreads, smem, stream, map_w,
-                           map_x, map_xhi, map_dw, map_dx, args));
+  TCRV_CUDA_TRY(launch_pdl(kernel, grid, kGemmThreads, smem, stream, map_w, map_x, map_xhi, map_dw, map_dx, args));
   TCRV_CUDA_TRY(cudaGetLastError());
   return TCRV_CUDA_OK;
 }

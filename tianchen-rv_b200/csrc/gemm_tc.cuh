@@ -69,7 +69,8 @@ constexpr int kGemmThreads = (kGemmEpilogueWarps + 4) * 32;  // TMA, MMA and one
 // The block starts with 384 x 168 registers; the third warpgroup keeps 128 x 40 of them and the epilogue's
 // two take 256 x 216 (60416 of 64512 in all).
 constexpr int kGemmEpilogueRegs = 216, kGemmOtherRegs = 40;
-static_assert(8 * kGemmEpilogueWarps * kGemmEpilogueRegs + 32 * kGemmOtherRegs <= 8 * 12 * 168, "the launch's registers");
+constexpr int kGemmSplitRegs = 32 * (kGemmEpilogueWarps * kGemmEpilogueRegs + 4 * kGemmOtherRegs);
+static_assert(kGemmSplitRegs <= kGemmThreads * 168, "the launch's registers");
 constexpr int kGemmCtrlBytes = 1024;  // barriers, TMEM base, abort flag
 
 // The shape of a work item: kRowTiles x 128 weight rows, kCols activation columns.
