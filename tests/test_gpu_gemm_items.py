@@ -1,6 +1,6 @@
-"""GPU parity, work items of the prefill GEMM: whole, half and narrow items at their edges (rows around
-128 and 256, columns around 32 and 64, block counts that end a stage early) equal the sequential oracle
-bit for bit, with both folds and with several destinations."""
+"""GPU parity, work items of the prefill GEMM: whole items, halves and narrow ones of 32 columns at their edges
+(ragged rows and columns, block counts that end a stage early) equal the sequential oracle bit for bit, with both
+folds and with several destinations.  (test_gpu_gemm_narrow_items.py has those of 16 columns.)"""
 import ctypes
 
 import numpy as np
@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nr,k,nc", [
-    (127, 32, 31), (129, 96, 33), (255, 160, 63), (257, 224, 65), (4096, 416, 77),  # narrow items
+    (127, 32, 31), (129, 96, 33), (255, 160, 63), (257, 224, 65),  # 128 x 16
+    (4096, 416, 77), (4001, 32, 77), (4081, 160, 95), (3900, 96, 97), (4111, 288, 65), (2049, 128, 160),  # 128 x 32
+    (4000, 160, 200), (3969, 32, 193), (4097, 224, 161),  # 256 x 64, all of them cut into halves
     (4864, 160, 512),   # 152 whole items: one round and four items cut into halves
     (4737, 96, 481),    # the same with a second row tile that does not exist and ragged columns
     (20480, 32, 128),   # 160 whole items of one block
@@ -39,9 +41,10 @@ def test_items_at_their_edges_are_bit_exact(cuda, pkg, O, nr, k, nc):
 
 
 # (tokens, weight rows, K): whole items with halves in the last round, a row tile that does not exist with
-# ragged columns, items of one block
-@pytest.mark.parametrize("tokens,rows,k", [(512, 4864, 160), (484, 4752, 96), (128, 20480, 32)])
-def test_whole_items_of_the_repacked_gemm_are_bit_exact(cuda, pkg, O, tokens, rows, k):
+# ragged columns, items of one block; halves only; items of 128 x 32
+@pytest.mark.parametrize("tokens,rows,k", [(512, 4864, 160), (484, 4752, 96), (128, 20480, 32), (200, 4000, 160), (76, 4016, 96), (80, 4112, 32),
+                                           (96, 4208, 288)])
+def test_items_of_the_repacked_gemm_are_bit_exact(cuda, pkg, O, tokens, rows, k):
     w = O.quantize_q4_0(O.fill_normal(rows * k, 53, 0, 0.02).reshape(rows, k))
     x = O.quantize_q8_0(O.fill_normal(tokens * k, 54).reshape(tokens, k))
     wx, xx = O.rows_to_q4_0x16(w), O.rows_to_q8_0x4(x)
