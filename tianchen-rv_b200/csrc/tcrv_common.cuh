@@ -36,16 +36,12 @@ __device__ __forceinline__ void raise_device_error(const DeviceErrorWords &w, in
   }
 }
 
+// Relocatable device code names the words itself.
 #ifdef __CUDACC_RDC__
 extern __device__ int g_device_error;
 extern __device__ int *g_host_error_mirror;
 __device__ __forceinline__ void raise_device_error(int code) {
-  atomicOr(&g_device_error, code);
-  int *mirror = g_host_error_mirror;
-  if (mirror != nullptr) {
-    *reinterpret_cast<volatile int *>(mirror) = code;
-    __threadfence_system();
-  }
+  raise_device_error(DeviceErrorWords{&g_device_error, &g_host_error_mirror}, code);
 }
 #endif
 // The words' addresses on the current device, for kernels that are compiled without relocatable device
