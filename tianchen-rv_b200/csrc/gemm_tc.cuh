@@ -6,8 +6,8 @@
 // Every ggml block (32 elements of K) has its own pair of fp16 scales, so the contraction
 // cannot accumulate across blocks inside the tensor core: each block gets fresh TMEM
 // accumulator tiles (128 weight rows x up to 64 activation columns, K = 32), and the epilogue
-// warps fold them into fp32 register accumulators with the two scales.  The fold runs in strict ascending block order per output element, in
-// the fused form fma((float)S * d_w, d_x, acc).
+// warps fold them into fp32 register accumulators with the two scales.  The fold runs in strict
+// ascending block order per output element, in the fused form fma((float)S * d_w, d_x, acc).
 //
 // The fold on the CUDA cores, not the tensor pipe, bounds this kernel, so the tensor core is
 // asked for the form that is cheapest to fold: the block sum arrives as an fp32 number.
@@ -23,7 +23,7 @@
 // Work items.  256 weight rows x 64 columns: the two row tiles share their columns, so one broadcast
 // load of activation scales serves two outputs of a thread (with 128 x 128 items those loads put 64 KB
 // per block through the shared-memory pipe beside the operands: 305 us for 512 x 32000 x 4096, 640
-// cycles per 128 x 128 x 32 of arithmetic that takes 276; they still cost 40 us of the 256).  8
+// cycles per 128 x 128 x 32 of arithmetic that takes 276; what they still cost stands below).  8
 // epilogue warps with 64 accumulators a thread: with 16 a hand-over's fixed cost is paid twice as often and
 // registers run out (252 us and more instead of 231), with 4 nothing covers a warp's waits (267).
 // Whole items are dealt round-robin to the CTAs; a last round that would leave more than half of
@@ -40,7 +40,9 @@
 //   warps 0..7  epilogue: warp w reads TMEM lanes 32*(w%4).. (its weight rows) and half of the
 //               columns of every accumulator tile
 //   warp 8      TMA producer (one elected lane)
-//   warps 9, 10 MMA issue (one elected lane each), by turns; warp 9 allocates TMEM
+//   warps 9, 10 MMA issue (one elected lane each), by turns; warp 9 allocates TMEM.  Two of a block's MMAs share
+//               A through the tensor core's operand buffer (without it 10 % slower on every shape), so the turns
+//               are kept by barriers: 1.4 % faster on 256 x 64 items, 2 to 4 % slower on 128 x 16
 // Pipelines: shared-memory stages of 4 blocks each (full/empty mbarriers) and TMEM stages of
 // several blocks each (full/empty mbarriers).  The epilogue warps wait on the accumulator barriers
 // only: a stage's scale tiles have landed when its first accumulator has.
@@ -48,7 +50,7 @@
 // What bounds it: per 256 x 64 block of outputs the fold's 128 packed operations a warp pair take about
 // 320 cycles of a scheduler's FMA pipe (a packed FMA of three different register pairs takes 3 cycles, not
 // 2), and the scale loads' 256 and the MMA operands' 128 cycles share the shared-memory pipe: without
-// the scale loads 210, without MMAs 206 of 230 us (512 x 32000 x 4096, operands in L2).  With one MMA warp,
+// the scale loads 210, without MMAs 206 of 230 us (512 x 32000 x 4096, operands in L2, before the turns).  With one MMA warp,
 // 16-register chunks and a single-lane producer it was 250; 512 x 11008 x 4096 92.7 -> 88.2 us, 77 x 4096 x
 // 11008 41.6 -> 32.5 us (there the producer's 780 cycles per stage were the limit).  32-register chunks need
 // more than the 168 registers a thread starts with; without setmaxnreg, 16-register chunks: 244 us.

@@ -226,7 +226,7 @@ int launch_mma(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t 
   args.nb = static_cast<uint32_t>(n / kQK);
   args.static_weights = (flags & TCRV_CUDA_FLAG_STATIC_WEIGHTS) ? 1u : 0u;
   args.x_aligned = multiple_of(vy, 16) && (nc == 1 || by % 16 == 0) ? 1u : 0u;
-  static_assert(kMmaSmemBytes<kQ8W> <= kMaxDynamicSmem, "two ring positions per warp");
+  static_assert(kMmaSmemBytes<kQ8W> <= kMaxDynamicSmem, "the ring of every warp");
   const bool far = bx >= kMmaFarStride;
   const auto kernel = far ? gemv_mma_kernel<kQ8W, true> : gemv_mma_kernel<kQ8W, false>;
   static std::atomic<bool> configured[64][2];
@@ -512,9 +512,11 @@ int launch_gemv(size_t n, float *s, const uint8_t *vx, const uint8_t *vy, size_t
   const bool bulk = nb > 0 && nb % 8 == 0 && nc <= kGemvMaxCols && multiple_of(vx, 16) && bx % 16 == 0 &&
                     multiple_of(vy, 2) && by % 2 == 0;
   // One or two columns in the reference's order: the streaming kernel with a term table per
-  // warp; also three columns of Q4_0 weights on rows too long for the tensor-core form
-  // (4096x11008: 16.7 us against 20.7).  Flags bit 13 keeps the table-per-CTA / tensor-core
-  // kernels, bit 14 takes this one for any 3 columns: tuning.
+  // warp; also three columns of Q4_0 weights on rows too long for the tensor-core form.  us, table per
+  // warp / per CTA: Q4_0 32000 x 4096 16.2 / 17.2, 2 columns 24.9 / 24.8; 4096 x 8192, 3 columns 11.2 / 12.9; the latter
+  // is the faster one on longer rows, though: 4096 x 11008 9.7 / 10.6, 2 columns 14.7 / 13.4, 3 columns 16.6 / 16.6, Q8_0
+  // 14.1 / 13.3, 2 columns 20.0 / 17.1.  Flags bit 13 keeps the table-per-CTA / tensor-core kernels, bit 14 takes this
+  // one for any 3 columns: tuning.
   const bool warp_tables =
       nc <= kStrictWarpTableCols ||
       (nc == 3 && ((flags & 0x4000u) != 0 || (!kQ8W && mma_strict_ring<kQ8W>(nb, nr, nc, vx, bx) == 0)));

@@ -1,24 +1,20 @@
 // Decode GEMV for several (4..8) activation columns on rows of at most 128 blocks (4096
 // elements): the same arithmetic and the same fp32 order as gemv_mma.cuh (16-way K split, one
 // mma.sync.m16n8k32.s8 per ggml block of a 16-row group), with the weights brought in as whole
-// rows by the 1-D bulk copy engine instead of as narrow tiled boxes.
+// rows by the 1-D bulk copy engine instead of chunk by chunk by the warps that use them.
 //
-// Why: a tiled TMA box that is only one K chunk wide (144 bytes of Q4_0 per row, two cache lines)
-// costs the copy engine about 8 cycles per row, so the time per 32-row slot grows with the
-// number of boxes (measured: 16 boxes of 32 rows 2.4 us, 32 boxes of 16 rows 3.5 us per slot)
-// and the ring cannot be made deeper by making the boxes smaller.  Contiguous copies of 4.6 KB
-// run at the engine's full rate (this kernel's ring and producer alone: 6.0 TB/s), and one
-// producer warp for the whole CTA takes the copy issue out of the consumer warps, which are
-// the bottleneck (instruction issue and dependency latency, not memory).  Measured against the
-// tiled kernel with the same activation staging, 8 columns: 17.9 vs 19.0 us on 32000 x 4096,
-// 9.6 vs 10.3 us on 11008 x 4096, 5.5 vs 6.2 us on 4096 x 4096.
+// Why: contiguous copies of 4.6 KB run at the engine's full rate (this kernel's ring and producer
+// alone: 6.0 TB/s), and one producer warp for the whole CTA takes the copy issue out of the consumer
+// warps, which are the bottleneck (instruction issue and dependency latency, not memory).  Longer
+// rows would leave the ring too few units.  us, 8 columns, weights from HBM, this kernel / the chunk-wise
+// one: Q4_0 32000 x 4096 18.9 / 24.1, 11008 x 4096 10.0 / 11.5, 4096 x 4096 5.3 / 6.4; Q8_0 24.4 / 28.8, 11.3 / 12.8, 6.3 / 7.1.
 //
 // Layout: a unit is one 16-row group, all of K, shared by the whole CTA: 8 row PAIRS (rows 2p,
 // 2p+1 are adjacent in memory and arrive in one copy) at a pitch of two rows plus 16 bytes.  The
 // MMA's row m is row 2 * (m % 8) + m / 8 of the group, so thread (g = lane / 4, t = lane % 4)
 // reads rows 2g and 2g+1: both lie in pair g, and the pitch (a multiple of 128 bytes plus 16)
 // puts the 8 pairs x 4 words of a fragment load into 32 different banks.  Which MMA row holds
-// which matrix row does not enter the arithmetic, so every output has the bits the tiled kernel
+// which matrix row does not enter the arithmetic, so every output has the bits the chunk-wise kernel
 // gives.
 //
 // Roles: 16 consumer warps (warp w owns K chunk w of every unit; its activation fragments stay

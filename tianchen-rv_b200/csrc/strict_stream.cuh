@@ -22,15 +22,14 @@
 // block in every row and keeps its activation words in registers.
 //
 // What bounds it: a slot's fold is one dependent operation per block, 4 cycles at best, whatever the number of
-// rows, so slots are as large as two of them fit, and the fold has its loads a batch ahead (strict_chain.cuh).
-// us before / after that, a launch that overlaps the one before, copies requested by the folding warp with
-// the fewest chains, and fewer instructions per term: Q5_0 11008 x 4096, 1 column 12.0 / 10.6, 32000 x 4096 23.4 /
-// 20.9; strict Q4_0 4096 x 11008, 4 columns 29.0 / 20.2, Q8_0 4096 x 8192, 3 columns 21.9 / 16.4; Q5_1 4096 x 11008, 6 columns
-// 31.7 / 26.2.  (More and smaller slots: Q5_0 11008 x 4096 with four of 16 rows 11.9.)
+// rows, so slots are large, the fold has its loads a batch ahead (strict_chain.cuh), and beyond that the workers'
+// rounds count (strict_stream_rows).  us without any of it / with the loads ahead, overlapping launches and fewer
+// instructions per term / with the rows by their rounds and columns on different banks: Q5_0 11008 x 4096, 1 column
+// 12.0 / 10.3 / 9.2; strict Q4_0 4096 x 11008, 4 columns 29.0 / 20.2 / 18.5, Q8_0 4096 x 8192, 3 columns 21.9 / 16.4 / 15.8; Q5_1 4096 x
+// 11008, 6 columns 31.7 / 26.2 / 25.6.  (More and smaller slots: Q5_0 11008 x 4096 with four of 16 rows 11.9.)
 //
-// It serves Q4_0 / Q8_0 rows on 16-byte boundaries that are too long for the tensor-core form, and the
-// sibling formats where its 512 workers on one slot beat the table per warp of gemv_any.cuh
-// (siblings.cu has the rule) or where the activations lie at an odd address.
+// It serves Q4_0 / Q8_0 rows on 16-byte boundaries that are too long for the tensor-core form, and most calls of
+// the sibling formats (siblings.cu has the rule), among them all with activations at an odd address.
 //
 // Folds (reference: lib/Conversion/RVV/RVVToEmitCBlockQuantLinear.cpp:322-356, 7538-7573,
 // 472-915, 916-1391, 6817-7263):
