@@ -112,7 +112,7 @@ def test_sibling_calls_take_the_faster_streaming_kernel(cuda, pkg, fmt, nr, nb, 
 
 # calls on both sides of the lines between the two streaming kernels, the shapes whose route was wrong among them
 @pytest.mark.parametrize("fmt,nr,nb,nc", [(1, 11008, 128, 4), (3, 11008, 128, 4), (1, 4096, 128, 3), (2, 1536, 128, 8), (1, 4096, 344, 1), (2, 512, 256, 1),
-                                          (1, 2048, 128, 1), (3, 32000, 128, 1), (2, 11008, 200, 2), (3, 11008, 344, 4), (3, 11008, 128, 8), (2, 512, 128, 8)])
+                                          (1, 2048, 128, 1), (2, 100, 16, 8), (3, 32000, 128, 1), (2, 11008, 200, 2), (3, 11008, 344, 4), (3, 11008, 128, 8), (2, 512, 128, 8)])
 def test_the_rule_takes_the_faster_of_both(cuda, pkg, fmt, nr, nb, nc):
     # weights off 16-byte boundaries leave only the table per warp, activations at an odd address only the one per CTA
     wb, ab = sd.STRIDES[fmt]

@@ -111,14 +111,19 @@ __global__ void __launch_bounds__(256) sibling_dot_kernel(const uint8_t *__restr
 //              11008 x 1024 6.7 / 7.0, 11008 x 6400 26.6 / 30.3; Q4_1 11008 x 4608 18.2 / 17.5; Q5_0 32000 x 512, 3 columns 9.3 / 16.8
 //   5..8       Q5_1 11008 x 4096, 8 columns 26.7 / 28.0, 4096 x 11008, 6 columns 25.6 / 41.9; a slot to a warp: Q5_0 1536 x 4096, 8
 //              columns 8.3 / 7.5, but 512 rows 4.7 / 6.5 (Q5_1)
+//   few rows   (1476 more calls with 64..1600) Q5_0 100 x 512, 8 columns 3.3 / 2.6, 444 x 1024, 4 columns 3.2 / 2.7, 450 rows 3.0 / 3.5,
+//              888 rows, 2 columns 2.9 / 2.6, 1100 rows 2.8 / 3.3; Q4_1 148 x 4096, 2 columns 3.0 / 3.4
 template <int kFormat>
 bool table_per_cta(const GemvAnyPlan &plan, uint32_t nb, size_t nr, size_t nc, int sms) {
   if (nc == 1)
     return true;
   const GemvAnyArgs &a = plan.args;
   const size_t blocks = nb * nc, n = static_cast<size_t>(sms);
-  if (nr <= n * a.nwarps * a.rps)
+  if (nr <= n * a.nwarps * a.rps) {
+    if (kFormat == 2 && nb <= 64 && (nr <= 3 * n || (nr >= 5 * n && nr <= 7 * n)))
+      return false;
     return nr < 5 * n || blocks < 256;
+  }
   if (nc > 4 || (kFormat == 2 && nc < 4))
     return true;
   return nr < 20 * n || nb > 160 || blocks < 256 || blocks > 600;
