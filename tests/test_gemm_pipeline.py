@@ -87,9 +87,7 @@ void roles(uint32_t nb, int count, char **items) {
     c.smem_empty = reinterpret_cast<uint64_t *>(8 * 100);
     c.tmem_full = reinterpret_cast<uint64_t *>(8 * 200);
     c.tmem_empty = reinterpret_cast<uint64_t *>(8 * 300);
-    c.turn = reinterpret_cast<uint64_t *>(8 * 400);
     c.mma_warp = role;
-    c.turn_phase = role ^ 1;
     for (int i = 0; i < count; ++i) {
       const GemmItem it = {0, 0, items[i][0] == 'w'};
       if (role < 0 && it.whole)
@@ -130,23 +128,23 @@ def program(tmp_path_factory):
 
 
 def record(program, multi, narrow, nb, items):
-    """(shared-memory stages, {role: [(what, barrier, parity)]}) of the epilogue (-1) and the MMA warps (0, 1)."""
+    """(shared-memory stages, TMEM stages, {role: [(what, barrier, parity)]}) of the epilogue (-1) and the MMA warps (0, 1)."""
     out = subprocess.run([program, str(multi), str(narrow), str(nb), *items], check=True, capture_output=True, text=True).stdout
-    stages, roles = 0, {}
+    stages, tmem, roles = 0, 0, {}
     for line in out.splitlines():
         what, number, parity = (line.split() + ["0", "0"])[:3]
         if what == "stages":
-            stages = int(number)
+            stages, tmem = int(number), int(parity)
         elif what == "role":
             trace = roles.setdefault(int(number), [])
         else:
             trace.append((what, int(number), int(parity)))
-    return stages, roles
+    return stages, tmem, roles
 
 
 def play(roles, late):
     """Every role runs as far as it can before `late` makes one step; the roles that never finish."""
-    phase, at = {}, dict.fromkeys(roles, 0)  # completed phases of a barrier; next step of a role
+    arrived, at = {}, dict.fromkeys(roles, 0)  # arrivals at a barrier; next step of a role
     filled = [None]  # whose A operand is in the tensor core's buffer
 
     def step(role):
@@ -154,12 +152,12 @@ def play(roles, late):
             return False
         what, bar, parity = roles[role][at[role]]
         if what == "arrive":
-            phase[bar] = phase.get(bar, 0) + 1
+            arrived[bar] = arrived.get(bar, 0) + 1
         elif what == "fill":
             filled[0] = role
         elif what == "use":
             assert filled[0] == role, "another warp's MMA came between the two that share an operand"
-        elif phase.get(bar, 0) % 2 == parity:
+        elif arrived.get(bar, 0) // (2 if bar // 100 == 3 else 1) % 2 == parity:  # free accumulators: epilogue and turn
             return False
         at[role] += 1
         return True
@@ -174,9 +172,12 @@ def play(roles, late):
     (0, 32, 1, "wwwwwwwwwwwwwwwwwwwwww"),
 ])
 def test_no_role_can_come_too_late_for_a_phase(program, multi, narrow, nb, items):
-    stages, roles = record(program, multi, narrow, nb, items)
+    stages, tmem, roles = record(program, multi, narrow, nb, items)
     fills = (nb + 3) // 4 * len(items)
-    # one epilogue warp stands for the eight, which do the same; the producer fills stage after stage
+    # one epilogue warp stands for the eight, which do the same; the producer fills stage after stage; before the
+    # first item the epilogue hands over all accumulators and the first MMA warp gives itself the first turn
+    roles[-1][:0] = [("arrive", 300 + i, 0) for i in range(tmem)]
+    roles[0][:0] = [("arrive", 300, 0)]
     roles["producer"] = [e for i in range(fills) for e in (("wait", 100 + i % stages, 1 - i // stages % 2), ("arrive", i % stages, 0))]
     for late in roles:
         assert play(roles, late) == [], f"role {late} comes too late"

@@ -360,8 +360,8 @@ inline int blocks_for(size_t items) {
 // fill no more than half of the SMs), 128 x 32 (32) or 128 x 16 (16).  Rounds of each kind times what an item
 // takes, in hundredths of a 256 x 64 one: with 128 blocks to a row a round takes 33 us whole, 20 in halves, 11.2 and
 // 7.4 to 8.3 narrow.  Narrow items win where the others leave SMs without work.  us a call (weights prepared), 256 x
-// 64 / 128 x 32 / 128 x 16: 77 x 4096 x 11008 51.6 / 34.2 / 47.6, 40 x 4096 x 4096 22.2 / 15.2 / 12.1, 16 x 32000 x 4096 39.3 / 34.2 / 31.4,
-// 33 x 20000 x 1024 14.3 / 16.1 / 14.7, 200 x 4096 x 4096 24.3 / 29.6 / 30.7, 512 x 11008 x 4096 92.0 / 119 / 156.
+// 64 / 128 x 32 / 128 x 16: 77 x 4096 x 11008 51.1 / 34.0 / 45.2, 40 x 4096 x 4096 22.1 / 15.0 / 11.6, 16 x 32000 x 4096 39.2 / 34.3 / 31.2,
+// 33 x 20000 x 1024 14.1 / 16.0 / 14.3, 200 x 4096 x 4096 24.6 / 29.3 / 29.2, 512 x 11008 x 4096 91.7 / 119 / 146.
 int narrow_items(size_t nr, size_t nc, size_t ctas) {
   const auto cdiv = [](size_t a, size_t b) { return (a + b - 1) / b; };
   const size_t tiles = cdiv(nr, 256) * cdiv(nc, 64), rem = tiles % ctas;

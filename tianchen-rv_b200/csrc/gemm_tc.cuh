@@ -42,7 +42,7 @@
 //   warp 8      TMA producer (one elected lane)
 //   warps 9, 10 MMA issue (one elected lane each), by turns; warp 9 allocates TMEM.  Two of a block's MMAs share
 //               A through the tensor core's operand buffer (without it 10 % slower on every shape), so the turns
-//               are kept by barriers: 1.4 % faster on 256 x 64 items, 2 to 4 % slower on 128 x 16
+//               are kept by the accumulators' barriers (0 to 1.5 % faster than without turns)
 // Pipelines: shared-memory stages of 4 blocks each (full/empty mbarriers) and TMEM stages of
 // several blocks each (full/empty mbarriers).  The epilogue warps wait on the accumulator barriers
 // only: a stage's scale tiles have landed when its first accumulator has.
@@ -255,12 +255,11 @@ __device__ __forceinline__ void fold_part(const uint32_t *v, uint64_t (&acc)[Sha
 struct GemmEpilogueCtx {
   uint8_t *stages;
   uint8_t *out_stage;
-  uint64_t *smem_full, *smem_empty, *tmem_full, *tmem_empty, *store_bar, *turn;
+  uint64_t *smem_full, *smem_empty, *tmem_full, *tmem_empty, *store_bar;
   volatile uint32_t *abort_flag;
   uint32_t tmem_base;
   uint32_t store_syncs;  // syncs of the epilogue warps done so far (parity of the next one)
   uint32_t mma_warp;     // an MMA warp fills the TMEM stages of its parity
-  uint32_t turn_phase;   // parity of its next turn
   PipeState ps, ts;
 };
 
@@ -536,12 +535,10 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
         // its accumulators have come, so it holds a stage for the warp that makes those and for no other.
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.smem_full[c.ps.stage], c.ps.phase, c.abort_flag)))
           return false;
-        // An MMA that takes A from the operand buffer has to follow the one that put it there: no MMA of the
-        // other warp may come between, so the hand-overs' MMAs are issued one after another.
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.turn[c.mma_warp], c.turn_phase, c.abort_flag)))
-          return false;
-        c.turn_phase ^= 1;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.tmem_empty[c.ts.stage], c.ts.phase ^ 1, c.abort_flag)))
+        // The accumulators are free, and it is this warp's turn: an MMA that takes A from the operand buffer has
+        // to follow the one that put it there, with no MMA of the other warp between.  So a hand-over's MMAs
+        // are issued after those of the one before, whose warp is the ninth to arrive here.
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&c.tmem_empty[c.ts.stage], c.ts.phase, c.abort_flag)))
           return false;
         tcgen05_fence_after_thread_sync();
         constexpr uint64_t kStep = (kQK >> 4);  // 32 bytes in 16-byte units
@@ -560,7 +557,7 @@ __device__ __forceinline__ bool gemm_mma_item(const GemmArgs &a, GemmEpilogueCtx
           }
           umma_commit(&c.tmem_full[c.ts.stage]);
           tcgen05_fence_before_thread_sync();
-          mbar_arrive(&c.turn[c.mma_warp ^ 1]);
+          mbar_arrive(&c.tmem_empty[c.ts.stage + 1 == Plan::kTmemStages ? 0 : c.ts.stage + 1]);
         }
         __syncwarp();
       }
@@ -592,8 +589,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   c.tmem_empty = c.tmem_full + Plan::kTmemStages;
   uint64_t *drain_bar = c.tmem_empty + Plan::kTmemStages;
   c.store_bar = drain_bar + 1;
-  c.turn = c.store_bar + 1;
-  uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(c.turn + kGemmMmaWarps);
+  uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(c.store_bar + 1);
   c.abort_flag = tmem_base_slot + 1;
   const uint32_t stage_base_addr = (smem_addr(smem_raw) + kGemmCtrlBytes + 1023u) & ~1023u;
   c.stages = smem_raw + (stage_base_addr - smem_addr(smem_raw));
@@ -612,12 +608,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int i = 0; i < Plan::kTmemStages; ++i) {
       mbar_init(&c.tmem_full[i], 1);
-      mbar_init(&c.tmem_empty[i], kGemmEpilogueWarps);
+      mbar_init(&c.tmem_empty[i], kGemmEpilogueWarps + 1);
     }
     mbar_init(drain_bar, kGemmMmaWarps);
     mbar_init(c.store_bar, kGemmEpilogueWarps);
-    for (int i = 0; i < kGemmMmaWarps; ++i)
-      mbar_init(&c.turn[i], 1);
     *c.abort_flag = 0;
     mbar_fence_init();
   }
@@ -706,7 +700,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // Two warps take turns at the TMEM stages: one warp's wait, wait, issue and commit for a hand-over
       // (640 cycles) is longer than what eight MMAs take (240 to 300).
       c.mma_warp = static_cast<uint32_t>(warp - kGemmEpilogueWarps - 1);
-      c.turn_phase = c.mma_warp ^ 1;  // the first turn is warp 9's
+      mbar_arrive_if(&c.tmem_empty[0], c.mma_warp == 0 && leader);  // the first turn
       for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
         const GemmItem it = gemm_item<kNarrow>(a, idx);
         if (it.n0 >= a.nr || it.m0 >= a.nc)
@@ -726,6 +720,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kGemmEpilogueRegs));
+    for (int i = 0; i < Plan::kTmemStages; ++i)  // all TMEM stages are free
+      mbar_arrive_if(&c.tmem_empty[i], lane == 0);
     // ------------------------------ epilogue warps ------------------------------
     for (uint32_t idx = blockIdx.x; idx < a.items && ok; idx += gridDim.x) {
       const GemmItem it = gemm_item<kNarrow>(a, idx);
