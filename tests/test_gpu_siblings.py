@@ -52,9 +52,9 @@ def test_sibling_vec_dot_entries_padded_and_unaligned(cuda, pkg, O, fmt, entry):
 @pytest.mark.parametrize("fmt", [1, 2, 3])
 @pytest.mark.parametrize("nr,nb,pad", [(2000, 128, 0), (777, 8, 0), (130, 40, 48), (4099, 64, 16)])
 def test_sibling_streaming_rows_bit_exact(cuda, pkg, O, fmt, nr, nb, pad):
-    # One column against many 16-byte aligned rows takes a streaming kernel: contiguous rows, rows with
-    # a stride, ragged last slots; the one with a table per warp, and at an odd address of the
-    # activation column the one with a table per CTA.
+    # One column against many rows takes a streaming kernel: contiguous rows, rows with a stride, ragged last
+    # slots; the one with a table per CTA at any address of the activation column, the one with a table per warp
+    # where the weights are off 16-byte boundaries, by whole words or not.
     w, x = sd.make(fmt, nr, 1, nb, 900 + fmt + nr)
     wb = w.shape[1]
     padded = np.zeros((nr, wb + pad), dtype=np.uint8)
@@ -65,9 +65,9 @@ def test_sibling_streaming_rows_bit_exact(cuda, pkg, O, fmt, nr, nb, pad):
     rows = np.unique(np.concatenate([np.arange(0, nr, max(1, nr // 60)), np.arange(max(0, nr - 40), nr)]))
     want = O.sibling_dot_rows(fmt, w[rows], x)
 
-    def run(x_ptr):
+    def run(x_ptr, w_ptr=wd.data_ptr()):
         out = cuda.full((nr, 1), float("nan"), dtype=cuda.float32, device="cuda")
-        assert L.tcrv_cuda_sibling_dot_rows(fmt, nb * 32, out.data_ptr(), wd.data_ptr(), x_ptr, x.shape[1], nr, 1,
+        assert L.tcrv_cuda_sibling_dot_rows(fmt, nb * 32, out.data_ptr(), w_ptr, x_ptr, x.shape[1], nr, 1,
                                             wb + pad, 1, None) == 0
         return out.cpu().numpy()
 
@@ -76,6 +76,10 @@ def test_sibling_streaming_rows_bit_exact(cuda, pkg, O, fmt, nr, nb, pad):
     flat = cuda.zeros(x.shape[1] + 1, dtype=cuda.uint8, device="cuda")
     flat[1:] = xd[0]
     assert np.array_equal(run(flat.data_ptr() + 1)[rows].view(np.uint32), want.view(np.uint32))
+    for shift in (4, 2):
+        moved = cuda.zeros(padded.size + shift, dtype=cuda.uint8, device="cuda")
+        moved[shift:] = wd.reshape(-1)
+        assert np.array_equal(run(xd.data_ptr(), moved.data_ptr() + shift)[rows].view(np.uint32), want.view(np.uint32))
     pkg.check_device_errors()
 
 
@@ -122,7 +126,7 @@ def test_the_rule_takes_the_faster_of_both(cuda, pkg, fmt, nr, nb, nc):
     fn = pkg.lib().tcrv_cuda_sibling_dot_rows
     rule, warp, cta = (graph_time.us(cuda, lambda st: fn(fmt, nb * 32, out.data_ptr(), w.data_ptr() + wo, x.data_ptr() + xo, nb * ab, nr, nc,
                                                          nb * wb, nc, st)) for wo, xo in ((0, 0), (4, 0), (0, 1)))
-    assert rule < 1.09 * min(warp, cta), f"{rule:.2f} us by the rule, {warp:.2f} with the table per warp, {cta:.2f} per CTA"
+    assert rule < 1.12 * min(warp, cta), f"{rule:.2f} us by the rule, {warp:.2f} with the table per warp, {cta:.2f} per CTA"
     pkg.check_device_errors()
 
 
